@@ -423,29 +423,128 @@ __global__ void __launch_bounds__(256) k_stats_final(StatParams p, const double 
     }
 }
 
-__global__ void k_mupdat(int32_t n, const int32_t *iv, const int32_t *jv, const double *add,
-                         int32_t matsto, int32_t nG, const int32_t *aig, const int32_t *p2g,
-                         const int64_t *off, const int32_t *col, double *matD, int32_t nVar,
-                         int32_t *errFlag) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    for (int32_t q = 0; q < n; ++q) {
-        const int32_t i = iv[q], j = jv[q];
-        const double a = add[q];
-        if (i <= 0 || j <= 0 || a == 0.0) continue;
-        if (i > nVar || j > nVar) { *errFlag = 23; continue; }
-        const int64_t ia = i > j ? i : j, ja = i > j ? j : i;
-        if (matsto == 2) {
-            if (ia == ja) { matD[ia - 1] += a; continue; }
-            int32_t lr;
-            const int32_t g1 = p2g[ia - 1], g2 = p2g[ja - 1];
-            const int64_t ij = d_ijpgrp(g1, g2, nG, aig, off, col, &lr);
-            if (ij == 0) continue;  // pair not stored (suppressed)
-            matD[ij + (ja - aig[g2 - 1]) + (ia - aig[g1 - 1]) * (int64_t)lr - 1] += a;
-        } else {
-            matD[(ia * ia - ia) / 2 + ja - 1] += a;
+// Ordered additions to scattered targets: target[addr(q)] += add(q) for q =
+// 0..n-1, the terms of one target added in the order of q (mupdat and the
+// vector side are called element by element in the reference).
+//
+// Bound: latency of the index loads and block searches.  Targets are
+// independent of each other, so each CTA owns the targets of one residue of
+// a hash and walks all terms in chunks of kOrdChunk; the terms of a chunk
+// that it owns are applied in rounds: every pending term enters its number
+// in a slot table (atomicMin by a second hash), the smallest of a slot is
+// applied, the others wait for the next round.  Terms of one target share a
+// slot, so they are applied in order; a chunk still pending after kOrdRounds
+// rounds (many terms of one target) is finished by one thread.  No memory is
+// allocated.  30,000 diagonal terms of a sparse matrix: 44 us, 8,740 us
+// with one thread for all of them (the first form).
+constexpr int kOrdThreads = 1024, kOrdItems = 4, kOrdChunk = kOrdThreads * kOrdItems, kOrdSlots = 4096;
+constexpr int kOrdRounds = 32, kOrdCtas = 64;
+
+__device__ __forceinline__ uint32_t ord_hash(int64_t a) {
+    return (uint32_t)(((uint64_t)a * 0x9E3779B97F4A7C15ull) >> 32);
+}
+
+// Terms: int64_t addr(q) (< 0: no target), double add(q)
+template <class Terms>
+__global__ void __launch_bounds__(kOrdThreads) k_ordered_add(int32_t n, Terms terms, double *target) {
+    __shared__ int32_t slot[kOrdSlots];
+    __shared__ uint32_t left[kOrdChunk / 32];
+    const int tid = threadIdx.x;
+    for (int k = tid; k < kOrdSlots; k += kOrdThreads) slot[k] = kOrdChunk;
+    for (int64_t base = 0; base < n; base += kOrdChunk) {
+        int64_t addr[kOrdItems];
+        double add[kOrdItems];
+        uint32_t h[kOrdItems];
+        unsigned pend = 0;
+#pragma unroll
+        for (int u = 0; u < kOrdItems; ++u) {
+            const int64_t q = base + u * kOrdThreads + tid;
+            addr[u] = q < n ? terms.addr((int32_t)q) : -1;
+            h[u] = ord_hash(addr[u]);
+            add[u] = 0.0;
+            if (addr[u] >= 0 && (h[u] >> 16) % gridDim.x == blockIdx.x) {
+                pend |= 1u << u;
+                add[u] = terms.add((int32_t)q);
+            }
+        }
+        int round = 0;
+        while (__syncthreads_or(pend != 0) && round < kOrdRounds) {
+#pragma unroll
+            for (int u = 0; u < kOrdItems; ++u)
+                if (pend >> u & 1) atomicMin(&slot[h[u] & (kOrdSlots - 1)], u * kOrdThreads + tid);
+            __syncthreads();
+            unsigned won = 0;
+#pragma unroll
+            for (int u = 0; u < kOrdItems; ++u)
+                if ((pend >> u & 1) && slot[h[u] & (kOrdSlots - 1)] == u * kOrdThreads + tid) {
+                    target[addr[u]] += add[u];
+                    won |= 1u << u;
+                }
+            __syncthreads();
+            // the slots of the applied terms are free for the next round
+#pragma unroll
+            for (int u = 0; u < kOrdItems; ++u)
+                if (won >> u & 1) slot[h[u] & (kOrdSlots - 1)] = kOrdChunk;
+            pend &= ~won;
+            ++round;
+        }
+        if (round == kOrdRounds) {   // uniform over the CTA
+            for (int k = tid; k < kOrdChunk / 32; k += kOrdThreads) left[k] = 0;
+            __syncthreads();
+#pragma unroll
+            for (int u = 0; u < kOrdItems; ++u)
+                if (pend >> u & 1) atomicOr(&left[(u * kOrdThreads + tid) >> 5], 1u << (tid & 31));
+            __syncthreads();
+            if (tid == 0)
+                for (int k = 0; k < kOrdChunk / 32; ++k)
+                    for (uint32_t w = left[k]; w; w &= w - 1) {
+                        const int32_t q = (int32_t)(base + 32 * k + __ffs(w) - 1);
+                        target[terms.addr(q)] += terms.add(q);
+                    }
+            __syncthreads();
         }
     }
 }
+
+// mupdat (pede.f90:3134-3204): element (i, j) of the packed or mpbits matrix
+struct MupdatTerms {
+    const int32_t *iv, *jv;
+    const double *a;
+    int32_t matsto, nG, nVar;
+    const int32_t *aig, *p2g;
+    const int64_t *off;
+    const int32_t *col;
+    int32_t *errFlag;
+    __device__ double add(int32_t q) const { return a[q]; }
+    __device__ int64_t addr(int32_t q) const {
+        const int32_t i = iv[q], j = jv[q];
+        if (i <= 0 || j <= 0 || a[q] == 0.0) return -1;
+        if (i > nVar || j > nVar) {
+            *errFlag = 23;
+            return -1;
+        }
+        const int64_t ia = i > j ? i : j, ja = i > j ? j : i;
+        if (matsto != 2) return (ia * ia - ia) / 2 + ja - 1;
+        if (ia == ja) return ia - 1;
+        int32_t lr;
+        const int32_t g1 = p2g[ia - 1], g2 = p2g[ja - 1];
+        const int64_t ij = d_ijpgrp(g1, g2, nG, aig, off, col, &lr);
+        // 0: pair not stored (suppressed)
+        return ij == 0 ? -1 : ij + (ja - aig[g2 - 1]) + (ia - aig[g1 - 1]) * (int64_t)lr - 1;
+    }
+};
+
+// global vector terms; indices outside the vector are ignored
+struct VectorTerms {
+    const int32_t *idx;
+    const double *a;
+    int32_t nVar;
+    __device__ double add(int32_t q) const { return a[q]; }
+    __device__ int64_t addr(int32_t q) const { return idx[q] >= 1 && idx[q] <= nVar ? idx[q] - 1 : -1; }
+};
+
+// CTAs: one per 128 terms, at most kOrdCtas (each walks all terms)
+unsigned ord_ctas(int32_t n) { return (unsigned)(n < 128 * kOrdCtas ? (n + 127) / 128 : kOrdCtas); }
 
 }  // namespace
 
@@ -489,7 +588,12 @@ cudaError_t launch_stats(const StatParams &p, cudaStream_t s) {
 
 cudaError_t launch_mupdat(int32_t n, const int32_t *i, const int32_t *j, const double *add,
                           const DevJob &d, int32_t *errFlag, cudaStream_t s) {
-    k_mupdat<<<1, 32, 0, s>>>(n, i, j, add, d.matsto, d.nG, d.aig, d.p2g, d.off, d.col, d.matD,
-                             d.nVar, errFlag);
+    const MupdatTerms t{i, j, add, d.matsto, d.nG, d.nVar, d.aig, d.p2g, d.off, d.col, errFlag};
+    k_ordered_add<<<ord_ctas(n), kOrdThreads, 0, s>>>(n, t, d.matD);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_vector_add(int32_t n, const int32_t *idx, const double *add, const DevJob &d, cudaStream_t s) {
+    k_ordered_add<<<ord_ctas(n), kOrdThreads, 0, s>>>(n, VectorTerms{idx, add, d.nVar}, d.gvec);
     return cudaGetLastError();
 }

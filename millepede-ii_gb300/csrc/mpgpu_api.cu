@@ -891,14 +891,6 @@ extern "C" int32_t mpgpu_mupdat(mpgpu_ctx *c, int32_t n, const int32_t *i, const
     return MPGPU_OK;
 }
 
-namespace {
-__global__ void k_vadd(int32_t n, const int32_t *idx, const double *v, double *gvec, int32_t nVar) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    for (int32_t q = 0; q < n; ++q)
-        if (idx[q] >= 1 && idx[q] <= nVar) gvec[idx[q] - 1] += v[q];
-}
-}  // namespace
-
 extern "C" int32_t mpgpu_vector_add(mpgpu_ctx *c, int32_t n, const int32_t *vidx, const double *vadd) {
     if (!c || n < 0) return MPGPU_ERR_ARG;
     if (n == 0) return MPGPU_OK;
@@ -910,8 +902,7 @@ extern "C" int32_t mpgpu_vector_add(mpgpu_ctx *c, int32_t n, const int32_t *vidx
     cudaStream_t s = c->stream;
     MPG_CUDA(c, dupload(b.di, vidx, n, s));
     MPG_CUDA(c, dupload(b.da, vadd, n, s));
-    k_vadd<<<1, 32, 0, s>>>(n, b.di, b.da, c->j.gvec, c->j.nVar);
-    MPG_CUDA(c, cudaGetLastError());
+    MPG_CUDA(c, launch_vector_add(n, b.di, b.da, c->j, s));
     MPG_CUDA(c, cudaStreamSynchronize(s));
     return MPGPU_OK;
 }

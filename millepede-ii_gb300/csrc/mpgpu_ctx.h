@@ -395,9 +395,11 @@ struct StatParams {
 };
 cudaError_t launch_stats(const StatParams &p, cudaStream_t s);
 
-// matrix-element updates (mupdat), applied in order by one thread
+// matrix-element updates (mupdat) and global-vector updates, the terms of
+// one element added in order
 cudaError_t launch_mupdat(int32_t n, const int32_t *i, const int32_t *j, const double *add,
                           const DevJob &d, int32_t *errFlag, cudaStream_t s);
+cudaError_t launch_vector_add(int32_t n, const int32_t *idx, const double *add, const DevJob &d, cudaStream_t s);
 
 // device version of ijpgrp (pede.f90:5371-5461); returns the 1-based index
 // of the first element of block (itema, itemb) and its row length

@@ -12,7 +12,7 @@
 //    device memory: a small allocation in the middle of the run can then
 //    fail, or fragment the memory the next large allocation needs.
 // mpgpu_mupdat_noalloc stages the triplets in one file-scope __device__
-// array of fixed size and runs the same k_mupdat kernel on them.  It never
+// array of fixed size and runs the same kernel (k_ordered_add) on them.  It never
 // allocates or frees device memory.
 //
 // Limits and rules of use:

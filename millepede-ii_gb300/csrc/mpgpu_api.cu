@@ -72,6 +72,9 @@ void free_layout(DevJob &j) {
     dfree(j.matD); dfree(j.gvec); dfree(j.gcnt); dfree(j.gpar); dfree(j.work);
     dfree(j.rowBlk0); dfree(j.blkJ); dfree(j.blkOff); dfree(j.blkLd);
     dfree(j.rowWidth);
+    dfree(j.br.val); dfree(j.br.col); dfree(j.br.stepBeg); dfree(j.br.itemBeg);
+    dfree(j.br.itemS0); dfree(j.br.itemS1); dfree(j.br.part); dfree(j.br.xp);
+    j.br = BlockRows();
 }
 
 void free_constraints(DevJob &j) {

@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "../../include/mpgpu.h"
+#include "mpgpu_bspmv.h"
 
 #define MPG_WARPS_FIT 8        // warps per CTA of the local-fit kernel
 #define MPG_FIT_BUCKETS 8      // size classes of records for the fit launches
@@ -157,9 +158,9 @@ struct DevJob {
     std::vector<int32_t> hR1, hR2;
     // host copies needed by the host-side control
     std::vector<int32_t> hAig;
-    // solver workspace
+    // workspace of the iterative solves, kept between the solves of a layout
     double *work = nullptr;
-    int64_t workLen = 0;
+    BlockRows br;
 };
 
 // Records kept on the device by mpgpu_loop1_device: copied once,
@@ -219,7 +220,9 @@ int32_t band_alloc(BandPre &P, int32_t nVar, int32_t nfit, int32_t w);
 void band_free(BandPre &P);
 cudaError_t band_fill(const BandPre &P, int32_t nVar, int32_t matsto, const double *matD, const int32_t *aig,
                       const int32_t *p2g, const int64_t *rowStart, const int32_t *bcol, const int64_t *boff,
-                      const int32_t *bld, cudaStream_t s);
+                      const int32_t *bld, int64_t nmat, cudaStream_t s);
+cudaError_t band_eliminate(const BandPre &P, int32_t nVar, int32_t m, const double *U, const double *Z,
+                           cudaStream_t s);
 cudaError_t band_reflect(const BandPre &P, int32_t nVar, const double *v, const double *y, const double *beta,
                          cudaStream_t s);
 cudaError_t band_factor(const BandPre &P, int32_t lprecm, cudaStream_t s);

@@ -40,7 +40,7 @@ inline int grid_for(int64_t n, int threads) {
 // block table of the row groups (blocks of group I ordered by column group)
 __global__ void k_band_fill(int32_t nVar, int32_t w, int32_t matsto, const double *matD, const int32_t *aig,
                             const int32_t *p2g, const int64_t *rowStart, const int32_t *bcol,
-                            const int64_t *boff, const int32_t *bld, double *B) {
+                            const int64_t *boff, const int32_t *bld, int64_t nmat, double *B) {
     const int32_t W1 = w + 1;
     const int64_t tot = (int64_t)nVar * W1;
     for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
@@ -59,7 +59,9 @@ __global__ void k_band_fill(int32_t nVar, int32_t w, int32_t matsto, const doubl
                     const int64_t mid = (lo + hi) >> 1;
                     const int32_t Jm = bcol[mid];
                     if (Jm == J) {
-                        a = matD[boff[mid] + (int64_t)(i - (aig[I - 1] - 1)) * bld[mid] + (j - (aig[J - 1] - 1))];
+                        // (blocks beyond the matrix: pairs left out of it)
+                        if (boff[mid] < nmat)
+                            a = matD[boff[mid] + (int64_t)(i - (aig[I - 1] - 1)) * bld[mid] + (j - (aig[J - 1] - 1))];
                         break;
                     }
                     if (Jm < J) lo = mid + 1;
@@ -68,6 +70,24 @@ __global__ void k_band_fill(int32_t nVar, int32_t w, int32_t matsto, const doubl
             }
         }
         B[e] = a;
+    }
+}
+
+// the band of Q^T A Q = A - Z U^T - U Z^T (all reflections at once, columns
+// of U and Z contiguous)
+__global__ void k_band_eliminate(int32_t nVar, int32_t w, int32_t m, const double *U, const double *Z, double *B) {
+    const int32_t W1 = w + 1;
+    const int64_t tot = (int64_t)nVar * W1;
+    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i = e / W1, j = i - w + (e - i * W1);
+        if (j < 0) continue;
+        double a = 0.0;
+        for (int64_t k = 0; k < m; ++k) {
+            const double *u = U + k * nVar, *z = Z + k * nVar;
+            a = fma(z[i], u[j], a);
+            a = fma(u[i], z[j], a);
+        }
+        B[e] = B[e] - a;
     }
 }
 
@@ -599,9 +619,15 @@ void band_free(BandPre &P) {
 
 cudaError_t band_fill(const BandPre &P, int32_t nVar, int32_t matsto, const double *matD, const int32_t *aig,
                       const int32_t *p2g, const int64_t *rowStart, const int32_t *bcol, const int64_t *boff,
-                      const int32_t *bld, cudaStream_t s) {
+                      const int32_t *bld, int64_t nmat, cudaStream_t s) {
     k_band_fill<<<grid_for((int64_t)nVar * (P.w + 1), kT), kT, 0, s>>>(nVar, P.w, matsto, matD, aig, p2g,
-                                                                        rowStart, bcol, boff, bld, P.B);
+                                                                        rowStart, bcol, boff, bld, nmat, P.B);
+    return cudaGetLastError();
+}
+
+cudaError_t band_eliminate(const BandPre &P, int32_t nVar, int32_t m, const double *U, const double *Z,
+                           cudaStream_t s) {
+    k_band_eliminate<<<grid_for((int64_t)nVar * (P.w + 1), kT), kT, 0, s>>>(nVar, P.w, m, U, Z, P.B);
     return cudaGetLastError();
 }
 

@@ -10,6 +10,7 @@
 #include <cstring>
 #include <vector>
 
+#include "mpgpu_bspmv.h"
 #include "mpgpu_ctx.h"
 
 namespace {
@@ -430,7 +431,6 @@ struct SparseBlocks {
     int64_t *colItemQ1 = nullptr;  // [nColItem] end
     int64_t *colItemBeg = nullptr; // [nG+1] first item of column group J
     double *colPart = nullptr;     // [nColItem * kSmallGroup]
-    int uniform = 0;               // every group has this many parameters (0: mixed)
 };
 
 // phase 1: warp per row group I: y_I = D_I x_I + sum_J A_IJ x_J, the
@@ -492,32 +492,31 @@ __global__ void k_spmv_cols(int32_t nG, const int32_t *aig, const int64_t *colSt
     }
 }
 
-// the same two phases for row groups of at most 8 parameters.  Phase 1,
+// the same two phases for row groups of at most 8 parameters of strongly
+// mixed sizes (others take the block-row copy, mpgpu_bspmv.cu).  Phase 1,
 // one thread per stored block (all blocks of all row groups, so the lanes
 // stay full whatever the row lengths): the block's rows times x_J into its
 // partial row sums (rowPart, 8 per block; the diagonal block adds both
 // triangles of its strictly-lower part there) and its columns times x_I
-// into tbuf (parameter-major per column group).  G > 0: every group has G
-// parameters (loops fully unrolled); G = 0: at most 8, predicated.  Phase
-// 2: the partial row sums of a group's blocks and the transposed products
-// of its incoming blocks summed by column items (long columns split over
-// several warps), then y = D x + the group's items in item order; no
-// atomics, the sums are reproducible.
+// into tbuf (parameter-major per column group).  Phase 2: the partial row
+// sums of a group's blocks and the transposed products of its incoming
+// blocks summed by column items (long columns split over several warps),
+// then y = D x + the group's items in item order; no atomics, the sums are
+// reproducible.
 constexpr int kSmallGroup = 8;
 
-template <int G>
 __global__ void __launch_bounds__(256) k_spmv_blocks(int64_t nb, const int32_t *brow, const int32_t *aig,
                                                      const int32_t *bcol, const int64_t *boff, const int32_t *bld,
                                                      const int64_t *tOff, const int32_t *tStr,
                                                      const double *matD, const double *x, double *tbuf,
                                                      double *rowPart) {
-    constexpr int M = G > 0 ? G : kSmallGroup;
+    constexpr int M = kSmallGroup;
     for (int64_t bl = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; bl < nb;
          bl += (int64_t)gridDim.x * blockDim.x) {
         const int32_t I = brow[bl], J = bcol[bl];
         const int32_t ia = aig[I - 1] - 1, ja = aig[J - 1] - 1;
-        const int np = G > 0 ? G : aig[I] - 1 - ia;
-        const int nj = G > 0 ? G : aig[J] - 1 - ja;
+        const int np = aig[I] - 1 - ia;
+        const int nj = aig[J] - 1 - ja;
         const double *blk = matD + boff[bl];
         const int32_t ld = bld[bl];
         double xi[M], sr[M];
@@ -628,62 +627,259 @@ __global__ void k_spmv_final(int32_t n, const int32_t *aig, const int32_t *p2g, 
 }
 
 // ---------------------------------------------------------------- MINRES state
+// Iteration scalars.  Two copies alternate from iteration to iteration: the
+// kernel that takes the scalar step (k_mr_w, k_qlp_w) computes it in every
+// CTA from one copy and writes the other, so no CTA reads what another one
+// is writing.
 struct MinresState {
     double beta1, beta, oldb, alfa, dbar, epsln, oldeps, delta, gbar, root, gamma, cs, sn, phi, phibar;
     double tnorm2, gmax, gmin, Anorm, ynorm, rnorm, denom, rtol;
-    double dotv;       // scratch result of the last dot
-    int itn, itnlim, istop, done;
+    int k;                        // iterations whose update is done
+    int itn, itnlim, istop;
 };
 
-__global__ void k_mr_init(MinresState *S, double rtol, int itnlim) {
+// MINRES-QLP (Choi, Paige & Saunders 2011; minresqlpModule.f90:411-1333 in
+// the reference): the Lanczos scalars of MinresState plus the rows of the
+// lower-triangular L = R P not yet final, the final u values and the
+// rotations of the current iteration for the vector kernel
+struct QlpState {
+    double etaA, thA, gA, tauA, etaB, thB, gB, tauB, uF1, uF2;
+    double c1, s1, c2, s2, uA, uB, uC;
+};
+
+// pend: the last test ended the iteration (written by k_mr_next); done:
+// promoted from it by the next operator product, read by every kernel.  The
+// scalar alfa stands between k_mr_y2 and the scalar step.
+struct MinresFlags {
+    int pend, done;
+    double alfa;
+};
+
+// sum over the CTA (kThreads threads) in a fixed order, in every thread
+__device__ __forceinline__ double cta_sum(double v, double *sh) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double r = sh[0];
+#pragma unroll
+    for (int q = 1; q < kThreads / 32; ++q) r += sh[q];
+    __syncthreads();
+    return r;
+}
+
+__device__ __forceinline__ double sum_of_partials(const double *part, int n, double *sh) {
+    double v = 0.0;
+    for (int i = threadIdx.x; i < n; i += kThreads) v += part[i];
+    return cta_sum(v, sh);
+}
+
+// beta1^2 = r1 . y
+__global__ void k_mr_init(MinresState *S, QlpState *Q, MinresFlags *F, const double *dotv, double rtol, int itnlim) {
     if (threadIdx.x) return;
-    // beta1 = sqrt(r1 . y) is in S->dotv
-    double b1 = S->dotv;
-    memset(S, 0, sizeof(MinresState));
+    memset(S, 0, 2 * sizeof(MinresState));
+    if (Q) memset(Q, 0, 2 * sizeof(QlpState));
+    F->pend = F->done = 0;
     S->rtol = rtol;
     S->itnlim = itnlim;
     S->cs = -1.0;
     S->gmin = 1.0e300;
-    if (b1 <= 0.0) { S->istop = b1 < 0.0 ? 9 : 0; S->done = 1; return; }
+    double b1 = *dotv;
+    if (b1 <= 0.0) { S->istop = b1 < 0.0 ? 9 : 0; F->pend = F->done = 1; return; }
     b1 = sqrt(b1);
     S->beta1 = b1;
     S->beta = b1;
     S->phibar = b1;
 }
 
-__global__ void k_mr_scale_v(int32_t n, const MinresState *S, const double *y, double *v) {
-    if (S->done) return;
-    const double s = 1.0 / S->beta;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        v[i] = s * y[i];
-}
+// One iteration is five launches: operator product (block_rows_spmv, or the
+// separate products of the other storages), k_mr_y1, k_mr_y2, k_mr_w or
+// k_qlp_w, k_mr_next.  The dot products that end one kernel are summed by
+// every CTA of the next one (at most kMrBlocks values).  They are bound by
+// launch and synchronisation latency, not by their 0.2 MB vectors; the first
+// form had 16 launches, with the sums in kernels of one CTA.
+constexpr int kMrBlocks = 1216;    // CTAs of the vector kernels (at most)
+constexpr int kNextRows = 128;     // rows per step of k_mr_next
+constexpr int kNextBlocks = 304;
+constexpr int kWyFused = 64;       // constraints whose products ride in the iteration's kernels
 
-__global__ void k_mr_y1(int32_t n, const MinresState *S, double *y, const double *r1) {
-    if (S->done || S->itn < 1) return;   // itn counts completed iterations
-    const double f = S->beta / S->oldb;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        y[i] = y[i] - f * r1[i];
-}
+// The convergence test of the iteration just updated (from x . x), the
+// commit of the MINRES-QLP iterate, then the next Lanczos vector v = y /
+// beta, padded with zeros for the operator (xa), and the partial dots of it
+// with the 2 m columns [U | W] of the constraint reflections (row-major
+// UWr: a thread owns a column and every nsub-th row, so that no sum crosses
+// lanes but the last nsub ones; 36 columns of 30,000 rows are 1.7 us of
+// FP64).
+struct NextParams {
+    int32_t n, nfit, m, R;
+    const int32_t *aig, *p2g;   // padded positions of xa (null: xa has the order of the parameters)
+    MinresState *S;
+    MinresFlags *F;
+    const double *partX;
+    int npX;
+    double maxxnorm;
+    const double *y, *xc, *UWr;
+    double *v, *x, *xa, *partUW;
+};
 
-__global__ void k_mr_alfa(MinresState *S) {
-    if (threadIdx.x || S->done) return;
-    S->alfa = S->dotv;
-}
-
-__global__ void k_mr_y2(int32_t n, const MinresState *S, double *y, double *r1, double *r2, const double *cu) {
-    if (S->done) return;
-    const double f = S->alfa / S->beta;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double yi = y[i] - f * r2[i];
-        r1[i] = r2[i];
-        r2[i] = yi;
-        y[i] = (yi * cu[i]) * cu[i];
+template <bool QLP>
+__global__ void __launch_bounds__(kThreads) k_mr_next(NextParams p) {
+    __shared__ double sh[kThreads / 32], xs[kNextRows], red[kThreads];
+    if (p.F->done) return;
+    const int tid = threadIdx.x;
+    MinresState *S = p.S;
+    const int k = S->k;
+    if (k > 0) {
+        if (S->istop == 9) {
+            if (blockIdx.x == 0 && tid == 0) p.F->pend = 1;
+            return;
+        }
+        const double xnorm = sqrt(sum_of_partials(p.partX, p.npX, sh));
+        const double Anorm = sqrt(S->tnorm2), rnorm = S->phibar;
+        const double test1 = rnorm / (Anorm * xnorm), test2 = S->root / Anorm;
+        int istop = 0;
+        if (k >= S->itnlim) istop = 6;
+        if (S->gmax / S->gmin >= 0.1 / 2.220446049250313e-16) istop = 4;
+        if (test2 <= S->rtol) istop = 2;
+        if (test1 <= S->rtol) istop = 1;
+        const bool commit = !(QLP && xnorm > p.maxxnorm);
+        if (!commit) istop = 5;
+        if (QLP && commit)
+            for (int64_t i = (int64_t)blockIdx.x * blockDim.x + tid; i < p.nfit; i += (int64_t)gridDim.x * blockDim.x)
+                p.x[i] = p.xc[i];
+        if (blockIdx.x == 0 && tid == 0) {
+            S->itn = k;
+            if (commit) {
+                S->Anorm = Anorm;
+                S->ynorm = xnorm;
+                S->rnorm = rnorm;
+            }
+            if (istop) {
+                S->istop = istop;
+                p.F->pend = 1;
+            }
+        }
+        if (istop) return;
+    }
+    const double f = 1.0 / S->beta;
+    const int C = 2 * p.m;
+    const int nsub = C ? kThreads / C : 0, sub = C ? tid / C : 0, cc = C ? tid - sub * C : 0;
+    double acc = 0.0;
+    for (int64_t r0 = (int64_t)blockIdx.x * kNextRows; r0 < p.n; r0 += (int64_t)gridDim.x * kNextRows) {
+        const int64_t i = r0 + tid;
+        if (tid < kNextRows) {
+            double vi = 0.0;
+            if (i < p.nfit) {
+                vi = f * p.y[i];
+                p.v[i] = vi;
+            }
+            if (i < p.n) {
+                int64_t at = i;
+                if (p.aig) {
+                    const int32_t g = p.p2g[i] - 1;
+                    at = (int64_t)g * p.R + i - (p.aig[g] - 1);
+                }
+                p.xa[at] = vi;
+            }
+            xs[tid] = vi;
+        }
+        if (!C) continue;
+        __syncthreads();
+        if (sub < nsub) {
+            const int rows = (int)min((int64_t)kNextRows, p.n - r0);
+            const double *u = p.UWr + r0 * C + cc;
+#pragma unroll 6
+            for (int r = sub; r < rows; r += nsub) acc = fma(u[(int64_t)r * C], xs[r], acc);
+        }
+        __syncthreads();
+    }
+    if (!C) return;
+    red[tid] = acc;
+    __syncthreads();
+    if (tid < C) {
+        double t = 0.0;
+        for (int q = 0; q < nsub; ++q) t += red[q * C + tid];
+        p.partUW[(int64_t)blockIdx.x * C + tid] = t;
     }
 }
 
-__device__ void mr_rot_body(MinresState *S) {
-    double b2 = S->dotv;
-    if (b2 < 0.0) { S->istop = 9; S->done = 1; return; }
+// (paths without block_rows_spmv's extra CTA)
+__global__ void k_mr_promote(MinresFlags *F) {
+    if (threadIdx.x == 0 && blockIdx.x == 0 && F->pend) F->done = 1;
+}
+
+// y = Q^T A Q v on the fitted rows: with the block-row copy the item sums
+// less [U | W] coef (coef of br_coef), else the separate products' ba; then
+// y -= (beta / oldbeta) r1 from the second iteration on, partials of v . y
+struct Y1Params {
+    int32_t nfit, n, m, R;
+    const int32_t *aig, *p2g;
+    const int64_t *itemBeg;
+    const double *part, *UWc, *coef, *ba, *r1, *v;
+    const MinresState *S;
+    const MinresFlags *F;
+    double *y, *partA;
+};
+
+template <bool ITEMS>
+__global__ void __launch_bounds__(kThreads) k_mr_y1(Y1Params p) {
+    __shared__ double sh[kThreads / 32], cs[2 * kWyFused];
+    if (p.F->done) return;
+    const int C = ITEMS ? 2 * p.m : 0;
+    if ((int)threadIdx.x < C) cs[threadIdx.x] = p.coef[threadIdx.x];
+    __syncthreads();
+    const bool upd = p.S->k >= 1;
+    const double f = upd ? p.S->beta / p.S->oldb : 0.0;
+    double acc = 0.0;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < p.nfit; i += (int64_t)gridDim.x * blockDim.x) {
+        double yi;
+        if (ITEMS) {
+            const int32_t g = p.p2g[i] - 1;
+            const int64_t ii = i - (p.aig[g] - 1);
+            yi = 0.0;
+            for (int64_t q = p.itemBeg[g]; q < p.itemBeg[g + 1]; ++q) yi += p.part[q * p.R + ii];
+            double a0 = 0.0, a1 = 0.0;
+#pragma unroll 6
+            for (int q = 0; q < p.m; ++q) {
+                a0 = fma(p.UWc[(int64_t)q * p.n + i], cs[q], a0);
+                a1 = fma(p.UWc[(int64_t)(p.m + q) * p.n + i], cs[p.m + q], a1);
+            }
+            yi -= a0 + a1;
+        } else {
+            yi = p.ba[i];
+        }
+        if (upd) yi = yi - f * p.r1[i];
+        p.y[i] = yi;
+        acc += p.v[i] * yi;
+    }
+    acc = cta_sum(acc, sh);
+    if (threadIdx.x == 0) p.partA[blockIdx.x] = acc;
+}
+
+// alfa = v . y; the new residual r = y - (alfa / beta) r2 into the buffer of
+// the one before r2; y = M^-1 r (diagonal cu), partials of r . y
+__global__ void __launch_bounds__(kThreads) k_mr_y2(int32_t n, const MinresState *S, MinresFlags *F,
+                                                    const double *partA, int npA, double *y, double *rOld,
+                                                    const double *r2, const double *cu, double *partB) {
+    __shared__ double sh[kThreads / 32];
+    if (F->done) return;
+    const double alfa = sum_of_partials(partA, npA, sh);
+    if (blockIdx.x == 0 && threadIdx.x == 0) F->alfa = alfa;
+    const double f = alfa / S->beta;
+    double acc = 0.0;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const double yi = y[i] - f * r2[i];
+        rOld[i] = yi;
+        const double zi = (yi * cu[i]) * cu[i];
+        y[i] = zi;
+        acc += yi * zi;
+    }
+    acc = cta_sum(acc, sh);
+    if (threadIdx.x == 0) partB[blockIdx.x] = acc;
+}
+
+__device__ void mr_rotate(MinresState *S, double b2) {
+    if (b2 < 0.0) { S->istop = 9; return; }
     S->oldb = S->beta;
     S->beta = sqrt(b2);
     S->tnorm2 += S->alfa * S->alfa + S->oldb * S->oldb + S->beta * S->beta;
@@ -705,146 +901,37 @@ __device__ void mr_rot_body(MinresState *S) {
     S->gmin = fmin(S->gmin, gamma);
 }
 
-__global__ void k_mr_rot(MinresState *S) {
-    if (threadIdx.x || S->done) return;
-    mr_rot_body(S);
-}
-
-__global__ void k_mr_w(int32_t n, const MinresState *S, const double *v, double *w, double *w1, double *w2,
-                       double *x) {
-    if (S->done) return;
-    const double oe = S->oldeps, de = S->delta, dn = S->denom, ph = S->phi;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double a = w2[i], b = w[i];
-        w1[i] = a;
-        w2[i] = b;
-        const double wn = (v[i] - oe * a - de * b) * dn;
-        w[i] = wn;
-        x[i] = x[i] + ph * wn;
+// beta^2 = r . y, the rotation (in every CTA), then w (into the buffer of
+// the older of the two kept) and x, partials of x . x
+__global__ void __launch_bounds__(kThreads) k_mr_w(int32_t n, const MinresState *Sin, MinresState *Sout,
+                                                   const MinresFlags *F, const double *partB, int npB,
+                                                   const double *v, double *wOld, const double *w, double *x,
+                                                   double *partX) {
+    __shared__ double sh[kThreads / 32];
+    __shared__ MinresState ss;
+    if (F->done) return;
+    const double b2 = sum_of_partials(partB, npB, sh);
+    if (threadIdx.x == 0) {
+        ss = *Sin;
+        ss.alfa = F->alfa;
+        mr_rotate(&ss, b2);
+        ss.k += 1;
+        if (blockIdx.x == 0) *Sout = ss;
     }
-}
-
-__device__ void mr_test_body(MinresState *S) {
-    S->itn += 1;
-    S->Anorm = sqrt(S->tnorm2);
-    S->ynorm = sqrt(S->dotv);
-    S->rnorm = S->phibar;
-    const double test1 = S->rnorm / (S->Anorm * S->ynorm);
-    const double test2 = S->root / S->Anorm;
-    const double Acond = S->gmax / S->gmin;
-    int istop = 0;
-    if (S->itn >= S->itnlim) istop = 6;
-    if (Acond >= 0.1 / 2.220446049250313e-16) istop = 4;
-    if (test2 <= S->rtol) istop = 2;
-    if (test1 <= S->rtol) istop = 1;
-    if (istop) { S->istop = istop; S->done = 1; }
-}
-
-__global__ void k_mr_test(MinresState *S) {
-    if (threadIdx.x || S->done) return;
-    mr_test_body(S);
-}
-
-// Fused forms of one MINRES iteration (diagonal or no preconditioner): each
-// vector update also forms its dot product's partial sums with the grid and
-// element order of k_dot_partial (kDotBlocks x kThreads, grid-stride), and
-// each scalar step sums the partials as k_sum_final does, so the iterates
-// are bit-identical to the unfused sequence with half the launches.
-__global__ void k_mr_v_pad(int32_t nfit, int32_t n, const MinresState *S, const double *y, double *v, double *xa) {
-    if (S->done) return;
-    const double s = 1.0 / S->beta;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        double vi = 0.0;
-        if (i < nfit) {
-            vi = s * y[i];
-            v[i] = vi;
-        }
-        xa[i] = vi;
-    }
-}
-
-// y = ba - (beta / oldbeta) r1 (from the second iteration on), partials of v . y
-__global__ void k_mr_y1_dot(int32_t n, const MinresState *S, const double *ba, double *y, const double *r1,
-                            const double *v, double *part) {
-    __shared__ double sh[kThreads];
-    if (S->done) return;
-    const bool upd = S->itn >= 1;
-    const double f = upd ? S->beta / S->oldb : 0.0;
+    __syncthreads();
+    if (ss.istop == 9) return;
+    const double oe = ss.oldeps, de = ss.delta, dn = ss.denom, ph = ss.phi;
     double acc = 0.0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        double yi = ba[i];
-        if (upd) yi = yi - f * r1[i];
-        y[i] = yi;
-        acc += v[i] * yi;
-    }
-    acc = block_sum(acc, sh);
-    if (threadIdx.x == 0) part[blockIdx.x] = acc;
-}
-
-// k_mr_y2, partials of r2 . y
-__global__ void k_mr_y2_dot(int32_t n, const MinresState *S, double *y, double *r1, double *r2, const double *cu,
-                            double *part) {
-    __shared__ double sh[kThreads];
-    if (S->done) return;
-    const double f = S->alfa / S->beta;
-    double acc = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double yi = y[i] - f * r2[i];
-        r1[i] = r2[i];
-        r2[i] = yi;
-        const double zi = (yi * cu[i]) * cu[i];
-        y[i] = zi;
-        acc += yi * zi;
-    }
-    acc = block_sum(acc, sh);
-    if (threadIdx.x == 0) part[blockIdx.x] = acc;
-}
-
-// k_mr_w, partials of x . x
-__global__ void k_mr_w_dot(int32_t n, const MinresState *S, const double *v, double *w, double *w1, double *w2,
-                           double *x, double *part) {
-    __shared__ double sh[kThreads];
-    if (S->done) return;
-    const double oe = S->oldeps, de = S->delta, dn = S->denom, ph = S->phi;
-    double acc = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double a = w2[i], b = w[i];
-        w1[i] = a;
-        w2[i] = b;
-        const double wn = (v[i] - oe * a - de * b) * dn;
-        w[i] = wn;
+        const double wn = (v[i] - oe * wOld[i] - de * w[i]) * dn;
+        wOld[i] = wn;
         const double xi = x[i] + ph * wn;
         x[i] = xi;
         acc += xi * xi;
     }
-    acc = block_sum(acc, sh);
-    if (threadIdx.x == 0) part[blockIdx.x] = acc;
+    acc = cta_sum(acc, sh);
+    if (threadIdx.x == 0) partX[blockIdx.x] = acc;
 }
-
-// the partials summed as k_sum_final, then the scalar step: 0 alfa, 1 the
-// rotation, 2 the convergence test
-__global__ void k_mr_sum_step(const double *part, int np, MinresState *S, int step) {
-    __shared__ double sh[kThreads];
-    if (S->done) return;
-    double acc = 0.0;
-    for (int i = threadIdx.x; i < np; i += blockDim.x) acc += part[i];
-    acc = block_sum(acc, sh);
-    if (threadIdx.x) return;
-    S->dotv = acc;
-    if (step == 0) S->alfa = acc;
-    else if (step == 1) mr_rot_body(S);
-    else mr_test_body(S);
-}
-
-// MINRES-QLP (Choi, Paige & Saunders 2011; minresqlpModule.f90:411-1333 in
-// the reference): the Lanczos scalars of MinresState plus the rows of the
-// lower-triangular L = R P not yet final, the final u values and the
-// rotations of the current iteration for the vector kernel
-struct QlpState {
-    double etaA, thA, gA, tauA, etaB, thB, gB, tauB, uF1, uF2;
-    double c1, s1, c2, s2, uA, uB, uC;
-    int k, commit;
-};
 
 __device__ __forceinline__ void d_sym_ortho(double a, double b, double *c, double *s, double *r) {
     *r = sqrt(a * a + b * b);
@@ -853,19 +940,11 @@ __device__ __forceinline__ void d_sym_ortho(double a, double b, double *c, doubl
     *s = b / *r;
 }
 
-__global__ void k_qlp_init(QlpState *Q) {
-    if (threadIdx.x) return;
-    memset(Q, 0, sizeof(QlpState));
-}
-
 // beta_{k+1}, the left reflection (column k of R, tau_k), the right
 // reflections P(k-2,k), P(k-1,k) and u; the same arithmetic as the oracle
-__global__ void k_qlp_rot(MinresState *S, QlpState *Q) {
-    if (threadIdx.x || S->done) return;
-    double b2 = S->dotv;
-    if (b2 < 0.0) { S->istop = 9; S->done = 1; return; }
-    const int k = S->itn + 1;
-    Q->k = k;
+__device__ void qlp_rotate(MinresState *S, QlpState *Q, double b2) {
+    if (b2 < 0.0) { S->istop = 9; return; }
+    const int k = S->k + 1;
     S->oldb = S->beta;
     S->beta = sqrt(b2);
     S->tnorm2 += S->alfa * S->alfa + S->oldb * S->oldb + S->beta * S->beta;
@@ -916,71 +995,121 @@ __global__ void k_qlp_rot(MinresState *S, QlpState *Q) {
     Q->etaB = etaC; Q->thB = thC; Q->gB = gC; Q->tauB = tau;
 }
 
-// W = V P (w_{k-2} final into xp) and the candidate iterate xc
-__global__ void k_qlp_w(int32_t n, const MinresState *S, const QlpState *Q, const double *v, double *wa,
-                        double *wb, double *xp, double *xc) {
-    if (S->done) return;
-    const int k = Q->k;
-    const double c1 = Q->c1, s1 = Q->s1, c2 = Q->c2, s2 = Q->s2, uA = Q->uA, uB = Q->uB, uC = Q->uC;
+// the scalar step of MINRES-QLP (in every CTA), then W = V P (w_{k-2} final
+// into xp) and the candidate iterate xc, partials of xc . xc
+__global__ void __launch_bounds__(kThreads) k_qlp_w(int32_t n, const MinresState *Sin, MinresState *Sout,
+                                                    const QlpState *Qin, QlpState *Qout, const MinresFlags *F,
+                                                    const double *partB, int npB, const double *v, double *wa,
+                                                    double *wb, double *xp, double *xc, double *partX) {
+    __shared__ double sh[kThreads / 32];
+    __shared__ MinresState ss;
+    __shared__ QlpState qs;
+    if (F->done) return;
+    const double b2 = sum_of_partials(partB, npB, sh);
+    if (threadIdx.x == 0) {
+        ss = *Sin;
+        qs = *Qin;
+        ss.alfa = F->alfa;
+        qlp_rotate(&ss, &qs, b2);
+        ss.k += 1;
+        if (blockIdx.x == 0) {
+            *Sout = ss;
+            *Qout = qs;
+        }
+    }
+    __syncthreads();
+    if (ss.istop == 9) return;
+    const int k = ss.k;
+    const double c1 = qs.c1, s1 = qs.s1, c2 = qs.c2, s2 = qs.s2, uA = qs.uA, uB = qs.uB, uC = qs.uC;
+    double acc = 0.0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        double a = wa[i], bb = wb[i], c = v[i];
+        double a = wa[i], bb = wb[i], c = v[i], xi = xp[i];
         if (k >= 3) {
             const double a2 = c1 * a + s1 * c;
             c = s1 * a - c1 * c;
             a = a2;
-            xp[i] = xp[i] + uA * a;
+            xi = xi + uA * a;
+            xp[i] = xi;
         }
         if (k >= 2) {
-            const double b2 = c2 * bb + s2 * c;
+            const double b2r = c2 * bb + s2 * c;
             c = s2 * bb - c2 * c;
-            bb = b2;
+            bb = b2r;
         }
         wa[i] = bb;
         wb[i] = c;
-        xc[i] = xp[i] + uB * bb + uC * c;
+        xi = xi + uB * bb + uC * c;
+        xc[i] = xi;
+        acc += xi * xi;
     }
-}
-
-__global__ void k_qlp_test(MinresState *S, QlpState *Q, double maxxnorm) {
-    if (threadIdx.x || S->done) return;
-    Q->commit = 0;
-    const double xnorm = sqrt(S->dotv);
-    if (xnorm > maxxnorm) { S->istop = 5; S->done = 1; S->itn += 1; return; }
-    Q->commit = 1;
-    S->itn += 1;
-    S->ynorm = xnorm;
-    S->rnorm = S->phibar;
-    const double test1 = S->rnorm / (S->Anorm * xnorm);
-    const double test2 = S->root / S->Anorm;
-    const double Acond = S->gmax / S->gmin;
-    int istop = 0;
-    if (S->itn >= S->itnlim) istop = 6;
-    if (Acond >= 0.1 / 2.220446049250313e-16) istop = 4;
-    if (test2 <= S->rtol) istop = 2;
-    if (test1 <= S->rtol) istop = 1;
-    if (istop) { S->istop = istop; S->done = 1; }
-}
-
-__global__ void k_qlp_commit(int32_t n, const QlpState *Q, const double *xc, double *x) {
-    if (!Q->commit) return;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        x[i] = xc[i];
-}
-
-__global__ void k_copy_pad(int32_t n, int32_t ntot, const double *x, double *xa) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < ntot; i += (int64_t)gridDim.x * blockDim.x)
-        xa[i] = i < n ? x[i] : 0.0;
-}
-
-__global__ void k_copy_if(int32_t n, const MinresState *S, const double *a, double *b) {
-    if (S && S->done) return;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        b[i] = a[i];
+    acc = cta_sum(acc, sh);
+    if (threadIdx.x == 0) partX[blockIdx.x] = acc;
 }
 
 __global__ void k_apply_precond(int32_t n, const double *r, const double *cu, double *y) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         y[i] = (r[i] * cu[i]) * cu[i];
+}
+
+// ---- the reflections as columns: U (n x m, column k = V_k with Vk at n - m + k)
+__global__ void k_u_columns(int32_t n, int32_t m, const double *V, const double *Vk, double *U) {
+    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < (int64_t)n * m;
+         e += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t k = e / n, i = e - k * n, kn = n - m + k;
+        U[e] = i < kn ? V[e] : (i == kn ? Vk[k] : 0.0);
+    }
+}
+
+// M = U^T W, one CTA per element
+__global__ void __launch_bounds__(kThreads) k_column_dots(int32_t n, int32_t m, const double *U, const double *W,
+                                                          double *M) {
+    __shared__ double sh[kThreads / 32];
+    const double *u = U + (int64_t)(blockIdx.x / m) * n, *w = W + (int64_t)(blockIdx.x % m) * n;
+    double v = 0.0;
+    for (int i = threadIdx.x; i < n; i += kThreads) v = fma(u[i], w[i], v);
+    v = cta_sum(v, sh);
+    if (threadIdx.x == 0) M[blockIdx.x] = v;
+}
+
+// S = T M T^T (T upper triangular), one CTA; X scratch
+__global__ void k_wy_s(int32_t m, const double *T, const double *M, double *X, double *S) {
+    for (int e = threadIdx.x; e < m * m; e += blockDim.x) {
+        const int r = e / m, c = e % m;
+        double v = 0.0;
+        for (int q = r; q < m; ++q) v = fma(T[r * m + q], M[q * m + c], v);
+        X[e] = v;
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < m * m; e += blockDim.x) {
+        const int r = e / m, c = e % m;
+        double v = 0.0;
+        for (int q = c; q < m; ++q) v = fma(X[r * m + q], T[c * m + q], v);
+        S[e] = v;
+    }
+}
+
+// Z = W T^T - U S / 2, so that Q^T A Q = A - Z U^T - U Z^T; [U | W] by rows
+__global__ void k_wy_zrows(int32_t n, int32_t m, const double *U, const double *W, const double *T, const double *S,
+                           double *Z, double *UWr) {
+    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < (int64_t)n * m;
+         e += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t k = e / n, i = e - k * n;
+        double z = 0.0, h = 0.0;
+        for (int64_t b = k; b < m; ++b) z = fma(W[b * n + i], T[k * m + b], z);
+        for (int64_t b = 0; b < m; ++b) h = fma(U[b * n + i], S[b * m + k], h);
+        Z[e] = z - 0.5 * h;
+        UWr[i * 2 * m + k] = U[e];
+        UWr[i * 2 * m + m + k] = W[e];
+    }
+}
+
+// diagonal of Q^T A Q
+__global__ void k_diag_eliminate(int32_t n, int32_t m, const double *U, const double *Z, double *dg) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    double a = 0.0;
+    for (int64_t k = 0; k < m; ++k) a = fma(Z[k * n + i], U[k * n + i], a);
+    dg[i] = dg[i] - 2.0 * a;
 }
 
 __global__ void k_precond(int32_t n, const double *dg, double *cu) {
@@ -1016,17 +1145,17 @@ struct Solver {
     cudaStream_t s;
     int nsm;
     SparseBlocks sb;
-    double *part = nullptr;
+    bool useRows = false;         // the product takes the job's block-row copy
+    double *part = nullptr, *partOwned = nullptr;   // partial sums of dot()
     explicit Solver(mpgpu_ctx *cc) : c(cc), j(cc->j), s(cc->stream) {
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
     }
     ~Solver() {
-        // part is stream-ordered (cudaMallocAsync on the context's stream)
-        if (part) cudaFreeAsync(part, s);
-        part = nullptr;
+        // stream-ordered (cudaMallocAsync on the context's stream)
+        if (partOwned) cudaFreeAsync(partOwned, s);
         dfree(wyPart); dfree(wyT);
         dfree(sb.rowStart); dfree(sb.bcol); dfree(sb.boff); dfree(sb.bld); dfree(sb.tOff);
-        dfree(sb.colStart); dfree(sb.colBlk); dfree(sb.tBase); dfree(sb.tbuf); dfree(part);
+        dfree(sb.colStart); dfree(sb.colBlk); dfree(sb.tBase); dfree(sb.tbuf);
         dfree(sb.tStr); dfree(sb.brow); dfree(sb.rowPart);
         dfree(sb.colItemJ); dfree(sb.colItemQ0); dfree(sb.colItemQ1); dfree(sb.colItemBeg); dfree(sb.colPart);
         dfree(pmvRow); dfree(pmvPart);
@@ -1170,9 +1299,6 @@ struct Solver {
         }
         ciBeg[j.nG] = (int64_t)ciJ.size();
         sb.nColItem = (int64_t)ciJ.size();
-        int32_t minnp = maxnp;
-        for (int32_t I = 1; I <= j.nG; ++I) minnp = std::min(minnp, aig[I] - aig[I - 1]);
-        sb.uniform = (sb.smallGroups && minnp == maxnp) ? maxnp : 0;
         sb.nblk = nb;
         sb.tlen = tl;
         auto up = [&](auto *&d, const auto &h) -> cudaError_t {
@@ -1202,25 +1328,24 @@ struct Solver {
         return MPGPU_OK;
     }
 
+    // what avprd0 needs for the current matrix
+    int32_t prepare_product() {
+        if (j.matsto != 2) {
+            MPG_CUDA(c, alloc_pmv(j.nVar));
+            return MPGPU_OK;
+        }
+        useRows = block_rows_fit(c);
+        return useRows ? block_rows_build(c) : build_blocks();
+    }
+
     // y = A x (full parameter space)
     void avprd0(const double *x, double *y) {
-        if (j.matsto == 2 && sb.smallGroups) {
+        if (useRows) {
+            block_rows_product(j.br, j.aig, j.p2g, x, y, s);
+        } else if (j.matsto == 2 && sb.smallGroups) {
             const unsigned gb = grid(sb.nblk);
-#define MPG_SPMV_BLOCKS(G)                                                                                  \
-    k_spmv_blocks<G><<<gb, kThreads, 0, s>>>(sb.nblk, sb.brow, j.aig, sb.bcol, sb.boff, sb.bld, sb.tOff, sb.tStr, \
-                                             j.matD, x, sb.tbuf, sb.rowPart)
-            switch (sb.uniform) {
-            case 1: MPG_SPMV_BLOCKS(1); break;
-            case 2: MPG_SPMV_BLOCKS(2); break;
-            case 3: MPG_SPMV_BLOCKS(3); break;
-            case 4: MPG_SPMV_BLOCKS(4); break;
-            case 5: MPG_SPMV_BLOCKS(5); break;
-            case 6: MPG_SPMV_BLOCKS(6); break;
-            case 7: MPG_SPMV_BLOCKS(7); break;
-            case 8: MPG_SPMV_BLOCKS(8); break;
-            default: MPG_SPMV_BLOCKS(0); break;
-            }
-#undef MPG_SPMV_BLOCKS
+            k_spmv_blocks<<<gb, kThreads, 0, s>>>(sb.nblk, sb.brow, j.aig, sb.bcol, sb.boff, sb.bld, sb.tOff, sb.tStr,
+                                                  j.matD, x, sb.tbuf, sb.rowPart);
             k_spmv_colitems<<<wgrid(sb.nColItem), kThreads, 0, s>>>(sb.nColItem, sb.colItemJ, sb.colItemQ0,
                                                                     sb.colItemQ1, j.aig, sb.rowStart, sb.rowPart,
                                                                     sb.colStart, sb.tBase, sb.tbuf, sb.colPart);
@@ -1252,6 +1377,39 @@ struct Solver {
             apply();
         }
     }
+    // Reflections of at most kWyFused constraints as n x m columns: U, W = A
+    // U, Z with Q^T A Q = A - Z U^T - U Z^T (its diagonal and band follow
+    // without applying reflection after reflection), S = T (U^T A U) T^T, and
+    // [U | W] by rows for the iteration's dot products.  Q^T A Q x = A x - W a
+    // - U c with a = T^T s, c = T t - S s, s = U^T x, t = W^T x: the 2 m dots
+    // and one product with the unreflected x, instead of a reflection pass
+    // before and after the product.
+    struct Wy {
+        int32_t m = 0;
+        double *UWc = nullptr, *UWr = nullptr, *Z = nullptr, *S = nullptr;
+    } wy;
+    bool wy_fits() const { return useRows && j.ncon > 0 && j.ncon <= kWyFused; }
+    int64_t wy_len() const { return wy_fits() ? 5 * (int64_t)j.ncon * j.nVar + 3 * (int64_t)j.ncon * j.ncon : 0; }
+    // buf: wy_len() doubles
+    int32_t wy_build(double *buf) {
+        const int32_t m = j.ncon, n = j.nVar;
+        const int64_t nm = (int64_t)n * m;
+        wy.UWc = buf;
+        wy.UWr = buf + 2 * nm;
+        wy.Z = buf + 4 * nm;
+        wy.S = buf + 5 * nm;
+        double *M = wy.S + m * m, *X = M + m * m;
+        k_u_columns<<<grid(nm), kThreads, 0, s>>>(n, m, j.qlV, j.qlVk, wy.UWc);
+        for (int32_t k = 0; k < m; ++k)
+            MPG_CUDA(c, block_rows_product(j.br, j.aig, j.p2g, wy.UWc + (int64_t)k * n, wy.UWc + nm + (int64_t)k * n, s));
+        k_column_dots<<<m * m, kThreads, 0, s>>>(n, m, wy.UWc, wy.UWc + nm, M);
+        k_wy_s<<<1, 1024, 0, s>>>(m, j.qlT, M, X, wy.S);
+        k_wy_zrows<<<grid(nm), kThreads, 0, s>>>(n, m, wy.UWc, wy.UWc + nm, j.qlT, wy.S, wy.Z, wy.UWr);
+        MPG_CUDA(c, cudaGetLastError());
+        wy.m = m;
+        return MPGPU_OK;
+    }
+
     // band of Q^T A Q (pede's preconditioner fill and qlpssq with band
     // width mbandw) and its lltdec factor with the block spikes
     int32_t band_build(BandPre &P, int32_t mbandw, int32_t lprecm, double *v, double *tmp, double *yk,
@@ -1259,12 +1417,16 @@ struct Solver {
         const int32_t n = j.nVar, nfit = j.nVar - j.ncon;
         if (mbandw > MPGPU_BAND_MAX) return set_err(c, MPGPU_ERR_LIMIT, "band preconditioner wider than 32");
         if (band_alloc(P, n, nfit, mbandw - 1)) return set_err(c, MPGPU_ERR_ALLOC, "band preconditioner");
-        MPG_CUDA(c, band_fill(P, n, j.matsto, j.matD, j.aig, j.p2g, sb.rowStart, sb.bcol, sb.boff, sb.bld, s));
-        cudaError_t e = cudaSuccess;
-        reflections(v, tmp, yk, dsc, [&] {
-            if (e == cudaSuccess) e = band_reflect(P, n, v, yk, dsc, s);
-        });
-        MPG_CUDA(c, e);
+        MPG_CUDA(c, band_fill(P, n, j.matsto, j.matD, j.aig, j.p2g, j.rowBlk0, j.blkJ, j.blkOff, j.blkLd, j.nmat, s));
+        if (wy.m > 0) {
+            MPG_CUDA(c, band_eliminate(P, n, wy.m, wy.UWc, wy.Z, s));
+        } else {
+            cudaError_t e = cudaSuccess;
+            reflections(v, tmp, yk, dsc, [&] {
+                if (e == cudaSuccess) e = band_reflect(P, n, v, yk, dsc, s);
+            });
+            MPG_CUDA(c, e);
+        }
         MPG_CUDA(c, band_factor(P, lprecm, s));
         return MPGPU_OK;
     }
@@ -1329,7 +1491,8 @@ int32_t solve_inversion(mpgpu_ctx *c, const double *consResiduals, double *corrO
     MPG_CUDA(c, cudaMallocAsync(&yv, sizeof(double) * (ncon + 1), s));
     MPG_CUDA(c, cudaMallocAsync(&used, sizeof(int32_t) * n, s));
     MPG_CUDA(c, cudaMallocAsync(&piv, sizeof(int32_t) * 4, s));
-    MPG_CUDA(c, cudaMallocAsync(&S.part, sizeof(double) * (kDotBlocks + 8), s));
+    MPG_CUDA(c, cudaMallocAsync(&S.partOwned, sizeof(double) * (kDotBlocks + 8), s));
+    S.part = S.partOwned;
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
@@ -1455,49 +1618,51 @@ int32_t solve_minres(mpgpu_ctx *c, const double *consResiduals, double rtol, int
     DevJob &j = c->j;
     cudaStream_t s = c->stream;
     const int32_t n = j.nVar, ncon = j.ncon, nfit = n - ncon;
-    if (j.matsto == 2) {
-        int32_t rc = S.build_blocks();
-        if (rc) return rc;
-    } else {
-        MPG_CUDA(c, S.alloc_pmv(n));
-    }
-    MPG_CUDA(c, cudaMallocAsync(&S.part, sizeof(double) * (kDotBlocks + 8), s));
-    // workspace released on every return
-    struct Scratch {
-        std::vector<double *> bufs;
-        MinresState *St = nullptr;
-        QlpState *Qs = nullptr;
-        cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
-        ~Scratch() {
-            for (double *p : bufs) cudaFree(p);
-            if (St) cudaFree(St);
-            if (Qs) cudaFree(Qs);
-            for (cudaEvent_t e : ev)
-                if (e) cudaEventDestroy(e);
+    // released on every return
+    struct Events {
+        cudaEvent_t e[3] = {nullptr, nullptr, nullptr};
+        ~Events() {
+            for (cudaEvent_t x : e)
+                if (x) cudaEventDestroy(x);
         }
-    } W;
-    auto vec = [&](int64_t len) -> double * {
-        double *p = nullptr;
-        if (cudaMalloc(&p, sizeof(double) * std::max<int64_t>(len, 1)) != cudaSuccess) return nullptr;
-        W.bufs.push_back(p);
+    } ev;
+    for (cudaEvent_t &x : ev.e) cudaEventCreate(&x);
+    cudaEvent_t e0 = ev.e[0], e1 = ev.e[1], ep = ev.e[2];
+    cudaEventRecord(e0, s);
+    int32_t rc = S.prepare_product();
+    if (rc) return rc;
+    // workspace, kept by the job: vectors, partial sums, the reflections'
+    // columns, the iteration's scalars
+    const bool fused = S.useRows && ncon <= kWyFused;
+    const int64_t nv = ((int64_t)std::max(n, 1) + 1) / 2 * 2;   // vectors stay 16-byte aligned
+    const int64_t nxp = fused ? ((int64_t)j.nG * j.br.R + 1) / 2 * 2 : nv;
+    const int nb = (int)std::min<int64_t>(kMrBlocks, (nfit + kThreads - 1) / kThreads + (nfit < 1));
+    const int nbNext = (int)std::min<int64_t>(kNextBlocks, (n + kNextRows - 1) / kNextRows);
+    const int64_t nUW = (int64_t)nbNext * 2 * kWyFused;
+    const int64_t scalLen = (2 * sizeof(MinresState) + 2 * sizeof(QlpState) + sizeof(MinresFlags)) / 8 + 8;
+    const int64_t len = 16 * nv + nxp + 3 * kMrBlocks + kDotBlocks + 8 + nUW + 2 * kWyFused + scalLen + S.wy_len();
+    MPG_CUDA(c, dgrow(j, j.work, len));
+    double *at = j.work;
+    auto vec = [&](int64_t l) {
+        double *p = at;
+        at += l;
         return p;
     };
-    double *rhs = vec(n), *xa = vec(n), *ba = vec(n), *dg = vec(n), *cu = vec(n), *tmp = vec(n), *yk = vec(n);
-    double *r1 = vec(n), *r2 = vec(n), *y = vec(n), *v = vec(n), *w = vec(n), *w1 = vec(n), *w2 = vec(n);
-    double *x = vec(n);
-    double *wa = nullptr, *wb = nullptr, *xp = nullptr, *xc = nullptr;
-    if (qlp) { wa = vec(n); wb = vec(n); xp = vec(n); xc = vec(n); }
-    MinresState *&St = W.St;
-    QlpState *&Qs = W.Qs;
-    MPG_CUDA(c, cudaMalloc(&St, sizeof(MinresState)));
-    if (qlp) MPG_CUDA(c, cudaMalloc(&Qs, sizeof(QlpState)));
-    for (double *p : W.bufs)
-        if (!p) return set_err(c, MPGPU_ERR_ALLOC, "MINRES workspace");
-    cudaEvent_t &e0 = W.ev[0], &e1 = W.ev[1], &ep = W.ev[2];
-    cudaEventCreate(&e0);
-    cudaEventCreate(&e1);
-    cudaEventRecord(e0, s);
+    double *xa = vec(nxp), *rhs = vec(nv), *ba = vec(nv), *dg = vec(nv), *cu = vec(nv), *tmp = vec(nv), *yk = vec(nv);
+    double *r[2] = {vec(nv), vec(nv)}, *y = vec(nv), *v = vec(nv), *w[2] = {vec(nv), vec(nv)}, *x = vec(nv);
+    double *xp = vec(nv), *xc = vec(nv), *xb = vec(nv);
+    double *partA = vec(kMrBlocks), *partB = vec(kMrBlocks), *partX = vec(kMrBlocks), *partD = vec(kDotBlocks + 8);
+    double *partUW = vec(nUW), *coef = vec(2 * kWyFused);
+    MinresState *St = reinterpret_cast<MinresState *>(at);
+    QlpState *Qs = reinterpret_cast<QlpState *>(St + 2);
+    MinresFlags *F = reinterpret_cast<MinresFlags *>(Qs + 2);
+    at += scalLen;
+    S.part = partD;
     MPG_CUDA(c, cudaMemcpyAsync(rhs, j.gvec, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
+    if (S.wy_fits()) {
+        rc = S.wy_build(at);
+        if (rc) return rc;
+    }
     std::vector<double> yc(ncon > 0 ? ncon : 1, 0.0);
     double *dsc = c->scal + 300;
     if (ncon > 0) {
@@ -1507,10 +1672,10 @@ int32_t solve_minres(mpgpu_ctx *c, const double *consResiduals, double rtol, int
             yc[k - 1] = ((consResiduals ? consResiduals[k - 1] : 0.0) - d) / j.hL[(size_t)(k - 1) * ncon + k - 1];
         }
         // rhs - A Q [0; y], then Q^T
-        MPG_CUDA(c, cudaMemsetAsync(xa, 0, sizeof(double) * n, s));
-        MPG_CUDA(c, cudaMemcpyAsync(xa + nfit, yc.data(), sizeof(double) * ncon, cudaMemcpyHostToDevice, s));
-        S.qlmlq(xa, 0);
-        S.avprd0(xa, ba);
+        MPG_CUDA(c, cudaMemsetAsync(xb, 0, sizeof(double) * n, s));
+        MPG_CUDA(c, cudaMemcpyAsync(xb + nfit, yc.data(), sizeof(double) * ncon, cudaMemcpyHostToDevice, s));
+        S.qlmlq(xb, 0);
+        S.avprd0(xb, ba);
         k_sub<<<S.grid(n), kThreads, 0, s>>>(n, rhs, ba);
         S.qlmlq(rhs, 1);
     }
@@ -1521,89 +1686,80 @@ int32_t solve_minres(mpgpu_ctx *c, const double *consResiduals, double rtol, int
     const int32_t mbandw = c->mbandw;
     BandPre P;
     struct BandGuard { BandPre &p; ~BandGuard() { band_free(p); } } bandGuard{P};
-    cudaEventCreate(&ep);
     if (mbandw == 0) {
         if (j.matsto == 2) k_sparse_diag<<<S.grid(n), kThreads, 0, s>>>(n, j.matD, dg);
         else k_get_diag<<<S.grid(n), kThreads, 0, s>>>(n, j.matD, dg);
-        S.reflections(v, tmp, yk, dsc, [&] { k_diag_update<<<S.grid(n), kThreads, 0, s>>>(n, dg, v, yk, dsc); });
+        if (S.wy.m > 0)
+            k_diag_eliminate<<<(n + kThreads - 1) / kThreads, kThreads, 0, s>>>(n, S.wy.m, S.wy.UWc, S.wy.Z, dg);
+        else
+            S.reflections(v, tmp, yk, dsc, [&] { k_diag_update<<<S.grid(n), kThreads, 0, s>>>(n, dg, v, yk, dsc); });
         k_precond<<<S.grid(nfit), kThreads, 0, s>>>(nfit, dg, cu);
     } else {
         k_fill<<<S.grid(nfit), kThreads, 0, s>>>(nfit, 1.0, cu);
         if (mbandw > 0) {
-            int32_t rc = S.band_build(P, mbandw, c->lprecm, v, tmp, yk, dsc);
+            rc = S.band_build(P, mbandw, c->lprecm, v, tmp, yk, dsc);
             if (rc) return rc;
         }
     }
     cudaEventRecord(ep, s);
-    const int *doneFlag = &St->done;
     // MINRES state: x = 0, r1 = r2 = b, y = M^-1 r1, beta1 = sqrt(r1.y)
     MPG_CUDA(c, cudaMemsetAsync(x, 0, sizeof(double) * n, s));
-    MPG_CUDA(c, cudaMemsetAsync(w, 0, sizeof(double) * n, s));
-    MPG_CUDA(c, cudaMemsetAsync(w1, 0, sizeof(double) * n, s));
-    MPG_CUDA(c, cudaMemsetAsync(w2, 0, sizeof(double) * n, s));
-    MPG_CUDA(c, cudaMemcpyAsync(r1, rhs, sizeof(double) * nfit, cudaMemcpyDeviceToDevice, s));
-    MPG_CUDA(c, cudaMemcpyAsync(r2, rhs, sizeof(double) * nfit, cudaMemcpyDeviceToDevice, s));
-    k_apply_precond<<<S.grid(nfit), kThreads, 0, s>>>(nfit, r1, cu, y);
+    MPG_CUDA(c, cudaMemsetAsync(xa, 0, sizeof(double) * nxp, s));
+    for (double *p : {w[0], w[1], xp}) MPG_CUDA(c, cudaMemsetAsync(p, 0, sizeof(double) * n, s));
+    for (double *p : {r[0], r[1]})
+        MPG_CUDA(c, cudaMemcpyAsync(p, rhs, sizeof(double) * nfit, cudaMemcpyDeviceToDevice, s));
+    k_apply_precond<<<S.grid(nfit), kThreads, 0, s>>>(nfit, r[0], cu, y);
     if (mbandw > 0) MPG_CUDA(c, band_solve(P, nullptr, y, s));
-    dot(r1, y, nfit, S.part, &St->dotv, s);
-    k_mr_init<<<1, 32, 0, s>>>(St, rtol, itnlim);
+    dot(r[0], y, nfit, partD, dsc, s);
+    k_mr_init<<<1, 32, 0, s>>>(St, qlp ? Qs : nullptr, F, dsc, rtol, itnlim);
     const double maxxnorm = (double)nfit / sqrt(2.220446049250313e-16);
-    if (qlp) {
-        k_qlp_init<<<1, 32, 0, s>>>(Qs);
-        MPG_CUDA(c, cudaMemsetAsync(wa, 0, sizeof(double) * n, s));
-        MPG_CUDA(c, cudaMemsetAsync(wb, 0, sizeof(double) * n, s));
-        MPG_CUDA(c, cudaMemsetAsync(xp, 0, sizeof(double) * n, s));
-    }
-    MinresState hs;
-    int it = 0;
-    const int batch = 16;
+    const bool pad = fused && !j.br.uniform;
+    NextParams np{n,  nfit, fused ? ncon : 0, fused ? j.br.R : 0, pad ? j.aig : nullptr, j.p2g, St, F,
+                  partX, nb, maxxnorm, y, xc, S.wy.UWr, v, x, xa, partUW};
+    Y1Params y1{nfit, n, fused ? ncon : 0, fused ? j.br.R : 0, j.aig, j.p2g, j.br.itemBeg, j.br.part, S.wy.UWc, coef,
+                ba, r[0], v, St, F, y, partA};
+    const BlockRowsCoef bc{fused ? ncon : 0, nbNext, partUW, j.qlT, S.wy.S, coef, &F->pend, &F->done};
+    auto next = [&](int cur) {
+        np.S = St + cur;
+        if (qlp) k_mr_next<true><<<nbNext, kThreads, 0, s>>>(np);
+        else k_mr_next<false><<<nbNext, kThreads, 0, s>>>(np);
+    };
+    next(0);
     // the iterations of one batch are recorded once as a CUDA graph and
     // replayed (all scalars live on the device); direct launches if the
-    // capture is refused
-    const bool fused = !qlp && mbandw <= 0;
+    // capture is refused.  An even number: the two copies of the scalars and
+    // the buffer pairs have swapped back at its end.
+    const int batch = 16;
     auto batchBody = [&] {
         for (int q = 0; q < batch; ++q) {
+            const int a = q & 1, b = 1 - a;   // current and next scalars; older and current of r and w
+            y1.S = St + a;
+            y1.r1 = r[a];
             if (fused) {
-                k_mr_v_pad<<<S.grid(n), kThreads, 0, s>>>(nfit, n, St, y, v, xa);
+                block_rows_spmv(j.br, xa, &F->done, &bc, s);
+                k_mr_y1<true><<<nb, kThreads, 0, s>>>(y1);
+            } else {
+                k_mr_promote<<<1, 32, 0, s>>>(F);
                 S.qlmlq(xa, 0);
                 S.avprd0(xa, ba);
                 S.qlmlq(ba, 1);
-                k_mr_y1_dot<<<kDotBlocks, kThreads, 0, s>>>(nfit, St, ba, y, r1, v, S.part);
-                k_mr_sum_step<<<1, kThreads, 0, s>>>(S.part, kDotBlocks, St, 0);
-                k_mr_y2_dot<<<kDotBlocks, kThreads, 0, s>>>(nfit, St, y, r1, r2, cu, S.part);
-                k_mr_sum_step<<<1, kThreads, 0, s>>>(S.part, kDotBlocks, St, 1);
-                k_mr_w_dot<<<kDotBlocks, kThreads, 0, s>>>(nfit, St, v, w, w1, w2, x, S.part);
-                k_mr_sum_step<<<1, kThreads, 0, s>>>(S.part, kDotBlocks, St, 2);
-                continue;
+                k_mr_y1<false><<<nb, kThreads, 0, s>>>(y1);
             }
-            k_mr_scale_v<<<S.grid(nfit), kThreads, 0, s>>>(nfit, St, y, v);
-            // y = (Q^T A Q v)(1:nfit)
-            k_copy_pad<<<S.grid(n), kThreads, 0, s>>>(nfit, n, v, xa);
-            S.qlmlq(xa, 0);
-            S.avprd0(xa, ba);
-            S.qlmlq(ba, 1);
-            k_copy_if<<<S.grid(nfit), kThreads, 0, s>>>(nfit, St, ba, y);
-            k_mr_y1<<<S.grid(nfit), kThreads, 0, s>>>(nfit, St, y, r1);
-            dot(v, y, nfit, S.part, &St->dotv, s);
-            k_mr_alfa<<<1, 32, 0, s>>>(St);
-            k_mr_y2<<<S.grid(nfit), kThreads, 0, s>>>(nfit, St, y, r1, r2, cu);
-            if (mbandw > 0) band_solve(P, doneFlag, y, s);
-            dot(r2, y, nfit, S.part, &St->dotv, s);
-            if (!qlp) {
-                k_mr_rot<<<1, 32, 0, s>>>(St);
-                k_mr_w<<<S.grid(nfit), kThreads, 0, s>>>(nfit, St, v, w, w1, w2, x);
-                dot(x, x, nfit, S.part, &St->dotv, s);
-                k_mr_test<<<1, 32, 0, s>>>(St);
-            } else {
-                k_qlp_rot<<<1, 32, 0, s>>>(St, Qs);
-                k_qlp_w<<<S.grid(nfit), kThreads, 0, s>>>(nfit, St, Qs, v, wa, wb, xp, xc);
-                dot(xc, xc, nfit, S.part, &St->dotv, s);
-                k_qlp_test<<<1, 32, 0, s>>>(St, Qs, maxxnorm);
-                k_qlp_commit<<<S.grid(nfit), kThreads, 0, s>>>(nfit, Qs, xc, x);
+            k_mr_y2<<<nb, kThreads, 0, s>>>(nfit, St + a, F, partA, nb, y, r[a], r[b], cu, partB);
+            int npB = nb;
+            if (mbandw > 0) {
+                band_solve(P, &F->done, y, s);
+                k_dot_partial<<<kDotBlocks, kThreads, 0, s>>>(nfit, r[a], y, partB);
+                npB = kDotBlocks;
             }
+            if (qlp)
+                k_qlp_w<<<nb, kThreads, 0, s>>>(nfit, St + a, St + b, Qs + a, Qs + b, F, partB, npB, v, w[0], w[1], xp,
+                                                xc, partX);
+            else
+                k_mr_w<<<nb, kThreads, 0, s>>>(nfit, St + a, St + b, F, partB, npB, v, w[a], w[b], x, partX);
+            next(b);
         }
     };
-    if (j.matsto != 2) MPG_CUDA(c, S.alloc_pmv(n));  // no allocation while the graph is recorded
     struct GraphGuard {
         cudaGraph_t g = nullptr;
         cudaGraphExec_t e = nullptr;
@@ -1618,16 +1774,20 @@ int32_t solve_minres(mpgpu_ctx *c, const double *consResiduals, double rtol, int
             gg.e = nullptr;
         cudaGetLastError();
     }
-    for (;;) {
+    MinresState hs[2];
+    MinresFlags hf;
+    for (int it = 0;;) {
         if (gg.e) MPG_CUDA(c, cudaGraphLaunch(gg.e, s));
         else batchBody();
         it += batch;
-        MPG_CUDA(c, cudaMemcpyAsync(&hs, St, sizeof(MinresState), cudaMemcpyDeviceToHost, s));
+        MPG_CUDA(c, cudaMemcpyAsync(hs, St, sizeof(hs), cudaMemcpyDeviceToHost, s));
+        MPG_CUDA(c, cudaMemcpyAsync(&hf, F, sizeof(hf), cudaMemcpyDeviceToHost, s));
         MPG_CUDA(c, cudaStreamSynchronize(s));
-        if (hs.done || it > itnlim + batch) break;
+        if (hf.pend || hf.done || it > itnlim + batch) break;
     }
-    info->itn = hs.itn;
-    info->istop = hs.istop;
+    const MinresState &last = hs[1].k > hs[0].k ? hs[1] : hs[0];   // the copy that the last step wrote
+    info->itn = last.itn;
+    info->istop = last.istop;
     if (ncon > 0) {
         MPG_CUDA(c, cudaMemcpyAsync(x + nfit, yc.data(), sizeof(double) * ncon, cudaMemcpyHostToDevice, s));
         S.qlmlq(x, 0);
@@ -1648,12 +1808,8 @@ int32_t avprod_host(mpgpu_ctx *c, int32_t n, const double *x, double *b) {
     Solver S(c);
     DevJob &j = c->j;
     cudaStream_t s = c->stream;
-    if (j.matsto == 2) {
-        int32_t rc = S.build_blocks();
-        if (rc) return rc;
-    } else {
-        MPG_CUDA(c, S.alloc_pmv(j.nVar));
-    }
+    const int32_t rcp = S.prepare_product();
+    if (rcp) return rcp;
     double *xa = nullptr, *ba = nullptr;
     MPG_CUDA(c, cudaMalloc(&xa, sizeof(double) * j.nVar));
     MPG_CUDA(c, cudaMalloc(&ba, sizeof(double) * j.nVar));
@@ -1678,13 +1834,10 @@ int32_t band_precond_factor(mpgpu_ctx *c, int32_t mbandw, int32_t lprecm, double
     cudaStream_t s = c->stream;
     const int32_t n = j.nVar, nfit = n - j.ncon;
     if (mbandw <= 0) return set_err(c, MPGPU_ERR_ARG, "band width must be positive");
-    if (j.matsto == 2) {
-        int32_t rc = S.build_blocks();
-        if (rc) return rc;
-    } else {
-        MPG_CUDA(c, S.alloc_pmv(n));
-    }
-    MPG_CUDA(c, cudaMallocAsync(&S.part, sizeof(double) * (kDotBlocks + 8), s));
+    const int32_t rcp = S.prepare_product();
+    if (rcp) return rcp;
+    MPG_CUDA(c, cudaMallocAsync(&S.partOwned, sizeof(double) * (kDotBlocks + 8), s));
+    S.part = S.partOwned;
     struct Bufs {
         double *v = nullptr, *tmp = nullptr, *yk = nullptr;
         BandPre P;

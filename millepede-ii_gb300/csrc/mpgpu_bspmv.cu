@@ -18,8 +18,8 @@
 // most itemSteps steps of one row group go to one warp each; their sums are
 // added in item order.  No atomics, fixed order: the product is reproducible.
 // 9.0M
-// stored elements: 46 us (62 % of the FP64 bound), 6.9M: 36 us (first form
-// 101 and 84 us).
+// stored elements: 44 us (FP64 pipe 83 % busy while the SMs are active),
+// 6.9M: 35 us (first form 101 and 84 us).
 #include <algorithm>
 #include <vector>
 
@@ -30,6 +30,7 @@ namespace {
 
 constexpr int kBrMax = 8;        // parameters per group
 constexpr int kBrWarps = 8;      // warps per CTA of the product
+constexpr int kBrUnroll = 4;     // steps whose loads are in flight together
 
 // per row group: its stored off-diagonal blocks in list order (ownBlk), its
 // diagonal block (diagBlk, -1: none stored); per block its column group as a
@@ -167,7 +168,7 @@ __global__ void k_br_fill(BrFill P, int32_t *col, double *val) {
 __device__ void br_coef(const BlockRowsCoef &k) {
     extern __shared__ double sc[];   // 2 m sums, then the partial sums
     const int C = 2 * k.m, tid = threadIdx.x;
-    if (tid == 0 && *k.pend) *k.done = 1;
+    mr_test(k.test);
     if (C == 0) return;
     const int nsub = blockDim.x / C, sub = tid / C, cc = tid - sub * C;
     double *red = sc + C;
@@ -203,15 +204,35 @@ __device__ void br_coef(const BlockRowsCoef &k) {
     }
 }
 
-__device__ __forceinline__ double2 ld_stream2(const double *p) {
-    double2 v;
-    asm("ld.global.nc.L1::no_allocate.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
-    return v;
+// a lane's R values of one step (column pairs for even R) and the R values of x
+template <int R>
+__device__ __forceinline__ void br_load(const double *p, double (&v)[R]) {
+    constexpr int L = 32 / R * R;
+    if constexpr (R % 2 == 0) {
+#pragma unroll
+        for (int q = 0; q < R / 2; ++q)
+            asm("ld.global.nc.L1::no_allocate.v2.f64 {%0, %1}, [%2];"
+                : "=d"(v[2 * q]), "=d"(v[2 * q + 1])
+                : "l"(p + q * 2 * L));
+    } else {
+#pragma unroll
+        for (int q = 0; q < R; ++q)
+            asm("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v[q]) : "l"(p + q * L));
+    }
 }
-__device__ __forceinline__ double ld_stream(const double *p) {
-    double v;
-    asm("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
-    return v;
+template <int R>
+__device__ __forceinline__ void br_load_x(const double *p, double (&x)[R]) {
+    if constexpr (R % 2 == 0) {
+#pragma unroll
+        for (int q = 0; q < R / 2; ++q) {
+            const double2 y = __ldg(reinterpret_cast<const double2 *>(p) + q);
+            x[2 * q] = y.x;
+            x[2 * q + 1] = y.y;
+        }
+    } else {
+#pragma unroll
+        for (int q = 0; q < R; ++q) x[q] = __ldg(p + q);
+    }
 }
 
 template <int R, bool COEF>
@@ -232,30 +253,30 @@ __global__ void __launch_bounds__(32 * kBrWarps) k_br_spmv(int64_t nitem, const 
     if (ln < L) {
         const int32_t *cp = col + (int64_t)a * NS + slot;
         const double *vp = val + (int64_t)a * R * L + (R % 2 == 0 ? 2 * ln : ln);
-#pragma unroll 2
-        for (int t = a; t < e; ++t, cp += NS, vp += R * L) {
-            const double *x = xp + (int64_t)*cp * R;
-            if constexpr (R % 2 == 0) {
-                double2 v[R / 2];
+        // kBrUnroll steps' loads in flight together: columns, then values and x
+        auto steps = [&](auto cnt) {
+            constexpr int U = decltype(cnt)::value;
+            int32_t c[U];
+            double v[U][R], x[U][R];
 #pragma unroll
-                for (int q = 0; q < R / 2; ++q) v[q] = ld_stream2(vp + q * 2 * L);
+            for (int u = 0; u < U; ++u) c[u] = __ldg(cp + u * NS);
 #pragma unroll
-                for (int q = 0; q < R / 2; ++q) {
-                    const double2 y = *reinterpret_cast<const double2 *>(x + 2 * q);
-                    acc0 = fma(v[q].x, y.x, acc0);
-                    acc1 = fma(v[q].y, y.y, acc1);
-                }
-            } else {
-                double v[R];
+            for (int u = 0; u < U; ++u) br_load<R>(vp + u * R * L, v[u]);
 #pragma unroll
-                for (int q = 0; q < R; ++q) v[q] = ld_stream(vp + q * L);
+            for (int u = 0; u < U; ++u) br_load_x<R>(xp + (int64_t)c[u] * R, x[u]);
+#pragma unroll
+            for (int u = 0; u < U; ++u)
 #pragma unroll
                 for (int q = 0; q < R; ++q) {
-                    if (q % 2 == 0) acc0 = fma(v[q], x[q], acc0);
-                    else acc1 = fma(v[q], x[q], acc1);
+                    if (q % 2 == 0) acc0 = fma(v[u][q], x[u][q], acc0);
+                    else acc1 = fma(v[u][q], x[u][q], acc1);
                 }
-            }
-        }
+            cp += U * NS;
+            vp += U * R * L;
+        };
+        int t = a;
+        for (; t + kBrUnroll <= e; t += kBrUnroll) steps(std::integral_constant<int, kBrUnroll>());
+        for (; t < e; ++t) steps(std::integral_constant<int, 1>());
     }
     double v = acc0 + acc1;
     if constexpr ((R & (R - 1)) == 0) {
@@ -383,8 +404,9 @@ int32_t block_rows_build(mpgpu_ctx *c) {
     if (nsteps >= (int64_t)1 << 31) return set_err(c, MPGPU_ERR_LIMIT, "sparse product: too many blocks");
     // steps per item: one item for every warp that fits on the device, so
     // that the sums across lanes (4 of them for R = 6) stay a small part;
-    // between 2 and 16 steps
-    const int itemSteps = (int)std::min<int64_t>(16, std::max<int64_t>(2, nsteps / ((int64_t)nsm * 64)));
+    // between 4 and 16 steps, whole rounds of loads
+    const int itemSteps =
+        (int)std::min<int64_t>(16, std::max<int64_t>(1, (nsteps / ((int64_t)nsm * 64) + 2) / kBrUnroll) * kBrUnroll);
     k_br_nitems<<<blocks_for(nG + 1), 256, 0, s>>>(nG, itemSteps, b.stepBeg, cnt);
     MPG_CUDA(c, scan_ex(cnt, b.itemBeg, nG + 1, tmp, s));
     int64_t nitem = 0;

@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "mpgpu_minres.cuh"
+
 struct mpgpu_ctx;
 
 // Device arrays of the copy, kept (with their capacities) in the job between
@@ -36,7 +38,7 @@ struct BlockRowsCoef {
     const double *partUW;     // [nblk][2 m] partial sums of x with the columns [U | W]
     const double *T, *S;      // m x m: compact WY factor, T (U^T A U) T^T
     double *coef;             // [2 m] c (of U), a (of W)
-    int32_t *pend, *done;     // convergence flag of the last test, promoted here
+    MinresTest test;          // of the last iteration, taken by the same CTA
 };
 cudaError_t block_rows_spmv(const BlockRows &b, const double *xp, const int32_t *done, const BlockRowsCoef *coef,
                             cudaStream_t s);

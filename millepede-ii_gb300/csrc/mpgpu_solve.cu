@@ -627,17 +627,6 @@ __global__ void k_spmv_final(int32_t n, const int32_t *aig, const int32_t *p2g, 
 }
 
 // ---------------------------------------------------------------- MINRES state
-// Iteration scalars.  Two copies alternate from iteration to iteration: the
-// kernel that takes the scalar step (k_mr_w, k_qlp_w) computes it in every
-// CTA from one copy and writes the other, so no CTA reads what another one
-// is writing.
-struct MinresState {
-    double beta1, beta, oldb, alfa, dbar, epsln, oldeps, delta, gbar, root, gamma, cs, sn, phi, phibar;
-    double tnorm2, gmax, gmin, Anorm, ynorm, rnorm, denom, rtol;
-    int k;                        // iterations whose update is done
-    int itn, itnlim, istop;
-};
-
 // MINRES-QLP (Choi, Paige & Saunders 2011; minresqlpModule.f90:411-1333 in
 // the reference): the Lanczos scalars of MinresState plus the rows of the
 // lower-triangular L = R P not yet final, the final u values and the
@@ -647,31 +636,19 @@ struct QlpState {
     double c1, s1, c2, s2, uA, uB, uC;
 };
 
-// pend: the last test ended the iteration (written by k_mr_next); done:
-// promoted from it by the next operator product, read by every kernel.  The
-// scalar alfa stands between k_mr_y2 and the scalar step.
-struct MinresFlags {
-    int pend, done;
-    double alfa;
-};
-
-// sum over the CTA (kThreads threads) in a fixed order, in every thread
+// sum over the CTA (T threads) in a fixed order, in thread 0; sh: T / 32
+template <int T>
 __device__ __forceinline__ double cta_sum(double v, double *sh) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
     __syncthreads();
     double r = sh[0];
+    if (threadIdx.x == 0) {
 #pragma unroll
-    for (int q = 1; q < kThreads / 32; ++q) r += sh[q];
-    __syncthreads();
+        for (int q = 1; q < T / 32; ++q) r += sh[q];
+    }
     return r;
-}
-
-__device__ __forceinline__ double sum_of_partials(const double *part, int n, double *sh) {
-    double v = 0.0;
-    for (int i = threadIdx.x; i < n; i += kThreads) v += part[i];
-    return cta_sum(v, sh);
 }
 
 // beta1^2 = r1 . y
@@ -679,97 +656,341 @@ __global__ void k_mr_init(MinresState *S, QlpState *Q, MinresFlags *F, const dou
     if (threadIdx.x) return;
     memset(S, 0, 2 * sizeof(MinresState));
     if (Q) memset(Q, 0, 2 * sizeof(QlpState));
-    F->pend = F->done = 0;
+    F->done = F->commit = 0;
     S->rtol = rtol;
     S->itnlim = itnlim;
     S->cs = -1.0;
     S->gmin = 1.0e300;
     double b1 = *dotv;
-    if (b1 <= 0.0) { S->istop = b1 < 0.0 ? 9 : 0; F->pend = F->done = 1; return; }
+    if (b1 <= 0.0) { S->istop = b1 < 0.0 ? 9 : 0; F->done = 1; return; }
     b1 = sqrt(b1);
     S->beta1 = b1;
     S->beta = b1;
+    S->invb = 1.0 / b1;
     S->phibar = b1;
 }
 
-// One iteration is five launches: operator product (block_rows_spmv, or the
-// separate products of the other storages), k_mr_y1, k_mr_y2, k_mr_w or
-// k_qlp_w, k_mr_next.  The dot products that end one kernel are summed by
-// every CTA of the next one (at most kMrBlocks values).  They are bound by
-// launch and synchronisation latency, not by their 0.2 MB vectors; the first
-// form had 16 launches, with the sums in kernels of one CTA.
+// One iteration is four launches: operator product with the convergence
+// test of the last update beside it (block_rows_spmv; k_mr_test and the
+// separate products of the other storages), k_mr_y1, k_mr_y2, k_mr_step.
+// The dot products that end one kernel are summed by every CTA of the next
+// one (at most kMrBlocks values).  They are bound by launch and
+// synchronisation latency, not by their 0.2 MB vectors, and by FP64
+// instructions that every warp would repeat (a warp's FP64 instruction holds
+// the pipe for 16 clocks, a division about 30 of them), so the scalars are
+// formed by one warp.  At 30,000 globals and 18 constraints: product 35 to
+// 44 us (mpgpu_bspmv.cu), 9.8, 6.2 and 10.9 us.  The first form had 16
+// launches, with the sums in kernels of one CTA.
 constexpr int kMrBlocks = 1216;    // CTAs of the vector kernels (at most)
-constexpr int kNextRows = 128;     // rows per step of k_mr_next
-constexpr int kNextBlocks = 304;
+constexpr int kY1Threads = 512, kY1Lanes = 4;   // k_mr_y1: lanes per row
+constexpr int kStepRows = 128;     // rows per round of k_mr_step
+constexpr int kStepBlocks = 304;
 constexpr int kWyFused = 64;       // constraints whose products ride in the iteration's kernels
 
-// The convergence test of the iteration just updated (from x . x), the
-// commit of the MINRES-QLP iterate, then the next Lanczos vector v = y /
+// the test alone (paths without block_rows_spmv's extra CTA)
+__global__ void k_mr_test(MinresTest t) {
+    if (t.F->done) return;
+    mr_test(t);
+}
+
+// y = Q^T A Q v on the fitted rows: with the block-row copy the item sums
+// less [U | W] coef (coef of br_coef), else the separate products' ba; then
+// y -= (beta / oldbeta) r1 from the second iteration on, partials of v . y.
+// With xc, the MINRES-QLP iterate that the test has just accepted is
+// committed first.  kY1Lanes lanes share a row's items and columns: one lane
+// per row waits for about ten dependent loads in a row of 20 items and 36
+// columns (14.2 us, 9.8 us with four).
+struct Y1Params {
+    int32_t nfit, n, m, R;
+    const int32_t *aig, *p2g;
+    const int64_t *itemBeg;
+    const double *part, *UWc, *coef, *ba, *r1, *v, *xc;
+    const MinresState *S;
+    const MinresFlags *F;
+    double *y, *x, *partA;
+};
+
+template <bool ITEMS>
+__global__ void __launch_bounds__(kY1Threads) k_mr_y1(Y1Params p) {
+    constexpr int L = kY1Lanes;
+    __shared__ double sh[kY1Threads / 32], cs[2 * kWyFused];
+    const int64_t t0 = (int64_t)blockIdx.x * kY1Threads + threadIdx.x, step = (int64_t)gridDim.x * kY1Threads;
+    if (p.xc && p.F->commit)
+        for (int64_t i = t0; i < p.nfit; i += step) p.x[i] = p.xc[i];
+    if (p.F->done) return;
+    const int C = ITEMS ? 2 * p.m : 0;
+    if ((int)threadIdx.x < C) cs[threadIdx.x] = p.coef[threadIdx.x];
+    __syncthreads();
+    const bool upd = p.S->k >= 1;
+    const double f = p.S->bo;
+    const int sub = threadIdx.x % L;
+    double acc = 0.0;
+    // (the loop bound is the same for the lanes of a row and rounded up to whole warps)
+    const int64_t rows = ((int64_t)p.nfit + 32 / L - 1) / (32 / L) * (32 / L);
+    for (int64_t i = t0 / L; i < rows; i += step / L) {
+        const bool in = i < p.nfit;
+        double yi = 0.0, vi = 0.0, ri = 0.0;
+        if (in && sub == 0) {
+            vi = p.v[i];
+            if (upd) ri = p.r1[i];
+            if (!ITEMS) yi = p.ba[i];
+        }
+        if (ITEMS) {
+            double a0 = 0.0, a1 = 0.0, s0 = 0.0, s1 = 0.0;
+            if (in) {
+#pragma unroll 9
+                for (int k = sub; k < C; k += L) a0 = fma(p.UWc[(int64_t)k * p.n + i], cs[k], a0);
+                const int32_t g = p.p2g[i] - 1;
+                const double *pt = p.part + (i - (p.aig[g] - 1));
+                const int64_t q1 = p.itemBeg[g + 1];
+                int64_t q = p.itemBeg[g] + sub;
+                for (; q + 3 * L < q1; q += 4 * L) {
+                    const double a = pt[q * p.R], b = pt[(q + L) * p.R], c = pt[(q + 2 * L) * p.R],
+                                 d = pt[(q + 3 * L) * p.R];
+                    s0 += a + b;
+                    s1 += c + d;
+                }
+                for (; q < q1; q += L) a1 += pt[q * p.R];
+            }
+            yi = ((s0 + s1) + a1) - a0;
+#pragma unroll
+            for (int o = L / 2; o > 0; o >>= 1) yi += __shfl_xor_sync(0xffffffffu, yi, o);
+        }
+        if (in && sub == 0) {
+            yi = yi - f * ri;
+            p.y[i] = yi;
+            acc += vi * yi;
+        }
+    }
+    acc = cta_sum<kY1Threads>(acc, sh);
+    if (threadIdx.x == 0) p.partA[blockIdx.x] = acc;
+}
+
+// alfa = v . y; the new residual r = y - (alfa / beta) r2 into the buffer of
+// the one before r2; y = M^-1 r (diagonal cu), partials of r . y
+__global__ void __launch_bounds__(kThreads) k_mr_y2(int32_t n, const MinresState *S, MinresFlags *F,
+                                                    const double *partA, int npA, double *y, double *rOld,
+                                                    const double *r2, const double *cu, double *partB) {
+    __shared__ double sh[kThreads / 32], sf;
+    if (F->done) return;
+    if (threadIdx.x < 32) {
+        const double alfa = warp_sum_of(partA, npA);
+        if (threadIdx.x == 0) {
+            sf = alfa * S->invb;
+            if (blockIdx.x == 0) F->alfa = alfa;
+        }
+    }
+    __syncthreads();
+    const double f = sf;
+    double acc = 0.0;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const double yi = y[i] - f * r2[i];
+        rOld[i] = yi;
+        const double zi = (yi * cu[i]) * cu[i];
+        y[i] = zi;
+        acc += yi * zi;
+    }
+    acc = cta_sum<kThreads>(acc, sh);
+    if (threadIdx.x == 0) partB[blockIdx.x] = acc;
+}
+
+// The scalar steps run in one warp on the CTA's copies; the square roots and
+// reciprocals that do not depend on each other are taken by different lanes
+// at once (a chain of them, 0.7 us each, was half of the kernel).
+__device__ __forceinline__ double lane_of(double v, int lane) { return __shfl_sync(0xffffffffu, v, lane); }
+
+// beta_{k+1} = sqrt(b2) and the left reflection
+__device__ void mr_rotate(MinresState *S, double b2) {
+    const int ln = threadIdx.x & 31;
+    if (b2 < 0.0) {
+        if (ln == 0) S->istop = 9;
+        return;
+    }
+    const double gbar = S->sn * S->dbar - S->cs * S->alfa;
+    double r = sqrt(ln == 0 ? b2 : gbar * gbar + b2);
+    if (ln != 0 && r < 2.220446049250313e-16) r = 2.220446049250313e-16;
+    const double inv = 1.0 / r;
+    const double beta = lane_of(r, 0), invb = lane_of(inv, 0), gamma = lane_of(r, 1), denom = lane_of(inv, 1);
+    if (ln) return;
+    S->oldb = S->beta;
+    S->beta = beta;
+    S->bo = beta * S->invb;
+    S->invb = invb;
+    S->tnorm2 += S->alfa * S->alfa + S->oldb * S->oldb + b2;
+    S->oldeps = S->epsln;
+    S->delta = S->cs * S->dbar + S->sn * S->alfa;
+    S->gbar = gbar;
+    S->epsln = S->sn * beta;
+    S->dbar = -S->cs * beta;
+    S->cs = gbar * denom;
+    S->sn = beta * denom;
+    S->phi = S->cs * S->phibar;
+    S->phibar = S->sn * S->phibar;
+    S->denom = denom;
+    S->gmax = fmax(S->gmax, gamma);
+    S->gmin = fmin(S->gmin, gamma);
+}
+
+// beta_{k+1}, the left reflection (column k of R, tau_k), the right
+// reflections P(k-2,k), P(k-1,k) and u: the oracle's steps, with products by
+// reciprocals for its quotients
+__device__ void qlp_rotate(MinresState *S, QlpState *Q, double b2) {
+    const int ln = threadIdx.x & 31;
+    if (b2 < 0.0) {
+        if (ln == 0) S->istop = 9;
+        return;
+    }
+    const int k = S->k + 1;
+    const double epsk = S->epsln, alfa = S->alfa, oldb = S->beta;
+    const double delta = S->cs * S->dbar + S->sn * alfa;
+    const double gbar = S->sn * S->dbar - S->cs * alfa;
+    const double tnorm2 = S->tnorm2 + (alfa * alfa + oldb * oldb + b2);
+    // lanes: beta, gamma, the first right reflection, ||T||
+    const double sq = ln == 0 ? b2 : ln == 1 ? gbar * gbar + b2 : ln == 2 ? Q->gA * Q->gA + epsk * epsk : tnorm2;
+    const double rt = sqrt(sq), inv = rt > 0.0 ? 1.0 / rt : 0.0;
+    const double beta = lane_of(rt, 0), invb = lane_of(inv, 0), gamma = lane_of(rt, 1), ig = lane_of(inv, 1);
+    const double rA = lane_of(rt, 2), iA = lane_of(inv, 2), Anorm = lane_of(rt, 3);
+    const double cs = gamma > 0.0 ? gbar * ig : 1.0, sn = gamma > 0.0 ? beta * ig : 0.0;
+    const double tau = cs * S->phibar;
+    double c1 = 1, s1 = 0, c2 = 1, s2 = 0, etaC = 0, thC = 0, gC, dk = delta, gk = gamma;
+    double gA = Q->gA, thB = Q->thB, gB = Q->gB, iB = 0.0;
+    if (k >= 3) {
+        if (rA > 0.0) { c1 = gA * iA; s1 = epsk * iA; }
+        gA = rA;
+        const double th = c1 * thB + s1 * dk;
+        dk = s1 * thB - c1 * dk;
+        thB = th;
+        etaC = s1 * gk;
+        gk = -c1 * gk;
+    }
+    if (k >= 2) {
+        const double r = sqrt(gB * gB + dk * dk);
+        if (r > 0.0) { iB = 1.0 / r; c2 = gB * iB; s2 = dk * iB; }
+        gB = r;
+        thC = s2 * gk;
+        gC = -c2 * gk;
+    } else {
+        gC = gk;
+    }
+    const double tiny = 2.220446049250313e-16 * Anorm;
+    double uA = 0.0, uB = 0.0;
+    if (k >= 3) uA = fabs(gA) > tiny ? (Q->tauA - Q->etaA * Q->uF2 - Q->thA * Q->uF1) * iA : 0.0;
+    if (k >= 2) uB = fabs(gB) > tiny ? (Q->tauB - Q->etaB * Q->uF1 - thB * uA) * iB : 0.0;
+    const double uC = fabs(gC) > tiny ? (tau - etaC * uA - thC * uB) / gC : 0.0;
+    __syncwarp();
+    if (ln) return;
+    S->oldb = oldb;
+    S->beta = beta;
+    S->bo = beta * S->invb;
+    S->invb = invb;
+    S->tnorm2 = tnorm2;
+    S->Anorm = Anorm;
+    S->gbar = gbar;
+    S->epsln = S->sn * beta;
+    S->dbar = -S->cs * beta;
+    S->cs = cs;
+    S->sn = sn;
+    S->phibar = sn * S->phibar;
+    S->gmax = fmax(S->gmax, gamma);
+    S->gmin = fmin(S->gmin, gamma);
+    Q->c1 = c1; Q->s1 = s1; Q->c2 = c2; Q->s2 = s2;
+    Q->uA = uA; Q->uB = uB; Q->uC = uC;
+    if (k >= 3) { Q->uF2 = Q->uF1; Q->uF1 = uA; }
+    Q->etaA = Q->etaB; Q->thA = thB; Q->gA = gB; Q->tauA = Q->tauB;
+    Q->etaB = etaC; Q->thB = thC; Q->gB = gC; Q->tauB = tau;
+}
+
+// The scalar step from beta^2 = r . y (in every CTA), the solution update
+// with the current Lanczos vector v (MINRES: w into the buffer of the older
+// of the two kept, x; MINRES-QLP: W = V P with w_{k-2} final into xp, and
+// the candidate iterate xc), partials of x . x; then the next vector v = y /
 // beta, padded with zeros for the operator (xa), and the partial dots of it
 // with the 2 m columns [U | W] of the constraint reflections (row-major
 // UWr: a thread owns a column and every nsub-th row, so that no sum crosses
 // lanes but the last nsub ones; 36 columns of 30,000 rows are 1.7 us of
-// FP64).
-struct NextParams {
+// FP64).  kStart: the first vector only.
+enum StepKind { kStart, kMinres, kQlp };
+
+struct StepParams {
     int32_t n, nfit, m, R;
-    const int32_t *aig, *p2g;   // padded positions of xa (null: xa has the order of the parameters)
-    MinresState *S;
-    MinresFlags *F;
-    const double *partX;
-    int npX;
-    double maxxnorm;
-    const double *y, *xc, *UWr;
-    double *v, *x, *xa, *partUW;
+    const int32_t *aig, *p2g;   // padded positions of xa (aig null: xa has the order of the parameters)
+    const MinresState *Sin;
+    MinresState *Sout;
+    const QlpState *Qin;
+    QlpState *Qout;
+    const MinresFlags *F;
+    const double *partB;
+    int npB;
+    const double *y, *UWr;
+    double *v, *xa, *partX, *partUW;
+    double *wa, *wb, *x, *xp, *xc;   // MINRES: wa the older, wb the newer w
 };
 
-template <bool QLP>
-__global__ void __launch_bounds__(kThreads) k_mr_next(NextParams p) {
-    __shared__ double sh[kThreads / 32], xs[kNextRows], red[kThreads];
+template <StepKind KIND>
+__global__ void __launch_bounds__(kThreads) k_mr_step(StepParams p) {
+    __shared__ double sh[kThreads / 32], xs[kStepRows], red[kThreads];
+    __shared__ MinresState ss;
+    __shared__ QlpState qs;
     if (p.F->done) return;
     const int tid = threadIdx.x;
-    MinresState *S = p.S;
-    const int k = S->k;
-    if (k > 0) {
-        if (S->istop == 9) {
-            if (blockIdx.x == 0 && tid == 0) p.F->pend = 1;
-            return;
-        }
-        const double xnorm = sqrt(sum_of_partials(p.partX, p.npX, sh));
-        const double Anorm = sqrt(S->tnorm2), rnorm = S->phibar;
-        const double test1 = rnorm / (Anorm * xnorm), test2 = S->root / Anorm;
-        int istop = 0;
-        if (k >= S->itnlim) istop = 6;
-        if (S->gmax / S->gmin >= 0.1 / 2.220446049250313e-16) istop = 4;
-        if (test2 <= S->rtol) istop = 2;
-        if (test1 <= S->rtol) istop = 1;
-        const bool commit = !(QLP && xnorm > p.maxxnorm);
-        if (!commit) istop = 5;
-        if (QLP && commit)
-            for (int64_t i = (int64_t)blockIdx.x * blockDim.x + tid; i < p.nfit; i += (int64_t)gridDim.x * blockDim.x)
-                p.x[i] = p.xc[i];
-        if (blockIdx.x == 0 && tid == 0) {
-            S->itn = k;
-            if (commit) {
-                S->Anorm = Anorm;
-                S->ynorm = xnorm;
-                S->rnorm = rnorm;
-            }
-            if (istop) {
-                S->istop = istop;
-                p.F->pend = 1;
+    // the CTA's copies of the scalars, by words
+    if (tid < (int)(sizeof(MinresState) / 8))
+        reinterpret_cast<double *>(&ss)[tid] = reinterpret_cast<const double *>(p.Sin)[tid];
+    if (KIND == kQlp && tid >= 32 && tid < 32 + (int)(sizeof(QlpState) / 8))
+        reinterpret_cast<double *>(&qs)[tid - 32] = reinterpret_cast<const double *>(p.Qin)[tid - 32];
+    __syncthreads();
+    if (KIND != kStart && tid < 32) {
+        const double b2 = warp_sum_of(p.partB, p.npB);
+        if (tid == 0) ss.alfa = p.F->alfa;
+        __syncwarp();
+        if (KIND == kQlp) qlp_rotate(&ss, &qs, b2);
+        else mr_rotate(&ss, b2);
+        if (tid == 0) {
+            ss.k += 1;
+            if (blockIdx.x == 0) {
+                *p.Sout = ss;
+                if (KIND == kQlp) *p.Qout = qs;
             }
         }
-        if (istop) return;
     }
-    const double f = 1.0 / S->beta;
+    __syncthreads();
+    if (ss.istop == 9) return;
+    const int k = ss.k;
+    const double f = ss.invb;
     const int C = 2 * p.m;
     const int nsub = C ? kThreads / C : 0, sub = C ? tid / C : 0, cc = C ? tid - sub * C : 0;
-    double acc = 0.0;
-    for (int64_t r0 = (int64_t)blockIdx.x * kNextRows; r0 < p.n; r0 += (int64_t)gridDim.x * kNextRows) {
+    double acc = 0.0, xx = 0.0;
+    for (int64_t r0 = (int64_t)blockIdx.x * kStepRows; r0 < p.n; r0 += (int64_t)gridDim.x * kStepRows) {
         const int64_t i = r0 + tid;
-        if (tid < kNextRows) {
+        if (tid < kStepRows) {
             double vi = 0.0;
             if (i < p.nfit) {
+                if (KIND == kMinres) {
+                    const double wn = (p.v[i] - ss.oldeps * p.wa[i] - ss.delta * p.wb[i]) * ss.denom;
+                    p.wa[i] = wn;
+                    const double xi = p.x[i] + ss.phi * wn;
+                    p.x[i] = xi;
+                    xx += xi * xi;
+                } else if (KIND == kQlp) {
+                    double a = p.wa[i], bb = p.wb[i], c = p.v[i], xi = p.xp[i];
+                    if (k >= 3) {
+                        const double a2 = qs.c1 * a + qs.s1 * c;
+                        c = qs.s1 * a - qs.c1 * c;
+                        a = a2;
+                        xi = xi + qs.uA * a;
+                        p.xp[i] = xi;
+                    }
+                    if (k >= 2) {
+                        const double b2r = qs.c2 * bb + qs.s2 * c;
+                        c = qs.s2 * bb - qs.c2 * c;
+                        bb = b2r;
+                    }
+                    p.wa[i] = bb;
+                    p.wb[i] = c;
+                    xi = xi + qs.uB * bb + qs.uC * c;
+                    p.xc[i] = xi;
+                    xx += xi * xi;
+                }
                 vi = f * p.y[i];
                 p.v[i] = vi;
             }
@@ -786,12 +1007,16 @@ __global__ void __launch_bounds__(kThreads) k_mr_next(NextParams p) {
         if (!C) continue;
         __syncthreads();
         if (sub < nsub) {
-            const int rows = (int)min((int64_t)kNextRows, p.n - r0);
+            const int rows = (int)min((int64_t)kStepRows, p.n - r0);
             const double *u = p.UWr + r0 * C + cc;
-#pragma unroll 6
+#pragma unroll 10
             for (int r = sub; r < rows; r += nsub) acc = fma(u[(int64_t)r * C], xs[r], acc);
         }
         __syncthreads();
+    }
+    if (KIND != kStart) {
+        xx = cta_sum<kThreads>(xx, sh);
+        if (tid == 0) p.partX[blockIdx.x] = xx;
     }
     if (!C) return;
     red[tid] = acc;
@@ -801,249 +1026,6 @@ __global__ void __launch_bounds__(kThreads) k_mr_next(NextParams p) {
         for (int q = 0; q < nsub; ++q) t += red[q * C + tid];
         p.partUW[(int64_t)blockIdx.x * C + tid] = t;
     }
-}
-
-// (paths without block_rows_spmv's extra CTA)
-__global__ void k_mr_promote(MinresFlags *F) {
-    if (threadIdx.x == 0 && blockIdx.x == 0 && F->pend) F->done = 1;
-}
-
-// y = Q^T A Q v on the fitted rows: with the block-row copy the item sums
-// less [U | W] coef (coef of br_coef), else the separate products' ba; then
-// y -= (beta / oldbeta) r1 from the second iteration on, partials of v . y
-struct Y1Params {
-    int32_t nfit, n, m, R;
-    const int32_t *aig, *p2g;
-    const int64_t *itemBeg;
-    const double *part, *UWc, *coef, *ba, *r1, *v;
-    const MinresState *S;
-    const MinresFlags *F;
-    double *y, *partA;
-};
-
-template <bool ITEMS>
-__global__ void __launch_bounds__(kThreads) k_mr_y1(Y1Params p) {
-    __shared__ double sh[kThreads / 32], cs[2 * kWyFused];
-    if (p.F->done) return;
-    const int C = ITEMS ? 2 * p.m : 0;
-    if ((int)threadIdx.x < C) cs[threadIdx.x] = p.coef[threadIdx.x];
-    __syncthreads();
-    const bool upd = p.S->k >= 1;
-    const double f = upd ? p.S->beta / p.S->oldb : 0.0;
-    double acc = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < p.nfit; i += (int64_t)gridDim.x * blockDim.x) {
-        double yi;
-        if (ITEMS) {
-            const int32_t g = p.p2g[i] - 1;
-            const int64_t ii = i - (p.aig[g] - 1);
-            yi = 0.0;
-            for (int64_t q = p.itemBeg[g]; q < p.itemBeg[g + 1]; ++q) yi += p.part[q * p.R + ii];
-            double a0 = 0.0, a1 = 0.0;
-#pragma unroll 6
-            for (int q = 0; q < p.m; ++q) {
-                a0 = fma(p.UWc[(int64_t)q * p.n + i], cs[q], a0);
-                a1 = fma(p.UWc[(int64_t)(p.m + q) * p.n + i], cs[p.m + q], a1);
-            }
-            yi -= a0 + a1;
-        } else {
-            yi = p.ba[i];
-        }
-        if (upd) yi = yi - f * p.r1[i];
-        p.y[i] = yi;
-        acc += p.v[i] * yi;
-    }
-    acc = cta_sum(acc, sh);
-    if (threadIdx.x == 0) p.partA[blockIdx.x] = acc;
-}
-
-// alfa = v . y; the new residual r = y - (alfa / beta) r2 into the buffer of
-// the one before r2; y = M^-1 r (diagonal cu), partials of r . y
-__global__ void __launch_bounds__(kThreads) k_mr_y2(int32_t n, const MinresState *S, MinresFlags *F,
-                                                    const double *partA, int npA, double *y, double *rOld,
-                                                    const double *r2, const double *cu, double *partB) {
-    __shared__ double sh[kThreads / 32];
-    if (F->done) return;
-    const double alfa = sum_of_partials(partA, npA, sh);
-    if (blockIdx.x == 0 && threadIdx.x == 0) F->alfa = alfa;
-    const double f = alfa / S->beta;
-    double acc = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double yi = y[i] - f * r2[i];
-        rOld[i] = yi;
-        const double zi = (yi * cu[i]) * cu[i];
-        y[i] = zi;
-        acc += yi * zi;
-    }
-    acc = cta_sum(acc, sh);
-    if (threadIdx.x == 0) partB[blockIdx.x] = acc;
-}
-
-__device__ void mr_rotate(MinresState *S, double b2) {
-    if (b2 < 0.0) { S->istop = 9; return; }
-    S->oldb = S->beta;
-    S->beta = sqrt(b2);
-    S->tnorm2 += S->alfa * S->alfa + S->oldb * S->oldb + S->beta * S->beta;
-    S->oldeps = S->epsln;
-    S->delta = S->cs * S->dbar + S->sn * S->alfa;
-    S->gbar = S->sn * S->dbar - S->cs * S->alfa;
-    S->epsln = S->sn * S->beta;
-    S->dbar = -S->cs * S->beta;
-    S->root = sqrt(S->gbar * S->gbar + S->dbar * S->dbar);
-    double gamma = sqrt(S->gbar * S->gbar + S->beta * S->beta);
-    if (gamma < 2.220446049250313e-16) gamma = 2.220446049250313e-16;
-    S->gamma = gamma;
-    S->cs = S->gbar / gamma;
-    S->sn = S->beta / gamma;
-    S->phi = S->cs * S->phibar;
-    S->phibar = S->sn * S->phibar;
-    S->denom = 1.0 / gamma;
-    S->gmax = fmax(S->gmax, gamma);
-    S->gmin = fmin(S->gmin, gamma);
-}
-
-// beta^2 = r . y, the rotation (in every CTA), then w (into the buffer of
-// the older of the two kept) and x, partials of x . x
-__global__ void __launch_bounds__(kThreads) k_mr_w(int32_t n, const MinresState *Sin, MinresState *Sout,
-                                                   const MinresFlags *F, const double *partB, int npB,
-                                                   const double *v, double *wOld, const double *w, double *x,
-                                                   double *partX) {
-    __shared__ double sh[kThreads / 32];
-    __shared__ MinresState ss;
-    if (F->done) return;
-    const double b2 = sum_of_partials(partB, npB, sh);
-    if (threadIdx.x == 0) {
-        ss = *Sin;
-        ss.alfa = F->alfa;
-        mr_rotate(&ss, b2);
-        ss.k += 1;
-        if (blockIdx.x == 0) *Sout = ss;
-    }
-    __syncthreads();
-    if (ss.istop == 9) return;
-    const double oe = ss.oldeps, de = ss.delta, dn = ss.denom, ph = ss.phi;
-    double acc = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double wn = (v[i] - oe * wOld[i] - de * w[i]) * dn;
-        wOld[i] = wn;
-        const double xi = x[i] + ph * wn;
-        x[i] = xi;
-        acc += xi * xi;
-    }
-    acc = cta_sum(acc, sh);
-    if (threadIdx.x == 0) partX[blockIdx.x] = acc;
-}
-
-__device__ __forceinline__ void d_sym_ortho(double a, double b, double *c, double *s, double *r) {
-    *r = sqrt(a * a + b * b);
-    if (*r == 0.0) { *c = 1.0; *s = 0.0; return; }
-    *c = a / *r;
-    *s = b / *r;
-}
-
-// beta_{k+1}, the left reflection (column k of R, tau_k), the right
-// reflections P(k-2,k), P(k-1,k) and u; the same arithmetic as the oracle
-__device__ void qlp_rotate(MinresState *S, QlpState *Q, double b2) {
-    if (b2 < 0.0) { S->istop = 9; return; }
-    const int k = S->k + 1;
-    S->oldb = S->beta;
-    S->beta = sqrt(b2);
-    S->tnorm2 += S->alfa * S->alfa + S->oldb * S->oldb + S->beta * S->beta;
-    S->Anorm = sqrt(S->tnorm2);
-    const double epsk = S->epsln;
-    const double delta = S->cs * S->dbar + S->sn * S->alfa;
-    const double gbar = S->sn * S->dbar - S->cs * S->alfa;
-    S->epsln = S->sn * S->beta;
-    S->dbar = -S->cs * S->beta;
-    S->root = sqrt(gbar * gbar + S->dbar * S->dbar);
-    double cs, sn, gamma;
-    d_sym_ortho(gbar, S->beta, &cs, &sn, &gamma);
-    S->cs = cs;
-    S->sn = sn;
-    const double tau = cs * S->phibar;
-    S->phibar = sn * S->phibar;
-    S->gmax = fmax(S->gmax, gamma);
-    S->gmin = fmin(S->gmin, gamma);
-    double c1 = 1, s1 = 0, c2 = 1, s2 = 0, etaC = 0, thC = 0, gC, dk = delta, gk = gamma;
-    if (k >= 3) {
-        double r;
-        d_sym_ortho(Q->gA, epsk, &c1, &s1, &r);
-        Q->gA = r;
-        const double th = c1 * Q->thB + s1 * dk;
-        dk = s1 * Q->thB - c1 * dk;
-        Q->thB = th;
-        etaC = s1 * gk;
-        gk = -c1 * gk;
-    }
-    if (k >= 2) {
-        double r;
-        d_sym_ortho(Q->gB, dk, &c2, &s2, &r);
-        Q->gB = r;
-        thC = s2 * gk;
-        gC = -c2 * gk;
-    } else {
-        gC = gk;
-    }
-    const double tiny = 2.220446049250313e-16 * S->Anorm;
-    double uA = 0.0, uB = 0.0, uC;
-    if (k >= 3) uA = fabs(Q->gA) > tiny ? (Q->tauA - Q->etaA * Q->uF2 - Q->thA * Q->uF1) / Q->gA : 0.0;
-    if (k >= 2) uB = fabs(Q->gB) > tiny ? (Q->tauB - Q->etaB * Q->uF1 - Q->thB * uA) / Q->gB : 0.0;
-    uC = fabs(gC) > tiny ? (tau - etaC * uA - thC * uB) / gC : 0.0;
-    Q->c1 = c1; Q->s1 = s1; Q->c2 = c2; Q->s2 = s2;
-    Q->uA = uA; Q->uB = uB; Q->uC = uC;
-    if (k >= 3) { Q->uF2 = Q->uF1; Q->uF1 = uA; }
-    Q->etaA = Q->etaB; Q->thA = Q->thB; Q->gA = Q->gB; Q->tauA = Q->tauB;
-    Q->etaB = etaC; Q->thB = thC; Q->gB = gC; Q->tauB = tau;
-}
-
-// the scalar step of MINRES-QLP (in every CTA), then W = V P (w_{k-2} final
-// into xp) and the candidate iterate xc, partials of xc . xc
-__global__ void __launch_bounds__(kThreads) k_qlp_w(int32_t n, const MinresState *Sin, MinresState *Sout,
-                                                    const QlpState *Qin, QlpState *Qout, const MinresFlags *F,
-                                                    const double *partB, int npB, const double *v, double *wa,
-                                                    double *wb, double *xp, double *xc, double *partX) {
-    __shared__ double sh[kThreads / 32];
-    __shared__ MinresState ss;
-    __shared__ QlpState qs;
-    if (F->done) return;
-    const double b2 = sum_of_partials(partB, npB, sh);
-    if (threadIdx.x == 0) {
-        ss = *Sin;
-        qs = *Qin;
-        ss.alfa = F->alfa;
-        qlp_rotate(&ss, &qs, b2);
-        ss.k += 1;
-        if (blockIdx.x == 0) {
-            *Sout = ss;
-            *Qout = qs;
-        }
-    }
-    __syncthreads();
-    if (ss.istop == 9) return;
-    const int k = ss.k;
-    const double c1 = qs.c1, s1 = qs.s1, c2 = qs.c2, s2 = qs.s2, uA = qs.uA, uB = qs.uB, uC = qs.uC;
-    double acc = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        double a = wa[i], bb = wb[i], c = v[i], xi = xp[i];
-        if (k >= 3) {
-            const double a2 = c1 * a + s1 * c;
-            c = s1 * a - c1 * c;
-            a = a2;
-            xi = xi + uA * a;
-            xp[i] = xi;
-        }
-        if (k >= 2) {
-            const double b2r = c2 * bb + s2 * c;
-            c = s2 * bb - c2 * c;
-            bb = b2r;
-        }
-        wa[i] = bb;
-        wb[i] = c;
-        xi = xi + uB * bb + uC * c;
-        xc[i] = xi;
-        acc += xi * xi;
-    }
-    acc = cta_sum(acc, sh);
-    if (threadIdx.x == 0) partX[blockIdx.x] = acc;
 }
 
 __global__ void k_apply_precond(int32_t n, const double *r, const double *cu, double *y) {
@@ -1067,7 +1049,7 @@ __global__ void __launch_bounds__(kThreads) k_column_dots(int32_t n, int32_t m, 
     const double *u = U + (int64_t)(blockIdx.x / m) * n, *w = W + (int64_t)(blockIdx.x % m) * n;
     double v = 0.0;
     for (int i = threadIdx.x; i < n; i += kThreads) v = fma(u[i], w[i], v);
-    v = cta_sum(v, sh);
+    v = cta_sum<kThreads>(v, sh);
     if (threadIdx.x == 0) M[blockIdx.x] = v;
 }
 
@@ -1637,8 +1619,9 @@ int32_t solve_minres(mpgpu_ctx *c, const double *consResiduals, double rtol, int
     const int64_t nv = ((int64_t)std::max(n, 1) + 1) / 2 * 2;   // vectors stay 16-byte aligned
     const int64_t nxp = fused ? ((int64_t)j.nG * j.br.R + 1) / 2 * 2 : nv;
     const int nb = (int)std::min<int64_t>(kMrBlocks, (nfit + kThreads - 1) / kThreads + (nfit < 1));
-    const int nbNext = (int)std::min<int64_t>(kNextBlocks, (n + kNextRows - 1) / kNextRows);
-    const int64_t nUW = (int64_t)nbNext * 2 * kWyFused;
+    const int nbY1 = (int)std::min<int64_t>(kMrBlocks, ((int64_t)nfit * kY1Lanes + kY1Threads - 1) / kY1Threads + (nfit < 1));
+    const int nbStep = (int)std::min<int64_t>(kStepBlocks, (n + kStepRows - 1) / kStepRows);
+    const int64_t nUW = (int64_t)nbStep * 2 * kWyFused;
     const int64_t scalLen = (2 * sizeof(MinresState) + 2 * sizeof(QlpState) + sizeof(MinresFlags)) / 8 + 8;
     const int64_t len = 16 * nv + nxp + 3 * kMrBlocks + kDotBlocks + 8 + nUW + 2 * kWyFused + scalLen + S.wy_len();
     MPG_CUDA(c, dgrow(j, j.work, len));
@@ -1714,17 +1697,18 @@ int32_t solve_minres(mpgpu_ctx *c, const double *consResiduals, double rtol, int
     k_mr_init<<<1, 32, 0, s>>>(St, qlp ? Qs : nullptr, F, dsc, rtol, itnlim);
     const double maxxnorm = (double)nfit / sqrt(2.220446049250313e-16);
     const bool pad = fused && !j.br.uniform;
-    NextParams np{n,  nfit, fused ? ncon : 0, fused ? j.br.R : 0, pad ? j.aig : nullptr, j.p2g, St, F,
-                  partX, nb, maxxnorm, y, xc, S.wy.UWr, v, x, xa, partUW};
-    Y1Params y1{nfit, n, fused ? ncon : 0, fused ? j.br.R : 0, j.aig, j.p2g, j.br.itemBeg, j.br.part, S.wy.UWc, coef,
-                ba, r[0], v, St, F, y, partA};
-    const BlockRowsCoef bc{fused ? ncon : 0, nbNext, partUW, j.qlT, S.wy.S, coef, &F->pend, &F->done};
-    auto next = [&](int cur) {
-        np.S = St + cur;
-        if (qlp) k_mr_next<true><<<nbNext, kThreads, 0, s>>>(np);
-        else k_mr_next<false><<<nbNext, kThreads, 0, s>>>(np);
-    };
-    next(0);
+    StepParams sp{};
+    sp.n = n; sp.nfit = nfit; sp.m = fused ? ncon : 0; sp.R = fused ? j.br.R : 0;
+    sp.aig = pad ? j.aig : nullptr; sp.p2g = j.p2g;
+    sp.F = F; sp.partB = partB; sp.y = y; sp.UWr = S.wy.UWr; sp.v = v; sp.xa = xa;
+    sp.partX = partX; sp.partUW = partUW; sp.x = x; sp.xp = xp; sp.xc = xc;
+    Y1Params y1{};
+    y1.nfit = nfit; y1.n = n; y1.m = sp.m; y1.R = sp.R; y1.aig = j.aig; y1.p2g = j.p2g;
+    y1.itemBeg = j.br.itemBeg; y1.part = j.br.part; y1.UWc = S.wy.UWc; y1.coef = coef; y1.ba = ba; y1.v = v;
+    y1.xc = qlp ? xc : nullptr; y1.F = F; y1.y = y; y1.x = x; y1.partA = partA;
+    BlockRowsCoef bc{sp.m, nbStep, partUW, j.qlT, S.wy.S, coef, {nullptr, F, partX, nbStep, qlp ? maxxnorm : -1.0}};
+    sp.Sin = St;
+    k_mr_step<kStart><<<nbStep, kThreads, 0, s>>>(sp);
     // the iterations of one batch are recorded once as a CUDA graph and
     // replayed (all scalars live on the device); direct launches if the
     // capture is refused.  An even number: the two copies of the scalars and
@@ -1733,31 +1717,32 @@ int32_t solve_minres(mpgpu_ctx *c, const double *consResiduals, double rtol, int
     auto batchBody = [&] {
         for (int q = 0; q < batch; ++q) {
             const int a = q & 1, b = 1 - a;   // current and next scalars; older and current of r and w
+            bc.test.S = St + a;
             y1.S = St + a;
             y1.r1 = r[a];
             if (fused) {
                 block_rows_spmv(j.br, xa, &F->done, &bc, s);
-                k_mr_y1<true><<<nb, kThreads, 0, s>>>(y1);
+                k_mr_y1<true><<<nbY1, kY1Threads, 0, s>>>(y1);
             } else {
-                k_mr_promote<<<1, 32, 0, s>>>(F);
+                k_mr_test<<<1, 32, 0, s>>>(bc.test);
                 S.qlmlq(xa, 0);
                 S.avprd0(xa, ba);
                 S.qlmlq(ba, 1);
-                k_mr_y1<false><<<nb, kThreads, 0, s>>>(y1);
+                k_mr_y1<false><<<nbY1, kY1Threads, 0, s>>>(y1);
             }
-            k_mr_y2<<<nb, kThreads, 0, s>>>(nfit, St + a, F, partA, nb, y, r[a], r[b], cu, partB);
-            int npB = nb;
+            k_mr_y2<<<nb, kThreads, 0, s>>>(nfit, St + a, F, partA, nbY1, y, r[a], r[b], cu, partB);
+            sp.npB = nb;
             if (mbandw > 0) {
                 band_solve(P, &F->done, y, s);
                 k_dot_partial<<<kDotBlocks, kThreads, 0, s>>>(nfit, r[a], y, partB);
-                npB = kDotBlocks;
+                sp.npB = kDotBlocks;
             }
-            if (qlp)
-                k_qlp_w<<<nb, kThreads, 0, s>>>(nfit, St + a, St + b, Qs + a, Qs + b, F, partB, npB, v, w[0], w[1], xp,
-                                                xc, partX);
-            else
-                k_mr_w<<<nb, kThreads, 0, s>>>(nfit, St + a, St + b, F, partB, npB, v, w[a], w[b], x, partX);
-            next(b);
+            sp.Sin = St + a; sp.Sout = St + b;
+            sp.Qin = Qs + a; sp.Qout = Qs + b;
+            sp.wa = qlp ? w[0] : w[a];
+            sp.wb = qlp ? w[1] : w[b];
+            if (qlp) k_mr_step<kQlp><<<nbStep, kThreads, 0, s>>>(sp);
+            else k_mr_step<kMinres><<<nbStep, kThreads, 0, s>>>(sp);
         }
     };
     struct GraphGuard {
@@ -1783,7 +1768,7 @@ int32_t solve_minres(mpgpu_ctx *c, const double *consResiduals, double rtol, int
         MPG_CUDA(c, cudaMemcpyAsync(hs, St, sizeof(hs), cudaMemcpyDeviceToHost, s));
         MPG_CUDA(c, cudaMemcpyAsync(&hf, F, sizeof(hf), cudaMemcpyDeviceToHost, s));
         MPG_CUDA(c, cudaStreamSynchronize(s));
-        if (hf.pend || hf.done || it > itnlim + batch) break;
+        if (hf.done || it > itnlim + batch) break;
     }
     const MinresState &last = hs[1].k > hs[0].k ? hs[1] : hs[0];   // the copy that the last step wrote
     info->itn = last.itn;

@@ -83,7 +83,8 @@ typedef struct mpgpu_ctx mpgpu_ctx;
 /* one record per CTA of one warp (no persistent loop), no size classes: the
  * plain launch form, for comparison */
 #define MPGPU_FLAG_ONE_RECORD_PER_BLOCK 4
-/* no timing of warps-per-CTA candidates on the first data loop */
+/* no timing of warps-per-CTA candidates on the first data loop (only classes
+ * of several 100,000 records are timed) */
 #define MPGPU_FLAG_NO_AUTOTUNE 8
 /* the tensor-core dense solve (metsol 31) factorises at every solve instead
  * of first preconditioning with the factor of the job's previous solve */
@@ -189,10 +190,10 @@ int32_t mpgpu_write_mon(const char *path, int32_t header, int32_t mode, int32_t 
 
 /* Fit size classes of the uploaded records (the shared memory each fit
  * needs: class k < 7 up to 4 KB << k, class 7 beyond one CTA): records per
- * class, warps per CTA chosen by the tuner on the first data loop (0: not
- * yet tuned, -1: no candidate fitted) and the sample times (ms) of 1, 2, 4
- * and 8 warps per CTA; arrays of MPGPU_FIT_BUCKETS (and 4x that for
- * tuneMs).  No counterpart in the reference. */
+ * class, warps per CTA chosen on the first data loop (0: no loop yet, -1:
+ * no candidate fitted), by the tuner for classes of several 100,000 records,
+ * else one, and the tuner's sample times (ms) of 1, 2, 4 and 8 warps per CTA
+ * (0: not sampled); arrays of MPGPU_FIT_BUCKETS (and 4x that for tuneMs).  No counterpart in the reference. */
 #define MPGPU_FIT_BUCKETS 8
 int32_t mpgpu_fit_buckets(const mpgpu_ctx *ctx, int64_t *count, int32_t *wpc, double *tuneMs);
 

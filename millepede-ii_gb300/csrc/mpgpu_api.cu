@@ -550,6 +550,9 @@ extern "C" int32_t mpgpu_upload_timing(const mpgpu_ctx *c, double *msCopy, doubl
 }
 
 // ------------------------------------------------------------------ data loop
+// share of a class that the warps-per-CTA tuner may sample
+constexpr int kTuneShare = 128;
+
 static int32_t run_loop(mpgpu_ctx *c, const mpgpu_fitopts *opt, mpgpu_fitstats *stats,
                         int32_t *naccf, float *chi2f, int32_t *ndff) {
     DevJob &j = c->j;
@@ -625,7 +628,7 @@ static int32_t run_loop(mpgpu_ctx *c, const mpgpu_fitopts *opt, mpgpu_fitstats *
         FitParams cap = q;
         cap.onePerBlock = 0;
         q.bigMode = (c->flags & MPGPU_FLAG_LARGE_RECORDS) || fit_warps_per_cta(cap) < 4 ? 1 : 0;
-        if (bucketed && !j.bucketWpc.empty() && j.bucketWpc[b] > 0) q.wpc = j.bucketWpc[b];
+        if (bucketed) q.wpc = !j.bucketWpc.empty() && j.bucketWpc[b] > 0 ? j.bucketWpc[b] : fit_default_wpc(q);
         if (q.bigMode) {
             // B and W, or the S-form's Y (neq x nalc), S (neq x neq) and its
             // group and equation lists, whichever is larger, so that the
@@ -647,24 +650,33 @@ static int32_t run_loop(mpgpu_ctx *c, const mpgpu_fitopts *opt, mpgpu_fitstats *
         MPG_CUDA(c, dgrow(j, j.bigDone, subMax));
         for (auto &q : bfp) { q.bw = j.bw; q.bigDone = j.bigDone; }
     }
-    if (fp.bandmax >= 0 && (opt->icalcm == 1 || mon.on)) {
+    bool anyBig = false;
+    for (const FitParams &q : bfp) anyBig = anyBig || q.bigMode != 0;
+    if (fp.bandmax >= 0 && (opt->icalcm == 1 || mon.on || anyBig)) {
         // every warp that can be resident: 64 per SM (one-record-per-block
         // launches take at most that many records)
-        const int64_t stride = 32 * (int64_t)fp.nalcmax + (int64_t)fp.nalcmax * (fp.nalcmax + 1) / 2 + 2;
+        const int64_t stride = anyBig ? band_scratch_total(fp.nalcmax, fp.neqmax) : band_scratch(fp.nalcmax, fp.neqmax);
         MPG_CUDA(c, dgrow(j, j.bscr, (int64_t)nsm * 64 * stride));
         for (auto &q : bfp) { q.bscr = j.bscr; q.bscrStride = stride; }
     }
-    // warps per CTA of each class, timed on a sample of the class on the
-    // first loop with matrix after an upload that changed the class's
-    // maxima; the records' results do not depend on it
+    // warps per CTA of each class: fit_default_wpc, or for the classes of large
+    // jobs the best of a timed sample on the first loop with matrix after an
+    // upload that changed the class's maxima.  The sample (five launches) is
+    // at most 1/kTuneShare of the class each, and a class whose share does
+    // not fill the device is not sampled: sampling four waves of every class
+    // took longer than the loop itself for jobs of some 10,000 records
+    // (broken lines, 50,000 records: first iteration 226 ms, the next 103).
+    // The records' results do not depend on it.
     if (bucketed && opt->icalcm == 1 && !(c->flags & MPGPU_FLAG_NO_AUTOTUNE) && nchunk > 0) {
         for (int b = 0; b < nb; ++b) {
             if (j.bucketWpc[b] != 0 || bfp[b].recList == nullptr) continue;
-            // sample: four waves of the most warps an SM holds
-            const int64_t sample = bfp[b].bigMode ? std::min<int64_t>(bsub[b], (int64_t)nsm * 64)
-                                                  : (int64_t)nsm * 64 * 4;
-            const int64_t i0 = j.bucketOff[b], i1 = std::min(j.bucketOff[b + 1], i0 + sample);
-            if (i1 <= i0) continue;
+            const int64_t inClass = j.bucketOff[b + 1] - j.bucketOff[b];
+            const int64_t sample = std::min<int64_t>(bfp[b].bigMode ? bsub[b] : inClass, inClass / kTuneShare);
+            if (sample < (int64_t)nsm * 16) {
+                j.bucketWpc[b] = bfp[b].wpc;
+                continue;
+            }
+            const int64_t i0 = j.bucketOff[b], i1 = i0 + sample;
             FitParams q = bfp[b];
             q.stage = j.stage;
             q.r0 = i0;
@@ -673,7 +685,7 @@ static int32_t run_loop(mpgpu_ctx *c, const mpgpu_fitopts *opt, mpgpu_fitstats *
             const int cand[4] = {1, 2, 4, 8};
             float best = 0.0f;
             int bestW = 0;
-            // more warps per CTA are kept unless fewer are at least 3 % faster
+            // fewer warps per CTA are kept unless more are at least 3 % faster
             cudaEvent_t t0, t1;
             cudaEventCreate(&t0);
             cudaEventCreate(&t1);
@@ -690,8 +702,8 @@ static int32_t run_loop(mpgpu_ctx *c, const mpgpu_fitopts *opt, mpgpu_fitstats *
                 float ms = 0.0f;
                 cudaEventElapsedTime(&ms, t0, t1);
                 j.bucketTuneMs[4 * b + k] = ms;
-                if (bestW == 0 || ms <= best * 1.03f) {
-                    if (bestW == 0 || ms < best) best = ms;
+                if (bestW == 0 || ms < best * 0.97f) {
+                    best = ms;
                     bestW = cand[k];
                 }
             }

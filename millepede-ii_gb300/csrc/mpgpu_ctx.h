@@ -281,12 +281,29 @@ __host__ __device__ inline int64_t band_doubles(int nalc, int bandmax, int bdrma
     return n * (b + 1) + 2 * n * d + 3 * n + d * d + 16;
 }
 
+// Per-warp global scratch of band records: the vectors or columns of the
+// band substitutions (32 per warp), the packed band inverse or the border
+// vectors of the equations (8 each), and the packed local matrix of large
+// records.  Of those it is read only by the forms that
+// do not work on the band storage; in shared memory it took a third of a
+// large record's area (22 of 60 KB at 74 locals), i.e. three instead of five
+// records per SM.
+__host__ __device__ inline bool clmat_in_global(bool big, int bandmax) { return big && bandmax >= 0; }
+__host__ __device__ inline int64_t band_scratch(int nalcmax, int neqmax) {
+    const int64_t inv = (int64_t)nalcmax * (nalcmax + 1) / 2, z = 8 * (int64_t)neqmax;
+    return 32 * (int64_t)nalcmax + (inv > z ? inv : z) + 2;
+}
+__host__ __device__ inline int64_t band_scratch_total(int nalcmax, int neqmax) {
+    return band_scratch(nalcmax, neqmax) + (int64_t)nalcmax * (nalcmax + 1) / 2;
+}
+
 __host__ __device__ inline int64_t warp_bytes(int wmax, int neqmax, int nalcmax, int nalgmax,
                                               int bandmax, int bdrmax, int ngrpmax, bool big = false) {
     int64_t d = 0;
     d += wmax;                          // gl
     d += 7 * (int64_t)neqmax;           // rm1 lcor lwgt res t1 t2 w0
-    d += (int64_t)nalcmax * (nalcmax + 1) / 2 + 4 * (int64_t)nalcmax;  // clmat blvec diag ocol scol
+    if (!clmat_in_global(big, bandmax)) d += (int64_t)nalcmax * (nalcmax + 1) / 2;  // clmat
+    d += 4 * (int64_t)nalcmax;          // blvec diag ocol scol
     if (!big) d += 2 * (int64_t)nalcmax * nalgmax;  // B W (global memory for large records)
     d += band_doubles(nalcmax, bandmax, bdrmax);
     int64_t i = 0;
@@ -350,6 +367,7 @@ struct FitParams {
 
 int fit_smem_per_warp(const FitParams &p);
 int fit_warps_per_cta(const FitParams &p);
+int fit_default_wpc(const FitParams &p);
 cudaError_t launch_fit(const FitParams &p, int nsm, int maxPerSM, cudaStream_t s);
 // W B^T of the accepted records r0..r1 added to their block-major staging
 // (large-record mode, one CTA per record, 64 x 64 FP64 tiles)

@@ -221,12 +221,14 @@ struct WarpMem {
     double *gl, *rm1, *lcor, *lwgt, *res, *t1, *t2, *w0, *clmat, *blvec, *diag, *ocol, *scol;
     double *B, *W;
     double *bnd;   // band scratch (may be null)
+    int bndLen;    // its length
     int32_t *in, *mq, *slots, *swS, *sw, *used, *goff;
 };
 
 __device__ WarpMem carve(char *base, const FitParams &p) {
     WarpMem m;
     double *d = (double *)base;
+    const int64_t wid = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     m.gl = d; d += p.wmax;
     m.rm1 = d; d += p.neqmax;
     m.lcor = d; d += p.neqmax;
@@ -235,7 +237,12 @@ __device__ WarpMem carve(char *base, const FitParams &p) {
     m.t1 = d; d += p.neqmax;
     m.t2 = d; d += p.neqmax;
     m.w0 = d; d += p.neqmax;
-    m.clmat = d; d += (int64_t)p.nalcmax * (p.nalcmax + 1) / 2;
+    if (clmat_in_global(p.bigMode != 0, p.bandmax)) {
+        m.clmat = p.bscr + wid * p.bscrStride + band_scratch(p.nalcmax, p.neqmax);
+    } else {
+        m.clmat = d;
+        d += (int64_t)p.nalcmax * (p.nalcmax + 1) / 2;
+    }
     m.blvec = d; d += p.nalcmax;
     m.diag = d; d += p.nalcmax;
     m.ocol = d; d += p.nalcmax;
@@ -247,6 +254,7 @@ __device__ WarpMem carve(char *base, const FitParams &p) {
         m.B = m.W = nullptr;   // per record in global memory
     }
     m.bnd = p.bandmax >= 0 ? d : nullptr;
+    m.bndLen = (int)band_doubles(p.nalcmax, p.bandmax, p.bdrmax);
     d += band_doubles(p.nalcmax, p.bandmax, p.bdrmax);
     int32_t *q = (int32_t *)d;
     m.in = q; q += p.wmax;
@@ -387,12 +395,14 @@ __device__ void w_dbcslv_multi(const double *w, int mp1, int n, int nrhs, int ex
 }
 #undef WB2
 
+// direct: the matrix is in vbnd and vbdr already (v is not used)
 __device__ void w_sqmibb0(int side, double *v, double *b, int n, int nbdr, int nbnd, int *nrank, double *evdmin,
-                          double *evdmax, const BandWork &wk) {
+                          double *evdmax, const BandWork &wk, bool direct) {
     const int ln = lane_id();
     double *vbnd = wk.vbnd, *vbdr = wk.vbdr, *aux = wk.aux, *vbk = wk.vbk, *vzru = wk.vzru;
     const int mp1 = nbnd + 1, nmb = n - nbdr;
-    if (side == 1) {
+    if (direct) {
+    } else if (side == 1) {
         const int nb1 = nbdr + 1;
         for (int q = ln; q < nmb * mp1; q += 32) {
             const int i = nb1 + q / mp1, d = q % mp1, j = i + d;
@@ -441,7 +451,8 @@ __device__ void w_sqmibb0(int side, double *v, double *b, int n, int nbdr, int n
     }
     if (__any_sync(0xffffffffu, bad)) {
         for (int q = 1 + ln; q <= n; q += 32) b[q] = 0.0;
-        for (int q = 1 + ln; q <= (n * n + n) / 2; q += 32) v[q] = 0.0;
+        if (!direct)
+            for (int q = 1 + ln; q <= (n * n + n) / 2; q += 32) v[q] = 0.0;
         __syncwarp();
         *nrank = 0;
         *evdmin = 0.0;
@@ -474,7 +485,7 @@ __device__ void w_sqmibb0(int side, double *v, double *b, int n, int nbdr, int n
             while (rem >= ib) { rem -= ib; ib++; }
             const int jb = rem + 1, ip = q + 1;
             const int ioff = nb1 + (ib - 1) * n, joff = nb1 + (jb - 1) * n;
-            double t = v[ip];
+            double t = vbdr[(jb - 1) * n + ib];   // element (ib, jb) of the border
             for (int i = 0; i <= nmb - 1; i++) t = t - vbdr[ioff + i] * aux[joff + i];
             vbk[ip] = t;
         }
@@ -633,6 +644,204 @@ __device__ void w_band_inverse(int side, double *v, int n, int nbdr, int nbnd, c
     __syncwarp();
 }
 #undef WB
+
+// Normal equations of records with few locals per equation, equations added
+// in order: base[target(ij, ik)] is element (ij >= ik).  An equation of nl
+// locals has nl (nl + 1) / 2 terms w g_j g_k and nl terms w r g_j, item q of
+// them in lane q mod 32 (FP64 instructions hold the pipe for 16 clocks
+// however few lanes take part, so both kinds share them).  The terms of
+// kNeBatch equations are formed first, then added equation by equation: an
+// addition waits for the shared-memory read and one FP64 add of the equation
+// before it only.  112,000 clocks per record of 140 equations, with
+// everything inside the loop over equations 145,000 at fewer records per SM.
+constexpr int kNeBatch = 4, kNeItems = 3;   // equations per batch, items per lane
+// most locals per equation (kNeItems x 32 items)
+constexpr int kNeLocals = 12;
+template <class Target>
+__device__ __forceinline__ void normal_equations(const WarpMem &m, int neq, double *base, Target &&target) {
+    const int ln = lane_id();
+    // pair (j, k) of each of the lane's items, the same in every equation
+    int pj[kNeItems], pk[kNeItems];
+#pragma unroll
+    for (int u = 0; u < kNeItems; ++u) {
+        int j = 1, k = ln + 32 * u + 1;
+        while (k > j) { k -= j; j++; }
+        pj[u] = j;
+        pk[u] = k;
+    }
+    constexpr int kNone = -1;   // below it: -2 - index of the right-hand side
+    for (int e0 = 0; e0 < neq; e0 += kNeBatch) {
+        double t[kNeBatch][kNeItems];
+        int a[kNeBatch][kNeItems];
+#pragma unroll
+        for (int x = 0; x < kNeBatch; ++x) {
+            const int e = e0 + x;
+            int sl = 0, nl = 0;
+            double wght = 0.0, rm = 0.0;
+            if (e < neq) {
+                sl = m.mq[3 * e];
+                nl = m.mq[3 * e + 1] - sl - 1;
+                wght = m.lwgt[e];
+                rm = m.rm1[e];
+            }
+            const int npair = (nl * nl + nl) / 2, nit = npair + nl;
+#pragma unroll
+            for (int u = 0; u < kNeItems; ++u) {
+                a[x][u] = kNone;
+                t[x][u] = 0.0;
+                const int q = ln + 32 * u;
+                if (q < nit) {
+                    const bool pair = q < npair;
+                    const int j = pair ? pj[u] : 0, k = pair ? pk[u] : q - npair + 1;
+                    const int ik = m.in[sl + k];
+                    t[x][u] = wght * (pair ? m.gl[sl + j] : rm) * m.gl[sl + k];
+                    a[x][u] = pair ? target(m.in[sl + j], ik) : -1 - ik;
+                }
+            }
+        }
+#pragma unroll
+        for (int x = 0; x < kNeBatch; ++x) {
+#pragma unroll
+            for (int u = 0; u < kNeItems; ++u)
+                if (a[x][u] != kNone) {
+                    double *to = a[x][u] >= 0 ? base + a[x][u] : m.blvec + (-2 - a[x][u]);
+                    *to = *to + t[x][u];
+                }
+            __syncwarp();
+        }
+    }
+}
+
+// place of element (ij >= ik) of a band record's local matrix in the band
+// storage of sqmibb (side 1) and sqmibb2 (side 2)
+// (offset from vbnd)
+__device__ __forceinline__ int band_element(const BandWork &wk, int side, int n, int nbdr, int mp1, int ij, int ik) {
+    const int bdr = (int)(wk.vbdr - wk.vbnd);
+    if (side == 1) return ik <= nbdr ? bdr + (ik - 1) * n + ij : ij - ik + 1 + (ik - nbdr - 1) * mp1;
+    const int nmb = n - nbdr;
+    return ij > nmb ? bdr + (ij - nmb - 1) * n + ik : ij - ik + 1 + (ik - 1) * mp1;
+}
+
+// S_ef = t2_e t2_f l_e^T Gamma^-1 l_f of a band record over the nge equations
+// geq, from the factors of w_sqmibb0.  With the band and border parts l = (b,
+// d), A the band matrix, C its border columns and K the inverse of the border
+// Schur complement, l_e^T Gamma^-1 l_f = b_f^T A^-1 b_e + z_f^T K z_e, z = d -
+// (A^-1 C)^T b (aux holds A^-1 C).  Lane per equation e: x = A^-1 b_e by the
+// band substitutions (the last W values of the recurrence in registers; x
+// lane-interleaved in X, nmb x 32), then the products with every f <= e.  The
+// full inverse with its products (Y = L Gamma^-1) took 594,000 clocks per
+// large record at three records per SM, its per-lane columns apart in memory;
+// this takes 390,000 at five.  Used up to W = kBandW bands and kBorder border locals.
+// Not part of the fit's decisions.  Z: nge x kBorder.
+constexpr int kBorder = 8;
+template <int W>
+__device__ __forceinline__ void w_band_schur(const WarpMem &m, const BandWork &wk, int side, int n, int nbdr, int nbnd,
+                                             const int32_t *geq, int nge, int neq, double *X, double *Z, double *S) {
+    const int ln = lane_id();
+    const int mp1 = nbnd + 1, nmb = n - nbdr;
+    const double *w = wk.vbnd, *vbk = wk.vbk;
+    const double *aux = wk.aux + (side == 1 ? nbdr + 1 : 1);   // aux[ib * n + i]: band index i (0-based), border ib
+    // locals (1-based) b0 + 1 .. b0 + nmb are the band, d0 + 1 .. the border
+    const int b0 = side == 1 ? nbdr : 0, d0 = side == 1 ? 0 : nmb;
+    double *x = X + ln;
+    for (int e0 = 0; e0 < nge; e0 += 32) {
+        const bool on = e0 + ln < nge;
+        const int E = geq[on ? e0 + ln : e0];
+        const int sl = m.mq[3 * E], sg = on ? m.mq[3 * E + 1] : m.mq[3 * E] + 1;
+        for (int i = 0; i < nmb; ++i) x[i * 32] = 0.0;
+        double zb[kBorder];
+#pragma unroll
+        for (int ib = 0; ib < kBorder; ++ib) zb[ib] = 0.0;
+        int first = nmb;
+        for (int q = sl + 1; q < sg; ++q) {
+            const int l = m.in[q], i = l - 1 - b0;
+            const double g = m.gl[q];
+            if ((unsigned)i < (unsigned)nmb) {
+                x[i * 32] += g;
+                first = min(first, i);
+#pragma unroll
+                for (int ib = 0; ib < kBorder; ++ib)
+                    if (ib < nbdr) zb[ib] = __fma_rn(-g, aux[ib * n + i], zb[ib]);
+            } else {
+#pragma unroll
+                for (int ib = 0; ib < kBorder; ++ib)
+                    if (ib == l - 1 - d0) zb[ib] += g;
+            }
+        }
+        double zk[kBorder];   // K z_e
+#pragma unroll
+        for (int ib = 0; ib < kBorder; ++ib) {
+            zk[ib] = 0.0;
+            if (ib < nbdr) {
+                if (on) Z[(e0 + ln) * kBorder + ib] = zb[ib];
+#pragma unroll
+                for (int jb = 0; jb < kBorder; ++jb)
+                    if (jb < nbdr) {
+                        const int hi = max(ib, jb) + 1, lo = min(ib, jb) + 1;
+                        zk[ib] = __fma_rn(vbk[(hi * hi - hi) / 2 + lo], zb[jb], zk[ib]);
+                    }
+            }
+        }
+        // forward: r[j] = x[i + j] with the updates of the rows before i
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) first = min(first, __shfl_xor_sync(0xffffffffu, first, o));
+        double r[W + 1];
+#pragma unroll
+        for (int j = 0; j <= W; ++j) r[j] = first + j < nmb ? x[(first + j) * 32] : 0.0;
+#pragma unroll 2
+        for (int i = first; i < nmb; ++i) {
+            const double nxt = i + 1 + W < nmb ? x[(i + 1 + W) * 32] : 0.0;
+            const double xi = r[0];
+            x[i * 32] = xi;
+            const double *c = w + i * mp1 + 1;   // c[j]: WB(j + 1, i + 1)
+#pragma unroll
+            for (int j = 1; j <= W; ++j) {
+                r[j - 1] = r[j];
+                if (j <= nbnd) r[j - 1] = __fma_rn(i + j < nmb ? -c[j] : 0.0, xi, r[j]);
+            }
+            r[W] = nxt;
+        }
+        // backward: y[j - 1] = x[i + j]
+        double y[W + 1];
+#pragma unroll
+        for (int j = 0; j <= W; ++j) y[j] = 0.0;
+#pragma unroll 2
+        for (int i = nmb - 1; i >= 0; --i) {
+            const double *c = w + i * mp1 + 1;
+            double v = i >= first ? x[i * 32] * c[0] : 0.0;
+#pragma unroll
+            for (int j = W; j >= 1; --j)
+                if (j <= nbnd) v = __fma_rn(i + j < nmb ? -c[j] : 0.0, y[j - 1], v);
+#pragma unroll
+            for (int j = W; j >= 1; --j) y[j] = y[j - 1];
+            y[0] = v;
+            x[i * 32] = v;
+        }
+        __syncwarp();
+        const double te = m.t2[E];
+        const int fEnd = min(nge, e0 + 32);
+        for (int fi = 0; fi < fEnd; ++fi) {
+            const int f = geq[fi];
+            const int fl = m.mq[3 * f], fg = m.mq[3 * f + 1];
+            double acc = 0.0;
+#pragma unroll
+            for (int ib = 0; ib < kBorder; ++ib)
+                if (ib < nbdr) acc = __fma_rn(Z[fi * kBorder + ib], zk[ib], acc);
+#pragma unroll 4
+            for (int q = fl + 1; q < fg; ++q) {
+                const int i = m.in[q] - 1 - b0;
+                if ((unsigned)i < (unsigned)nmb) acc = __fma_rn(x[i * 32], m.gl[q], acc);
+            }
+            if (on && fi <= e0 + ln) {
+                const double v = te * m.t2[f] * acc;
+                S[f * neq + E] = v;
+                S[E * neq + f] = v;
+            }
+        }
+        __syncwarp();
+    }
+}
+constexpr int kBandW = 4;
 
 __device__ __forceinline__ double wsum_serial(const double *a, int n) {
     // sequential sum in index order on lane 0, broadcast to the warp
@@ -885,8 +1094,101 @@ __device__ __forceinline__ void sform_dispatch(const WarpMem &m, const double *S
     }
 }
 
-template <bool BIG>
-__global__ void __launch_bounds__(32 * MPG_WARPS_FIT, 2)
+// Off-diagonal and diagonal blocks of the S-form update of a large record
+// (S in global memory), group by group: H = G_p S over the record's
+// equations (H: rows of the group x nge, in shared memory; a lane per
+// equation, S read once per equation of the group), then a lane per column b
+// of the groups before: U(a, b) = sum_f H(a, f) g_bf over the equations of b,
+// row after row, so that the lanes of a group write consecutive elements.
+// A lane per block (S's block in registers, 36 elements written per lane to
+// places apart) took 311,000 clocks per record at three records per SM, this
+// 280,000 at five.  (The kernel is short of instruction cache: loads a few
+// steps ahead in w_band_schur, or a flag that spares eq_lists_meet, made it
+// slower, 32.6 to 38.7 ms for 50,000 broken lines.)
+template <int M>
+__device__ __forceinline__ void sform_columns(const WarpMem &m, const double *H, const int32_t *fpos, int nge, int pg,
+                                              const int32_t *grp, const int64_t *pdst, double *stage) {
+    const int ln = lane_id();
+    const int a0 = m.goff[pg], np = m.goff[pg + 1] - a0;
+    for (int b0 = 0; b0 < a0; b0 += 32) {
+        const int b = b0 + ln;
+        if (b >= a0) continue;
+        const int q = grp[b], c0 = m.goff[q], nj = m.goff[q + 1] - c0;
+        const int s0 = m.swS[b], mq = m.swS[b + 1] - s0;
+        double g[M];
+        int f[M];
+#pragma unroll
+        for (int i = 0; i < M; ++i) {
+            const int ent = i < mq ? m.sw[s0 + i] : 0;
+            g[i] = i < mq ? m.gl[ent & 0xffff] : 0.0;
+            f[i] = i < mq ? fpos[ent >> 16] : 0;
+        }
+        double *out = stage + __ldg(pdst + pg * (pg + 1) / 2 + q) + (b - c0);
+        const bool meet = eq_lists_meet(m, a0, c0);
+#pragma unroll 2
+        for (int ii = 0; ii < np; ++ii) {
+            double u = meet ? gtwg_element(m, a0 + ii, b, false) : 0.0;
+#pragma unroll
+            for (int i = 0; i < M; ++i) u = __fma_rn(H[ii * nge + f[i]], g[i], u);
+            out[(int64_t)ii * nj] = u;
+        }
+    }
+}
+
+__device__ void sform_large(const WarpMem &m, const double *S, int neq, int ngrp, const int32_t *geq, int nge,
+                            int32_t *fpos, int32_t *grp, double *H, int mmax, const int64_t *pdst, double *stage) {
+    const int ln = lane_id();
+    for (int i = ln; i < nge; i += 32) fpos[geq[i]] = i;
+    for (int g = ln; g < ngrp; g += 32)
+        for (int b = m.goff[g]; b < m.goff[g + 1]; ++b) grp[b] = g;
+    __syncwarp();
+    for (int pg = 0; pg < ngrp; ++pg) {
+        const int a0 = m.goff[pg], np = m.goff[pg + 1] - a0;
+        const int s0 = m.swS[a0], mp = m.swS[a0 + 1] - s0;
+        for (int fi = ln; fi < nge; fi += 32) {
+            const int f = geq[fi];
+            for (int ii = 0; ii < np; ++ii) {
+                const int sa = m.swS[a0 + ii];
+                double h = 0.0;
+                for (int i = 0; i < mp; ++i) {
+                    const int ent = m.sw[sa + i];
+                    h = __fma_rn(m.gl[ent & 0xffff], S[(ent >> 16) * neq + f], h);
+                }
+                H[ii * nge + fi] = h;
+            }
+        }
+        __syncwarp();
+        if (mmax <= 2) sform_columns<2>(m, H, fpos, nge, pg, grp, pdst, stage);
+        else if (mmax <= 4) sform_columns<4>(m, H, fpos, nge, pg, grp, pdst, stage);
+        else sform_columns<kSformMaxEq>(m, H, fpos, nge, pg, grp, pdst, stage);
+        // the diagonal block: the G^T W G part folded into H
+        const int64_t base = __ldg(pdst + pg * (pg + 1) / 2 + pg);
+        const int nel = np * (np + 1) / 2;
+        for (int t = ln; t < nel; t += 32) {
+            int ii = 0;
+            while ((ii + 1) * (ii + 2) / 2 <= t) ii++;
+            const int jj = t - ii * (ii + 1) / 2;
+            const int sa = m.swS[a0 + ii], sb = m.swS[a0 + jj];
+            double u = 0.0;
+            for (int i = 0; i < mp; ++i) {
+                const int ent = m.sw[sa + i], e = ent >> 16;
+                const double z = __fma_rn(-m.w0[e], m.gl[ent & 0xffff], H[ii * nge + fpos[e]]);
+                u = __fma_rn(z, m.gl[m.sw[sb + i] & 0xffff], u);
+            }
+            stage[base + t] = u;
+        }
+        __syncwarp();
+    }
+}
+
+// BAND: the launch's class holds records with a band structure (without, the
+// band code's registers would spill into the dense fits: 16.1 against 16.9 ms
+// for 400,000 barrel records)
+// Registers: 128 per thread for 16 warps per SM; large records' shared memory
+// leaves room for ten warps at most, so they may use 200 (at 128 their loops
+// spill).
+template <bool BIG, bool BAND>
+__global__ void __launch_bounds__(BIG ? 320 : 32 * MPG_WARPS_FIT, BIG ? 1 : 2)
 k_fit(FitParams p, int perWarp) {
     extern __shared__ __align__(16) char smem[];
     const int ln = lane_id();
@@ -944,12 +1246,21 @@ k_fit(FitParams p, int perWarp) {
             }
             __syncwarp();
             const int nter = (p.nloopn != 1 && p.lhuber != 0) ? p.lhuber : 1;
-            const bool band = ri.mbnd >= 0 && p.lfitbb > 0 && nalc > 5;
+            const bool band = BAND && ri.mbnd >= 0 && p.lfitbb > 0 && nalc > 5;
             const bool seqNormal = ((ri.mside >> 8) & 1) != 0;
             const bool denseLoc = ((ri.mside >> 9) & 1) != 0;
             const bool simpleWords = ((ri.mside >> 10) & 1) != 0;
             const bool needResing = p.lhuber > 1 && p.dwcut != 0.0f;
             const int npk = (nalc * nalc + nalc) / 2;
+            // few locals in every equation: terms batched over equations; of
+            // a band record summed into the band storage
+            bool batched = BAND && !denseLoc && !seqNormal;
+            if (batched) {
+                bool few = true;
+                for (int e = ln; e < neq; e += 32) few = few && m.mq[3 * e + 1] - m.mq[3 * e] - 1 <= kNeLocals;
+                batched = __all_sync(0xffffffffu, few);
+            }
+            const bool direct = batched && band;
             int nrank = 0, ndf = 0;
             double summ = 0.0;
             float cndl10 = 0.0f, resing = 0.0f;
@@ -1030,11 +1341,22 @@ k_fit(FitParams p, int perWarp) {
                         else m.blvec[j - 1] = acc;
                     }
                     __syncwarp();
+                } else if (direct) {
+                    const BandWork wk = band_work(m, ri, nalc);
+                    const int side = ri.mside & 0xff, nb = ri.mbdr, mp1 = ri.mbnd + 1;
+                    for (int i = ln; i < nalc * mp1; i += 32) wk.vbnd[1 + i] = 0.0;
+                    for (int i = ln; i < nalc * nb; i += 32) wk.vbdr[1 + i] = 0.0;
+                    for (int i = ln; i < nalc; i += 32) m.blvec[i] = 0.0;
+                    __syncwarp();
+                    normal_equations(m, neq, wk.vbnd,
+                                     [&](int ij, int ik) { return band_element(wk, side, nalc, nb, mp1, ij, ik); });
                 } else {
                 for (int i = ln; i < npk; i += 32) m.clmat[i] = 0.0;
                 for (int i = ln; i < nalc; i += 32) m.blvec[i] = 0.0;
                 __syncwarp();
-                for (int e = 0; e < neq; ++e) {
+                if (batched)
+                    normal_equations(m, neq, m.clmat, [](int ij, int ik) { return (ij * ij - ij) / 2 + ik - 1; });
+                for (int e = batched ? neq : 0; e < neq; ++e) {
                     const int sl = m.mq[3 * e], sg = m.mq[3 * e + 1];
                     const int nl = sg - sl - 1;
                     const double wght = m.lwgt[e], rm = m.rm1[e];
@@ -1078,7 +1400,7 @@ k_fit(FitParams p, int perWarp) {
                     int nr = 0;
                     const BandWork wk = band_work(m, ri, nalc);
                     w_sqmibb0(ri.mside & 0xff, m.clmat - 1, m.blvec - 1, nalc, ri.mbdr, ri.mbnd, &nr, &evdmin,
-                              &evdmax, wk);
+                              &evdmax, wk, direct);
                     cndl10 = evdmin > 0.0 ? log10f((float)(evdmax / evdmin)) : 0.0f;
                     nrank = nr;
                     if (p.monOn && p.monPull && iter == 1 && nr == nalc) {
@@ -1246,8 +1568,9 @@ k_fit(FitParams p, int perWarp) {
                 // records with simple word lists, at most four equations per
                 // group, room for Y and S in the B/W area and a lower count.
                 bool sform = false;
+                int mmax = 0;
                 if (p.icalcm == 1 && simpleWords) {
-                    int mmax = 0, nnz = 0;
+                    int nnz = 0;
                     for (int g = ln; g < ngrp; g += 32) {
                         const int c0 = m.goff[g];
                         mmax = max(mmax, m.swS[c0 + 1] - m.swS[c0]);
@@ -1295,7 +1618,9 @@ k_fit(FitParams p, int perWarp) {
                     p.vstage[ri.slotOff + s] = v;
                 }
                 __syncwarp();
-                if (p.icalcm == 1 && band) {
+                // band records with a narrow border take S from the factors
+                const bool bandSchur = sform && band && ri.mbdr <= kBorder && ri.mbnd <= kBandW;
+                if (p.icalcm == 1 && band && !bandSchur) {
                     const BandWork wk = band_work(m, ri, nalc);
                     const int64_t wid = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
                     double *X = p.bscr + wid * p.bscrStride;
@@ -1319,8 +1644,14 @@ k_fit(FitParams p, int perWarp) {
                         nge += __popc(bal);
                     }
                     __syncwarp();
+                    if (bandSchur) {
+                        const int64_t wid = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+                        double *X = p.bscr + wid * p.bscrStride;
+                        w_band_schur<kBandW>(m, band_work(m, ri, nalc), ri.mside & 0xff, nalc, ri.mbdr, ri.mbnd, geq, nge,
+                                             neq, X, X + 32 * (int64_t)p.nalcmax, S);
+                    }
                     // Y_ek = sum over the locals j of equation e of l_ej Gamma^-1_jk
-                    for (int t = ln; t < nge * nalc; t += 32) {
+                    for (int t = ln; !bandSchur && t < nge * nalc; t += 32) {
                         const int e = geq[t / nalc], k = t - (t / nalc) * nalc + 1;
                         const int sl = m.mq[3 * e], sg = m.mq[3 * e + 1];
                         double y = 0.0;
@@ -1344,7 +1675,7 @@ k_fit(FitParams p, int perWarp) {
                     __syncwarp();
                     // S_ef = t2_e t2_f sum over the locals k of equation f of Y_ek l_fk
                     const int ns = nge * (nge + 1) / 2;
-                    for (int t = ln; t < ns; t += 32) {
+                    for (int t = ln; !bandSchur && t < ns; t += 32) {
                         int ie = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
                         while (ie > 0 && ie * (ie + 1) / 2 > t) ie--;
                         while ((ie + 1) * (ie + 2) / 2 <= t) ie++;
@@ -1363,7 +1694,21 @@ k_fit(FitParams p, int perWarp) {
                     // a in block (p, q).  Off-diagonal blocks first (every
                     // task the same size), then the diagonal ones, one per slot
                     const int ntask = BIG ? 0 : tpre[ngrp];
+                    // large records: H of a group in the band work area (the
+                    // factors are not needed any more), the index lists in
+                    // the record's slot list and equation weights
+                    int npmax = 0;
                     if (BIG) {
+                        for (int g = ln; g < ngrp; g += 32) npmax = max(npmax, m.goff[g + 1] - m.goff[g]);
+#pragma unroll
+                        for (int o = 16; o > 0; o >>= 1)
+                            npmax = max(npmax, __shfl_xor_sync(0xffffffffu, npmax, o));
+                    }
+                    const bool byGroup = BIG && m.bnd && npmax * nge <= m.bndLen;
+                    if (byGroup) {
+                        sform_large(m, S, neq, ngrp, geq, nge, reinterpret_cast<int32_t *>(m.rm1), m.slots, m.bnd,
+                                    mmax, pdst, p.stage);
+                    } else if (BIG) {
                         // large records (S in global memory): a lane per
                         // off-diagonal block (pg, q), q < pg, t = pg (pg - 1) / 2 + q
                         const int nblk = ngrp * (ngrp - 1) / 2;
@@ -1385,7 +1730,7 @@ k_fit(FitParams p, int perWarp) {
                         const int a = m.goff[pg] + loc / pg, q = loc % pg;
                         sform_dispatch<false>(m, S, neq, a, pg, q, pdst, p.stage);
                     }
-                    for (int a = ln; a < nalg; a += 32) {
+                    for (int a = ln; !byGroup && a < nalg; a += 32) {
                         int lo = 0, hi = ngrp - 1;
                         while (lo < hi) {
                             const int mid = (lo + hi + 1) >> 1;
@@ -1544,9 +1889,37 @@ cudaError_t launch_update_big(const FitParams &p, cudaStream_t s) {
     return cudaGetLastError();
 }
 
+static auto fit_kernel(const FitParams &p) -> void (*)(FitParams, int) {
+    const bool band = p.bandmax >= 0;
+    return p.bigMode ? (band ? k_fit<true, true> : k_fit<true, false>) : (band ? k_fit<false, true> : k_fit<false, false>);
+}
+
 int fit_smem_per_warp(const FitParams &p) {
     return (int)warp_bytes(p.wmax, p.neqmax, p.nalcmax, p.nalgmax, p.bandmax, p.bdrmax, p.ngrpmax,
                            p.bigMode != 0);
+}
+
+// Warps per CTA of a class that is not tuned: the form with the most warps
+// resident on an SM (fewest warps on equal counts: a record is one warp's
+// work, and single-warp CTAs leave no warp waiting for the others).  At 1, 2,
+// 4 and 8 warps: the largest broken-line records 16.9, 22.4, -, - ms (3, 2
+// warps resident); those below 10.5, 10.5, 10.5, -; barrel records 16.4, -, -,
+// 16.1 ms per 400,000 (15, 16 resident); telescope records 2.31, -, 2.44, -.
+int fit_default_wpc(const FitParams &p) {
+    FitParams q = p;
+    q.onePerBlock = 0;
+    int best = 0, bestW = 1;
+    for (int w = 1; w <= MPG_WARPS_FIT; w *= 2) {
+        q.wpc = w;
+        if (fit_warps_per_cta(q) != w) break;
+        int perSM = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, fit_kernel(q), 32 * w, (size_t)fit_smem_per_warp(q) * w);
+        if (perSM * w > best) {
+            best = perSM * w;
+            bestW = w;
+        }
+    }
+    return bestW;
 }
 
 // warps per CTA so that one CTA fits the 227 KB of shared memory (at most
@@ -1560,7 +1933,7 @@ int fit_warps_per_cta(const FitParams &p) {
 
 cudaError_t launch_fit(const FitParams &p, int nsm, int maxPerSM, cudaStream_t s) {
     const int per = fit_smem_per_warp(p);
-    void (*kern)(FitParams, int) = p.bigMode ? k_fit<true> : k_fit<false>;
+    void (*kern)(FitParams, int) = fit_kernel(p);
     const int wpc = fit_warps_per_cta(p);
     if (wpc < 1) return cudaErrorInvalidConfiguration;
     const int bytes = per * wpc;

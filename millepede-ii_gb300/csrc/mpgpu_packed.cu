@@ -1,0 +1,519 @@
+// mpgpu_packed.cu -- pede's own inversion (sqminl) and decomposition (chdec2,
+// chslv2) of the packed symmetric matrix, in blocks of kPb pivots.
+//
+// Both sweep the matrix once per pivot with a rank-1 update, in the
+// reference's order.  One launch pair per pivot was bound by launches and by
+// reading and writing the whole matrix for one multiply-add per element
+// (1,500 rows: 27 us per pivot, 9 MB twice).  Here a panel kernel forms the
+// rows of kPb pivots in turn, each brought up to date with the pivots of its
+// block before it, and one update kernel then applies the block's pivots to
+// every element in their order: the same operations on every element in the
+// same order as pivot by pivot, with kPb multiply-adds per element read and
+// written.  The update is FP64-bound (n^3 / 2 multiply-adds for sqminl, n^3 /
+// 6 for chdec2 at 2 per SM and clock), the panels are bound by the latency of
+// a chain of pivots.  Measured: sqminl of 1,500 rows 17.4 ms (per block 299 us
+// panel, 71 us update) from 40.5 ms; chdec2 and chslv2 of 2,000 rows 8.7 ms
+// (per block 37 + 35 us panel, 61 us update) from 64 ms.
+#include <cooperative_groups.h>
+
+#include <algorithm>
+
+#include "mpgpu_packed.h"
+
+namespace cg = cooperative_groups;
+
+namespace {
+
+constexpr int kPb = 32;        // pivots per block
+constexpr int kTile = 64;      // update tiles
+
+__device__ __forceinline__ int64_t prow(int64_t r) { return r * (r + 1) / 2; }   // offset of row r
+
+// tile (bi, bj <= bi) of the lower triangle
+__device__ __forceinline__ void tri_tile(int64_t t, int &bi, int &bj) {
+    int i = (int)((sqrt(8.0 * (double)t + 1.0) - 1.0) * 0.5);
+    while ((int64_t)i * (i + 1) / 2 > t) i--;
+    while ((int64_t)(i + 1) * (i + 2) / 2 <= t) i++;
+    bi = i;
+    bj = (int)(t - (int64_t)i * (i + 1) / 2);
+}
+
+// ------------------------------------------------------------ sqminl
+// Panel state: the pivots of the block and how many there are.
+struct SqState {
+    int32_t k[kPb];
+    double vkk[kPb];
+    int32_t count, stop;
+};
+
+// Rows of a CTA: warps of 32 rows dealt to the CTAs in turn.
+struct SqParams {
+    int32_t n, tmax;
+    const double *V, *diag;
+    double *b, *d;             // right-hand side, current diagonal
+    int32_t *used;
+    int8_t *step;              // pivot step of a row in this block (-1: none)
+    double *S, *C;             // [kPb][n] scaled and unscaled pivot columns
+    SqState *st;
+    int32_t *deficit;
+};
+
+constexpr int kSqThreads = 256;
+
+// One cluster takes the pivots of a block.  Per pivot: the candidates of the
+// CTAs (largest |d_j| above 1e-10 of the original diagonal, lowest index on
+// ties: the choice of the reference's scan) are exchanged through distributed
+// shared memory with one cluster barrier; every thread then brings its rows of
+// the pivot column up to date with the block's earlier pivots, scales them and
+// updates its diagonal elements, so that the next choice needs no pass over
+// the matrix.
+__global__ void __launch_bounds__(kSqThreads) k_sqminl_panel(SqParams p) {
+    cg::cluster_group cl = cg::this_cluster();
+    struct Msg {
+        unsigned long long bits;
+        double d, b;
+        int k;
+    };
+    __shared__ Msg msg[2];
+    __shared__ unsigned long long wbits[kSqThreads / 32];
+    __shared__ int wk[kSqThreads / 32];
+    __shared__ double Sk[kPb], Ck[kPb], sv[2];
+    __shared__ int spiv;
+    const int tid = threadIdx.x, ln = tid & 31, wib = tid >> 5;
+    const int nc = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+    const int n = p.n, rowStep = nc * kSqThreads;
+    const int row0 = (wib * nc + rank) * 32 + ln;
+    if (p.st->stop) {   // uniform: set by an earlier launch
+        if (rank == 0 && tid == 0) p.st->count = 0;   // nothing for this block's update
+        return;
+    }
+    for (int j = row0; j < n; j += rowStep) p.step[j] = -1;
+    int t = 0;
+    for (; t < p.tmax; ++t) {
+        unsigned long long best = 0;
+        int bk = -1;
+        for (int j = row0; j < n; j += rowStep) {
+            if (p.used[j]) continue;
+            const double a = fabs(p.d[j]);
+            const unsigned long long ab = (unsigned long long)__double_as_longlong(a);
+            if (a > 1.0E-10 * p.diag[j] && (bk < 0 || ab > best)) { best = ab; bk = j; }
+        }
+        auto take = [&](unsigned long long ob, int ok) {
+            if (ok >= 0 && (bk < 0 || ob > best || (ob == best && ok < bk))) { best = ob; bk = ok; }
+        };
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long ob = __shfl_xor_sync(0xffffffffu, best, o);
+            const int ok = __shfl_xor_sync(0xffffffffu, bk, o);
+            take(ob, ok);
+        }
+        if (ln == 0) { wbits[wib] = best; wk[wib] = bk; }
+        __syncthreads();
+        if (tid == 0) {
+#pragma unroll
+            for (int w = 1; w < kSqThreads / 32; ++w) take(wbits[w], wk[w]);
+            Msg &m = msg[t & 1];
+            m.bits = best;
+            m.k = bk;
+            m.d = bk >= 0 ? p.d[bk] : 0.0;
+            m.b = bk >= 0 ? p.b[bk] : 0.0;
+        }
+        cl.sync();
+        if (wib == 0) {
+            Msg m{0, 0.0, 0.0, -1};
+            if (ln < nc) m = *cl.map_shared_rank(&msg[t & 1], ln);
+            best = m.bits;
+            bk = m.k;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const unsigned long long ob = __shfl_xor_sync(0xffffffffu, best, o);
+                const int ok = __shfl_xor_sync(0xffffffffu, bk, o);
+                take(ob, ok);
+            }
+            const unsigned own = __ballot_sync(0xffffffffu, bk >= 0 && m.k == bk);
+            const int src = own ? __ffs(own) - 1 : 0;
+            const double dk = __shfl_sync(0xffffffffu, m.d, src), bb = __shfl_sync(0xffffffffu, m.b, src);
+            if (ln == 0) {
+                const double vkk = bk >= 0 ? 1.0 / dk : 0.0;
+                spiv = bk;
+                sv[0] = vkk;
+                sv[1] = bb * vkk;
+                if (rank == 0) {
+                    p.st->k[t] = bk;
+                    p.st->vkk[t] = vkk;
+                }
+            }
+            // the earlier pivots' columns at row k (other CTAs' writes: past L1)
+            if (bk >= 0 && ln < t) {
+                Sk[ln] = __ldcg(p.S + (int64_t)ln * n + bk);
+                Ck[ln] = __ldcg(p.C + (int64_t)ln * n + bk);
+            }
+        }
+        __syncthreads();
+        const int k = spiv;
+        if (k < 0) break;
+        const double vkk = sv[0], bnew = sv[1];
+        for (int j = row0; j < n; j += rowStep) {
+            const int64_t at = (int64_t)t * n + j;
+            if (j == k) {
+                p.S[at] = 0.0;
+                p.C[at] = 0.0;
+                p.step[j] = (int8_t)t;
+                p.used[j] = 1;
+                p.b[j] = bnew;
+                continue;
+            }
+            const int ps = p.step[j];
+            double w = ps < 0 ? p.V[j > k ? prow(j) + k : prow(k) + j] : Sk[ps];
+            if (j > k) {
+#pragma unroll 4
+                for (int q = ps + 1; q < t; ++q) w = fma(-Sk[q], p.C[(int64_t)q * n + j], w);
+            } else {
+#pragma unroll 4
+                for (int q = ps + 1; q < t; ++q) w = fma(-p.S[(int64_t)q * n + j], Ck[q], w);
+            }
+            const double sc = w * vkk;
+            p.S[at] = sc;
+            p.C[at] = w;
+            p.b[j] = fma(-bnew, w, p.b[j]);
+            if (!p.used[j]) p.d[j] = fma(-sc, w, p.d[j]);
+        }
+        // (the next candidates read this thread's own rows only)
+    }
+    if (rank == 0 && tid == 0) {
+        p.st->count = t;
+        if (t < p.tmax) {
+            p.st->stop = 1;
+            *p.deficit = -1;
+        }
+    }
+    cl.sync();   // no CTA leaves while another may read its messages
+}
+
+// every element brought up to date with the block's pivots in their order;
+// elements of a pivot row or column start from what its step left there
+__global__ void __launch_bounds__(256) k_sqminl_update(int32_t n, double *V, const int8_t *step, const double *S,
+                                                       const double *C, SqState *st) {
+    __shared__ double ss[kPb][kTile + 2], cc[kPb][kTile + 2];
+    __shared__ int8_t sr[kTile], sc[kTile];
+    const int T = st->count;
+    if (T <= 0) return;
+    int bi, bj;
+    tri_tile(blockIdx.x, bi, bj);
+    const int r0 = bi * kTile, c0 = bj * kTile, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    for (int e = tid; e < T * kTile; e += 256) {
+        const int q = e / kTile, i = e % kTile;
+        cc[q][i] = r0 + i < n ? C[(int64_t)q * n + r0 + i] : 0.0;
+        ss[q][i] = c0 + i < n ? S[(int64_t)q * n + c0 + i] : 0.0;
+    }
+    bool any = false;
+    if (tid < kTile) {
+        sr[tid] = r0 + tid < n ? step[r0 + tid] : -1;
+        sc[tid] = c0 + tid < n ? step[c0 + tid] : -1;
+        any = sr[tid] >= 0 || sc[tid] >= 0;
+    }
+    const bool pivots = __syncthreads_or(any);
+    double w[4][4];
+    int p0[4][4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const int i = ty + 16 * a, jj = tx + 16 * b, r = r0 + i, c = c0 + jj;
+            w[a][b] = 0.0;
+            p0[a][b] = -1;
+            if (r >= n || c > r) continue;
+            if (pivots) {
+                const int pr = sr[i], pc = sc[jj], q = max(pr, pc);
+                p0[a][b] = q;
+                if (q >= 0) {
+                    w[a][b] = r == c ? -st->vkk[q] : S[(int64_t)q * n + (pr == q ? c : r)];
+                    continue;
+                }
+            }
+            w[a][b] = V[prow(r) + c];
+        }
+    if (!pivots) {
+        for (int q = 0; q < T; ++q) {
+            double x[4], y[4];
+#pragma unroll
+            for (int a = 0; a < 4; ++a) { x[a] = -cc[q][ty + 16 * a]; y[a] = ss[q][tx + 16 * a]; }
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int b = 0; b < 4; ++b) w[a][b] = fma(y[b], x[a], w[a][b]);
+        }
+    } else {
+        for (int q = 0; q < T; ++q) {
+            double x[4], y[4];
+#pragma unroll
+            for (int a = 0; a < 4; ++a) { x[a] = -cc[q][ty + 16 * a]; y[a] = ss[q][tx + 16 * a]; }
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int b = 0; b < 4; ++b) {
+                    const double v = fma(y[b], x[a], w[a][b]);
+                    w[a][b] = q > p0[a][b] ? v : w[a][b];
+                }
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const int r = r0 + ty + 16 * a, c = c0 + tx + 16 * b;
+            if (r < n && c <= r) V[prow(r) + c] = w[a][b];
+        }
+}
+
+__global__ void k_sq_init(int32_t n, const double *V, double *d, int32_t *used, SqState *st, int32_t *deficit) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) {
+        d[i] = V[prow(i) + i];
+        used[i] = 0;
+    }
+    if (i == 0) {
+        st->count = st->stop = 0;
+        *deficit = 0;
+    }
+}
+
+// ------------------------------------------------------------ chdec2
+// Rows i1-1 .. i0 (at most kPb) are the pivots of a block, from the last.
+// First their own triangle, by one warp: lane c holds column i0 + c; row i is
+// scaled by f_i = 1 / G(i, i) (the element itself where it is not positive, as
+// chdec2 leaves it) and taken from the rows above.  The backward substitution
+// of chslv2 uses the same rows in the same order and rides along.
+__global__ void __launch_bounds__(32) k_chdec_diag(int32_t i0, int32_t nb, double *g, double *x, double *stat) {
+    __shared__ double rat[kPb];
+    const int c = threadIdx.x;
+    double w[kPb];
+#pragma unroll
+    for (int r = 0; r < kPb; ++r) w[r] = (r < nb && c <= r) ? g[prow(i0 + r) + i0 + c] : 0.0;
+    double xc = c < nb ? x[i0 + c] : 0.0;
+    double gmax = stat[0], gmin = stat[1], cnt = stat[2];
+#pragma unroll
+    for (int i = kPb - 1; i >= 0; --i) {
+        if (i >= nb) continue;
+        const double d = __shfl_sync(0xffffffffu, w[i], i);
+        double f = d;
+        if (d > 0.0) {
+            f = 1.0 / d;
+            gmax = cnt == 0.0 ? d : fmax(gmax, d);
+            gmin = cnt == 0.0 ? d : fmin(gmin, d);
+            cnt += 1.0;
+        }
+        const double q = c < i ? w[i] * f : 0.0;
+        __syncwarp();
+        rat[c] = q;
+        __syncwarp();
+        const double xi = __shfl_sync(0xffffffffu, xc, i);
+        if (c < i) xc = fma(-q, xi, xc);
+#pragma unroll
+        for (int r = 0; r < i; ++r) w[r] = fma(-w[i], rat[r], w[r]);   // used for c <= r
+        w[i] = c < i ? q : f;
+    }
+#pragma unroll
+    for (int r = 0; r < kPb; ++r)
+        if (r < nb && c <= r) g[prow(i0 + r) + i0 + c] = w[r];
+    if (c < nb) x[i0 + c] = xc;
+    if (c == 0) { stat[0] = gmax; stat[1] = gmin; stat[2] = cnt; }
+}
+
+// then the columns c < i0 of those rows, a thread per column: U the unscaled,
+// R the scaled rows (also left in g); x of the columns
+__global__ void __launch_bounds__(32) k_chdec_rows(int32_t i0, int32_t nb, double *g, double *x, double *U, double *R,
+                                                   int64_t ld) {
+    __shared__ double rat[kPb][kPb], f[kPb], xb[kPb];
+    for (int e = threadIdx.x; e < nb * nb; e += 32) {
+        const int i = e / nb, r = e % nb;
+        if (r <= i) {
+            const double v = g[prow(i0 + i) + i0 + r];
+            if (r < i) rat[i][r] = v;
+            else f[i] = v;
+        }
+    }
+    if ((int)threadIdx.x < nb) xb[threadIdx.x] = x[i0 + threadIdx.x];
+    __syncwarp();
+    const int64_t c = (int64_t)blockIdx.x * 32 + threadIdx.x;
+    if (c >= i0) return;
+    double w[kPb];
+#pragma unroll
+    for (int r = 0; r < kPb; ++r) w[r] = r < nb ? g[prow(i0 + r) + c] : 0.0;
+    double xc = x[c];
+#pragma unroll
+    for (int i = kPb - 1; i >= 0; --i) {
+        if (i >= nb) continue;
+#pragma unroll
+        for (int r = 0; r < i; ++r) w[r] = fma(-w[i], rat[i][r], w[r]);
+        const double q = w[i] * f[i];
+        U[i * ld + c] = w[i];
+        R[i * ld + c] = q;
+        g[prow(i0 + i) + c] = q;
+        xc = fma(-q, xb[i], xc);
+    }
+    x[c] = xc;
+}
+
+// the leading i0 x i0 triangle: G(r, c) -= U(i, c) R(i, r), i from the last
+__global__ void __launch_bounds__(256) k_chdec_update(int32_t i0, int32_t nb, double *g, const double *U,
+                                                      const double *R, int64_t ld) {
+    __shared__ double su[kPb][kTile + 2], sr[kPb][kTile + 2];
+    int bi, bj;
+    tri_tile(blockIdx.x, bi, bj);
+    const int r0 = bi * kTile, c0 = bj * kTile, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    for (int e = tid; e < nb * kTile; e += 256) {
+        const int q = e / kTile, i = e % kTile;
+        sr[q][i] = r0 + i < i0 ? R[q * ld + r0 + i] : 0.0;
+        su[q][i] = c0 + i < i0 ? U[q * ld + c0 + i] : 0.0;
+    }
+    __syncthreads();
+    double w[4][4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const int r = r0 + ty + 16 * a, c = c0 + tx + 16 * b;
+            w[a][b] = (r < i0 && c <= r) ? g[prow(r) + c] : 0.0;
+        }
+    for (int q = nb - 1; q >= 0; --q) {
+        double x[4], y[4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) { x[a] = -sr[q][ty + 16 * a]; y[a] = su[q][tx + 16 * a]; }
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) w[a][b] = fma(y[b], x[a], w[a][b]);
+    }
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const int r = r0 + ty + 16 * a, c = c0 + tx + 16 * b;
+            if (r < i0 && c <= r) g[prow(r) + c] = w[a][b];
+        }
+}
+
+// ------------------------------------------------------------ chslv2, forward
+// x(i) = x(i) G(i, i) - sum_{k < i} G(i, k) x(k).  Per block of kFb rows every
+// CTA solves the block's triangle (one warp, two rows per lane) and takes it
+// off its rows below; the solved block goes to out, as other CTAs still read
+// x.
+constexpr int kFb = 64;
+__global__ void k_chslv_scale(int32_t n, const double *g, double *x) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) x[i] *= g[prow(i) + i];
+}
+__global__ void __launch_bounds__(256) k_chslv_fwd(int32_t n, int32_t i0, const double *g, double *x, double *out) {
+    __shared__ double t[kFb][kFb + 1], xs[kFb];
+    const int tid = threadIdx.x, ln = tid & 31, wib = tid >> 5, nb = min(kFb, n - i0);
+    for (int e = tid; e < nb * kFb; e += 256) {
+        const int r = e / kFb, c = e % kFb;
+        t[r][c] = c < r ? g[prow(i0 + r) + i0 + c] : 0.0;
+    }
+    __syncthreads();
+    if (wib == 0) {
+        double a = ln < nb ? x[i0 + ln] : 0.0, b = ln + 32 < nb ? x[i0 + ln + 32] : 0.0;
+        for (int k = 0; k < nb; ++k) {
+            const double xk = __shfl_sync(0xffffffffu, k < 32 ? a : b, k & 31);
+            if (ln > k && ln < nb) a = fma(-t[ln][k], xk, a);
+            if (ln + 32 > k && ln + 32 < nb) b = fma(-t[ln + 32][k], xk, b);
+        }
+        xs[ln] = a;
+        xs[ln + 32] = b;
+        if (blockIdx.x == 0) {
+            if (ln < nb) out[i0 + ln] = a;
+            if (ln + 32 < nb) out[i0 + ln + 32] = b;
+        }
+    }
+    __syncthreads();
+    for (int64_t r = i0 + kFb + (int64_t)blockIdx.x * 8 + wib; r < n; r += (int64_t)gridDim.x * 8) {
+        const double *row = g + prow(r) + i0;
+        double v = row[ln] * xs[ln] + row[ln + 32] * xs[ln + 32];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (ln == 0) x[r] -= v;
+    }
+}
+
+int64_t tiles_of(int64_t n) {
+    const int64_t t = (n + kTile - 1) / kTile;
+    return t * (t + 1) / 2;
+}
+
+}  // namespace
+
+// S, C (or U, R): 2 kPb n; d or out: n; step: n bytes; state
+int64_t packed_work_len(int32_t n) {
+    return (2 * kPb + 1) * (int64_t)n + ((int64_t)n + 7) / 8 + (int64_t)(sizeof(SqState) + 7) / 8 + 8;
+}
+
+cudaError_t packed_sqminl(int32_t n, double *V, double *b, const double *diag, int32_t *used, int32_t *deficit,
+                          double *work, cudaStream_t s) {
+    SqParams p{};
+    p.n = n;
+    p.V = V;
+    p.diag = diag;
+    p.b = b;
+    p.used = used;
+    p.deficit = deficit;
+    p.S = work;
+    p.C = p.S + (int64_t)kPb * n;
+    p.d = p.C + (int64_t)kPb * n;
+    p.st = reinterpret_cast<SqState *>(p.d + n);
+    p.step = reinterpret_cast<int8_t *>(p.st + 1);
+    k_sq_init<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, V, p.d, used, p.st, deficit);
+    // CTAs of the panel's cluster: enough for one row per thread, more while
+    // that shortens the pivot columns (the FP64 work of a column is spread
+    // over them; a barrier of more CTAs costs little); 16 where the device
+    // takes such clusters
+    int cl = n <= 512 ? 4 : 8;
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    cfg.blockDim = dim3(kSqThreads);
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    if (n > 1024) {
+        int nclust = 0;
+        at.val.clusterDim.x = 16;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.gridDim = dim3(16);
+        if (cudaFuncSetAttribute(k_sqminl_panel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+            cudaOccupancyMaxActiveClusters(&nclust, k_sqminl_panel, &cfg) == cudaSuccess && nclust > 0)
+            cl = 16;
+        else
+            cudaGetLastError();
+    }
+    at.val.clusterDim.x = cl;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(cl);
+    const unsigned nt = (unsigned)tiles_of(n);
+    for (int32_t i = 0; i < n; i += kPb) {
+        p.tmax = std::min(kPb, n - i);
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, k_sqminl_panel, p);
+        if (e != cudaSuccess) return e;
+        k_sqminl_update<<<nt, 256, 0, s>>>(n, V, p.step, p.S, p.C, p.st);
+    }
+    return cudaGetLastError();
+}
+
+cudaError_t packed_chdec_solve(int32_t n, double *g, double *x, double *stat, double *work, cudaStream_t s) {
+    double *U = work, *R = U + (int64_t)kPb * n, *out = R + (int64_t)kPb * n;
+    for (int32_t i1 = n; i1 > 0; i1 -= kPb) {
+        const int32_t i0 = std::max(0, i1 - kPb), nb = i1 - i0;
+        k_chdec_diag<<<1, 32, 0, s>>>(i0, nb, g, x, stat);
+        if (i0 == 0) break;
+        k_chdec_rows<<<(unsigned)((i0 + 31) / 32), 32, 0, s>>>(i0, nb, g, x, U, R, n);
+        k_chdec_update<<<(unsigned)tiles_of(i0), 256, 0, s>>>(i0, nb, g, U, R, n);
+    }
+    k_chslv_scale<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, g, x);
+    for (int32_t i0 = 0; i0 < n; i0 += kFb) {
+        const int64_t rest = std::max<int64_t>(0, (int64_t)n - i0 - kFb);
+        const unsigned gb = (unsigned)std::max<int64_t>(1, std::min<int64_t>((rest + 7) / 8, 304));
+        k_chslv_fwd<<<gb, 256, 0, s>>>(n, i0, g, x, out);
+    }
+    cudaMemcpyAsync(x, out, sizeof(double) * n, cudaMemcpyDeviceToDevice, s);
+    return cudaGetLastError();
+}

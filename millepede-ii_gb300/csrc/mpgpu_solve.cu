@@ -12,6 +12,7 @@
 
 #include "mpgpu_bspmv.h"
 #include "mpgpu_ctx.h"
+#include "mpgpu_packed.h"
 
 namespace {
 
@@ -233,75 +234,7 @@ __global__ void k_vec_with_kn(const double *v, int32_t ilast, double vk, int32_t
         out[i] = i < ilast ? v[i] : (i == kn - 1 ? vk : 0.0);
 }
 
-// sqminl pivot step part 1 (one CTA): choose the pivot (first remaining
-// index with the largest |v_jj| above 1e-10 * |original diagonal|, the
-// choice of the reference's linked-list scan), scale the pivot row/column.
-__global__ void k_sqminl_pivot(int32_t n, double *v, double *b, const double *diag, int32_t *used,
-                               double *vk, double *scal, int32_t *pivot) {
-    __shared__ double sb[1024];
-    __shared__ int sk[1024];
-    const double eps = 1.0E-10;
-    double best = -1.0;
-    int bk = -1;
-    for (int j = threadIdx.x; j < n; j += blockDim.x) {
-        if (used[j]) continue;
-        const double a = fabs(v[(int64_t)(j + 1) * (j + 2) / 2 - 1]);
-        if (a > eps * diag[j] && a > best) { best = a; bk = j; }
-    }
-    sb[threadIdx.x] = best;
-    sk[threadIdx.x] = bk;
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if ((int)threadIdx.x < s) {
-            const double ob = sb[threadIdx.x + s];
-            const int ok = sk[threadIdx.x + s];
-            if (ob > sb[threadIdx.x] || (ob == sb[threadIdx.x] && ok >= 0 && (sk[threadIdx.x] < 0 || ok < sk[threadIdx.x]))) {
-                sb[threadIdx.x] = ob;
-                sk[threadIdx.x] = ok;
-            }
-        }
-        __syncthreads();
-    }
-    const int k = sk[0];
-    if (threadIdx.x == 0) *pivot = k;
-    if (k < 0) return;
-    const int64_t kk = (int64_t)(k + 1) * (k + 2) / 2 - 1;
-    const double vkk = 1.0 / v[kk];
-    for (int j = threadIdx.x; j < n; j += blockDim.x) {
-        if (j == k) { vk[j] = 0.0; continue; }
-        const int64_t jk = j > k ? (int64_t)j * (j + 1) / 2 + k : (int64_t)k * (k + 1) / 2 + j;
-        const double s = v[jk] * vkk;
-        v[jk] = s;
-        vk[j] = s;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        v[kk] = -vkk;
-        b[k] = b[k] * vkk;
-        used[k] = 1;
-        scal[0] = vkk;
-    }
-}
-
-// sqminl pivot step part 2: rank-1 elimination of rows j != k
-__global__ void k_sqminl_elim(int32_t n, double *v, double *b, const double *vk, const double *scal,
-                              const int32_t *pivot) {
-    const int k = *pivot;
-    if (k < 0) return;
-    const double vkk = scal[0];
-    const int ln = threadIdx.x & 31;
-    const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    const double bk = b[k];
-    for (int64_t j = w; j < n; j += nw) {
-        if (j == k) continue;
-        const double vjk = vk[j] / vkk;
-        if (ln == 0) b[j] = b[j] - bk * vjk;
-        double *row = v + j * (j + 1) / 2;
-        for (int64_t c = ln; c <= j; c += 32) row[c] = row[c] - vk[c] * vjk;
-    }
-}
-
+// sqminl without a pivot left: rows and columns of the unused rows zeroed
 __global__ void k_sqminl_deficit(int32_t n, double *v, double *b, const int32_t *used, const int32_t *pivot) {
     if (*pivot >= 0) return;
     for (int64_t j = blockIdx.x; j < n; j += gridDim.x) {
@@ -321,61 +254,6 @@ __global__ void k_negate(int64_t n, double *v) {
 __global__ void k_diag_abs(int32_t n, const double *v, double *d) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         d[i] = fabs(v[(i + 1) * (i + 2) / 2 - 1]);
-}
-
-// chdec2 step i (1-based): pivot, then the rank-1 update of rows 1..i-1
-__global__ void k_chdec_pivot(int64_t i, double *g, double *stat) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    const int64_t ii = i * (i + 1) / 2 - 1;
-    if (g[ii] > 0.0) {
-        const double d = g[ii];
-        if (stat[2] == 0.0) { stat[0] = d; stat[1] = d; }
-        else { stat[0] = fmax(stat[0], d); stat[1] = fmin(stat[1], d); }
-        stat[2] += 1.0;
-        g[ii] = 1.0 / d;
-    }
-}
-
-__global__ void k_chdec_update(int64_t i, double *g) {
-    const int64_t rowi = (i * i - i) / 2 - 1;   // g[rowi + c] = G(i, c), c 1-based
-    const double gii = g[rowi + i];
-    const int ln = threadIdx.x & 31;
-    const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t j = 1 + w; j <= i - 1; j += nw) {
-        const double ratio = g[rowi + j] * gii;
-        if (ratio == 0.0) continue;
-        double *rowj = g + (j * j - j) / 2 - 1;
-        for (int64_t c = 1 + ln; c <= j; c += 32) rowj[c] = rowj[c] - g[rowi + c] * ratio;
-    }
-}
-
-__global__ void k_chdec_scale(int64_t i, double *g) {
-    const int64_t rowi = (i * i - i) / 2 - 1;
-    const double gii = g[rowi + i];
-    for (int64_t c = 1 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c <= i - 1; c += (int64_t)gridDim.x * blockDim.x)
-        g[rowi + c] = g[rowi + c] * gii;
-}
-
-// chslv2 (mpnum.f90:953-987), one CTA: backward then forward substitution
-__global__ void k_chslv2(const double *g, double *x, int32_t n) {
-    __shared__ double sh[1024];
-    // backward: x(i) -= sum_{k>i} G(k,i) x(k)
-    for (int64_t i = n; i >= 1; --i) {
-        double s = 0.0;
-        for (int64_t k = i + 1 + threadIdx.x; k <= n; k += blockDim.x) s += g[(k * k - k) / 2 + i - 1] * x[k - 1];
-        s = block_sum(s, sh);
-        if (threadIdx.x == 0) x[i - 1] = x[i - 1] - s;
-        __syncthreads();
-    }
-    for (int64_t i = 1; i <= n; ++i) {
-        const int64_t ro = (i * i - i) / 2 - 1;
-        double s = 0.0;
-        for (int64_t k = 1 + threadIdx.x; k <= i - 1; k += blockDim.x) s += g[ro + k] * x[k - 1];
-        s = block_sum(s, sh);
-        if (threadIdx.x == 0) x[i - 1] = x[i - 1] * g[ro + i] - s;
-        __syncthreads();
-    }
 }
 
 // corr(i) -= sum_j A'(nfit+j, i) y(j), i <= nfit (minver/mchdec rhs)
@@ -1455,20 +1333,20 @@ int32_t solve_inversion(mpgpu_ctx *c, const double *consResiduals, double *corrO
     // for the whole device, i.e. for the other jobs' work in a served mix
     struct Tmp {
         cudaStream_t s;
-        double *corr = nullptr, *vbuf = nullptr, *Av = nullptr, *vk = nullptr, *diag = nullptr, *yv = nullptr;
+        double *corr = nullptr, *vbuf = nullptr, *Av = nullptr, *work = nullptr, *diag = nullptr, *yv = nullptr;
         int32_t *used = nullptr, *piv = nullptr;
         ~Tmp() {
-            for (void *p : {(void *)corr, (void *)vbuf, (void *)Av, (void *)vk, (void *)diag, (void *)yv,
+            for (void *p : {(void *)corr, (void *)vbuf, (void *)Av, (void *)work, (void *)diag, (void *)yv,
                             (void *)used, (void *)piv})
                 if (p) cudaFreeAsync(p, s);
         }
     } T{s};
-    double *&corr = T.corr, *&vbuf = T.vbuf, *&Av = T.Av, *&vk = T.vk, *&diag = T.diag, *&yv = T.yv;
+    double *&corr = T.corr, *&vbuf = T.vbuf, *&Av = T.Av, *&work = T.work, *&diag = T.diag, *&yv = T.yv;
     int32_t *&used = T.used, *&piv = T.piv;
     MPG_CUDA(c, cudaMallocAsync(&corr, sizeof(double) * n, s));
     MPG_CUDA(c, cudaMallocAsync(&vbuf, sizeof(double) * n, s));
     MPG_CUDA(c, cudaMallocAsync(&Av, sizeof(double) * n, s));
-    MPG_CUDA(c, cudaMallocAsync(&vk, sizeof(double) * n, s));
+    if (dense < 0) MPG_CUDA(c, cudaMallocAsync(&work, sizeof(double) * packed_work_len(nfit), s));
     MPG_CUDA(c, cudaMallocAsync(&diag, sizeof(double) * n, s));
     MPG_CUDA(c, cudaMallocAsync(&yv, sizeof(double) * (ncon + 1), s));
     MPG_CUDA(c, cudaMallocAsync(&used, sizeof(int32_t) * n, s));
@@ -1519,12 +1397,7 @@ int32_t solve_inversion(mpgpu_ctx *c, const double *consResiduals, double *corrO
     if (!decomposition && dense < 0) {
         // sqminl (mpnum.f90:230-355) on the leading nfit x nfit block
         k_diag_abs<<<S.grid(nfit), kThreads, 0, s>>>(nfit, j.matD, diag);
-        MPG_CUDA(c, cudaMemsetAsync(used, 0, sizeof(int32_t) * nfit, s));
-        MPG_CUDA(c, cudaMemsetAsync(piv, 0, sizeof(int32_t) * 4, s));
-        for (int i = 0; i < nfit; ++i) {
-            k_sqminl_pivot<<<1, 1024, 0, s>>>(nfit, j.matD, corr, diag, used, vk, scal + 8, piv);
-            k_sqminl_elim<<<S.wgrid(nfit), kThreads, 0, s>>>(nfit, j.matD, corr, vk, scal + 8, piv);
-        }
+        MPG_CUDA(c, packed_sqminl(nfit, j.matD, corr, diag, used, piv, work, s));
         k_sqminl_deficit<<<S.grid(nfit, 1), kThreads, 0, s>>>(nfit, j.matD, corr, used, piv);
         k_negate<<<S.grid((int64_t)nfit * (nfit + 1) / 2), kThreads, 0, s>>>((int64_t)nfit * (nfit + 1) / 2, j.matD);
         std::vector<int32_t> hu(nfit);
@@ -1547,14 +1420,7 @@ int32_t solve_inversion(mpgpu_ctx *c, const double *consResiduals, double *corrO
     } else {
         // chdec2 + chslv2 (mpnum.f90:891-987)
         MPG_CUDA(c, cudaMemsetAsync(scal + 16, 0, sizeof(double) * 3, s));
-        for (int64_t i = nfit; i >= 1; --i) {
-            k_chdec_pivot<<<1, 32, 0, s>>>(i, j.matD, scal + 16);
-            if (i > 1) {
-                k_chdec_update<<<S.wgrid(i - 1), kThreads, 0, s>>>(i, j.matD);
-                k_chdec_scale<<<S.grid(i - 1), kThreads, 0, s>>>(i, j.matD);
-            }
-        }
-        k_chslv2<<<1, 1024, 0, s>>>(j.matD, corr, nfit);
+        MPG_CUDA(c, packed_chdec_solve(nfit, j.matD, corr, scal + 16, work, s));
         double st[3];
         MPG_CUDA(c, cudaMemcpyAsync(st, scal + 16, sizeof(double) * 3, cudaMemcpyDeviceToHost, s));
         MPG_CUDA(c, cudaStreamSynchronize(s));

@@ -26,81 +26,227 @@ namespace {
 constexpr int kNB = 128;   // panel width = tile size
 constexpr int kSuperPanels = 4;   // panels per block column of the tensor-core factorisation
 
-// ------------------------------------------------------------ panel kernels
-// Cholesky of the 128 x 128 diagonal block at (k0, k0), in shared memory.
-__global__ void __launch_bounds__(512) k_potrf128(double *A, int64_t ld, int64_t k0, int32_t *err) {
-    extern __shared__ __align__(16) double sa[];   // 128 x 129
-    constexpr int S = kNB + 1;
-    __shared__ int bad;
-    __shared__ double sinv;   // reciprocal of the pivot: one FP64 division per column, not one per thread
-    const int tid = threadIdx.x, nt = blockDim.x;
-    if (tid == 0) bad = 0;
-    for (int e = tid; e < kNB * kNB; e += nt) {
-        const int i = e / kNB, j = e % kNB;
-        sa[i * S + j] = j <= i ? A[(k0 + i) * ld + k0 + j] : 0.0;
-    }
-    __syncthreads();
-    for (int j = 0; j < kNB; ++j) {
-        if (tid == 0) {
-            const double d = sa[j * S + j];
-            const double piv = d > 0.0 ? sqrt(d) : 1.0;
-            if (!(d > 0.0)) bad = 1;
-            sa[j * S + j] = piv;
-            sinv = 1.0 / piv;
-        }
-        __syncthreads();
-        const double inv = sinv;
-        for (int i = j + 1 + tid; i < kNB; i += nt) sa[i * S + j] *= inv;
-        __syncthreads();
-        const int m = kNB - 1 - j;
-        for (int e = tid; e < m * m; e += nt) {
-            const int i = j + 1 + e / m, k = j + 1 + e % m;
-            if (k <= i) sa[i * S + k] -= sa[i * S + j] * sa[k * S + j];
-        }
-        __syncthreads();
-    }
-    for (int e = tid; e < kNB * kNB; e += nt) {
-        const int i = e / kNB, j = e % kNB;
-        if (j <= i) A[(k0 + i) * ld + k0 + j] = sa[i * S + j];
-    }
-    if (tid == 0 && bad) atomicExch(err, (int)(k0 / kNB) + 1);
+// ------------------------------------------------------------ panel kernel
+// A 128-wide panel is factorised in four launches of 32 columns each, left-
+// looking within the panel: every CTA factorises the 32 x 32 diagonal block
+// for itself (its warps 0..3; no launch and no wait between that and its
+// use), while its other warps take the panel's earlier columns off their rows;
+// then the rows are solved.  The CTAs with the panel's own later rows also
+// bring those rows' diagonal blocks up to date, so that the next launch starts
+// on a finished one.
+//
+// Bound: a warp's FP64 instruction holds its quarter of the SM for 64 clocks
+// (2 multiply-adds per SM and clock), so that the chain of 32 pivots takes
+// some ten instructions (640 clocks) each, and the rows 8,256 multiply-adds
+// each over the four launches.  One CTA factorising 128 x 128 by itself (287
+// us, nearly all of it FP64 instructions of a single warp) followed by a
+// triangular solve of one warp per row (98 us at 3,000 rows, 306 us at 10,000)
+// took 385 and 593 us per panel; the four launches take 191 and 437 us.
+constexpr int kPc = 32;                 // columns per launch
+constexpr int kPcWarps = 16;            // warps 0..3 the diagonal block, 4..15 rows
+constexpr int kRowWarps = kPcWarps - 4;
+constexpr int kTld = kPc + 2;           // rows of the factor in shared memory
+constexpr int kLld = kNB - kPc + 2;     // rows of the earlier columns
+
+__device__ __forceinline__ void bar_n(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+
+// Reciprocal by Newton's iteration from an FP32 seed, |d| within 2^+-120; the
+// conversions in integers, as a conversion costs a slot of the FP64 pipe.
+__device__ __forceinline__ double newton_rcp(double d) {
+    const uint32_t hi = (uint32_t)__double2hiint(d), lo = (uint32_t)__double2loint(d);
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__uint_as_float((hi - (896u << 20)) << 3 | lo >> 29)));
+    const uint32_t f = __float_as_uint(y);
+    double z = __hiloint2double((int)((f >> 3) + (896u << 20)), (int)(f << 29));
+    z = fma(z, fma(-d, z, 1.0), z);
+    return fma(z, fma(-d, z, 1.0), z);
 }
 
-// L21 = A21 L11^-T: one warp per row below the diagonal block; L11 held
-// transposed in shared memory so that a column of L11 is contiguous.
-__global__ void __launch_bounds__(256) k_trsm128(double *A, int64_t ld, int64_t k0, int64_t nrows) {
-    extern __shared__ __align__(16) double lt[];   // 128 x 128 (lt[j * 128 + c] = L11[c][j]) + 128 inverse diagonal
-    double *dinv = lt + kNB * kNB;
-    const int tid = threadIdx.x, ln = tid & 31, wib = tid >> 5;
-    for (int e = tid; e < kNB * kNB; e += blockDim.x) {
-        const int c = e / kNB, j = e % kNB;
-        lt[j * kNB + c] = j <= c ? A[(k0 + c) * ld + k0 + j] : 0.0;
+// Cholesky factor of the 32 x 32 block at D into T, the reciprocals of its
+// diagonal into rs; by 128 threads (lane = row, warp w the columns 4 q + w in
+// registers).  Per column the owner's warp leaves it in shared memory, then
+// every warp takes its product with the reciprocal pivot off its own columns:
+// the next one at once, the others while the next pivot's reciprocal is under
+// way.  Square roots only at the end, for all columns at once.  False (T not
+// written) where a pivot is not within 2^+-120.
+__device__ __forceinline__ bool triangle_fast(const double *D, int64_t ld, double *T, double *rs, double (*col)[kPc],
+                                              double *dv) {
+    const int ln = threadIdx.x & 31, w = threadIdx.x >> 5;
+    double v[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = 4 * q + w <= ln ? D[ln * ld + 4 * q + w] : 0.0;
+    if (w == 0) col[0][ln] = v[0];
+    bool good = true;
+    double t = 0.0;
+#pragma unroll
+    for (int j = 0; j < kPc; ++j) {
+        bar_n(1, 128);
+        const double *cj = col[j & 3], *cp = col[(j + 3) & 3];
+        const double d = cj[j], x = cj[ln];
+        good = good && d > 0x1p-120 && d < 0x1p120;
+        const double rd = newton_rcp(d);
+        if (j > 0) {   // the column before, off the columns after this one
+#pragma unroll
+            for (int q = j >> 2; q < 8; ++q)
+                if (4 * q + w > j) v[q] = fma(-t, cp[4 * q + w], v[q]);
+        }
+        t = x * rd;
+        if (j + 1 < kPc && w == ((j + 1) & 3)) {
+            const int q = (j + 1) >> 2;
+            v[q] = fma(-t, cj[j + 1], v[q]);
+            col[(j + 1) & 3][ln] = v[q];
+        }
+        if (threadIdx.x == 0) dv[j] = d;
+    }
+    bar_n(1, 128);
+    if (!good) return false;
+    const double d = dv[ln], r = rsqrt(d);
+    double root = d * r;
+    root = fma(fma(-root, root, d), 0.5 * r, root);
+    if (w == 0) rs[ln] = r;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int c = 4 * q + w;
+        const double rc = __shfl_sync(0xffffffffu, r, c);
+        if (c <= ln) T[ln * kTld + c] = c == ln ? root : v[q] * rc;
+    }
+    return true;
+}
+
+// the same by one warp with the library's root, for any pivot (1 in place of
+// one that is not positive); returns whether there was such a pivot
+__device__ __noinline__ bool triangle_any(const double *D, int64_t ld, double *T, double *rs) {
+    const int ln = threadIdx.x & 31;
+    double *row = T + ln * kTld;
+    for (int c = 0; c <= ln; ++c) row[c] = D[ln * ld + c];
+    __syncwarp();
+    bool neg = false;
+    for (int j = 0; j < kPc; ++j) {
+        const double d = T[j * kTld + j];
+        double inv = 1.0, piv = 1.0;
+        if (d > 0.0) {
+            piv = sqrt(d);
+            inv = 1.0 / piv;
+        } else {
+            neg = true;
+        }
+        __syncwarp();
+        const double l = ln > j ? row[j] * inv : piv;
+        if (ln >= j) row[j] = l;
+        if (ln == 0) rs[j] = inv;
+        __syncwarp();
+        for (int c = j + 1; c <= ln; ++c) row[c] = fma(-l, T[c * kTld + j], row[c]);
+        __syncwarp();
+    }
+    return neg;
+}
+
+// Columns k0 + b .. k0 + b + 31 of the panel at k0 for the rows below.  LPR
+// lanes per row, lane q of a row the columns c = q mod LPR.  The first ns =
+// 3 - b / 32 CTAs take the panel's own later blocks of 32 rows, the others the
+// rows below the panel, a unit of 32 / LPR rows per warp in turn.  The factor
+// of the diagonal block goes to diag, as other CTAs may still have to read the
+// block itself.
+template <int LPR>
+__global__ void __launch_bounds__(32 * kPcWarps) k_panel32(double *A, int64_t ld, int64_t k0, int32_t b, int64_t nrows,
+                                                            double *diag, int32_t *err) {
+    constexpr int NC = kPc / LPR, RPU = 32 / LPR;   // columns per lane, rows per unit
+    __shared__ __align__(16) double L[kPc][kLld];   // the diagonal rows' earlier columns
+    __shared__ __align__(16) double T[kPc * kTld];
+    __shared__ double rs[kPc], dv[kPc], col[4][kPc], X[kPc][kPc + 1];
+    const int tid = threadIdx.x, ln = tid & 31, wib = tid >> 5, sub = ln % LPR, rowBase = ln - sub;
+    const int ns = (kNB - kPc - b) / kPc;
+    const bool own = (int)blockIdx.x < ns;   // a block of the panel's own rows
+    const int64_t r0 = k0 + b;               // first row and column of the diagonal block
+    const double *D = A + r0 * ld + r0;
+    double a[NC];
+    const int64_t nunit = own ? kPc / RPU : (nrows + RPU - 1) / RPU;
+    const int64_t ustep = own ? 1 : gridDim.x - ns;
+    int64_t u = own ? wib - 4 : (int64_t)(wib - 4) * ustep + blockIdx.x - ns;
+    double *row = nullptr;
+    bool in = false;
+    auto start = [&]() {   // the unit's rows, less the panel's earlier columns
+        const int64_t r = u * RPU + ln / LPR;
+        in = own || r < nrows;
+        row = A + ((own ? r0 + kPc * (blockIdx.x + 1) : k0 + kNB) + (in ? r : 0)) * ld + k0;
+#pragma unroll
+        for (int i = 0; i < NC; ++i) a[i] = row[b + LPR * i + sub];
+        if (b == 0) return;
+        double2 xn = *reinterpret_cast<const double2 *>(row);
+#pragma unroll 2
+        for (int k = 0; k < b; k += 2) {
+            const double2 x = xn;
+            if (k + 2 < b) xn = *reinterpret_cast<const double2 *>(row + k + 2);
+            double2 l[NC];
+#pragma unroll
+            for (int i = 0; i < NC; ++i) l[i] = *reinterpret_cast<const double2 *>(&L[LPR * i + sub][k]);
+#pragma unroll
+            for (int i = 0; i < NC; ++i) a[i] = fma(-x.x, l[i].x, a[i]);
+#pragma unroll
+            for (int i = 0; i < NC; ++i) a[i] = fma(-x.y, l[i].y, a[i]);
+        }
+    };
+    if (wib < 4) {
+        if (!triangle_fast(D, ld, T, rs, col, dv) && wib == 0) {
+            const bool neg = triangle_any(D, ld, T, rs);
+            if (neg && blockIdx.x == 0 && tid == 0) atomicExch(err, (int)(k0 / kNB) + 1);
+        }
+    } else {
+        for (int e = tid - 128; e < kPc * (b / 2); e += 32 * kRowWarps) {
+            const int c = e / (b / 2), k = 2 * (e % (b / 2));
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&L[c][k]);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(A + (r0 + c) * ld + k0 + k)
+                         : "memory");
+        }
+        asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+        bar_n(2, 32 * kRowWarps);
+        if (u < nunit) start();
     }
     __syncthreads();
-    for (int j = tid; j < kNB; j += blockDim.x) dinv[j] = 1.0 / lt[j * kNB + j];
-    __syncthreads();
-    const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t r = (int64_t)blockIdx.x * (blockDim.x >> 5) + wib; r < nrows; r += nw) {
-        double *row = A + (k0 + kNB + r) * ld + k0;
-        double a[4];
+    if (wib >= 4) {
+        while (u < nunit) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) a[q] = row[q * 32 + ln];
+            for (int j = 0; j < kPc; ++j) {
+                const double x = __shfl_sync(0xffffffffu, a[j / LPR], rowBase | (j % LPR)) * rs[j];
+                if (sub == j % LPR) a[j / LPR] = x;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            for (int l = 0; l < 32; ++l) {
-                const int j = q * 32 + l;
-                const double xj = __shfl_sync(0xffffffffu, a[q], l) * dinv[j];
-                if (ln == l) a[q] = xj;
-#pragma unroll
-                for (int q2 = 0; q2 < 4; ++q2) {
-                    if (q2 < q) continue;
-                    const int c = q2 * 32 + ln;
-                    if (c > j) a[q2] -= xj * lt[j * kNB + c];
-                }
+                for (int i = j / LPR; i < NC; ++i)
+                    if (i > j / LPR || sub > j % LPR) a[i] = fma(-x, T[(LPR * i + sub) * kTld + j], a[i]);
             }
-        }
+            if (in)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) row[q * 32 + ln] = a[q];
+                for (int i = 0; i < NC; ++i) row[b + LPR * i + sub] = a[i];
+            if (own)
+#pragma unroll
+                for (int i = 0; i < NC; ++i) X[u * RPU + ln / LPR][LPR * i + sub] = a[i];
+            u += kRowWarps * ustep;
+            if (u < nunit) start();
+        }
+    } else if (blockIdx.x == 0) {
+        double *o = diag + (r0 / kPc) * kPc * kPc;
+        for (int e = tid; e < kPc * kPc; e += 128) o[e] = e % kPc <= e / kPc ? T[(e / kPc) * kTld + e % kPc] : 0.0;
+    }
+    if (!own) return;
+    __syncthreads();
+    double *Dn = A + (r0 + kPc * (blockIdx.x + 1)) * (ld + 1);
+    for (int e = tid; e < kPc * (kPc + 1) / 2; e += 32 * kPcWarps) {
+        int i = (int)((sqrtf(8.0f * (float)e + 1.0f) - 1.0f) * 0.5f);
+        while (i * (i + 1) / 2 > e) i--;
+        while ((i + 1) * (i + 2) / 2 <= e) i++;
+        const int c = e - i * (i + 1) / 2;
+        double acc = Dn[i * ld + c];
+#pragma unroll 8
+        for (int k = 0; k < kPc; ++k) acc = fma(-X[i][k], X[c][k], acc);
+        Dn[i * ld + c] = acc;
+    }
+}
+
+// the factors of the diagonal blocks to their places
+__global__ void __launch_bounds__(256) k_put_diag(double *A, int64_t ld, const double *diag) {
+    const int64_t r0 = (int64_t)blockIdx.x * kPc;
+    for (int e = threadIdx.x; e < kPc * kPc; e += 256) {
+        const int i = e / kPc, c = e % kPc;
+        if (c <= i) A[(r0 + i) * ld + r0 + c] = diag[r0 * kPc + e];
     }
 }
 
@@ -167,18 +313,27 @@ int32_t dense_cholesky_device(mpgpu_ctx *c, double *A, int64_t npad, int mode, f
     const int32_t np = (int32_t)(npad / kNB);
     int nsm = 0;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
-    const int potrfSmem = kNB * (kNB + 1) * (int)sizeof(double);
-    const int trsmSmem = (kNB * kNB + kNB) * (int)sizeof(double);
-    MPG_CUDA(c, smem_optin((const void *)k_potrf128));
-    MPG_CUDA(c, smem_optin((const void *)k_trsm128));
     MPG_CUDA(c, cudaMemsetAsync(dErr, 0, sizeof(int32_t), s));
-    auto panel = [&](int32_t p, cudaStream_t st) -> int64_t {   // potrf + trsm of panel p; rows below it
-        const int64_t k0 = (int64_t)p * kNB;
-        k_potrf128<<<1, 512, potrfSmem, st>>>(A, ld, k0, dErr);
-        const int64_t rows = npad - k0 - kNB;
-        if (rows > 0) {
-            const int64_t tb = std::min<int64_t>((rows + 7) / 8, (int64_t)nsm);
-            k_trsm128<<<(unsigned)tb, 256, trsmSmem, st>>>(A, ld, k0, rows);
+    struct Diag {   // factors of the diagonal blocks, freed on the caller's stream
+        cudaStream_t s;
+        double *p = nullptr;
+        ~Diag() { if (p) cudaFreeAsync(p, s); }
+    } D{s};
+    MPG_CUDA(c, cudaMallocAsync(&D.p, sizeof(double) * npad * kPc, s));
+    double *diag = D.p;
+    auto panel = [&](int32_t p, cudaStream_t st) -> int64_t {   // panel p; rows below it
+        const int64_t k0 = (int64_t)p * kNB, rows = npad - k0 - kNB;
+        for (int b = 0; b < kNB; b += kPc) {
+            // 4 lanes per row take 176 + 8 b FP64 instructions per unit of 8
+            // rows, 8 lanes 112 + 4 b per unit of 4 rows: whichever ends first
+            // where the units go to the quarters of the SMs in turn
+            const int ns = (kNB - kPc - b) / kPc;
+            const int64_t G = std::max(1, nsm - ns), u4 = (rows + 7) / 8, u8 = (rows + 3) / 4;
+            const int64_t c4 = (u4 + 4 * G - 1) / (4 * G) * (176 + 8 * b), c8 = (u8 + 4 * G - 1) / (4 * G) * (112 + 4 * b);
+            const bool wide = c8 <= c4;
+            const unsigned grid = (unsigned)std::max<int64_t>(1, ns + std::min<int64_t>(G, wide ? u8 : u4));
+            if (wide) k_panel32<8><<<grid, 32 * kPcWarps, 0, st>>>(A, ld, k0, b, rows, diag, dErr);
+            else k_panel32<4><<<grid, 32 * kPcWarps, 0, st>>>(A, ld, k0, b, rows, diag, dErr);
         }
         return rows;
     };
@@ -191,6 +346,8 @@ int32_t dense_cholesky_device(mpgpu_ctx *c, double *A, int64_t npad, int mode, f
             k_syrk_fp64<<<(unsigned)ntile, 256, 0, s>>>(A, ld, (int64_t)p * kNB, (int64_t)(p + 1) * kNB, T);
             MPG_CUDA(c, cudaGetLastError());
         }
+        k_put_diag<<<(unsigned)(npad / kPc), 256, 0, s>>>(A, ld, diag);
+        MPG_CUDA(c, cudaGetLastError());
     } else {
         // Task lists, copied once: (1) the updates inside every block
         // column (panel p updates the tiles (i, j) of the later panels j of
@@ -288,6 +445,7 @@ int32_t dense_cholesky_device(mpgpu_ctx *c, double *A, int64_t npad, int mode, f
                 MPG_CUDA(c, tc_tile_gemm(op, op, A, ld, nullptr, T * (T + 1) / 2, e2, e - s0, -1.0, 1.0, dErr, R.sb));
             MPG_CUDA(c, cudaEventRecord(evBulk, R.sb));
         }
+        k_put_diag<<<(unsigned)(npad / kPc), 256, 0, R.sp>>>(A, ld, diag);
         MPG_CUDA(c, cudaGetLastError());
         MPG_CUDA(c, cudaEventRecord(evEnd, R.sb));
         MPG_CUDA(c, cudaStreamWaitEvent(s, evEnd, 0));

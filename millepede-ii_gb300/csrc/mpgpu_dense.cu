@@ -1,8 +1,9 @@
 // mpgpu_dense.cu -- blocked dense Cholesky of the global matrix (the dense
 // solve of `method cholesky`, pede.f90:7951-8054 / chdec2 mpnum.f90:891-987,
 // re-blocked for the GPU) in two forms:
-//   mode 0: FP64 throughout (panel, triangular solve, trailing update on the
-//           FP64 CUDA cores);
+//   mode 0: FP64 throughout: panel and triangular solve on the FP64 units,
+//           trailing update in FP64 by exact slices on the tensor cores
+//           (mpgpu_ozaki.cu);
 //   mode 1: FP64 panel factorisation and triangular solve; the trailing
 //           update A22 -= L21 L21^T, which carries the N^3/3 work, on the
 //           tcgen05 tensor cores in 3xTF32 (x = hi + lo, products
@@ -19,6 +20,7 @@
 #include <vector>
 
 #include "mpgpu_ctx.h"
+#include "mpgpu_ozaki.h"
 #include "mpgpu_tc.cuh"
 
 namespace {
@@ -250,45 +252,6 @@ __global__ void __launch_bounds__(256) k_put_diag(double *A, int64_t ld, const d
     }
 }
 
-// ------------------------------------------------ FP64 trailing update
-// 64 x 64 tiles (bi >= bj), 256 threads with 4 x 4 outputs each, K = 128
-// in chunks of 16 from the FP64 panel.
-__global__ void __launch_bounds__(256) k_syrk_fp64(double *A, int64_t ld, int64_t k0, int64_t r0, int32_t T) {
-    __shared__ double sa[16][64 + 1], sb[16][64 + 1];
-    const int64_t t = blockIdx.x;
-    int bi = (int)((sqrt(8.0 * (double)t + 1.0) - 1.0) * 0.5);
-    while ((int64_t)bi * (bi + 1) / 2 > t) bi--;
-    while ((int64_t)(bi + 1) * (bi + 2) / 2 <= t) bi++;
-    const int bj = (int)(t - (int64_t)bi * (bi + 1) / 2);
-    if (bi >= T) return;
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int64_t i0 = r0 + (int64_t)bi * 64, j0 = r0 + (int64_t)bj * 64;
-    double acc[4][4] = {};
-    for (int kc = 0; kc < kNB; kc += 16) {
-        for (int e = tid; e < 64 * 16; e += 256) {
-            const int r = e >> 4, k = e & 15;
-            sa[k][r] = A[(i0 + r) * ld + k0 + kc + k];
-            sb[k][r] = A[(j0 + r) * ld + k0 + kc + k];
-        }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < 16; ++k) {
-            double a[4], b[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) { a[q] = sa[k][ty * 4 + q]; b[q] = sb[k][tx * 4 + q]; }
-#pragma unroll
-            for (int p = 0; p < 4; ++p)
-#pragma unroll
-                for (int q = 0; q < 4; ++q) acc[p][q] = fma(a[p], b[q], acc[p][q]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int p = 0; p < 4; ++p)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) A[(i0 + ty * 4 + p) * ld + j0 + tx * 4 + q] -= acc[p][q];
-}
-
 __global__ void k_pad_identity(double *A, int64_t ld, int64_t n, int64_t npad) {
     const int64_t i = n + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < npad) A[i * ld + i] = 1.0;
@@ -299,8 +262,7 @@ __global__ void k_pad_identity(double *A, int64_t ld, int64_t n, int64_t npad) {
 // Factorise the dense padded matrix A (npad x npad, row-major, lower
 // triangle) in place.  Returns 0, MPGPU_ERR_FACTOR (non-positive pivot in
 // panel *badPanel) or a CUDA/timeout error.
-// mode 0: right-looking by 128-wide panels, FP64 trailing updates.
-// mode 1: block columns of kSuperPanels panels: inside a block column the
+// Block columns of kSuperPanels panels: inside a block column the
 // 128-wide panels are factorised and update the rest of the block column;
 // the trailing matrix then receives the whole block column at once, K = 512
 // accumulated in tensor memory before one FP64 read-modify-write per tile
@@ -337,18 +299,7 @@ int32_t dense_cholesky_device(mpgpu_ctx *c, double *A, int64_t npad, int mode, f
         }
         return rows;
     };
-    if (mode == 0) {
-        for (int32_t p = 0; p < np; ++p) {
-            const int64_t rows = panel(p, s);
-            if (rows <= 0) break;
-            const int32_t T = (int32_t)(rows / 64);
-            const int64_t ntile = (int64_t)T * (T + 1) / 2;
-            k_syrk_fp64<<<(unsigned)ntile, 256, 0, s>>>(A, ld, (int64_t)p * kNB, (int64_t)(p + 1) * kNB, T);
-            MPG_CUDA(c, cudaGetLastError());
-        }
-        k_put_diag<<<(unsigned)(npad / kPc), 256, 0, s>>>(A, ld, diag);
-        MPG_CUDA(c, cudaGetLastError());
-    } else {
+    {
         // Task lists, copied once: (1) the updates inside every block
         // column (panel p updates the tiles (i, j) of the later panels j of
         // its block column, i >= j); (2) per block column, the trailing
@@ -361,8 +312,9 @@ int32_t dense_cholesky_device(mpgpu_ctx *c, double *A, int64_t npad, int mode, f
             const int32_t e = std::min(s0 + kSuperPanels, np);
             for (int32_t p = s0; p < e; ++p) {
                 off[p] = (int64_t)tk.size();
+                const int32_t kp = mode == 0 ? 0 : p - s0;   // K tile of the panel in its operand
                 for (int32_t jj = p + 1; jj < e; ++jj)
-                    for (int32_t i = jj; i < np; ++i) tk.push_back({i, jj, p - s0, p - s0 + 1, i, jj});
+                    for (int32_t i = jj; i < np; ++i) tk.push_back({i, jj, kp, kp + 1, i, jj});
             }
         }
         off[np] = (int64_t)tk.size();
@@ -377,18 +329,21 @@ int32_t dense_cholesky_device(mpgpu_ctx *c, double *A, int64_t npad, int mode, f
         // panels (and the tiles the next panels need) on a high-priority
         // stream, the bulk of each trailing update on a second stream: the
         // panels of block column b + 1 run while the bulk of block column b
-        // is updated (look-ahead); the TF32 split of a block column is
+        // is updated (look-ahead); the operands of a block column are
         // double-buffered for that overlap
         struct Res {
             tc::TileTask *task = nullptr;
             float *hl[4] = {nullptr, nullptr, nullptr, nullptr};
+            uint8_t *img[3] = {nullptr, nullptr, nullptr};
+            int32_t *ex[3] = {nullptr, nullptr, nullptr};
             cudaStream_t sp = nullptr, sb = nullptr;
             cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
             cudaStream_t s0 = nullptr;   // the caller's stream (the buffers are ordered on it)
             ~Res() {
                 if (sp) cudaStreamSynchronize(sp);
                 if (sb) cudaStreamSynchronize(sb);
-                for (void *p : {(void *)task, (void *)hl[2], (void *)hl[3]})   // hl[0], hl[1] are the caller's
+                for (void *p : {(void *)task, (void *)hl[2], (void *)hl[3], (void *)img[0], (void *)img[1],
+                                (void *)img[2], (void *)ex[0], (void *)ex[1], (void *)ex[2]})   // hl[0], hl[1] are the caller's
                     if (p) cudaFreeAsync(p, s0);
                 for (cudaEvent_t e : ev)
                     if (e) cudaEventDestroy(e);
@@ -399,10 +354,23 @@ int32_t dense_cholesky_device(mpgpu_ctx *c, double *A, int64_t npad, int mode, f
         const int64_t splitLen = npad * kNB * kSuperPanels;
         R.s0 = s;
         MPG_CUDA(c, cudaMallocAsync(&R.task, sizeof(tc::TileTask) * std::max<size_t>(tk.size(), 1), s));
-        R.hl[0] = hiBuf;
-        R.hl[1] = loBuf;
-        MPG_CUDA(c, cudaMallocAsync(&R.hl[2], sizeof(float) * splitLen, s));
-        MPG_CUDA(c, cudaMallocAsync(&R.hl[3], sizeof(float) * splitLen, s));
+        // operands: mode 1 TF32 hi and lo of a block column; mode 0 the
+        // slices of a block column (one scale group, K = 512) and of one
+        // panel (K = 128) for the updates inside the block column
+        oz::Op col[2] = {}, pan{};
+        if (mode == 1) {
+            R.hl[0] = hiBuf;
+            R.hl[1] = loBuf;
+            MPG_CUDA(c, cudaMallocAsync(&R.hl[2], sizeof(float) * splitLen, s));
+            MPG_CUDA(c, cudaMallocAsync(&R.hl[3], sizeof(float) * splitLen, s));
+        } else {
+            for (int q = 0; q < 3; ++q) {
+                MPG_CUDA(c, cudaMallocAsync(&R.img[q], (size_t)(np * (q < 2 ? kSuperPanels : 1) * oz::kTileBytes), s));
+                MPG_CUDA(c, cudaMallocAsync(&R.ex[q], sizeof(int32_t) * npad, s));
+            }
+            for (int q = 0; q < 2; ++q) col[q] = oz::Op{R.img[q], R.ex[q], kSuperPanels, 1};
+            pan = oz::Op{R.img[2], R.ex[2], 1, 1};
+        }
         int lo = 0, hiPrio = 0;
         MPG_CUDA(c, cudaDeviceGetStreamPriorityRange(&lo, &hiPrio));
         MPG_CUDA(c, cudaStreamCreateWithPriority(&R.sp, cudaStreamNonBlocking, hiPrio));
@@ -423,26 +391,36 @@ int32_t dense_cholesky_device(mpgpu_ctx *c, double *A, int64_t npad, int mode, f
             const int32_t e2 = std::min(e + kSuperPanels, np);
             float *hb = R.hl[2 * (b & 1)], *lb = R.hl[2 * (b & 1) + 1];
             const tc::TcOp op{hb, lb, kSuperPanels};
+            const oz::Op &co = col[b & 1];
+            // tile products with the block column's operands (K tiles 0..e - s0)
+            auto update = [&](const tc::TileTask *tasks, int64_t n, int32_t trail0, int32_t trailK, cudaStream_t st) {
+                return mode == 1 ? tc_tile_gemm(op, op, A, ld, tasks, n, trail0, trailK, -1.0, 1.0, dErr, st)
+                                 : oz_tile_gemm(co, co, A, ld, tasks, n, trail0, trailK, 2, -1.0, 1.0, dErr, st);
+            };
             bool last = false;
             for (int32_t p = s0; p < e; ++p) {
                 const int64_t rows = panel(p, R.sp);
                 if (rows <= 0) { last = true; break; }
-                MPG_CUDA(c, tc_split_tiles(A, ld, p + 1, np, p, p + 1, hb, lb, kSuperPanels, s0, R.sp));
-                MPG_CUDA(c, tc_tile_gemm(op, op, A, ld, R.task + off[p], off[p + 1] - off[p], 0, 0, -1.0, 1.0,
-                                         dErr, R.sp));
+                const int64_t n = off[p + 1] - off[p];
+                if (mode == 1) {
+                    MPG_CUDA(c, tc_split_tiles(A, ld, p + 1, np, p, p + 1, hb, lb, kSuperPanels, s0, R.sp));
+                    MPG_CUDA(c, tc_tile_gemm(op, op, A, ld, R.task + off[p], n, 0, 0, -1.0, 1.0, dErr, R.sp));
+                } else if (p + 1 < e) {
+                    MPG_CUDA(c, oz_split(A, ld, p + 1, np, p, p + 1, 0, 0, pan, 0, p, 0, R.sp));
+                    MPG_CUDA(c, oz_tile_gemm(pan, pan, A, ld, R.task + off[p], n, 0, 0, 0, -1.0, 1.0, dErr, R.sp));
+                }
             }
             if (last) break;
             if (e >= np) break;
+            if (mode == 0) MPG_CUDA(c, oz_split(A, ld, e, np, s0, e, 0, 0, co, 0, s0, 2, R.sp));
             // the next block column's tiles, after the previous bulk update
             MPG_CUDA(c, cudaStreamWaitEvent(R.sp, evBulk, 0));
-            MPG_CUDA(c, tc_tile_gemm(op, op, A, ld, R.task + offN[b], offN[b + 1] - offN[b], 0, 0, -1.0, 1.0, dErr,
-                                     R.sp));
+            MPG_CUDA(c, update(R.task + offN[b], offN[b + 1] - offN[b], 0, 0, R.sp));
             MPG_CUDA(c, cudaEventRecord(evPanels, R.sp));
             // the bulk: tiles (i, j >= e2), on the second stream
             const int64_t T = np - e2;
             MPG_CUDA(c, cudaStreamWaitEvent(R.sb, evPanels, 0));
-            if (T > 0)
-                MPG_CUDA(c, tc_tile_gemm(op, op, A, ld, nullptr, T * (T + 1) / 2, e2, e - s0, -1.0, 1.0, dErr, R.sb));
+            if (T > 0) MPG_CUDA(c, update(nullptr, T * (T + 1) / 2, e2, e - s0, R.sb));
             MPG_CUDA(c, cudaEventRecord(evBulk, R.sb));
         }
         k_put_diag<<<(unsigned)(npad / kPc), 256, 0, R.sp>>>(A, ld, diag);

@@ -2,22 +2,28 @@
 // blocked Cholesky factor: the dense form of the inversion that gives pede
 // its parameter errors (minver, pede.f90:7838-7945, which inverts with
 // sqminl, mpnum.f90:230-355).  With A = L L^T (mpgpu_dense.cu):
-//   trtri  X = L^-1, in place, block column by block column from the last
-//          (LAPACK's blocked order): for panel p, T = X_trail P (the panel
-//          P below the diagonal block times the already inverted trailing
-//          part, lower triangular), then X_panel = -T D_p with D_p = L_pp^-1;
+//   trtri  X = L^-1, in place, from the inverses of the diagonal blocks;
 //   lauum  Z = X^T X (lower part), Z_ij = sum_{k >= i} X_ki^T X_kj.
 // Both are lists of 128 x 128 tile products C = alpha sum_k A_k B_k^T +
-// beta C run by one of two kernels: FP64 on the CUDA cores (64 x 64 per CTA,
-// the form of the FP64 trailing update) or tcgen05 3xTF32 with FP32
-// accumulation in tensor memory over the whole K range (operands split
-// once into TF32 hi/lo tiles).  Work: N^3/3 for each of trtri and lauum.
+// beta C run by one of two kernels: FP64 by exact slices on the tensor cores
+// (mpgpu_ozaki.cu) or tcgen05 3xTF32 with FP32 accumulation in tensor memory
+// over the whole K range (operands split once into TF32 hi/lo tiles).  Work:
+// N^3/3 for each of trtri and lauum.
+// trtri in FP64 doubles the inverted diagonal blocks: X_21 = -X_22 (L_21 X_11)
+// for all pairs of blocks of b tiles at once, b = 1, 2, 4, ...: twelve products
+// for 4,200 rows, the largest of 512 halves of tiles.  In 3xTF32 it goes block
+// column by block column from the last: for panel p, T = X_trail P (the panel P
+// below the diagonal block times the already inverted trailing part), then
+// X_panel = -T D_p with D_p = L_pp^-1.
+// Measured in FP64, 4,200 rows: trtri 2.8 ms, lauum 1.6 ms (together 101 ms on
+// the CUDA cores' FP64 units, trtri by panels).
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <vector>
 
 #include "mpgpu_ctx.h"
+#include "mpgpu_ozaki.h"
 #include "mpgpu_tc.cuh"
 
 namespace {
@@ -276,9 +282,10 @@ __global__ void __launch_bounds__(kTcThreads) k_tile_gemm_tc(TcOp A, TcOp B, dou
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(kNB));
 }
 
-// diagonal block p of X: D_p = L_pp^-1 from its transposed copy
+// diagonal blocks p0 + blockIdx.y of X: D_p = L_pp^-1 from its transposed copy
 // (DinvT[p][r][c] = D_p[c][r]), zero above the diagonal
-__global__ void k_set_diag_inverse(double *L, int64_t ld, int32_t p, const double *DinvT) {
+__global__ void k_set_diag_inverse(double *L, int64_t ld, int32_t p0, const double *DinvT) {
+    const int32_t p = p0 + blockIdx.y;
     const double *D = DinvT + (int64_t)p * kTileEl;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < kTileEl; e += gridDim.x * blockDim.x) {
         const int i = e / kNB, j = e % kNB;
@@ -302,20 +309,39 @@ __global__ void k_dense_lower_to_packed(const double *Z, int64_t ld, int64_t n, 
 // L (npad x npad, dense row-major, the lower Cholesky factor with the
 // inverses of its diagonal blocks in DinvT) is replaced by X = L^-1; Z =
 // X^T X (lower part) is written to Zd and its leading n x n block packed
-// into Zp.  mode 0: FP64 tile products; mode 1: tensor-core 3xTF32.
+// into Zp.  mode 0: FP64 tile products by slices; mode 1: tensor-core 3xTF32.
 int32_t dense_inverse_device(mpgpu_ctx *c, double *L, int64_t npad, int64_t n, int mode, const double *DinvT,
                              double *Zd, double *Zp, int32_t *dErr) {
     cudaStream_t s = c->stream;
     const int32_t np = (int32_t)(npad / kNB);
     const int64_t ld = npad;
-    // tasks of every trtri step (T products, then the panel scaling) and of lauum
+    // tasks of every trtri step (mode 0: T = L_21 X_11, then X_21 = -X_22 T,
+    // for every block size; mode 1: T products, then the panel scaling) and of
+    // lauum
     std::vector<TileTask> tk;
-    std::vector<int64_t> stepT(np + 1), stepS(np + 1);
-    for (int32_t p = np - 1; p >= 0; --p) {
-        stepT[p] = (int64_t)tk.size();
-        for (int32_t r = p + 1; r < np; ++r) tk.push_back({r, p, p + 1, r + 1, r - p - 1, 0});
-        stepS[p] = (int64_t)tk.size();
-        for (int32_t r = p + 1; r < np; ++r) tk.push_back({r - p - 1, 0, 0, 1, r, p});
+    std::vector<int64_t> stepT(np + 2), stepS(np + 2);
+    if (mode == 0) {
+        int lv = 0;
+        for (int32_t b = 1; b < np; b *= 2, ++lv)
+            for (int sec = 0; sec < 2; ++sec) {
+                (sec ? stepS : stepT)[lv] = (int64_t)tk.size();
+                std::vector<TileTask> t;
+                for (int32_t base = 0; base + b < np; base += 2 * b)
+                    for (int32_t i = base + b; i < std::min(base + 2 * b, np); ++i)
+                        for (int32_t j = base; j < base + b; ++j)
+                            t.push_back(sec ? TileTask{i, j, base + b, i + 1, i, j} : TileTask{i, j, j, base + b, i, j});
+                std::stable_sort(t.begin(), t.end(),
+                                 [](const TileTask &a, const TileTask &b) { return a.k1 - a.k0 > b.k1 - b.k0; });
+                tk.insert(tk.end(), t.begin(), t.end());
+            }
+        stepT[lv] = (int64_t)tk.size();
+    } else {
+        for (int32_t p = np - 1; p >= 0; --p) {
+            stepT[p] = (int64_t)tk.size();
+            for (int32_t r = p + 1; r < np; ++r) tk.push_back({r, p, p + 1, r + 1, r - p - 1, 0});
+            stepS[p] = (int64_t)tk.size();
+            for (int32_t r = p + 1; r < np; ++r) tk.push_back({r - p - 1, 0, 0, 1, r, p});
+        }
     }
     const int64_t lauum0 = (int64_t)tk.size();
     {
@@ -331,15 +357,22 @@ int32_t dense_inverse_device(mpgpu_ctx *c, double *L, int64_t npad, int64_t n, i
     double *T = nullptr;
     float *xhi = nullptr, *xlo = nullptr, *thi = nullptr, *tlo = nullptr, *phi = nullptr, *plo = nullptr,
           *dhi = nullptr, *dlo = nullptr;
+    // mode 0: slices of the two operands, W tiles of every row at a time
+    uint8_t *img[2] = {nullptr, nullptr};
+    int32_t *ex[2] = {nullptr, nullptr};
     auto release = [&] {
+        for (int q = 0; q < 2; ++q) {
+            cudaFree(img[q]);
+            cudaFree(ex[q]);
+        }
         cudaFree(dTask); cudaFree(T);
         cudaFree(xhi); cudaFree(xlo); cudaFree(thi); cudaFree(tlo); cudaFree(phi); cudaFree(plo);
         cudaFree(dhi); cudaFree(dlo);
     };
     cudaError_t e = cudaMalloc(&dTask, sizeof(TileTask) * tk.size());
-    if (e == cudaSuccess) e = cudaMalloc(&T, sizeof(double) * npad * kNB);
     const int64_t full = (int64_t)np * np * kTileEl;
     if (mode == 1) {
+        if (e == cudaSuccess) e = cudaMalloc(&T, sizeof(double) * npad * kNB);
         // X (non-transposed) and L^T, later X^T, split tile by tile; the
         // panel T and the diagonal inverse D_p split per step
         if (e == cudaSuccess) e = cudaMalloc(&xhi, sizeof(float) * full);
@@ -351,6 +384,27 @@ int32_t dense_inverse_device(mpgpu_ctx *c, double *L, int64_t npad, int64_t n, i
         if (e == cudaSuccess) e = cudaMalloc(&dhi, sizeof(float) * kTileEl);
         if (e == cudaSuccess) e = cudaMalloc(&dlo, sizeof(float) * kTileEl);
     }
+    // W: all K tiles up to 64 (C is read and written once per W tiles, 64 of
+    // them take 400 us), fewer where the memory does not suffice
+    int32_t W = std::min(64, (np + 3) / 4 * 4);
+    oz::Op oa{}, ob{};
+    if (mode == 0 && e == cudaSuccess) {
+        for (;; W = std::max(4, W / 8 * 4)) {
+            const size_t bytes = (size_t)np * W * oz::kTileBytes;
+            e = cudaMalloc(&img[0], bytes);
+            if (e == cudaSuccess) e = cudaMalloc(&img[1], bytes);
+            if (e == cudaSuccess || W == 4) break;
+            cudaGetLastError();
+            for (uint8_t *&p : img) {
+                cudaFree(p);
+                p = nullptr;
+            }
+        }
+        for (int q = 0; q < 2; ++q)
+            if (e == cudaSuccess) e = cudaMalloc(&ex[q], sizeof(int32_t) * np * (W / 4) * kNB);
+        oa = oz::Op{img[0], ex[0], W, W / 4};
+        ob = oz::Op{img[1], ex[1], W, W / 4};
+    }
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(dTask, tk.data(), sizeof(TileTask) * tk.size(), cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) { release(); return cuda_err(c, e, "blocked inverse workspace"); }
@@ -361,42 +415,68 @@ int32_t dense_inverse_device(mpgpu_ctx *c, double *L, int64_t npad, int64_t n, i
             k_split_tiles<<<np - 1 - p, 256, 0, s>>>(L, ld, p + 1, np, p, p + 1, 1, phi, plo, np, 0);
     }
     MPG_CUDA(c, cudaMemsetAsync(dErr, 0, sizeof(int32_t), s));
-    // ---- trtri, panels from the last
-    for (int32_t p = np - 1; p >= 0; --p) {
-        const int32_t m = np - 1 - p;
-        if (m > 0) {
-            if (mode == 1) {
+    // launches of mode 0 release the workspace when they fail
+#define MPG_OZ(call)                                                        \
+    do {                                                                    \
+        const cudaError_t oe_ = (call);                                     \
+        if (oe_ != cudaSuccess) {                                           \
+            release();                                                      \
+            return cuda_err(c, oe_, #call);                                 \
+        }                                                                   \
+    } while (0)
+    const int64_t nla = (int64_t)np * (np + 1) / 2;
+    if (mode == 0) {
+        // ---- trtri: T in Zd, which lauum fills afterwards
+        k_set_diag_inverse<<<dim3(16, np), 256, 0, s>>>(L, ld, 0, DinvT);
+        int lv = 0;
+        for (int32_t b = 1; b < np; b *= 2, ++lv) {
+            const int32_t pairs = (np - b + 2 * b - 1) / (2 * b);
+            for (int32_t w0 = 0; w0 < b; w0 += W) {
+                const int32_t w1 = std::min(w0 + W, b);
+                MPG_OZ(oz_split(L, ld, b, 2 * b, w0, w1, 0, 0, oa, 0, w0, 2, s, pairs, 2 * b, np));
+                MPG_OZ(oz_split(L, ld, 0, b, w0, w1, 1, 2, ob, 0, w0, 2, s, pairs, 2 * b, np));
+                MPG_OZ(oz_tile_gemm(oa, ob, Zd, ld, dTask + stepT[lv], stepS[lv] - stepT[lv], 0, 0, 2, 1.0, 0.0, dErr,
+                                    s, oz::Window{2 * b, w0, w1 - w0}));
+            }
+            for (int32_t w0 = b; w0 < 2 * b; w0 += W) {
+                const int32_t w1 = std::min(w0 + W, 2 * b);
+                MPG_OZ(oz_split(L, ld, b, 2 * b, w0, w1, 0, 1, oa, 0, w0, 2, s, pairs, 2 * b, np));
+                MPG_OZ(oz_split(Zd, ld, 0, b, w0, w1, 1, 0, ob, 0, w0, 2, s, pairs, 2 * b, np));
+                MPG_OZ(oz_tile_gemm(oa, ob, L, ld, dTask + stepS[lv], stepT[lv + 1] - stepS[lv], 0, 0, 2, -1.0, 0.0,
+                                    dErr, s, oz::Window{2 * b, w0, w1 - w0}));
+            }
+        }
+        // ---- lauum
+        for (int32_t w0 = 0; w0 < np; w0 += W) {
+            const int32_t w1 = std::min(w0 + W, np);
+            MPG_OZ(oz_split(L, ld, 0, np, w0, w1, 1, 2, oa, 0, w0, 2, s));
+            MPG_OZ(oz_tile_gemm(oa, oa, Zd, ld, dTask + lauum0, nla, 0, 0, 2, 1.0, 0.0, dErr, s,
+                                oz::Window{0, w0, w1 - w0}));
+        }
+    } else {
+        // ---- trtri, panels from the last
+        for (int32_t p = np - 1; p >= 0; --p) {
+            const int32_t m = np - 1 - p;
+            if (m > 0) {
                 k_tile_gemm_tc<<<m, kTcThreads, kTcSmem, s>>>(TcOp{xhi, xlo, np}, TcOp{phi, plo, np}, T, kNB,
                                                               dTask + stepT[p], 0, 0, 1.0, 0.0, dErr);
                 k_split_tiles<<<m, 256, 0, s>>>(T, kNB, 0, m, 0, 1, 0, thi, tlo, 1, 0);
                 k_split_tiles<<<1, 256, 0, s>>>(DinvT + (int64_t)p * kTileEl, kNB, 0, 1, 0, 1, 0, dhi, dlo, 1, 0);
                 k_tile_gemm_tc<<<m, kTcThreads, kTcSmem, s>>>(TcOp{thi, tlo, 1}, TcOp{dhi, dlo, 1}, L, ld,
                                                               dTask + stepS[p], 0, 0, -1.0, 0.0, dErr);
-            } else {
-                k_tile_gemm_fp64<<<4 * m, 256, 0, s>>>(Fp64Op{L, ld, 0}, Fp64Op{L, ld, 1}, T, kNB, dTask + stepT[p],
-                                                       1.0, 0.0);
-                k_tile_gemm_fp64<<<4 * m, 256, 0, s>>>(Fp64Op{T, kNB, 0},
-                                                       Fp64Op{DinvT + (int64_t)p * kTileEl, kNB, 0}, L, ld,
-                                                       dTask + stepS[p], -1.0, 0.0);
             }
+            k_set_diag_inverse<<<16, 256, 0, s>>>(L, ld, p, DinvT);
+            // the finished column of X, split for the later steps' products
+            k_split_tiles<<<m + 1, 256, 0, s>>>(L, ld, p, np, p, p + 1, 0, xhi, xlo, np, 0);
+            MPG_CUDA(c, cudaGetLastError());
         }
-        k_set_diag_inverse<<<16, 256, 0, s>>>(L, ld, p, DinvT);
-        // the finished column of X, split for the later steps' products
-        if (mode == 1) k_split_tiles<<<m + 1, 256, 0, s>>>(L, ld, p, np, p, p + 1, 0, xhi, xlo, np, 0);
-        MPG_CUDA(c, cudaGetLastError());
-    }
-    // ---- lauum
-    const int64_t nla = (int64_t)np * (np + 1) / 2;
-    if (mode == 1) {
-        // X^T tiles (i, k) for k >= i (into the L^T area)
+        // ---- lauum: X^T tiles (i, k) for k >= i (into the L^T area)
         for (int32_t i = 0; i < np; ++i)
             k_split_tiles<<<np - i, 256, 0, s>>>(L, ld, i, np, i, i + 1, 1, phi, plo, np, 0);
         k_tile_gemm_tc<<<(unsigned)nla, kTcThreads, kTcSmem, s>>>(TcOp{phi, plo, np}, TcOp{phi, plo, np}, Zd, ld,
                                                                   dTask + lauum0, 0, 0, 1.0, 0.0, dErr);
-    } else {
-        k_tile_gemm_fp64<<<(unsigned)(4 * nla), 256, 0, s>>>(Fp64Op{L, ld, 1}, Fp64Op{L, ld, 1}, Zd, ld,
-                                                             dTask + lauum0, 1.0, 0.0);
     }
+#undef MPG_OZ
     MPG_CUDA(c, cudaGetLastError());
     k_dense_lower_to_packed<<<4096, 256, 0, s>>>(Zd, ld, n, Zp);
     int32_t h = 0;

@@ -156,76 +156,155 @@ __global__ void k_wy_apply(int32_t n, int32_t m, const double *V, const double *
 
 // ---------------------------------------------------------------- packed products
 // y = A x for the packed symmetric matrix in two deterministic passes.
-// Pass 1, one CTA per block of 64 rows: the lower part of each row (one
-// warp per row, contiguous) and, per column j left of the block's last row,
-// the partial column sum over the block's rows (one thread per column,
-// contiguous across threads).  Pass 2 adds, per j, the row part and the
-// partial column sums of the blocks below j in block order.
+// Pass 1, one CTA per 16 rows x 1,024 columns, a thread per column: every
+// element is read once and used for its row's sum and for its column's.  Pass 2
+// adds, per j, the row parts by column range and the column parts of the blocks
+// below j, eight threads per j.
+// FP64-bound: two multiply-adds per stored element (62 us for 6,000 rows; the
+// matrix once takes 22 us).  Reading it once per row and once per column took
+// 248 + 85 us, now 99 + 15 (1,500 rows: 21 + 14 us, now 20 + 4).
 constexpr int kMvRows = 16;
+constexpr int kMvCols = 1024;
 
-__global__ void __launch_bounds__(256) k_pmv_blocks(int32_t n, const double *A, const double *x, double *yrow,
-                                                     double *part) {
-    const int64_t b = blockIdx.x;
-    const int64_t i0 = b * kMvRows, i1 = min((int64_t)n, i0 + kMvRows);
-    const int ln = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    __shared__ double xs[kMvRows];
-    if (threadIdx.x < kMvRows) xs[threadIdx.x] = i0 + threadIdx.x < n ? x[i0 + threadIdx.x] : 0.0;
-    __syncthreads();
-    for (int64_t i = i0 + wib; i < i1; i += 8) {
-        const double *row = A + i * (i + 1) / 2;
-        double s = 0.0;
-        for (int64_t j = ln; j <= i; j += 32) s += row[j] * x[j];
+// sums of v[0..15] over the warp, v[r] in lanes 2 r and 2 r + 1
+__device__ __forceinline__ double warp_sum16(double (&v)[kMvRows]) {
+    const int ln = threadIdx.x & 31;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (ln == 0) yrow[i] = s;
+    for (int h = kMvRows / 2; h > 0; h >>= 1) {
+        const bool up = ln & (2 * h);
+#pragma unroll
+        for (int r = 0; r < h; ++r) {
+            const double give = up ? v[r] : v[r + h];
+            const double keep = up ? v[r + h] : v[r];
+            v[r] = keep + __shfl_xor_sync(0xffffffffu, give, 2 * h);
+        }
     }
-    for (int64_t j = threadIdx.x; j < i1 - 1; j += blockDim.x) {
-        double s = 0.0;
-        const int64_t ifirst = j + 1 > i0 ? j + 1 : i0;
-        for (int64_t i = ifirst; i < i1; ++i) s += A[i * (i + 1) / 2 + j] * xs[i - i0];
-        part[b * (int64_t)n + j] = s;
+    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
+__global__ void __launch_bounds__(256, 3) k_pmv_blocks(int32_t n, const double *A, const double *x, double *yrow,
+                                                     double *part) {
+    __shared__ double xs[kMvRows], ws[8][kMvRows];
+    const int64_t b = gridDim.x - 1 - blockIdx.x;   // the longest rows first
+    const int64_t i0 = b * kMvRows, i1 = min((int64_t)n, i0 + kMvRows), j0 = (int64_t)blockIdx.y * kMvCols;
+    if (j0 >= i1) return;
+    const int tid = threadIdx.x, ln = tid & 31, wib = tid >> 5;
+    if (tid < kMvRows) xs[tid] = i0 + tid < n ? x[i0 + tid] : 0.0;
+    __syncthreads();
+    const int64_t j1 = min(i1, j0 + kMvCols);
+    const double *base = A + i0 * (i0 + 1) / 2;
+    double r[kMvRows] = {};
+    for (int64_t j = j0 + tid; j < j1; j += 256) {
+        const double xj = x[j];
+        double a[kMvRows], c = 0.0;
+        if (j < i0 && i1 == i0 + kMvRows) {
+#pragma unroll
+            for (int q = 0; q < kMvRows; ++q) a[q] = base[q * i0 + q * (q + 1) / 2 + j];
+#pragma unroll
+            for (int q = 0; q < kMvRows; ++q) {
+                r[q] = fma(a[q], xj, r[q]);
+                c = fma(a[q], xs[q], c);
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < kMvRows; ++q) {
+                a[q] = (i0 + q < i1 && j <= i0 + q) ? base[q * i0 + q * (q + 1) / 2 + j] : 0.0;
+                if (i0 + q < i1 && j <= i0 + q) r[q] = fma(a[q], xj, r[q]);
+                if (i0 + q < i1 && j < i0 + q) c = fma(a[q], xs[q], c);
+            }
+        }
+        if (j < i1 - 1) part[b * (int64_t)n + j] = c;
+    }
+    const double t = warp_sum16(r);
+    // lane bits 4..1 select the row: bit 4 the upper half, ...
+    if (!(ln & 1)) ws[wib][ln >> 1] = t;
+    __syncthreads();
+    if (tid < kMvRows && i0 + tid < i1) {
+        double sum = ws[0][tid];
+#pragma unroll
+        for (int w = 1; w < 8; ++w) sum += ws[w][tid];
+        yrow[blockIdx.y * (int64_t)n + i0 + tid] = sum;
     }
 }
 
-__global__ void k_pmv_final(int32_t n, int64_t nb, const double *yrow, const double *part, double *y) {
-    const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    double s = yrow[j];
-    for (int64_t b = (j + 1) / kMvRows; b < nb; ++b) {
-        const int64_t i1 = min((int64_t)n, (b + 1) * kMvRows);
-        if (j < i1 - 1) s += part[b * (int64_t)n + j];
+__global__ void __launch_bounds__(256) k_pmv_final(int32_t n, int64_t nb, const double *yrow, const double *part,
+                                                   double *y) {
+    __shared__ double ps[8][32];
+    const int ln = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int64_t j = (int64_t)blockIdx.x * 32 + ln;
+    double s = 0.0;
+    if (j < n) {
+        for (int64_t b = (j + 1) / kMvRows + wib; b < nb; b += 8) {
+            const int64_t i1 = min((int64_t)n, (b + 1) * kMvRows);
+            if (j < i1 - 1) s += part[b * (int64_t)n + j];
+        }
     }
-    y[j] = s;
+    ps[wib][ln] = s;
+    __syncthreads();
+    if (wib == 0 && j < n) {
+        double t = yrow[j];
+        // row j's CTA covers all columns of its block of rows
+        const int64_t last = min((int64_t)n, (j / kMvRows + 1) * kMvRows) - 1;
+        for (int64_t q = 1; q <= last / kMvCols; ++q) t += yrow[q * (int64_t)n + j];
+#pragma unroll
+        for (int w = 0; w < 8; ++w) t += ps[w][ln];
+        y[j] = t;
+    }
 }
 
 // qlssq update of one reflection on the packed matrix (mpqldec.f90:
 // 644-686): rows 1..kn get 2(2 v_i vtAv - Av_i) v_c for c in [1, min(ilast,i)],
 // rows ilast and below in [1, ilast] get -2 Av_c v_i, the diagonal (kn,kn)
-// its combined term and rows > kn their -2 v_c Av_i parts.
-__global__ void k_qlssq_update(int32_t n, double *A, const double *v, double vk, const double *Av,
-                               const double *vtAvp, int32_t ilast, int32_t kn) {
+// its combined term and rows > kn their -2 v_c Av_i parts.  Tiles of 16 rows x
+// 256 columns, a thread per column: the row's and the column's factors are
+// read once per tile.  FP64-bound: two multiply-adds per element (62 us for
+// 6,000 rows, reading and writing the matrix 43 us); a warp per row took 210
+// us, now 104.
+constexpr int kQlRows = 16;
+constexpr int kQlCols = 256;
+__global__ void __launch_bounds__(256, 2) k_qlssq_update(int32_t n, double *A, const double *v, double vk,
+                                                      const double *Av, const double *vtAvp, int32_t ilast,
+                                                      int32_t kn) {
+    __shared__ double fa[kQlRows], fb[kQlRows];
+    const int64_t i0 = (int64_t)(gridDim.x - 1 - blockIdx.x) * kQlRows, j0 = (int64_t)blockIdx.y * kQlCols;   // 0-based
+    const int64_t i1 = min((int64_t)n, i0 + kQlRows);
+    if (j0 >= i1) return;
     const double vtAv = *vtAvp;
-    const int ln = threadIdx.x & 31;
-    const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t i1 = 1 + w; i1 <= n; i1 += nw) {   // 1-based row
-        double *row = A + (i1 * i1 - i1) / 2 - 1;     // row[c] = A(i1, c), c 1-based
-        const double vi = (i1 <= ilast) ? v[i1 - 1] : (i1 == kn ? vk : 0.0);
-        if (i1 <= ilast) {
-            // both corrections of the reference, in its order, in one pass
-            const double f = 2.0 * vi * vtAv - Av[i1 - 1];
-            for (int64_t cc = 1 + ln; cc <= i1; cc += 32)
-                row[cc] = (row[cc] + 2.0 * (f * v[cc - 1])) - 2.0 * Av[cc - 1] * vi;
-        } else if (i1 <= kn) {
-            const double f = 2.0 * vi * vtAv - Av[i1 - 1];
-            for (int64_t cc = 1 + ln; cc <= ilast; cc += 32) row[cc] = row[cc] + 2.0 * (f * v[cc - 1]);
+    const int tid = threadIdx.x;
+    if (tid < kQlRows && i0 + tid < i1) {
+        const int64_t i = i0 + tid + 1;   // 1-based
+        const double vi = i <= ilast ? v[i - 1] : (i == kn ? vk : 0.0), av = Av[i - 1];
+        fa[tid] = i <= kn ? 2.0 * (2.0 * vi * vtAv - av) : -2.0 * av;   // times v_c
+        fb[tid] = -2.0 * vi;                                           // times Av_c, rows up to ilast
+    }
+    __syncthreads();
+    double *base = A + i0 * (i0 + 1) / 2;
+    const int64_t j1 = min(min(i1, j0 + kQlCols), (int64_t)ilast);
+    for (int64_t j = j0 + tid; j < j1; j += 256) {
+        const double vc = v[j], ac = Av[j];
+        if (j < i0 && i1 == i0 + kQlRows && i1 <= ilast) {
+            double a[kQlRows];
+#pragma unroll
+            for (int q = 0; q < kQlRows; ++q) a[q] = base[q * i0 + q * (q + 1) / 2 + j];
+#pragma unroll
+            for (int q = 0; q < kQlRows; ++q)
+                base[q * i0 + q * (q + 1) / 2 + j] = fma(fb[q], ac, fma(fa[q], vc, a[q]));
+        } else {
+            for (int q = 0; q < (int)(i1 - i0); ++q) {
+                if (j > i0 + q) continue;
+                double *p = base + q * i0 + q * (q + 1) / 2 + j;
+                double a = fma(fa[q], vc, *p);
+                if (i0 + q < ilast) a = fma(fb[q], ac, a);
+                *p = a;
+            }
         }
-        if (i1 == kn && ln == 0) row[kn] = row[kn] + 2.0 * ((2.0 * vk * vtAv - Av[kn - 1]) * vk - Av[kn - 1] * vk);
-        if (i1 > kn) {
-            const double avi = Av[i1 - 1];
-            for (int64_t cc = 1 + ln; cc <= ilast; cc += 32) row[cc] = row[cc] - 2.0 * v[cc - 1] * avi;
-            if (ln == 0) row[kn] = row[kn] - 2.0 * vk * avi;
-        }
+    }
+    // column kn: the diagonal element and the rows below it
+    if (tid < (int)(i1 - i0) && kn - 1 >= j0 && kn - 1 < j0 + kQlCols) {
+        const int64_t i = i0 + tid + 1;
+        double *p = base + tid * i0 + tid * (tid + 1) / 2 + kn - 1;
+        if (i == kn) *p = *p + 2.0 * ((2.0 * vk * vtAv - Av[kn - 1]) * vk - Av[kn - 1] * vk);
+        if (i > kn) *p = *p - 2.0 * vk * Av[i - 1];
     }
 }
 
@@ -1039,7 +1118,8 @@ struct Solver {
         dfree(pmvRow);
         dfree(pmvPart);
         pmvN = -1;
-        cudaError_t e = cudaMalloc(&pmvRow, sizeof(double) * std::max<int64_t>(n, 1));
+        const int64_t nch = ((int64_t)n + kMvCols - 1) / kMvCols;
+        cudaError_t e = cudaMalloc(&pmvRow, sizeof(double) * std::max<int64_t>(nch * n, 1));
         if (e == cudaSuccess) e = cudaMalloc(&pmvPart, sizeof(double) * std::max<int64_t>(nb * n, 1));
         if (e != cudaSuccess) {
             dfree(pmvRow);
@@ -1054,8 +1134,9 @@ struct Solver {
     void packed_matvec(int32_t n, const double *A, const double *x, double *y) {
         const int64_t nb = ((int64_t)n + kMvRows - 1) / kMvRows;
         if (alloc_pmv(n) != cudaSuccess) return;
-        k_pmv_blocks<<<(unsigned)nb, 256, 0, s>>>(n, A, x, pmvRow, pmvPart);
-        k_pmv_final<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, nb, pmvRow, pmvPart, y);
+        const dim3 grid((unsigned)nb, (unsigned)(((int64_t)n + kMvCols - 1) / kMvCols));
+        k_pmv_blocks<<<grid, 256, 0, s>>>(n, A, x, pmvRow, pmvPart);
+        k_pmv_final<<<(unsigned)((n + 31) / 32), 256, 0, s>>>(n, nb, pmvRow, pmvPart, y);
     }
 
     // block table of the sparse storage, built from the host copies
@@ -1370,7 +1451,8 @@ int32_t solve_inversion(mpgpu_ctx *c, const double *consResiduals, double *corrO
             k_vec_with_kn<<<S.grid(n), kThreads, 0, s>>>(v, ilast, vkv, kn, n, vbuf);
             S.avprd0(vbuf, Av);
             dot(vbuf, Av, n, S.part, scal, s);   // vtAv
-            k_qlssq_update<<<S.wgrid(n), kThreads, 0, s>>>(n, j.matD, v, vkv, Av, scal, ilast, kn);
+            const dim3 tiles((unsigned)((n + kQlRows - 1) / kQlRows), (unsigned)((n + kQlCols - 1) / kQlCols));
+            k_qlssq_update<<<tiles, 256, 0, s>>>(n, j.matD, v, vkv, Av, scal, ilast, kn);
         }
     };
     // tensor-core forms with up to 128 constraints: Q^T A Q is formed inside

@@ -2,8 +2,8 @@
 // tensor cores by error-free slices (the scheme of Ozaki, Ogita, Oishi & Rump
 // 2012, with the operands' rows scaled to fixed point).
 //
-// GB300's FP64 units give 2 multiply-adds per SM and clock (0.63 T/s), its
-// bf16 tensor cores some 8,000.  Every operand row is scaled by a power of two
+// GB300's FP64 units give 2 multiply-adds per SM and clock (0.58 T/s), its
+// bf16 tensor cores some 4,000.  Every operand row is scaled by a power of two
 // over a group of at most 512 K values, rounded to 56-bit fixed point and cut
 // into eight balanced 7-bit digits, which bf16 holds exactly.  The products of
 // digits i and j with i + j = d share one FP32 accumulator: at most 8 pairs x
@@ -23,9 +23,11 @@
 // that oz_split lays out in the tensor cores' core-matrix order), its
 // accumulators fill the 512 columns of tensor memory.  Bounds: operand reads
 // of the 64-column instructions (6 KB of shared memory each), then the
-// epilogue's FP64 (4 instructions per element and group) and 70 KB per chunk
-// from L2.  Measured: X^T X of 33 x 33 triangular tiles
-// (561 tiles, 12 K tiles on average) 1.50 ms, 54 clocks per instruction.
+// epilogue (some 100 integer instructions per element and group) and 70 KB per chunk
+// from L2.  Measured: X^T X of 33 x 33 triangular tiles (561 tiles, 12 K tiles
+// on average) 1.31 ms, two thirds of it the instructions (54 clocks each), one
+// fifth the epilogue; with C read and written once per group and the integers
+// converted by FP64 instructions 1.50 ms.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -49,7 +51,8 @@ constexpr int kImagesB = kImages - 1;                // B needs no scaled digit 
 constexpr int kStageBytes = kChunkBytes + kImagesB * (kSliceBytes / 2);
 constexpr int kStages = 3;
 constexpr int kSmem = kStages * kStageBytes + 128;
-constexpr int kThreads = 192;                        // 4 epilogue warps, producer, MMA issuer
+constexpr int kEpi = 8;                              // epilogue warps
+constexpr int kThreads = 32 * (kEpi + 2);            // and producer, MMA issuer
 constexpr int kNanEx = 1 << 28;                      // row with an infinity or NaN
 
 // K-major core matrices of 8 rows x 16 bytes: 128 bytes apart along K, 256
@@ -105,13 +108,29 @@ __device__ __forceinline__ void tmem_ld4x8(uint32_t t, uint32_t (&r)[4][8]) {
         : "memory");
 }
 
-// t 2^e
-__device__ __forceinline__ double scale2(double t, int e) {
-    const long long b = __double_as_longlong(t);
-    const int f = (int)((b >> 52) & 0x7ff);
-    if (f == 0) return scalbn(t, e);   // zero (or subnormal)
-    if (f + e > 0 && f + e < 2047) return __longlong_as_double(b + ((long long)e << 52));
-    return scalbn(t, e);
+// (hi 2^28 + lo) 2^e rounded to nearest, |hi| and |lo| below 2^46.  In integers,
+// as the two conversions and the product took three FP64 instructions (64
+// clocks of a quarter of the SM each).
+__device__ __forceinline__ double combine(long long hi, long long lo, int e) {
+    long long h = hi + (lo >> 28);
+    uint32_t l = (uint32_t)lo & 0xfffffffu;
+    const long long sign = h & (long long)0x8000000000000000ull;
+    if (h < 0) {   // the magnitude
+        h = l ? ~h : -h;
+        l = (0u - l) & 0xfffffffu;
+    }
+    const unsigned long long u = (unsigned long long)h;
+    if (u == 0) return scalbn(sign ? -(double)l : (double)l, e);
+    const int z = __clzll((long long)u);   // 17..63
+    const unsigned long long ll = (unsigned long long)l << 36;
+    const unsigned long long w = (u << z) | (ll >> (64 - z));
+    const unsigned long long rest = ll << z;
+    unsigned long long m = w >> 11;   // 53 bits
+    const uint32_t low = (uint32_t)w & 0x7ffu;
+    m += (low > 0x400u || (low == 0x400u && ((m & 1) || rest != 0))) ? 1 : 0;
+    const int f = 1023 + 91 - z + e;   // exponent field of 2^63 2^(28 - z) 2^e
+    if (f > 0 && f < 2046) return __longlong_as_double(sign | (long long)(((unsigned long long)(f - 1) << 52) + m));
+    return scalbn(__longlong_as_double(sign | (long long)((1022ull << 52) + m)), f - 1023);
 }
 
 __global__ void __launch_bounds__(kThreads, 1) k_oz_gemm(Op A, Op B, double *C, int64_t ldc, const tc::TileTask *tasks,
@@ -149,7 +168,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz_gemm(Op A, Op B, double *C, 
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(tc::smem_u32(&empty[st])));
         }
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(tc::smem_u32(&accFull)));
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 128;\n" ::"r"(tc::smem_u32(&accEmpty)));
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(tc::smem_u32(&accEmpty)), "n"(32 * kEpi));
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -161,7 +180,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz_gemm(Op A, Op B, double *C, 
     // waits that run out leave *err = -1; every role then leaves its loop, and
     // the copies and MMAs already issued are waited for (bounded) below
     int issued = 0;   // producer: chunks whose copies were issued; MMA warp: chunks committed
-    if (wib == 4) {
+    if (wib == kEpi) {
         if (ln == 0) {
             int c = 0;
             for (int k = t.k0; k < t.k1 && ok; ++k) {
@@ -189,7 +208,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz_gemm(Op A, Op B, double *C, 
             for (int d = issued > kStages ? issued - kStages : 0; d < issued; ++d)
                 if (!tc::mbar_wait(tc::smem_u32(&full[d % kStages]), (d / kStages) & 1)) ok = false;
         }
-    } else if (wib == 5) {
+    } else if (wib == kEpi + 1) {
         if (ln == 0) {
             int c = 0, grp = 0;
             for (int k = t.k0; k < t.k1 && ok; ++k) {
@@ -245,26 +264,35 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz_gemm(Op A, Op B, double *C, 
                 if (!tc::mbar_wait(tc::smem_u32(&empty[d % kStages]), (d / kStages) & 1)) ok = false;
         }
     } else {
-        const int64_t row = (int64_t)t.cRow * kNB + wib * 32 + ln;
-        double *cp = C + row * ldc + (int64_t)t.cCol * kNB + half * kN;
+        // warps w and w + 4 take 32 columns each of the rows of tensor memory
+        // that they can read; C stays in registers over the groups
+        constexpr int kC = kN / (kEpi / 4);
+        const int rw = (wib & 3) * 32, c0 = (wib >> 2) * kC;
+        const int64_t row = (int64_t)t.cRow * kNB + rw + ln;
+        double *cp = C + row * ldc + (int64_t)t.cCol * kNB + half * kN + c0;
+        double c[kC];
+        const bool add = began || beta != 0.0;
+#pragma unroll
+        for (int q = 0; q < kC; q += 2) {
+            const double2 v = add ? *reinterpret_cast<const double2 *>(cp + q) : make_double2(0.0, 0.0);
+            c[q] = v.x;
+            c[q + 1] = v.y;
+        }
         int grp = 0;
         for (int k = t.k0; k < t.k1; ++k) {
             if (!(k == t.k1 - 1 || (k >> gs) != ((k + 1) >> gs))) continue;
             const int64_t g = k >> gs;
-            const int er = A.ex[((int64_t)t.aRow * A.ng + g) * kNB + wib * 32 + ln];
-            const int32_t *ecp = B.ex + ((int64_t)t.bRow * B.ng + g) * kNB + half * kN;
+            const int er = A.ex[((int64_t)t.aRow * A.ng + g) * kNB + rw + ln];
+            const int el = B.ex[((int64_t)t.bRow * B.ng + g) * kNB + half * kN + c0 + ln];   // lane = column
             if (!tc::mbar_wait(tc::smem_u32(&accFull), grp & 1)) {
                 ok = false;
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             __syncwarp();
-            const bool add = grp > 0 || began || beta != 0.0;
-            for (int cb = 0; cb < kN / 8; ++cb) {
-                double c[8];
 #pragma unroll
-                for (int q = 0; q < 8; ++q) c[q] = add ? cp[cb * 8 + q] : 0.0;
-                const uint32_t tc0 = tmem + ((uint32_t)(wib * 32) << 16) + (uint32_t)(cb * 8);
+            for (int cb = 0; cb < kC / 8; ++cb) {
+                const uint32_t tc0 = tmem + ((uint32_t)rw << 16) + (uint32_t)(c0 + cb * 8);
                 uint32_t vh[4][8], vl[4][8];
                 tmem_ld4x8(tc0, vh);
                 tmem_ld4x8(tc0 + 4 * kN, vl);
@@ -276,22 +304,19 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz_gemm(Op A, Op B, double *C, 
                         hi = (hi << 7) + (long long)__float2int_rn(__uint_as_float(vh[d][q]));
                         lo = (lo << 7) + (long long)__float2int_rn(__uint_as_float(vl[d][q]));
                     }
-                    // both below 2^46: exact doubles by the shifted-mantissa form
-                    const double M = 6755399441055744.0;   // 1.5 x 2^52
-                    const double dh = __longlong_as_double(0x4338000000000000ll + hi) - M;
-                    const double dl = __longlong_as_double(0x4338000000000000ll + lo) - M;
-                    const int ec = __ldg(ecp + cb * 8 + q);
-                    double x = scale2(fma(dh, 268435456.0, dl), er + ec - 61);
+                    const int ec = __shfl_sync(0xffffffffu, el, cb * 8 + q);
+                    double x = combine(hi, lo, er + ec - 61);
                     if (er == kNanEx || ec == kNanEx) x = __longlong_as_double(0x7ff8000000000000ll);
-                    c[q] = fma(alpha, x, c[q]);
+                    c[cb * 8 + q] += alpha < 0.0 ? -x : x;
                 }
-#pragma unroll
-                for (int q = 0; q < 8; ++q) cp[cb * 8 + q] = c[q];
             }
             asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
             asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(tc::smem_u32(&accEmpty)) : "memory");
             ++grp;
         }
+        if (ok)
+#pragma unroll
+            for (int q = 0; q < kC; q += 2) *reinterpret_cast<double2 *>(cp + q) = make_double2(c[q], c[q + 1]);
     }
     if (!ok) atomicExch(err, -1);
     __syncwarp();

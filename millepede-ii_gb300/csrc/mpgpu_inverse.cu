@@ -121,42 +121,73 @@ using tc::TcOp;
 // the tiles of M^T: tile (c, r) of the destination receives tile (r, c) of
 // M transposed) split into TF32 hi + lo; the destination's tile column is
 // the source's column less cOff (rows keep their index).
-__global__ void k_split_tiles(const double *M, int64_t ld, int32_t r0, int32_t r1, int32_t c0, int32_t c1,
-                              int32_t trans, float *hi, float *lo, int64_t ntDst, int32_t cOff) {
-    const int64_t nc = c1 - c0;
-    const int32_t tr = r0 + (int32_t)(blockIdx.x / nc), tcc = c0 + (int32_t)(blockIdx.x % nc);
+// A warp takes eight rows x 16 K: reads 128 bytes of each row (trans: 64 bytes
+// of 16 rows), writes 512 contiguous bytes.  Four CTAs per tile: a CTA per tile
+// with one element per thread at a time took 39 us for 156 tiles, now 24 (FP64
+// conversions and the remainder: three instructions of 64 clocks per 32
+// elements, 13 us).
+constexpr int kSplitParts = 4;
+__device__ __forceinline__ double widen(float f) {   // (double)f without the FP64 pipe
+    const uint32_t b = __float_as_uint(f), e = (b >> 23) & 255u;
+    if (e - 1u < 254u)
+        return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + (896u << 20))), (int)(b << 29));
+    return (double)f;
+}
+__global__ void __launch_bounds__(256) k_split_tiles(const double *M, int64_t ld, int32_t r0, int32_t r1, int32_t c0,
+                                                     int32_t c1, int32_t trans, float *hi, float *lo, int64_t ntDst,
+                                                     int32_t cOff) {
+    const int64_t nc = c1 - c0, tile = blockIdx.x / kSplitParts;
+    const int32_t tr = r0 + (int32_t)(tile / nc), tcc = c0 + (int32_t)(tile % nc);
     if (tr >= r1) return;
     const int64_t dst = trans ? ((int64_t)tcc * ntDst + tr) * kTileEl
                               : ((int64_t)tr * ntDst + (tcc - cOff)) * kTileEl;
-    for (int e = threadIdx.x; e < kTileEl; e += blockDim.x) {
-        // destination element (u, v) contiguous; source element (u, v) or (v, u)
-        const int u = e / kNB, v = e % kNB;
-        const int64_t src = trans ? ((int64_t)tr * kNB + v) * ld + (int64_t)tcc * kNB + u
-                                  : ((int64_t)tr * kNB + u) * ld + (int64_t)tcc * kNB + v;
-        const double x = M[src];
-        uint32_t h, l;
-        asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"((float)x));
-        const double rest = x - (double)__uint_as_float(h);
-        asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(l) : "f"((float)rest));
-        hi[dst + e] = __uint_as_float(h);
-        lo[dst + e] = __uint_as_float(l);
+    const int ln = threadIdx.x & 31, wib = threadIdx.x >> 5, r7 = ln & 7, k4 = ln >> 3;
+    constexpr int kItems = 128 / kSplitParts;   // 8 chunks x 16 row groups
+    const int part = (int)(blockIdx.x % kSplitParts) * kItems;
+#pragma unroll
+    for (int i = 0; i < kItems / 8; ++i) {
+        const int it = part + i * 8 + wib, u = (it & 15) * 8 + r7, k = (it >> 4) * kTK + k4 * 4;
+        double x[4];
+        if (!trans) {
+            const double2 *p = reinterpret_cast<const double2 *>(M + ((int64_t)tr * kNB + u) * ld + (int64_t)tcc * kNB + k);
+            const double2 v = p[0], w = p[1];
+            x[0] = v.x; x[1] = v.y; x[2] = w.x; x[3] = w.y;
+        } else {
+            const double *p = M + ((int64_t)tr * kNB + k) * ld + (int64_t)tcc * kNB + u;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) x[q] = p[q * ld];
+        }
+        uint32_t h[4], l[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h[q]) : "f"((float)x[q]));
+            const double rest = x[q] - widen(__uint_as_float(h[q]));
+            asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(l[q]) : "f"((float)rest));
+        }
+        const int64_t o = dst + (it >> 4) * (kNB * kTK) + ((it & 15) * 4 + k4) * 32 + r7 * 4;
+        *reinterpret_cast<uint4 *>(hi + o) = make_uint4(h[0], h[1], h[2], h[3]);
+        *reinterpret_cast<uint4 *>(lo + o) = make_uint4(l[0], l[1], l[2], l[3]);
     }
 }
 
 // One CTA per task: the K range of the task streamed chunk by chunk (16
-// columns of one K tile per chunk) through the 3-stage pipeline, hi*hi +
-// hi*lo + lo*hi accumulated in one FP32 tensor-memory accumulator over all
-// chunks, then C = alpha acc + beta C in FP64 (coalesced through shared
-// memory).  Bounded mbarrier waits: a wait that runs out sets *err = -1
-// and the CTA finishes without writing C.  Without a task list the CTAs
-// take the lower triangle of tiles from tile (trail0, trail0) on, each
-// with K tiles [0, trailK) of rows i and j: the trailing update of a
-// block column.
-__global__ void __launch_bounds__(kTcThreads) k_tile_gemm_tc(TcOp A, TcOp B, double *C, int64_t ldc,
-                                                             const TileTask *tasks, int32_t trail0, int32_t trailK,
-                                                             double alpha, double beta, int32_t *err) {
+// columns of one K tile per chunk) through three stages by a producer thread,
+// hi*hi + hi*lo + lo*hi accumulated in one FP32 tensor-memory accumulator over
+// all chunks, then C = alpha acc + beta C in FP64 (coalesced through shared
+// memory; alpha +-1, beta 0 or 1).  Bounded mbarrier waits: a wait that runs out
+// sets *err = -1 and the CTA finishes without writing C.  Without a task list
+// the CTAs take the lower triangle of tiles from tile (trail0, trail0) on, each
+// with K tiles [0, trailK) of rows i and j: the trailing update of a block
+// column.  Two CTAs per SM, so that one's epilogue (one FP64 addition per
+// element, 8,200 clocks) runs beside the other's products (6 instructions of 64
+// clocks per chunk); 32 KB per chunk from L2.  With the copies issued by all
+// threads and three FP64 instructions per element a trailing update of 11,175
+// tiles with K = 512 took 5.0 ms, now 2.2 (beside the panels).
+__global__ void __launch_bounds__(kTcThreads, 2) k_tile_gemm_tc(TcOp A, TcOp B, double *C, int64_t ldc,
+                                                                const TileTask *tasks, int32_t trail0, int32_t trailK,
+                                                                double alpha, double beta, int32_t *err) {
     extern __shared__ __align__(128) char tsm[];
-    __shared__ uint64_t mbar[kStages];
+    __shared__ uint64_t full[kStages], empty[kStages], done;
     __shared__ uint32_t tbase;
     const int tid = threadIdx.x, wib = tid >> 5, ln = tid & 31;
     TileTask t;
@@ -173,111 +204,114 @@ __global__ void __launch_bounds__(kTcThreads) k_tile_gemm_tc(TcOp A, TcOp B, dou
     const int per = kNB / kTK;   // chunks per K tile
     const int nch = (t.k1 - t.k0) * per;
     if (nch <= 0) return;
-    const uint32_t sbase = tc::smem_u32(tsm);
-    float *epi = reinterpret_cast<float *>(tsm) + wib * 32 * 33;   // after the last MMA only
+    const uint32_t sbase = (tc::smem_u32(tsm) + 127u) & ~127u;
     if (wib == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(tc::smem_u32(&tbase)),
                      "r"(kNB));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
     }
     if (tid == 0) {
-        for (int st = 0; st < kStages; ++st)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(tc::smem_u32(&mbar[st])));
+        for (int st = 0; st < kStages; ++st) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(tc::smem_u32(&full[st])));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(tc::smem_u32(&empty[st])));
+        }
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(tc::smem_u32(&done)));
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t tmem = tbase;
-    auto load = [&](int c, int st) {
-        const int64_t k = t.k0 + c / per;
-        const int kc0 = (c % per) * kTK;
-        const int64_t ta = ((int64_t)t.aRow * A.nt + k) * kTileEl, tb = ((int64_t)t.bRow * B.nt + k) * kTileEl;
-        const uint32_t s0 = sbase + st * kStageBytes;
-        tc::load_chunk_async(A.hi + ta, kc0, s0);
-        tc::load_chunk_async(A.lo + ta, kc0, s0 + kOpBytes);
-        tc::load_chunk_async(B.hi + tb, kc0, s0 + 2 * kOpBytes);
-        tc::load_chunk_async(B.lo + tb, kc0, s0 + 3 * kOpBytes);
-    };
-    uint32_t ph = 0;   // bit st: parity of the next completion of stage st's barrier
     bool ok = true;
-    for (int c = 0; c < kStages - 1; ++c) {
-        if (c < nch) load(c, c);
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-    }
-    for (int c = 0; c < nch; ++c) {
-        const int st = c % kStages;
-        asm volatile("cp.async.wait_group %0;\n" ::"n"(kStages - 2) : "memory");
-        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-        __syncthreads();
-        if (tid == 0) {
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            const uint32_t sb = sbase + st * kStageBytes;
+    int issued = 0;   // producer: chunks whose copies were issued; MMA warp: chunks committed
+    if (wib == 4) {
+        if (ln == 0) {
+            for (int c = 0; c < nch; ++c) {
+                const int st = c % kStages;
+                if (c >= kStages && !tc::mbar_wait(tc::smem_u32(&empty[st]), ((c / kStages) - 1) & 1)) {
+                    ok = false;
+                    break;
+                }
+                const int64_t k = t.k0 + c / per, in = (int64_t)(c % per) * (kNB * kTK);
+                const int64_t ta = ((int64_t)t.aRow * A.nt + k) * kTileEl + in;
+                const int64_t tb = ((int64_t)t.bRow * B.nt + k) * kTileEl + in;
+                const uint32_t bar = tc::smem_u32(&full[st]), s0 = sbase + st * kStageBytes;
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(kStageBytes)
+                             : "memory");
+                tc::bulk_load(s0, A.hi + ta, kOpBytes, bar);
+                tc::bulk_load(s0 + kOpBytes, A.lo + ta, kOpBytes, bar);
+                tc::bulk_load(s0 + 2 * kOpBytes, B.hi + tb, kOpBytes, bar);
+                tc::bulk_load(s0 + 3 * kOpBytes, B.lo + tb, kOpBytes, bar);
+                issued = c + 1;
+            }
+            // the last chunks' copies have landed (also after a failed wait)
+            for (int d = issued > kStages ? issued - kStages : 0; d < issued; ++d)
+                if (!tc::mbar_wait(tc::smem_u32(&full[d % kStages]), (d / kStages) & 1)) ok = false;
+        }
+    } else if (wib == 5) {
+        if (ln == 0) {
+            for (int c = 0; c < nch; ++c) {
+                const int st = c % kStages;
+                if (!tc::mbar_wait(tc::smem_u32(&full[st]), (c / kStages) & 1)) {
+                    ok = false;
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                const uint32_t sb = sbase + st * kStageBytes;
 #pragma unroll
-            for (int kk = 0; kk < kTK / 8; ++kk) {
-                const uint32_t off = kk * 256;   // 8 tf32 = 2 core matrices along K
-                const uint64_t dah = tc::umma_desc(sb + off), dal = tc::umma_desc(sb + kOpBytes + off);
-                const uint64_t dbh = tc::umma_desc(sb + 2 * kOpBytes + off), dbl = tc::umma_desc(sb + 3 * kOpBytes + off);
-                tc::mma_tf32(tmem, dah, dbh, (c > 0 || kk > 0) ? 1u : 0u);
-                tc::mma_tf32(tmem, dah, dbl, 1u);
-                tc::mma_tf32(tmem, dal, dbh, 1u);
+                for (int kk = 0; kk < kTK / 8; ++kk) {
+                    const uint32_t off = kk * 256;   // 8 tf32 = 2 core matrices along K
+                    const uint64_t dah = tc::umma_desc(sb + off), dal = tc::umma_desc(sb + kOpBytes + off);
+                    const uint64_t dbh = tc::umma_desc(sb + 2 * kOpBytes + off), dbl = tc::umma_desc(sb + 3 * kOpBytes + off);
+                    tc::mma_tf32(tmem, dah, dbh, (c > 0 || kk > 0) ? 1u : 0u);
+                    tc::mma_tf32(tmem, dah, dbl, 1u);
+                    tc::mma_tf32(tmem, dal, dbh, 1u);
+                }
+                tc::commit_to(tc::smem_u32(&empty[st]));
+                issued = c + 1;
             }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                             tc::smem_u32(&mbar[st]))
-                         : "memory");
-        }
-        // the stage of chunk c + kStages - 1 held chunk c - 1: wait for its MMAs
-        const int cn = c + kStages - 1;
-        if (cn < nch) {
-            const int sn = cn % kStages;
-            if (c >= 1) {
-                if (!tc::mbar_wait(tc::smem_u32(&mbar[sn]), (ph >> sn) & 1)) ok = false;
-                ph ^= 1u << sn;
-            }
-            if (ok) load(cn, sn);
-        }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-        if (!__syncthreads_and(ok)) { ok = false; break; }
-    }
-    // the MMAs of the chunks not yet waited for (the last kStages - 1)
-    if (ok) {
-        for (int c = (nch > kStages - 1 ? nch - (kStages - 1) : 0); c < nch; ++c) {
-            const int st = c % kStages;
-            if (!tc::mbar_wait(tc::smem_u32(&mbar[st]), (ph >> st) & 1)) ok = false;
-            ph ^= 1u << st;
+            if (ok) tc::commit_to(tc::smem_u32(&done));
+            // the MMAs issued are done (also after a failed wait)
+            for (int d = issued > kStages ? issued - kStages : 0; d < issued; ++d)
+                if (!tc::mbar_wait(tc::smem_u32(&empty[d % kStages]), (d / kStages) & 1)) ok = false;
         }
     } else {
-        for (int st = 0; st < kStages; ++st) tc::mbar_wait(tc::smem_u32(&mbar[st]), (ph >> st) & 1);
-    }
-    asm volatile("cp.async.wait_all;\n" ::: "memory");
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    if (__syncthreads_and(ok)) {
-        const int64_t rowBase = (int64_t)t.cRow * kNB + wib * 32;
-        const int64_t colBase = (int64_t)t.cCol * kNB;
-        for (int cb = 0; cb < kNB / 32; ++cb) {
-            uint32_t v[32];
-            tc::tmem_ld32(tmem + ((uint32_t)(wib * 32) << 16) + (uint32_t)(cb * 32), v);
+        if (!tc::mbar_wait(tc::smem_u32(&done), 0)) ok = false;
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        ok = __all_sync(0xffffffffu, ok);
+        if (ok) {
+            // all MMAs are done, so that the stages are free
+            float *epi = reinterpret_cast<float *>(tsm + (sbase - tc::smem_u32(tsm))) + wib * 32 * 33;
+            const int64_t rowBase = (int64_t)t.cRow * kNB + wib * 32;
+            const int64_t colBase = (int64_t)t.cCol * kNB;
+            const uint32_t flip = alpha < 0.0 ? 0x80000000u : 0u;
+            for (int cb = 0; cb < kNB / 32; ++cb) {
+                double *cp = C + rowBase * ldc + colBase + cb * 32 + ln;
+                uint32_t v[32];
+                tc::tmem_ld32(tmem + ((uint32_t)(wib * 32) << 16) + (uint32_t)(cb * 32), v);
 #pragma unroll
-            for (int q = 0; q < 32; ++q) epi[ln * 33 + q] = __uint_as_float(v[q]);
-            __syncwarp();
-            double *cp = C + rowBase * ldc + colBase + cb * 32 + ln;
-            if (beta != 0.0) {
-                double cv[32];
+                for (int q = 0; q < 32; ++q) epi[ln * 33 + q] = __uint_as_float(v[q] ^ flip);
+                __syncwarp();
+#pragma unroll 1
+                for (int r0 = 0; r0 < 32; r0 += 16) {
+                    double cv[16];
 #pragma unroll
-                for (int r = 0; r < 32; ++r) cv[r] = cp[r * ldc];
+                    for (int r = 0; r < 16; ++r) cv[r] = beta != 0.0 ? cp[(r0 + r) * ldc] : 0.0;
 #pragma unroll
-                for (int r = 0; r < 32; ++r) cp[r * ldc] = alpha * (double)epi[r * 33 + ln] + beta * cv[r];
-            } else {
-#pragma unroll
-                for (int r = 0; r < 32; ++r) cp[r * ldc] = alpha * (double)epi[r * 33 + ln];
+                    for (int r = 0; r < 16; ++r) {
+                        const double x = widen(epi[(r0 + r) * 33 + ln]);
+                        cp[(r0 + r) * ldc] = beta != 0.0 ? cv[r] + x : x;
+                    }
+                }
+                __syncwarp();
             }
-            __syncwarp();
         }
-    } else if (tid == 0) {
-        atomicExch(err, -1);
     }
+    if (!ok) atomicExch(err, -1);
+    __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     if (wib == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(kNB));
 }
@@ -412,7 +446,7 @@ int32_t dense_inverse_device(mpgpu_ctx *c, double *L, int64_t npad, int64_t n, i
         MPG_CUDA(c, smem_optin((const void *)k_tile_gemm_tc));
         // L^T tiles (p, k) for k > p: the panels of the original factor
         for (int32_t p = 0; p < np - 1; ++p)
-            k_split_tiles<<<np - 1 - p, 256, 0, s>>>(L, ld, p + 1, np, p, p + 1, 1, phi, plo, np, 0);
+            k_split_tiles<<<kSplitParts * (np - 1 - p), 256, 0, s>>>(L, ld, p + 1, np, p, p + 1, 1, phi, plo, np, 0);
     }
     MPG_CUDA(c, cudaMemsetAsync(dErr, 0, sizeof(int32_t), s));
     // launches of mode 0 release the workspace when they fail
@@ -460,19 +494,19 @@ int32_t dense_inverse_device(mpgpu_ctx *c, double *L, int64_t npad, int64_t n, i
             if (m > 0) {
                 k_tile_gemm_tc<<<m, kTcThreads, kTcSmem, s>>>(TcOp{xhi, xlo, np}, TcOp{phi, plo, np}, T, kNB,
                                                               dTask + stepT[p], 0, 0, 1.0, 0.0, dErr);
-                k_split_tiles<<<m, 256, 0, s>>>(T, kNB, 0, m, 0, 1, 0, thi, tlo, 1, 0);
-                k_split_tiles<<<1, 256, 0, s>>>(DinvT + (int64_t)p * kTileEl, kNB, 0, 1, 0, 1, 0, dhi, dlo, 1, 0);
+                k_split_tiles<<<kSplitParts * m, 256, 0, s>>>(T, kNB, 0, m, 0, 1, 0, thi, tlo, 1, 0);
+                k_split_tiles<<<kSplitParts, 256, 0, s>>>(DinvT + (int64_t)p * kTileEl, kNB, 0, 1, 0, 1, 0, dhi, dlo, 1, 0);
                 k_tile_gemm_tc<<<m, kTcThreads, kTcSmem, s>>>(TcOp{thi, tlo, 1}, TcOp{dhi, dlo, 1}, L, ld,
                                                               dTask + stepS[p], 0, 0, -1.0, 0.0, dErr);
             }
             k_set_diag_inverse<<<16, 256, 0, s>>>(L, ld, p, DinvT);
             // the finished column of X, split for the later steps' products
-            k_split_tiles<<<m + 1, 256, 0, s>>>(L, ld, p, np, p, p + 1, 0, xhi, xlo, np, 0);
+            k_split_tiles<<<kSplitParts * (m + 1), 256, 0, s>>>(L, ld, p, np, p, p + 1, 0, xhi, xlo, np, 0);
             MPG_CUDA(c, cudaGetLastError());
         }
         // ---- lauum: X^T tiles (i, k) for k >= i (into the L^T area)
         for (int32_t i = 0; i < np; ++i)
-            k_split_tiles<<<np - i, 256, 0, s>>>(L, ld, i, np, i, i + 1, 1, phi, plo, np, 0);
+            k_split_tiles<<<kSplitParts * (np - i), 256, 0, s>>>(L, ld, i, np, i, i + 1, 1, phi, plo, np, 0);
         k_tile_gemm_tc<<<(unsigned)nla, kTcThreads, kTcSmem, s>>>(TcOp{phi, plo, np}, TcOp{phi, plo, np}, Zd, ld,
                                                                   dTask + lauum0, 0, 0, 1.0, 0.0, dErr);
     }
@@ -493,7 +527,7 @@ cudaError_t tc_split_tiles(const double *M, int64_t ld, int32_t r0, int32_t r1, 
                            float *lo, int64_t ntDst, int32_t cOff, cudaStream_t s) {
     const int64_t n = (int64_t)(r1 - r0) * (c1 - c0);
     if (n <= 0) return cudaSuccess;
-    k_split_tiles<<<(unsigned)n, 256, 0, s>>>(M, ld, r0, r1, c0, c1, 0, hi, lo, ntDst, cOff);
+    k_split_tiles<<<(unsigned)(kSplitParts * n), 256, 0, s>>>(M, ld, r0, r1, c0, c1, 0, hi, lo, ntDst, cOff);
     return cudaGetLastError();
 }
 

@@ -81,15 +81,8 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem, uint64_t ad, uint64_t bd
 #undef MPG_MMA
 }
 
-__device__ __forceinline__ void commit_to(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
-}
-
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst),
-                 "l"(src), "r"(bytes), "r"(bar)
-                 : "memory");
-}
+using tc::bulk_load;
+using tc::commit_to;
 
 // eight columns of four accumulators, kN columns apart, and the wait for them
 __device__ __forceinline__ void tmem_ld4x8(uint32_t t, uint32_t (&r)[4][8]) {

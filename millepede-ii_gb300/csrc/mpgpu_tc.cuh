@@ -1,9 +1,9 @@
 // mpgpu_tc.cuh -- building blocks of the tcgen05 3xTF32 tile products
 // (dense Cholesky trailing update, mpgpu_dense.cu; blocked inverse,
 // mpgpu_inverse.cu): 128 x 128 FP32 accumulators in tensor memory, operand
-// chunks of 128 rows x 16 K staged in shared memory by cp.async in the
-// K-major no-swizzle core-matrix layout, one elected thread issuing the
-// MMAs, and mbarrier waits with an iteration limit.
+// chunks of 128 rows x 16 K laid out in the K-major no-swizzle core-matrix
+// order and staged in shared memory by bulk copies, one elected thread issuing
+// the MMAs, and mbarrier waits with an iteration limit.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -18,25 +18,26 @@ struct TileTask {
 };
 
 // Tile-major TF32 operands: tile (r, c) of an array with nt tiles per row at
-// ((r * nt + c) << 14) floats, row-major inside the tile.
+// ((r * nt + c) << 14) floats, inside the tile by chunks of 16 K in the layout
+// of the chunk in shared memory.
 struct TcOp {
     const float *hi, *lo;
     int64_t nt;
 };
 
-// Operands stream in chunks of K = 16 through a 3-stage cp.async pipeline;
-// one thread issues the tcgen05.mma of a chunk (hi*hi, hi*lo, lo*hi for two
-// K = 8 steps) and commits them to the stage's mbarrier, which frees the
-// stage for the chunk three ahead.  Shared-memory operand layout: K-major,
-// no swizzle, core matrices of 8 rows x 16 bytes; core (row group g, k
-// group c) at (g * 4 + c) * 128 bytes: leading (K) byte offset 128, stride
-// (row) byte offset 512.
+// Operands stream in chunks of K = 16 through three stages, filled by bulk
+// copies of 8 KB; one thread issues the tcgen05.mma of a chunk (hi*hi, hi*lo,
+// lo*hi for two K = 8 steps) and commits them to the stage's mbarrier, which
+// frees the stage for the chunk three ahead.  Operand layout: K-major, no
+// swizzle, core matrices of 8 rows x 16 bytes; core (row group g, k group c) at
+// (g * 4 + c) * 128 bytes: leading (K) byte offset 128, stride (row) byte
+// offset 512.
 constexpr int kTK = 16;                          // K per chunk
 constexpr int kStages = 3;
 constexpr int kOpBytes = kNB * kTK * 4;          // 8 KB per operand chunk
 constexpr int kStageBytes = 4 * kOpBytes;        // hi/lo of both operands
-constexpr int kTcSmem = kStages * kStageBytes;  // the epilogue transposes reuse stage 0
-constexpr int kTcThreads = 128;
+constexpr int kTcSmem = kStages * kStageBytes + 128;   // the epilogue transposes reuse stage 0
+constexpr int kTcThreads = 192;                  // 4 epilogue warps, producer, MMA issuer
 constexpr int kWaitLimit = 1 << 22;
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
@@ -84,23 +85,19 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 }
 
-// asynchronous copy of a 128 x 16 fp32 chunk (rows of 128 in global) into
-// the core-matrix layout; 4 x 16-byte copies per thread
-__device__ __forceinline__ void load_chunk_async(const float *g, int kc0, uint32_t s) {
-#pragma unroll
-    for (int i = 0; i < kNB * (kTK / 4) / kTcThreads; ++i) {
-        const int idx = threadIdx.x + i * kTcThreads;
-        const int row = idx >> 2, k4 = idx & 3;
-        const float *src = g + (int64_t)row * kNB + kc0 + k4 * 4;
-        const uint32_t dst = s + ((row >> 3) * 4 + k4) * 128 + (row & 7) * 16;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
-    }
+__device__ __forceinline__ void commit_to(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
 }
 
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
 
 }  // namespace tc
 
-// tile products and operand splits (mpgpu_inverse.cu)
+// tile products and operand splits (mpgpu_inverse.cu); alpha +-1, beta 0 or 1
 cudaError_t tc_split_tiles(const double *M, int64_t ld, int32_t r0, int32_t r1, int32_t c0, int32_t c1, float *hi,
                            float *lo, int64_t ntDst, int32_t cOff, cudaStream_t s);
 cudaError_t tc_tile_gemm(const tc::TcOp &A, const tc::TcOp &B, double *C, int64_t ldc, const tc::TileTask *tasks,

@@ -529,27 +529,33 @@ __global__ void k_copy_lower_shift(const double *F, double *Lo, int64_t npad, do
 }
 
 // inverses of the 128 x 128 diagonal blocks of L, stored transposed:
-// DinvT[p][r][*] = column r of L_pp^-1 (one CTA per block, one warp per r)
+// DinvT[p][r][*] = column r of L_pp^-1.  Four CTAs per block, one warp per r in
+// turn, from row r on (the column is zero above).  FP64-bound; one CTA per block
+// and all rows took 490 us for 47 blocks, now 130.
+constexpr int kTriParts = 4;
 __global__ void __launch_bounds__(256) k_trtri_blocks(const double *A, int64_t ld, double *DinvT) {
-    extern __shared__ __align__(16) double lt[];   // lt[j * 128 + c] = L_pp[c][j], then 1 / diagonal
-    double *dinv = lt + kNB * kNB;
-    const int64_t k0 = (int64_t)blockIdx.x * kNB;
+    extern __shared__ __align__(16) double lt[];   // lt[j * kLt + c] = L_pp[c][j], then 1 / diagonal
+    constexpr int kLt = kNB + 1;
+    double *dinv = lt + kNB * kLt;
+    const int64_t p = blockIdx.x / kTriParts, k0 = p * kNB;
     const int tid = threadIdx.x, ln = tid & 31, wib = tid >> 5;
-    for (int e = tid; e < kNB * kNB; e += blockDim.x) {
+#pragma unroll 8
+    for (int e = tid; e < kNB * kNB; e += 256) {
         const int c = e / kNB, j = e % kNB;
-        lt[j * kNB + c] = j <= c ? A[(k0 + c) * ld + k0 + j] : 0.0;
+        lt[j * kLt + c] = j <= c ? A[(k0 + c) * ld + k0 + j] : 0.0;
     }
     __syncthreads();
-    for (int j = tid; j < kNB; j += blockDim.x) dinv[j] = 1.0 / lt[j * kNB + j];
+    for (int j = tid; j < kNB; j += blockDim.x) dinv[j] = 1.0 / lt[j * kLt + j];
     __syncthreads();
-    double *out = DinvT + (int64_t)blockIdx.x * kNB * kNB;
-    for (int r = wib; r < kNB; r += blockDim.x >> 5) {
+    double *out = DinvT + p * kNB * kNB;
+    for (int r = (int)(blockIdx.x % kTriParts) + kTriParts * wib; r < kNB; r += kTriParts * 8) {
         double a[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) a[q] = (q * 32 + ln == r) ? 1.0 : 0.0;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            for (int l = 0; l < 32; ++l) {
+            if (q < r / 32) continue;
+            for (int l = q == r / 32 ? r % 32 : 0; l < 32; ++l) {
                 const int j = q * 32 + l;
                 const double xj = __shfl_sync(0xffffffffu, a[q], l) * dinv[j];
                 if (ln == l) a[q] = xj;
@@ -557,7 +563,7 @@ __global__ void __launch_bounds__(256) k_trtri_blocks(const double *A, int64_t l
                 for (int q2 = 0; q2 < 4; ++q2) {
                     if (q2 < q) continue;
                     const int c = q2 * 32 + ln;
-                    if (c > j) a[q2] -= xj * lt[j * kNB + c];
+                    if (c > j) a[q2] -= xj * lt[j * kLt + c];
                 }
             }
         }
@@ -666,53 +672,95 @@ __global__ void k_sb_transpose(const double *XS, int64_t npad, double *XT) {
 }
 
 // out[row0 + r] = sum_c X[row0 + r][c] in[row0 + c] over c <= r (lower) or
-// c >= r, c < size; a warp per row, lanes over c, tree sum over the lanes
-__global__ void k_sb_diag(const double *X, int64_t row0, int size, const double *in, double *out, int lower) {
+// c >= r, c < size; a warp per row, lanes over c, tree sum over the lanes.
+// Latency-bound: all loads of a row are issued at once (in a loop 9.7 us per
+// block, now 4.9).
+__global__ void __launch_bounds__(256) k_sb_diag(const double *X, int64_t row0, int size, const double *in, double *out,
+                                                 int lower) {
     const int ln = threadIdx.x & 31;
     const int r = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     if (r >= size) return;
     const double *xr = X + (row0 + r) * kSB;
     const int c0 = lower ? 0 : r, c1 = lower ? r + 1 : size;
-    double sum = 0.0;
-    for (int c = c0 + ln; c < c1; c += 32) sum += xr[c] * in[row0 + c];
+    constexpr int kQ = kSB / 32;
+    double x[kQ], v[kQ];
+#pragma unroll
+    for (int q = 0; q < kQ; ++q) {
+        const int c = ln + 32 * q;
+        const bool on = c >= c0 && c < c1;
+        x[q] = on ? xr[c] : 0.0;
+        v[q] = on ? in[row0 + c] : 0.0;
+    }
+    double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+    for (int q = 0; q < kQ; q += 2) {
+        s0 = fma(x[q], v[q], s0);
+        s1 = fma(x[q + 1], v[q + 1], s1);
+    }
+    double sum = s0 + s1;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
     if (ln == 0) out[row0 + r] = sum;
 }
 
-// v_R -= L[R][row0 .. row0 + size) z_b for the rows R >= row0 + size (warp per row)
-__global__ void k_sb_fwd_upd(const double *L, int64_t ld, int64_t row0, int size, int64_t npad, const double *z,
-                             double *v) {
+// v_R -= L[R][row0 .. row0 + kSB) z_b for the rows R >= row0 + kSB (there are
+// none below a shorter block), two rows per warp with all their loads issued at
+// once.  FP64-bound (512 multiply-adds per row, 8.8 us for 10,000 rows); with a
+// row per warp and a loop of dependent loads 19.5 us, now 14.8.  (Four rows per
+// warp leave too few warps for a few thousand rows.)
+__global__ void __launch_bounds__(256) k_sb_fwd_upd(const double *L, int64_t ld, int64_t row0, int64_t npad,
+                                                    const double *z, double *v) {
     const int ln = threadIdx.x & 31;
-    const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t R = row0 + size + w; R < npad; R += nw) {
-        const double *row = L + R * ld + row0;
-        double sum = 0.0;
-        for (int c = ln; c < size; c += 32) sum += row[c] * z[row0 + c];
+    const int64_t R = row0 + kSB + 2 * (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    if (R >= npad) return;   // (npad is even)
+    constexpr int kQ = kSB / 32;
+    const double *r0 = L + R * ld + row0 + ln, *r1 = r0 + ld;
+    double a[kQ], b[kQ], s0 = 0.0, s1 = 0.0;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        if (ln == 0) v[R] -= sum;
+    for (int q = 0; q < kQ; ++q) {
+        a[q] = r0[32 * q];
+        b[q] = r1[32 * q];
     }
+#pragma unroll
+    for (int q = 0; q < kQ; ++q) {
+        const double zq = z[row0 + ln + 32 * q];
+        s0 = fma(a[q], zq, s0);
+        s1 = fma(b[q], zq, s1);
+    }
+    const bool up = ln & 16;
+    double sum = (up ? s1 : s0) + __shfl_xor_sync(0xffffffffu, up ? s0 : s1, 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if ((ln & 15) == 0) v[R + (up ? 1 : 0)] -= sum;
 }
 
-// z_c -= sum_m L[row0 + m][c] o[row0 + m] for the columns c < row0: 64
-// columns per CTA, the m range in four quarters summed in order
+// z_c -= sum_m L[row0 + m][c] o[row0 + m] for the columns c < row0: 32
+// columns per CTA, the m range in eight parts summed in order.  FP64-bound as
+// the forward update; with 64 columns in four parts too few loads were in
+// flight: 28.9 us for 10,000 columns, now 15.5.
 __global__ void __launch_bounds__(256) k_sb_bwd_upd(const double *L, int64_t ld, int64_t row0, int size,
                                                     const double *o, double *z) {
-    __shared__ double part[4][64];
-    const int cl = threadIdx.x & 63, g = threadIdx.x >> 6;
-    const int64_t c = (int64_t)blockIdx.x * 64 + cl;
-    const int q = (size + 3) / 4, m0 = g * q, m1 = min(size, m0 + q);
-    double sum = 0.0;
-    if (c < row0) {
-        const double *col = L + row0 * ld + c;
-#pragma unroll 8
-        for (int m = m0; m < m1; ++m) sum += col[(int64_t)m * ld] * o[row0 + m];
-    }
-    part[g][cl] = sum;
+    __shared__ double part[8][32], os[kSB];
+    const int cl = threadIdx.x & 31, g = threadIdx.x >> 5;
+    for (int m = threadIdx.x; m < size; m += 256) os[m] = o[row0 + m];
     __syncthreads();
-    if (g == 0 && c < row0) z[c] -= ((part[0][cl] + part[1][cl]) + part[2][cl]) + part[3][cl];
+    const int64_t c = (int64_t)blockIdx.x * 32 + cl;   // row0 is a multiple of 32
+    const int q = size / 8, m0 = g * q;                // size is a multiple of 128
+    const double *col = L + (row0 + m0) * ld + c;
+    double s0 = 0.0, s1 = 0.0;
+#pragma unroll 8
+    for (int m = 0; m < q; m += 2) {
+        s0 = fma(col[(int64_t)m * ld], os[m0 + m], s0);
+        s1 = fma(col[(int64_t)(m + 1) * ld], os[m0 + m + 1], s1);
+    }
+    part[g][cl] = s0 + s1;
+    __syncthreads();
+    if (g == 0) {
+        double sum = part[0][cl];
+#pragma unroll
+        for (int w = 1; w < 8; ++w) sum += part[w][cl];
+        z[c] -= sum;
+    }
 }
 
 struct DenseWork {
@@ -733,40 +781,73 @@ struct DenseWork {
     }
 };
 
-// X_b for every super-block from L and the 128-row inverse blocks:
-// X_jj = L_jj^-1, and for i = j + d (d = 1, 2, 3) T = sum_{k=j}^{i-1} L_ik X_kj,
-// X_ij = -L_ii^-1 T (one wave of tile products per d over all super-blocks)
+// X_b for every super-block from L and the 128-row inverse blocks, doubling the
+// inverted blocks: X_21 = -X_22 (L_21 X_11) for blocks of one and then of two
+// tiles, exact tile products on the tensor cores (on the FP64 units, which 16
+// tile products per super-block keep busy, 1.3 ms for 6,000 rows, now 0.3).
 cudaError_t build_super_inverse(DenseWork &w, cudaStream_t s) {
-    const int64_t np = w.np, nsb = (np + 3) / 4;
+    const int32_t np = (int32_t)w.np;
     cudaError_t e = cudaMemsetAsync(w.XS, 0, sizeof(double) * w.npad * kSB, s);
     if (e != cudaSuccess) return e;
-    k_sb_set_diag<<<(unsigned)std::min<int64_t>(np * 64, 4096), 256, 0, s>>>(w.DinvT, np, w.XS);
+    k_sb_set_diag<<<(unsigned)std::min<int64_t>((int64_t)np * 64, 4096), 256, 0, s>>>(w.DinvT, np, w.XS);
     std::vector<tc::TileTask> tk;
-    std::vector<int64_t> wave(7, 0);
-    for (int d = 1; d <= 3; ++d) {
-        wave[2 * d - 2] = (int64_t)tk.size();
-        for (int64_t b = 0; b < nsb; ++b) {
-            const int32_t t0 = (int32_t)(4 * b), npb = (int32_t)std::min<int64_t>(4, np - 4 * b);
-            for (int32_t j = 0; j + d < npb; ++j) tk.push_back({t0 + j + d, j, t0 + j, t0 + j + d, t0 + j + d, j});
-        }
-        wave[2 * d - 1] = (int64_t)tk.size();
-        for (int64_t b = 0; b < nsb; ++b) {
-            const int32_t t0 = (int32_t)(4 * b), npb = (int32_t)std::min<int64_t>(4, np - 4 * b);
-            for (int32_t j = 0; j + d < npb; ++j) tk.push_back({0, j, t0 + j + d, t0 + j + d + 1, t0 + j + d, j});
+    int64_t first[5] = {0};
+    for (int lv = 0; lv < 2; ++lv) {
+        const int32_t b = 1 << lv;
+        for (int sec = 0; sec < 2; ++sec) {
+            for (int32_t base = 0; base + b < np; base += 2 * b)
+                for (int32_t i = base + b; i < std::min(base + 2 * b, np); ++i)
+                    for (int32_t j = base; j < base + b; ++j)
+                        tk.push_back(sec ? tc::TileTask{i, j, base + b, i + 1, i, j % 4}
+                                         : tc::TileTask{i, j, j, base + b, i, j % 4});
+            first[2 * lv + sec + 1] = (int64_t)tk.size();
         }
     }
-    wave[6] = (int64_t)tk.size();
     if (!tk.empty()) {
-        e = cudaMemcpyAsync(w.sbTask, tk.data(), sizeof(tc::TileTask) * tk.size(), cudaMemcpyHostToDevice, s);
-        if (e != cudaSuccess) return e;
-        for (int d = 1; d <= 3 && e == cudaSuccess; ++d) {
-            const int64_t a0 = wave[2 * d - 2], a1 = wave[2 * d - 1], a2 = wave[2 * d];
-            e = fp64_tile_gemm(w.L, w.npad, 0, w.XS, kSB, 1, w.XW, kSB, w.sbTask + a0, a1 - a0, 1.0, 0.0, s);
-            if (e == cudaSuccess)
-                e = fp64_tile_gemm(w.DinvT, kNB, 1, w.XW, kSB, 1, w.XS, kSB, w.sbTask + a1, a2 - a1, -1.0, 0.0, s);
+        struct Images {   // sliced operands, two tiles of every row
+            cudaStream_t s;
+            uint8_t *img[2] = {nullptr, nullptr};
+            int32_t *ex[2] = {nullptr, nullptr};
+            ~Images() {
+                for (int q = 0; q < 2; ++q) {
+                    if (img[q]) cudaFreeAsync(img[q], s);
+                    if (ex[q]) cudaFreeAsync(ex[q], s);
+                }
+            }
+        } I{s};
+        for (int q = 0; q < 2 && e == cudaSuccess; ++q) {
+            e = cudaMallocAsync(&I.img[q], (size_t)np * 2 * oz::kTileBytes, s);
+            if (e == cudaSuccess) e = cudaMallocAsync(&I.ex[q], sizeof(int32_t) * np * kNB, s);
+        }
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(w.sbTask, tk.data(), sizeof(tc::TileTask) * tk.size(), cudaMemcpyHostToDevice, s);
+        const oz::Op oa{I.img[0], I.ex[0], 2, 1}, ob{I.img[1], I.ex[1], 2, 1};
+        for (int lv = 0; lv < 2 && e == cudaSuccess; ++lv) {
+            const int32_t b = 1 << lv, pairs = (np - b + 2 * b - 1) / (2 * b);
+            if (pairs <= 0) break;
+            auto split = [&](const double *M, int64_t ld, int32_t r0, int32_t k0, int trans, int tri, const oz::Op &dst,
+                             int32_t wrap) {
+                if (e == cudaSuccess)
+                    e = oz_split(M, ld, r0, r0 + b, k0, k0 + b, trans, tri, dst, 0, k0, 1, s, pairs, 2 * b, np, wrap);
+            };
+            auto product = [&](double *C, int sec, double alpha) {
+                const int64_t t0 = first[2 * lv + sec], t1 = first[2 * lv + sec + 1];
+                if (e == cudaSuccess)
+                    e = oz_tile_gemm(oa, ob, C, kSB, w.sbTask + t0, t1 - t0, 0, 0, 1, alpha, 0.0, w.err, s,
+                                     oz::Window{2 * b, sec * b, b});
+            };
+            split(w.L, w.npad, b, 0, 0, 0, oa, 0);
+            split(w.XS, kSB, 0, 0, 1, 2, ob, 4);
+            product(w.XW, 0, 1.0);
+            split(w.XS, kSB, b, b, 0, 1, oa, 4);
+            split(w.XW, kSB, 0, b, 1, 0, ob, 4);
+            product(w.XS, 1, -1.0);
         }
         // the host task list must live until the copy has run
+        int32_t h = 0;
+        if (e == cudaSuccess) e = cudaMemcpyAsync(&h, w.err, sizeof(int32_t), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (e == cudaSuccess && h < 0) e = cudaErrorLaunchTimeout;   // a wait of a tile product ran out
     }
     if (e != cudaSuccess) return e;
     k_sb_transpose<<<(unsigned)std::min<int64_t>((w.npad * kSB + 255) / 256, 8192), 256, 0, s>>>(w.XS, w.npad, w.XT);
@@ -784,14 +865,13 @@ void precond(const DenseWork &w, const double *in, double *out, cudaStream_t s) 
         k_sb_diag<<<(unsigned)((size + 7) / 8), 256, 0, s>>>(w.XS, row0, size, v, zz, 1);
         const int64_t rows = w.npad - row0 - size;
         if (rows > 0)
-            k_sb_fwd_upd<<<(unsigned)std::min<int64_t>((rows + 7) / 8, 1216), 256, 0, s>>>(w.L, w.npad, row0, size,
-                                                                                           w.npad, zz, v);
+            k_sb_fwd_upd<<<(unsigned)((rows + 15) / 16), 256, 0, s>>>(w.L, w.npad, row0, w.npad, zz, v);
     }
     for (int64_t b = nsb - 1; b >= 0; --b) {
         const int64_t row0 = b * kSB;
         const int size = (int)std::min<int64_t>(kSB, w.npad - row0);
         k_sb_diag<<<(unsigned)((size + 7) / 8), 256, 0, s>>>(w.XT, row0, size, zz, out, 0);
-        if (row0 > 0) k_sb_bwd_upd<<<(unsigned)((row0 + 63) / 64), 256, 0, s>>>(w.L, w.npad, row0, size, out, zz);
+        if (row0 > 0) k_sb_bwd_upd<<<(unsigned)(row0 / 32), 256, 0, s>>>(w.L, w.npad, row0, size, out, zz);
     }
 }
 
@@ -1177,9 +1257,9 @@ int32_t dense_solve_pcg(mpgpu_ctx *c, int32_t n, const double *Ap, double *bx, i
             shift = shift == 0.0 ? 1e-7 : shift * 10.0;
         }
         if (r != MPGPU_OK) return r;
-        const int trtriSmem = (kNB * kNB + kNB) * (int)sizeof(double);
+        const int trtriSmem = (kNB * (kNB + 1) + kNB) * (int)sizeof(double);
         MPG_CUDA(c, smem_optin((const void *)k_trtri_blocks));
-        k_trtri_blocks<<<(unsigned)w.np, 256, trtriSmem, s>>>(w.L, w.npad, w.DinvT);
+        k_trtri_blocks<<<(unsigned)(kTriParts * w.np), 256, trtriSmem, s>>>(w.L, w.npad, w.DinvT);
         MPG_CUDA(c, build_super_inverse(w, s));
         MPG_CUDA(c, cudaGetLastError());
         D->factorValid = true;
@@ -1271,7 +1351,7 @@ int32_t dense_solve_pcg(mpgpu_ctx *c, int32_t n, const double *Ap, double *bx, i
     cudaEventRecord(eR, s);
     int32_t rcInv = MPGPU_OK;
     if (invOut && istop != 9) {
-        rcInv = dense_inverse_device(c, w.L, w.npad, nfit, mode, w.DinvT, w.F, invOut, w.err);
+        rcInv = dense_inverse_device(c, w.L, w.npad, nfit, mode, w.DinvT, w.XS, w.F, invOut, w.err);
         // the inverse overwrites L and F
         D->factorValid = false;
     }

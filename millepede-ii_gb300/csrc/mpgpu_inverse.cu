@@ -10,8 +10,9 @@
 // over the whole K range (operands split once into TF32 hi/lo tiles).  Work:
 // N^3/3 for each of trtri and lauum.
 // trtri in FP64 doubles the inverted diagonal blocks: X_21 = -X_22 (L_21 X_11)
-// for all pairs of blocks of b tiles at once, b = 1, 2, 4, ...: twelve products
-// for 4,200 rows, the largest of 512 halves of tiles.  In 3xTF32 it goes block
+// for all pairs of blocks of b tiles at once, b = 4, 8, ... (blocks of four tiles
+// come from the factorisation's super-blocks): eight products for 4,200 rows,
+// the largest of 512 halves of tiles.  In 3xTF32 it goes block
 // column by block column from the last: for panel p, T = X_trail P (the panel P
 // below the diagonal block times the already inverted trailing part), then
 // X_panel = -T D_p with D_p = L_pp^-1.
@@ -39,81 +40,6 @@ constexpr int64_t kTileEl = (int64_t)kNB * kNB;
 
 using tc::TileTask;
 
-// ------------------------------------------------------------ FP64 form
-// An operand tile (row, k) of a dense row-major FP64 matrix M, or of M^T
-// (trans: element (m, kk) of the tile is M[k*128 + kk][row*128 + m]).
-struct Fp64Op {
-    const double *M;
-    int64_t ld;
-    int32_t trans;
-};
-
-__global__ void __launch_bounds__(256) k_tile_gemm_fp64(Fp64Op A, Fp64Op B, double *C, int64_t ldc,
-                                                        const TileTask *tasks, double alpha, double beta) {
-    __shared__ double sa[16][64 + 1], sb[16][64 + 1];
-    const TileTask t = tasks[blockIdx.x >> 2];
-    const int sub = blockIdx.x & 3, si = sub >> 1, sj = sub & 1;
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int64_t ar = (int64_t)t.aRow * kNB + si * 64, br = (int64_t)t.bRow * kNB + sj * 64;
-    double acc[4][4] = {};
-    for (int k = t.k0; k < t.k1; ++k) {
-        for (int kc = 0; kc < kNB; kc += 16) {
-            const int64_t kb = (int64_t)k * kNB + kc;
-            for (int e = tid; e < 64 * 16; e += 256) {
-                if (!A.trans) {
-                    const int r = e >> 4, kk = e & 15;
-                    sa[kk][r] = A.M[(ar + r) * A.ld + kb + kk];
-                } else {
-                    const int r = e & 63, kk = e >> 6;
-                    sa[kk][r] = A.M[(kb + kk) * A.ld + ar + r];
-                }
-                if (!B.trans) {
-                    const int r = e >> 4, kk = e & 15;
-                    sb[kk][r] = B.M[(br + r) * B.ld + kb + kk];
-                } else {
-                    const int r = e & 63, kk = e >> 6;
-                    sb[kk][r] = B.M[(kb + kk) * B.ld + br + r];
-                }
-            }
-            __syncthreads();
-#pragma unroll
-            for (int kk = 0; kk < 16; ++kk) {
-                double a[4], b[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) { a[q] = sa[kk][ty * 4 + q]; b[q] = sb[kk][tx * 4 + q]; }
-#pragma unroll
-                for (int p = 0; p < 4; ++p)
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) acc[p][q] = fma(a[p], b[q], acc[p][q]);
-            }
-            __syncthreads();
-        }
-    }
-#pragma unroll
-    for (int p = 0; p < 4; ++p)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            double *cp = C + ((int64_t)t.cRow * kNB + si * 64 + ty * 4 + p) * ldc + (int64_t)t.cCol * kNB + sj * 64 +
-                         tx * 4 + q;
-            *cp = beta != 0.0 ? alpha * acc[p][q] + beta * *cp : alpha * acc[p][q];
-        }
-}
-
-}  // namespace
-
-// FP64 tile products C(cRow, cCol) = alpha sum_k op(A)(aRow, k) op(B)(k, bRow)
-// + beta C over a device task list (op: trans 0 takes tile (r, k) of A or
-// (bRow, k) of B transposed, trans 1 the tile as stored)
-cudaError_t fp64_tile_gemm(const double *A, int64_t lda, int32_t ta, const double *B, int64_t ldb, int32_t tb,
-                           double *C, int64_t ldc, const tc::TileTask *tasks, int64_t ntask, double alpha,
-                           double beta, cudaStream_t s) {
-    if (ntask <= 0) return cudaSuccess;
-    k_tile_gemm_fp64<<<(unsigned)(ntask * 4), 256, 0, s>>>(Fp64Op{A, lda, ta}, Fp64Op{B, ldb, tb}, C, ldc, tasks,
-                                                            alpha, beta);
-    return cudaGetLastError();
-}
-
-namespace {
 // ------------------------------------------------------------ tensor-core form
 using tc::TcOp;
 
@@ -316,14 +242,24 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_tile_gemm_tc(TcOp A, TcOp B, 
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(kNB));
 }
 
-// diagonal blocks p0 + blockIdx.y of X: D_p = L_pp^-1 from its transposed copy
+// diagonal block p of X: D_p = L_pp^-1 from its transposed copy
 // (DinvT[p][r][c] = D_p[c][r]), zero above the diagonal
-__global__ void k_set_diag_inverse(double *L, int64_t ld, int32_t p0, const double *DinvT) {
-    const int32_t p = p0 + blockIdx.y;
+__global__ void k_set_diag_inverse(double *L, int64_t ld, int32_t p, const double *DinvT) {
     const double *D = DinvT + (int64_t)p * kTileEl;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < kTileEl; e += gridDim.x * blockDim.x) {
         const int i = e / kNB, j = e % kNB;
         L[((int64_t)p * kNB + i) * ld + (int64_t)p * kNB + j] = j <= i ? D[(int64_t)j * kNB + i] : 0.0;
+    }
+}
+
+// the inverted blocks of four tiles (XS: rows of 4 kNB columns, zero above the
+// diagonal) to the tiles on and below the diagonal; eight rows per CTA
+__global__ void __launch_bounds__(256) k_set_super_inverse(double *L, int64_t ld, const double *XS) {
+    const int64_t r0 = (int64_t)blockIdx.x * 8, c0 = r0 / (4 * kNB) * (4 * kNB);
+    const int cols = (int)((r0 / kNB + 1) * kNB - c0);
+    for (int e = threadIdx.x; e < 8 * cols; e += 256) {
+        const int64_t r = r0 + e / cols;
+        L[r * ld + c0 + e % cols] = XS[r * 4 * kNB + e % cols];
     }
 }
 
@@ -341,11 +277,12 @@ __global__ void k_dense_lower_to_packed(const double *Z, int64_t ld, int64_t n, 
 }  // namespace
 
 // L (npad x npad, dense row-major, the lower Cholesky factor with the
-// inverses of its diagonal blocks in DinvT) is replaced by X = L^-1; Z =
+// inverses of its diagonal blocks in DinvT and of its blocks of four tiles in
+// XS) is replaced by X = L^-1; Z =
 // X^T X (lower part) is written to Zd and its leading n x n block packed
 // into Zp.  mode 0: FP64 tile products by slices; mode 1: tensor-core 3xTF32.
 int32_t dense_inverse_device(mpgpu_ctx *c, double *L, int64_t npad, int64_t n, int mode, const double *DinvT,
-                             double *Zd, double *Zp, int32_t *dErr) {
+                             const double *XS, double *Zd, double *Zp, int32_t *dErr) {
     cudaStream_t s = c->stream;
     const int32_t np = (int32_t)(npad / kNB);
     const int64_t ld = npad;
@@ -356,7 +293,7 @@ int32_t dense_inverse_device(mpgpu_ctx *c, double *L, int64_t npad, int64_t n, i
     std::vector<int64_t> stepT(np + 2), stepS(np + 2);
     if (mode == 0) {
         int lv = 0;
-        for (int32_t b = 1; b < np; b *= 2, ++lv)
+        for (int32_t b = 4; b < np; b *= 2, ++lv)
             for (int sec = 0; sec < 2; ++sec) {
                 (sec ? stepS : stepT)[lv] = (int64_t)tk.size();
                 std::vector<TileTask> t;
@@ -461,9 +398,9 @@ int32_t dense_inverse_device(mpgpu_ctx *c, double *L, int64_t npad, int64_t n, i
     const int64_t nla = (int64_t)np * (np + 1) / 2;
     if (mode == 0) {
         // ---- trtri: T in Zd, which lauum fills afterwards
-        k_set_diag_inverse<<<dim3(16, np), 256, 0, s>>>(L, ld, 0, DinvT);
+        k_set_super_inverse<<<(unsigned)np * 16, 256, 0, s>>>(L, ld, XS);
         int lv = 0;
-        for (int32_t b = 1; b < np; b *= 2, ++lv) {
+        for (int32_t b = 4; b < np; b *= 2, ++lv) {
             const int32_t pairs = (np - b + 2 * b - 1) / (2 * b);
             for (int32_t w0 = 0; w0 < b; w0 += W) {
                 const int32_t w1 = std::min(w0 + W, b);

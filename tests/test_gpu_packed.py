@@ -69,3 +69,23 @@ def test_packed(mp, orc, n, metsol, deficient):
     if metsol == 1:
         diag = A[np.cumsum(np.arange(1, n + 1)) - 1]
         assert np.max(np.abs(err - diag)) <= 1e-10 * np.max(np.abs(diag))
+
+
+def test_inversion_above_one_row_per_thread(mp):
+    """More rows than the threads of the largest cluster, against numpy:
+    eigenvalues between 1 and 7, within 10 n cond(A) u."""
+    n = 4200
+    M, b = matrix(n, 4, 0)
+    with context(mp, n, M, b) as ctx:
+        p = ctx.matrix()
+        g = np.zeros(n)
+        ctx.check(ctx.L.mpgpu_download_vector(ctx.h, mp.ptr(g, mp.f64p), None))
+        x, err, info = ctx.solve(1, errors=True)
+    A = np.zeros((n, n))
+    A[np.tril_indices(n)] = p
+    A = A + np.tril(A, -1).T
+    inv = np.linalg.inv(A)
+    tol = 10 * n * 7 * 2.0 ** -53
+    assert info.nrank == n
+    assert np.max(np.abs(x - inv @ g)) <= tol * np.max(np.abs(inv @ g))
+    assert np.max(np.abs(err - np.diag(inv))) <= tol * np.max(np.diag(inv))

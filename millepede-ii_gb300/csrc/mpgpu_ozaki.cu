@@ -25,9 +25,10 @@
 // of the 64-column instructions (6 KB of shared memory each), then the
 // epilogue (some 100 integer instructions per element and group) and 70 KB per chunk
 // from L2.  Measured: X^T X of 33 x 33 triangular tiles (561 tiles, 12 K tiles
-// on average) 1.31 ms, two thirds of it the instructions (54 clocks each), one
-// fifth the epilogue; with C read and written once per group and the integers
-// converted by FP64 instructions 1.50 ms.
+// on average) 1.20 ms, three quarters of it the instructions (54 clocks each),
+// one seventh the epilogue (with eight warps for it 1.31 ms; with C read and
+// written once per group and the integers converted by FP64 instructions, by
+// four warps, 1.50 ms).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -51,7 +52,7 @@ constexpr int kImagesB = kImages - 1;                // B needs no scaled digit 
 constexpr int kStageBytes = kChunkBytes + kImagesB * (kSliceBytes / 2);
 constexpr int kStages = 3;
 constexpr int kSmem = kStages * kStageBytes + 128;
-constexpr int kEpi = 8;                              // epilogue warps
+constexpr int kEpi = 16;                             // epilogue warps
 constexpr int kThreads = 32 * (kEpi + 2);            // and producer, MMA issuer
 constexpr int kNanEx = 1 << 28;                      // row with an infinity or NaN
 
@@ -257,7 +258,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz_gemm(Op A, Op B, double *C, 
                 if (!tc::mbar_wait(tc::smem_u32(&empty[d % kStages]), (d / kStages) & 1)) ok = false;
         }
     } else {
-        // warps w and w + 4 take 32 columns each of the rows of tensor memory
+        // warps w, w + 4, ... take kC columns each of the rows of tensor memory
         // that they can read; C stays in registers over the groups
         constexpr int kC = kN / (kEpi / 4);
         const int rw = (wib & 3) * 32, c0 = (wib >> 2) * kC;
@@ -276,7 +277,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz_gemm(Op A, Op B, double *C, 
             if (!(k == t.k1 - 1 || (k >> gs) != ((k + 1) >> gs))) continue;
             const int64_t g = k >> gs;
             const int er = A.ex[((int64_t)t.aRow * A.ng + g) * kNB + rw + ln];
-            const int el = B.ex[((int64_t)t.bRow * B.ng + g) * kNB + half * kN + c0 + ln];   // lane = column
+            const int el = B.ex[((int64_t)t.bRow * B.ng + g) * kNB + half * kN + c0 + ln % kC];   // lane = column
             if (!tc::mbar_wait(tc::smem_u32(&accFull), grp & 1)) {
                 ok = false;
                 break;

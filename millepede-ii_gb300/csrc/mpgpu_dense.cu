@@ -20,6 +20,7 @@
 #include <vector>
 
 #include "mpgpu_ctx.h"
+#include "mpgpu_fp64.cuh"
 #include "mpgpu_ozaki.h"
 #include "mpgpu_tc.cuh"
 
@@ -51,18 +52,6 @@ constexpr int kTld = kPc + 2;           // rows of the factor in shared memory
 constexpr int kLld = kNB - kPc + 2;     // rows of the earlier columns
 
 __device__ __forceinline__ void bar_n(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
-
-// Reciprocal by Newton's iteration from an FP32 seed, |d| within 2^+-120; the
-// conversions in integers, as a conversion costs a slot of the FP64 pipe.
-__device__ __forceinline__ double newton_rcp(double d) {
-    const uint32_t hi = (uint32_t)__double2hiint(d), lo = (uint32_t)__double2loint(d);
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__uint_as_float((hi - (896u << 20)) << 3 | lo >> 29)));
-    const uint32_t f = __float_as_uint(y);
-    double z = __hiloint2double((int)((f >> 3) + (896u << 20)), (int)(f << 29));
-    z = fma(z, fma(-d, z, 1.0), z);
-    return fma(z, fma(-d, z, 1.0), z);
-}
 
 // Cholesky factor of the 32 x 32 block at D into T, the reciprocals of its
 // diagonal into rs; by 128 threads (lane = row, warp w the columns 4 q + w in

@@ -12,12 +12,13 @@
 // written.  The update is FP64-bound (n^3 / 2 multiply-adds for sqminl, n^3 /
 // 6 for chdec2 at 2 per SM and clock), the panels are bound by the latency of
 // a chain of pivots.  Measured: sqminl of 1,500 rows 10.0 ms (per block 143 us
-// panel, 71 us update) from 40.5 ms; chdec2 and chslv2 of 2,000 rows 8.7 ms
-// (per block 37 + 35 us panel, 61 us update) from 64 ms.
+// panel, 71 us update) from 40.5 ms; chdec2 and chslv2 of 2,000 rows 5.3 ms
+// (per block 22 + 11 us panel, 46 us update) from 64 ms.
 #include <cooperative_groups.h>
 
 #include <algorithm>
 
+#include "mpgpu_fp64.cuh"
 #include "mpgpu_packed.h"
 
 namespace cg = cooperative_groups;
@@ -398,52 +399,88 @@ __global__ void k_sq_init(int32_t n, const double *V, double *d, int32_t *used, 
 
 // ------------------------------------------------------------ chdec2
 // Rows i1-1 .. i0 (at most kPb) are the pivots of a block, from the last.
-// First their own triangle, by one warp: lane c holds column i0 + c; row i is
-// scaled by f_i = 1 / G(i, i) (the element itself where it is not positive, as
-// chdec2 leaves it) and taken from the rows above.  The backward substitution
-// of chslv2 uses the same rows in the same order and rides along.
-__global__ void __launch_bounds__(32) k_chdec_diag(int32_t i0, int32_t nb, double *g, double *x, double *stat) {
-    __shared__ double rat[kPb];
-    const int c = threadIdx.x;
-    double w[kPb];
+// First their own triangle, by four warps: lane c holds column i0 + c, warp w
+// the rows 4 q + w of it in registers.  Row i is scaled by f_i = 1 / G(i, i)
+// (the element itself where it is not positive, as chdec2 leaves it) and taken
+// from the rows above: the next one at once, the others while the next pivot's
+// reciprocal is under way.  The backward substitution of chslv2 uses the same
+// rows in the same order and rides along.  Bound by the chain of pivots, some
+// ten FP64 instructions of 64 clocks each: with one warp for all rows 37 us, now
+// 22.
+__device__ __forceinline__ void bar4(void) { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+
+__global__ void __launch_bounds__(128) k_chdec_diag(int32_t i0, int32_t nb, double *g, double *x, double *stat) {
+    __shared__ double rowb[4][kPb], dv[kPb];
+    const int c = threadIdx.x & 31, wq = threadIdx.x >> 5;
+    double w[8];
 #pragma unroll
-    for (int r = 0; r < kPb; ++r) w[r] = (r < nb && c <= r) ? g[prow(i0 + r) + i0 + c] : 0.0;
+    for (int q = 0; q < 8; ++q) {
+        const int r = 4 * q + wq;
+        w[q] = (r < nb && c <= r) ? g[prow(i0 + r) + i0 + c] : 0.0;
+    }
     double xc = c < nb ? x[i0 + c] : 0.0;
-    double gmax = stat[0], gmin = stat[1], cnt = stat[2];
+    double t = 0.0;
+    const int top = nb - 1;
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+        if (4 * q + wq == top) rowb[top & 3][c] = w[q];
 #pragma unroll
     for (int i = kPb - 1; i >= 0; --i) {
         if (i >= nb) continue;
-        const double d = __shfl_sync(0xffffffffu, w[i], i);
-        double f = d;
-        if (d > 0.0) {
-            f = 1.0 / d;
-            gmax = cnt == 0.0 ? d : fmax(gmax, d);
-            gmin = cnt == 0.0 ? d : fmin(gmin, d);
-            cnt += 1.0;
+        bar4();
+        const double *cur = rowb[i & 3], *prev = rowb[(i + 1) & 3];
+        const double d = cur[i], wi = cur[c];
+        const double f = d > 0x1p-120 && d < 0x1p120 ? newton_rcp(d) : (d > 0.0 ? 1.0 / d : d);
+        if (threadIdx.x == 0) dv[i] = d;
+        if (i + 1 < nb) {   // the pivot before, from the rows above this one
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+                if (4 * q + wq < i) w[q] = fma(-t, prev[4 * q + wq], w[q]);   // used for c <= r
         }
-        const double q = c < i ? w[i] * f : 0.0;
-        __syncwarp();
-        rat[c] = q;
-        __syncwarp();
+        t = wi * f;   // (scaled element of column c)
+        if (i > 0 && wq == ((i - 1) & 3)) {
+            const int q = (i - 1) >> 2;
+            w[q] = fma(-t, cur[i - 1], w[q]);
+            rowb[(i - 1) & 3][c] = w[q];
+        }
         const double xi = __shfl_sync(0xffffffffu, xc, i);
-        if (c < i) xc = fma(-q, xi, xc);
-#pragma unroll
-        for (int r = 0; r < i; ++r) w[r] = fma(-w[i], rat[r], w[r]);   // used for c <= r
-        w[i] = c < i ? q : f;
+        if (c < i) xc = fma(-t, xi, xc);
+        if (wq == (i & 3) && c <= i) g[prow(i0 + i) + i0 + c] = c < i ? t : f;
     }
+    if (wq == 0) {
+        if (c < nb) x[i0 + c] = xc;
+        __syncwarp();
+        // largest, smallest and number of the positive pivots
+        const double d = c < nb ? dv[c] : 0.0, cnt = stat[2];
+        const unsigned pos = __ballot_sync(0xffffffffu, d > 0.0);
+        double hi = d > 0.0 ? d : 0.0, lo = d > 0.0 ? d : __longlong_as_double(0x7ff0000000000000ll);
 #pragma unroll
-    for (int r = 0; r < kPb; ++r)
-        if (r < nb && c <= r) g[prow(i0 + r) + i0 + c] = w[r];
-    if (c < nb) x[i0 + c] = xc;
-    if (c == 0) { stat[0] = gmax; stat[1] = gmin; stat[2] = cnt; }
+        for (int o = 16; o > 0; o >>= 1) {
+            hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+            lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        }
+        if (c == 0 && pos) {
+            stat[0] = cnt == 0.0 ? hi : fmax(stat[0], hi);
+            stat[1] = cnt == 0.0 ? lo : fmin(stat[1], lo);
+            stat[2] = cnt + (double)__popc(pos);
+        }
+    }
 }
 
-// then the columns c < i0 of those rows, a thread per column: U the unscaled,
-// R the scaled rows (also left in g); x of the columns
-__global__ void __launch_bounds__(32) k_chdec_rows(int32_t i0, int32_t nb, double *g, double *x, double *U, double *R,
-                                                   int64_t ld) {
-    __shared__ double rat[kPb][kPb], f[kPb], xb[kPb];
-    for (int e = threadIdx.x; e < nb * nb; e += 32) {
+// then the columns c < i0 of those rows, four lanes per column (lane s the rows
+// 4 q + s): U the unscaled, R the scaled rows (also left in g); x of the
+// columns.  FP64 instructions of single warps again: a thread per column took
+// 35 us for 1,000 columns, now 11.
+__global__ void __launch_bounds__(128) k_chdec_rows(int32_t i0, int32_t nb, double *g, double *x, double *U, double *R,
+                                                    int64_t ld) {
+    __shared__ double rat[kPb][kPb + 1], f[kPb], xb[kPb];
+    const int tid = threadIdx.x, ln = tid & 31, sub = ln & 3, quad = ln & 28;
+    const int64_t c = (int64_t)blockIdx.x * 32 + (tid >> 5) * 8 + (ln >> 2);
+    const bool in = c < i0;
+    double w[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) w[q] = (in && 4 * q + sub < nb) ? g[prow(i0 + 4 * q + sub) + c] : 0.0;
+    for (int e = tid; e < nb * nb; e += 128) {
         const int i = e / nb, r = e % nb;
         if (r <= i) {
             const double v = g[prow(i0 + i) + i0 + r];
@@ -451,62 +488,73 @@ __global__ void __launch_bounds__(32) k_chdec_rows(int32_t i0, int32_t nb, doubl
             else f[i] = v;
         }
     }
-    if ((int)threadIdx.x < nb) xb[threadIdx.x] = x[i0 + threadIdx.x];
-    __syncwarp();
-    const int64_t c = (int64_t)blockIdx.x * 32 + threadIdx.x;
-    if (c >= i0) return;
-    double w[kPb];
-#pragma unroll
-    for (int r = 0; r < kPb; ++r) w[r] = r < nb ? g[prow(i0 + r) + c] : 0.0;
-    double xc = x[c];
+    if (tid < nb) xb[tid] = x[i0 + tid];
+    __syncthreads();
+    double xs = 0.0;
 #pragma unroll
     for (int i = kPb - 1; i >= 0; --i) {
         if (i >= nb) continue;
+        const double u = __shfl_sync(0xffffffffu, w[i >> 2], quad | (i & 3));
 #pragma unroll
-        for (int r = 0; r < i; ++r) w[r] = fma(-w[i], rat[i][r], w[r]);
-        const double q = w[i] * f[i];
-        U[i * ld + c] = w[i];
-        R[i * ld + c] = q;
-        g[prow(i0 + i) + c] = q;
-        xc = fma(-q, xb[i], xc);
+        for (int q = 0; q <= i >> 2; ++q)
+            if (q < i >> 2 || sub < (i & 3)) w[q] = fma(-u, rat[i][4 * q + sub], w[q]);
     }
-    x[c] = xc;
+#pragma unroll
+    for (int q = 7; q >= 0; --q) {
+        const int i = 4 * q + sub;
+        if (i >= nb) continue;
+        const double v = w[q] * f[i];
+        if (in) {
+            U[i * ld + c] = w[q];
+            R[i * ld + c] = v;
+            g[prow(i0 + i) + c] = v;
+        }
+        xs = fma(-v, xb[i], xs);
+    }
+    xs += __shfl_xor_sync(0xffffffffu, xs, 1);
+    xs += __shfl_xor_sync(0xffffffffu, xs, 2);
+    if (in && sub == 0) x[c] += xs;
 }
 
-// the leading i0 x i0 triangle: G(r, c) -= U(i, c) R(i, r), i from the last
+// the leading i0 x i0 triangle: G(r, c) -= U(i, c) R(i, r), i from the last.
+// Tiles of 32 x 32: the work of a tile of 64 (65,000 clocks) was the time of
+// every launch with fewer tiles than SMs (61 us per block of 2,000 rows on
+// average, now 46; FP64 floor 36).
+constexpr int kCt = 32;
 __global__ void __launch_bounds__(256) k_chdec_update(int32_t i0, int32_t nb, double *g, const double *U,
                                                       const double *R, int64_t ld) {
-    __shared__ double su[kPb][kTile + 2], sr[kPb][kTile + 2];
+    __shared__ double su[kPb][kCt + 2], sr[kPb][kCt + 2];
     int bi, bj;
     tri_tile(blockIdx.x, bi, bj);
-    const int r0 = bi * kTile, c0 = bj * kTile, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    for (int e = tid; e < nb * kTile; e += 256) {
-        const int q = e / kTile, i = e % kTile;
+    const int r0 = bi * kCt, c0 = bj * kCt, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    for (int e = tid; e < nb * kCt; e += 256) {
+        const int q = e / kCt, i = e % kCt;
         sr[q][i] = r0 + i < i0 ? R[q * ld + r0 + i] : 0.0;
         su[q][i] = c0 + i < i0 ? U[q * ld + c0 + i] : 0.0;
     }
-    __syncthreads();
-    double w[4][4];
+    double w[2][2];
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int a = 0; a < 2; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
+        for (int b = 0; b < 2; ++b) {
             const int r = r0 + ty + 16 * a, c = c0 + tx + 16 * b;
             w[a][b] = (r < i0 && c <= r) ? g[prow(r) + c] : 0.0;
         }
+    __syncthreads();
+#pragma unroll 4
     for (int q = nb - 1; q >= 0; --q) {
-        double x[4], y[4];
+        double x[2], y[2];
 #pragma unroll
-        for (int a = 0; a < 4; ++a) { x[a] = -sr[q][ty + 16 * a]; y[a] = su[q][tx + 16 * a]; }
+        for (int a = 0; a < 2; ++a) { x[a] = -sr[q][ty + 16 * a]; y[a] = su[q][tx + 16 * a]; }
 #pragma unroll
-        for (int a = 0; a < 4; ++a)
+        for (int a = 0; a < 2; ++a)
 #pragma unroll
-            for (int b = 0; b < 4; ++b) w[a][b] = fma(y[b], x[a], w[a][b]);
+            for (int b = 0; b < 2; ++b) w[a][b] = fma(y[b], x[a], w[a][b]);
     }
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int a = 0; a < 2; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
+        for (int b = 0; b < 2; ++b) {
             const int r = r0 + ty + 16 * a, c = c0 + tx + 16 * b;
             if (r < i0 && c <= r) g[prow(r) + c] = w[a][b];
         }
@@ -554,8 +602,8 @@ __global__ void __launch_bounds__(256) k_chslv_fwd(int32_t n, int32_t i0, const 
     }
 }
 
-int64_t tiles_of(int64_t n) {
-    const int64_t t = (n + kTile - 1) / kTile;
+int64_t tiles_of(int64_t n, int tile) {
+    const int64_t t = (n + tile - 1) / tile;
     return t * (t + 1) / 2;
 }
 
@@ -630,7 +678,7 @@ cudaError_t packed_sqminl(int32_t n, double *V, double *b, const double *diag, i
             cfg.gridDim = dim3(cl);
         }
     }
-    const unsigned nt = (unsigned)tiles_of(n);
+    const unsigned nt = (unsigned)tiles_of(n, kTile);
     for (int32_t i = 0; i < n; i += kPb) {
         p.tmax = std::min(kPb, n - i);
         const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p);
@@ -644,10 +692,10 @@ cudaError_t packed_chdec_solve(int32_t n, double *g, double *x, double *stat, do
     double *U = work, *R = U + (int64_t)kPb * n, *out = R + (int64_t)kPb * n;
     for (int32_t i1 = n; i1 > 0; i1 -= kPb) {
         const int32_t i0 = std::max(0, i1 - kPb), nb = i1 - i0;
-        k_chdec_diag<<<1, 32, 0, s>>>(i0, nb, g, x, stat);
+        k_chdec_diag<<<1, 128, 0, s>>>(i0, nb, g, x, stat);
         if (i0 == 0) break;
-        k_chdec_rows<<<(unsigned)((i0 + 31) / 32), 32, 0, s>>>(i0, nb, g, x, U, R, n);
-        k_chdec_update<<<(unsigned)tiles_of(i0), 256, 0, s>>>(i0, nb, g, U, R, n);
+        k_chdec_rows<<<(unsigned)((i0 + 31) / 32), 128, 0, s>>>(i0, nb, g, x, U, R, n);
+        k_chdec_update<<<(unsigned)tiles_of(i0, kCt), 256, 0, s>>>(i0, nb, g, U, R, n);
     }
     k_chslv_scale<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, g, x);
     for (int32_t i0 = 0; i0 < n; i0 += kFb) {

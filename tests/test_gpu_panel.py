@@ -27,8 +27,10 @@ def matrix(n, kind):
     return M + np.diag(1e-3 * np.diag(M) + 1e-6)
 
 
-@pytest.mark.parametrize("n", [1, 31, 33, 96, 127, 129, 160, 385, 513, 650, 1160])
-@pytest.mark.parametrize("kind", ["dense", "scaled", "spiky"])
+# (2,700 and 5,400 rows: the first panels take four lanes per row, the last eight)
+@pytest.mark.parametrize("n,kind", [(n, kind) for kind in ("dense", "scaled", "spiky")
+                                    for n in (1, 31, 33, 96, 127, 129, 160, 385, 513, 650, 1160)]
+                         + [(2700, "scaled"), (5400, "dense")])
 def test_backward_error(mp, n, kind):
     A = matrix(n, kind)
     with mp.Context() as ctx:

@@ -195,7 +195,8 @@ __global__ void __launch_bounds__(kSqThreads) k_sqminl_panel(SqParams p) {
 // cluster): the row's state stays in registers, its columns of the block in
 // shared memory, where the other CTAs read the pivot row's.  The candidates are
 // pushed to every CTA before the one cluster barrier of a pivot, after which
-// each warp picks the pivot for itself.  Bound: the chain of a pivot (exchange,
+// each warp picks the pivot for itself.  (One barrier per launch besides, so
+// that no CTA is pushed to before it has started.)  Bound: the chain of a pivot (exchange,
 // barrier, the pivot column's element from L2, up to 31 dependent multiply-
 // adds); 9.3 us per pivot with the state in global memory, now 4.5 (1,500
 // rows).
@@ -235,6 +236,7 @@ __global__ void __launch_bounds__(THREADS) k_sqminl_panel_sm(SqParams p) {
     const double lim = in ? 1.0E-10 * p.diag[j] : 0.0;
     int ps = -1;
     int t = 0;
+    cl.sync();   // every CTA runs: the first candidates are pushed before any other barrier
     for (; t < p.tmax; ++t) {
         SqMsg m{(unsigned long long)__double_as_longlong(fabs(dj)), dj, bj, j};
         if (used || !(fabs(dj) > lim)) m.k = -1;

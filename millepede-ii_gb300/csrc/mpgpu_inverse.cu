@@ -202,9 +202,8 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_tile_gemm_tc(TcOp A, TcOp B, 
                 if (!tc::mbar_wait(tc::smem_u32(&empty[d % kStages]), (d / kStages) & 1)) ok = false;
         }
     } else {
-        if (!tc::mbar_wait(tc::smem_u32(&done), 0)) ok = false;
+        ok = tc::mbar_wait_warp(tc::smem_u32(&done), 0);
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        ok = __all_sync(0xffffffffu, ok);
         if (ok) {
             // all MMAs are done, so that the stages are free
             float *epi = reinterpret_cast<float *>(tsm + (sbase - tc::smem_u32(tsm))) + wib * 32 * 33;

@@ -278,12 +278,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz_gemm(Op A, Op B, double *C, 
             const int64_t g = k >> gs;
             const int er = A.ex[((int64_t)t.aRow * A.ng + g) * kNB + rw + ln];
             const int el = B.ex[((int64_t)t.bRow * B.ng + g) * kNB + half * kN + c0 + ln % kC];   // lane = column
-            if (!tc::mbar_wait(tc::smem_u32(&accFull), grp & 1)) {
+            if (!tc::mbar_wait_warp(tc::smem_u32(&accFull), grp & 1)) {
                 ok = false;
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            __syncwarp();
 #pragma unroll
             for (int cb = 0; cb < kC / 8; ++cb) {
                 const uint32_t tc0 = tmem + ((uint32_t)rw << 16) + (uint32_t)(c0 + cb * 8);

@@ -73,6 +73,13 @@ __device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t parity) {
     return false;
 }
 
+// the same by all lanes of a warp with one answer: where the limit runs out while
+// the phase completes, lanes that left the warp would be missing from its next
+// .aligned instruction
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t addr, uint32_t parity) {
+    return __all_sync(0xffffffffu, mbar_wait(addr, parity)) != 0;
+}
+
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"

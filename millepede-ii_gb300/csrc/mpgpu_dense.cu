@@ -180,7 +180,8 @@ __global__ void __launch_bounds__(32 * kPcWarps) k_panel32(double *A, int64_t ld
     if (wib < 4) {
         if (!triangle_fast(D, ld, T, rs, col, dv) && wib == 0) {
             const bool neg = triangle_any(D, ld, T, rs);
-            if (neg && blockIdx.x == 0 && tid == 0) atomicExch(err, (int)(k0 / kNB) + 1);
+            // (-1, a wait that ran out, stays: what follows it is no statement on the matrix)
+            if (neg && blockIdx.x == 0 && tid == 0) atomicCAS(err, 0, (int)(k0 / kNB) + 1);
         }
     } else {
         for (int e = tid - 128; e < kPc * (b / 2); e += 32 * kRowWarps) {
@@ -249,8 +250,8 @@ __global__ void k_pad_identity(double *A, int64_t ld, int64_t n, int64_t npad) {
 }  // namespace
 
 // Factorise the dense padded matrix A (npad x npad, row-major, lower
-// triangle) in place.  Returns 0, MPGPU_ERR_FACTOR (non-positive pivot in
-// panel *badPanel) or a CUDA/timeout error.
+// triangle) in place.  Returns 0, MPGPU_ERR_FACTOR (non-positive pivot, first
+// in panel *badPanel) or a CUDA/timeout error.
 // Block columns of kSuperPanels panels: inside a block column the
 // 128-wide panels are factorised and update the rest of the block column;
 // the trailing matrix then receives the whole block column at once, K = 512

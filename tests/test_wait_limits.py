@@ -39,3 +39,14 @@ def test_warps_agree_on_a_wait(name, body):
     assert waits
     for at in waits:
         assert any(re.search(r"\(ln == 0\)|\(tid == 0\)", h) for h in open_blocks(body, at)), (name, body[at:at + 60])
+
+
+def test_a_bad_pivot_does_not_hide_it():
+    """The error word of the dense factorisation is -1 after a wait that ran
+    out, reported as such; a panel number is only put where it was 0.  Every
+    unconditional store into an error word is the -1."""
+    for f in sorted(os.listdir(CSRC)):
+        if f.endswith((".cu", ".cuh")):
+            with open(os.path.join(CSRC, f)) as fh:
+                for value in re.findall(r"atomicExch\((?:\w+[.>-]+)?err,\s*(.*)\);", fh.read()):
+                    assert value == "-1", (f, value)

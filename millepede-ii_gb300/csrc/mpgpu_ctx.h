@@ -453,7 +453,7 @@ void dense_release(mpgpu_ctx *c);
 void dense_invalidate(mpgpu_ctx *c);
 // blocked inverse from the dense Cholesky factor (mpgpu_inverse.cu)
 int32_t dense_inverse_device(mpgpu_ctx *c, double *L, int64_t npad, int64_t n, int mode, const double *DinvT, const double *XS,
-                             double *Zd, double *Zp, int32_t *dErr);
+                             const int32_t *kexp, double *Zd, double *Zp, int32_t *dErr);
 int32_t solve_minres(mpgpu_ctx *c, const double *consResiduals, double rtol, int32_t itnlim,
                      double *corr, mpgpu_solveinfo *info, bool qlp = false);
 int32_t avprod_host(mpgpu_ctx *c, int32_t n, const double *x, double *b);

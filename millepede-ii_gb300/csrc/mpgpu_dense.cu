@@ -765,6 +765,14 @@ __global__ void __launch_bounds__(256) k_sb_bwd_upd(const double *L, int64_t ld,
     }
 }
 
+// exponents q with 2^q the size of sqrt(a_ii), the norm of row i of the factor
+__global__ void k_unit_exponents(const double *A, int64_t ld, int64_t n, int32_t *q) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int f = (int)((__double_as_longlong(A[i * ld + i]) >> 52) & 0x7ff);
+    q[i] = f == 2047 ? 0 : (f - 1022) >> 1;
+}
+
 struct DenseWork {
     int64_t npad = 0, np = 0;
     double *L = nullptr, *F = nullptr, *DinvT = nullptr;   // factor, matrix, inverse 128-row blocks (transposed)
@@ -775,18 +783,21 @@ struct DenseWork {
     double *t1 = nullptr, *t2 = nullptr;                   // the preconditioner's working vectors
     double *part = nullptr, *sc = nullptr;
     int32_t *err = nullptr;
+    int32_t *kexp = nullptr;                               // exponents of the units of the factor's rows
     void release() {
         cudaFree(L); cudaFree(F); cudaFree(DinvT); cudaFree(XS); cudaFree(XT); cudaFree(XW); cudaFree(sbTask);
         cudaFree(hi); cudaFree(lo);
         cudaFree(b); cudaFree(x); cudaFree(r); cudaFree(z); cudaFree(p); cudaFree(q); cudaFree(t1); cudaFree(t2);
-        cudaFree(part); cudaFree(sc); cudaFree(err);
+        cudaFree(part); cudaFree(sc); cudaFree(err); cudaFree(kexp);
     }
 };
 
 // X_b for every super-block from L and the 128-row inverse blocks, doubling the
 // inverted blocks: X_21 = -X_22 (L_21 X_11) for blocks of one and then of two
 // tiles, exact tile products on the tensor cores (on the FP64 units, which 16
-// tile products per super-block keep busy, 1.3 ms for 6,000 rows, now 0.3).
+// tile products per super-block keep busy, 1.3 ms for 6,000 rows, now 0.3).  The
+// second product's operands vary with the unit of parameter k along K and are
+// sliced with kexp.
 cudaError_t build_super_inverse(DenseWork &w, cudaStream_t s) {
     const int32_t np = (int32_t)w.np;
     cudaError_t e = cudaMemsetAsync(w.XS, 0, sizeof(double) * w.npad * kSB, s);
@@ -828,9 +839,10 @@ cudaError_t build_super_inverse(DenseWork &w, cudaStream_t s) {
             const int32_t b = 1 << lv, pairs = (np - b + 2 * b - 1) / (2 * b);
             if (pairs <= 0) break;
             auto split = [&](const double *M, int64_t ld, int32_t r0, int32_t k0, int trans, int tri, const oz::Op &dst,
-                             int32_t wrap) {
+                             int32_t wrap, int ksign = 0) {
                 if (e == cudaSuccess)
-                    e = oz_split(M, ld, r0, r0 + b, k0, k0 + b, trans, tri, dst, 0, k0, 1, s, pairs, 2 * b, np, wrap);
+                    e = oz_split(M, ld, r0, r0 + b, k0, k0 + b, trans, tri, dst, 0, k0, 1, s, pairs, 2 * b, np, wrap,
+                                 ksign ? w.kexp : nullptr, ksign);
             };
             auto product = [&](double *C, int sec, double alpha) {
                 const int64_t t0 = first[2 * lv + sec], t1 = first[2 * lv + sec + 1];
@@ -841,8 +853,8 @@ cudaError_t build_super_inverse(DenseWork &w, cudaStream_t s) {
             split(w.L, w.npad, b, 0, 0, 0, oa, 0);
             split(w.XS, kSB, 0, 0, 1, 2, ob, 4);
             product(w.XW, 0, 1.0);
-            split(w.XS, kSB, b, b, 0, 1, oa, 4);
-            split(w.XW, kSB, 0, b, 1, 0, ob, 4);
+            split(w.XS, kSB, b, b, 0, 1, oa, 4, 1);
+            split(w.XW, kSB, 0, b, 1, 0, ob, 4, -1);
             product(w.XS, 1, -1.0);
         }
         // the host task list must live until the copy has run
@@ -1119,6 +1131,7 @@ int32_t dense_workspace(mpgpu_ctx *c, int64_t npad, bool wy, DenseResident *&out
     if (e == cudaSuccess) e = cudaMalloc(&w.part, sizeof(double) * kDotBlk);
     if (e == cudaSuccess) e = cudaMalloc(&w.sc, sizeof(double) * 16);
     if (e == cudaSuccess) e = cudaMalloc(&w.err, sizeof(int32_t));
+    if (e == cudaSuccess) e = cudaMalloc(&w.kexp, sizeof(int32_t) * w.npad);
     if (wy) {
         for (double **v : {&y.U, &y.UT, &y.W, &y.ZU, &y.UZ}) {
             const int64_t len = (v == &y.ZU || v == &y.UZ) ? 2 * w.npad * kWy : w.npad * kWy;
@@ -1290,6 +1303,7 @@ int32_t dense_solve_pcg(mpgpu_ctx *c, int32_t n, const double *Ap, double *bx, i
         for (int tries = 0;; ++tries) {
             r = prepare(shift);
             if (r != MPGPU_OK) break;
+            k_unit_exponents<<<(unsigned)((w.npad + 255) / 256), 256, 0, s>>>(w.L, w.npad, w.npad, w.kexp);
             int32_t bad = -1;
             r = dense_cholesky_device(c, w.L, w.npad, mode, w.hi, w.lo, w.err, &bad);
             if (r != MPGPU_ERR_FACTOR || tries >= 6) break;
@@ -1390,7 +1404,7 @@ int32_t dense_solve_pcg(mpgpu_ctx *c, int32_t n, const double *Ap, double *bx, i
     cudaEventRecord(eR, s);
     int32_t rcInv = MPGPU_OK;
     if (invOut && istop != 9) {
-        rcInv = dense_inverse_device(c, w.L, w.npad, nfit, mode, w.DinvT, w.XS, w.F, invOut, w.err);
+        rcInv = dense_inverse_device(c, w.L, w.npad, nfit, mode, w.DinvT, w.XS, w.kexp, w.F, invOut, w.err);
         // the inverse overwrites L and F
         D->factorValid = false;
     }

@@ -12,7 +12,9 @@
 // trtri in FP64 doubles the inverted diagonal blocks: X_21 = -X_22 (L_21 X_11)
 // for all pairs of blocks of b tiles at once, b = 4, 8, ... (blocks of four tiles
 // come from the factorisation's super-blocks): eight products for 4,200 rows,
-// the largest of 512 halves of tiles.  In 3xTF32 it goes block
+// the largest of 512 halves of tiles.  X_22 has the inverse unit of parameter k in
+// column k and L_21 X_11 the unit in row k: the slices of these two are scaled by
+// it.  In 3xTF32 it goes block
 // column by block column from the last: for panel p, T = X_trail P (the panel P
 // below the diagonal block times the already inverted trailing part), then
 // X_panel = -T D_p with D_p = L_pp^-1.
@@ -277,11 +279,11 @@ __global__ void __launch_bounds__(256) k_dense_lower_to_packed(const double *Z, 
 
 // L (npad x npad, dense row-major, the lower Cholesky factor with the
 // inverses of its diagonal blocks in DinvT and of its blocks of four tiles in
-// XS) is replaced by X = L^-1; Z =
+// XS, and the exponents of its rows' units in kexp) is replaced by X = L^-1; Z =
 // X^T X (lower part) is written to Zd and its leading n x n block packed
 // into Zp.  mode 0: FP64 tile products by slices; mode 1: tensor-core 3xTF32.
 int32_t dense_inverse_device(mpgpu_ctx *c, double *L, int64_t npad, int64_t n, int mode, const double *DinvT,
-                             const double *XS, double *Zd, double *Zp, int32_t *dErr) {
+                             const double *XS, const int32_t *kexp, double *Zd, double *Zp, int32_t *dErr) {
     cudaStream_t s = c->stream;
     const int32_t np = (int32_t)(npad / kNB);
     const int64_t ld = npad;
@@ -410,8 +412,8 @@ int32_t dense_inverse_device(mpgpu_ctx *c, double *L, int64_t npad, int64_t n, i
             }
             for (int32_t w0 = b; w0 < 2 * b; w0 += W) {
                 const int32_t w1 = std::min(w0 + W, 2 * b);
-                MPG_OZ(oz_split(L, ld, b, 2 * b, w0, w1, 0, 1, oa, 0, w0, 2, s, pairs, 2 * b, np));
-                MPG_OZ(oz_split(Zd, ld, 0, b, w0, w1, 1, 0, ob, 0, w0, 2, s, pairs, 2 * b, np));
+                MPG_OZ(oz_split(L, ld, b, 2 * b, w0, w1, 0, 1, oa, 0, w0, 2, s, pairs, 2 * b, np, 0, kexp, 1));
+                MPG_OZ(oz_split(Zd, ld, 0, b, w0, w1, 1, 0, ob, 0, w0, 2, s, pairs, 2 * b, np, 0, kexp, -1));
                 MPG_OZ(oz_tile_gemm(oa, ob, L, ld, dTask + stepS[lv], stepT[lv + 1] - stepS[lv], 0, 0, 2, -1.0, 0.0,
                                     dErr, s, oz::Window{2 * b, w0, w1 - w0}));
             }

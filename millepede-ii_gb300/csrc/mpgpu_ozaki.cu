@@ -15,8 +15,15 @@
 // up to 3.7 times that of an FP64 sum where rows have a few large elements
 // (and the digits' squares gave the diagonal a bias).  What is left out or
 // rounded is below 2^-56 of (row maximum of A) x (row maximum of B) per term,
-// of either sign, against 2^-53 of the partial sums in FP64: over factors of
-// the barrel and telescope matrices 5 to 100 times below the FP64 sum's error.
+// of either sign, against 2^-53 of the partial sums in FP64.  That is as good
+// as an FP64 sum where the elements of a row are of like size, as they are in a
+// Cholesky factor, whose row k has the unit of parameter k (over factors of the
+// barrel and telescope matrices 5 to 100 times below the FP64 sum's error) and
+// in its inverse's columns.  Where the unit runs along K (a row of the inverse
+// times a column of a product of the factor) both operands are scaled by powers
+// of two per K value, which cancel in the product: without, the error grew by the
+// ratio of the units (relative errors of the inverse of 1,024 rows 2e-13 for
+// units 2e4 apart, 2e-9 for 1e8; with the scales as for equal units).
 //
 // Per chunk of 16 K a CTA multiplies 128 x 16 by 16 x 64 in 43 instructions
 // from 70 KB of shared memory (three stages, filled by bulk copies of images
@@ -324,11 +331,15 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz_gemm(Op A, Op B, double *C, 
 // exponents over the group's K tiles, then every eight consecutive K values of
 // a row as 16-byte pieces, one per slice, in core-matrix order (eight rows of a
 // piece are 128 contiguous bytes).  Integer arithmetic on the bit patterns
-// throughout.
+// throughout.  KS: the K values are scaled by powers of two, kexp[k] (or -kexp[k])
+// added to their exponents.
 constexpr int kSplitRows = 32;
+constexpr int kZeroEx = -(1 << 20);   // exponent of zero in scaled rows
+template <bool KS>
 __global__ void __launch_bounds__(256) k_oz_split(const double *M, int64_t ld, int32_t r0, int32_t k0, int32_t k1,
                                                   int trans, int tri, Op dst, int32_t rOff, int32_t cOff, int gs,
-                                                  int32_t step, int32_t lim, int32_t wrap) {
+                                                  int32_t step, int32_t lim, int32_t wrap, const int32_t *kexp,
+                                                  int ksign) {
     __shared__ int emax[kSplitRows];
     const int tid = threadIdx.x, ln = tid & 31, wib = tid >> 5;
     r0 += blockIdx.z * step;
@@ -349,17 +360,23 @@ __global__ void __launch_bounds__(256) k_oz_split(const double *M, int64_t ld, i
     // first row and K value in M
     const int64_t row0 = (int64_t)(trans && wrap > 0 ? R % wrap : R) * kNB + h0;
     const int64_t kk0 = (int64_t)(!trans && wrap > 0 ? k0 % wrap : k0) * kNB;
-    if (tid < kSplitRows) emax[tid] = 0;
+    const int32_t *ke = KS ? kexp + (int64_t)k0 * kNB : nullptr;
+    if (tid < kSplitRows) emax[tid] = KS ? kZeroEx : 0;
     __syncthreads();
-    auto field = [](double x) { return (int)((__double_as_longlong(x) >> 52) & 0x7ff); };
+    // exponent field of K value q of a row, scaled
+    auto field = [&](double x, int q) {
+        const int f = (int)((__double_as_longlong(x) >> 52) & 0x7ff);
+        if (!KS) return f;
+        return f == 2047 ? kNanEx : x == 0.0 ? kZeroEx : max(f, 1) + ksign * __ldg(ke + q);
+    };
     if (!trans) {
         for (int r = wib; r < kSplitRows; r += 8) {
             const double2 *p = reinterpret_cast<const double2 *>(M + (row0 + r) * ld + kk0);
-            int e = 0;
+            int e = KS ? kZeroEx : 0;
 #pragma unroll 4
             for (int q = ln; q < K / 2; q += 32) {
                 const double2 v = p[q];
-                e = max(e, max(field(v.x), field(v.y)));
+                e = max(e, max(field(v.x, 2 * q), field(v.y, 2 * q + 1)));
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
@@ -367,15 +384,16 @@ __global__ void __launch_bounds__(256) k_oz_split(const double *M, int64_t ld, i
         }
     } else {
         const double *p = M + kk0 * ld + row0 + ln;
-        int e = 0;
+        int e = KS ? kZeroEx : 0;
 #pragma unroll 8
-        for (int q = wib; q < K; q += 8) e = max(e, field(p[(int64_t)q * ld]));
+        for (int q = wib; q < K; q += 8) e = max(e, field(p[(int64_t)q * ld], q));
         atomicMax(&emax[ln], e);
     }
     __syncthreads();
     if (tid < kSplitRows)
         dst.ex[((int64_t)Rd * dst.ng + ((k0 - cOff) >> gs)) * kNB + h0 + tid] =
-            emax[tid] == 2047 ? kNanEx : max(emax[tid], 1) - 1022;
+            KS ? (emax[tid] == kNanEx ? kNanEx : emax[tid] - 1022)
+               : (emax[tid] == 2047 ? kNanEx : max(emax[tid], 1) - 1022);
     uint8_t *out = dst.img + ((int64_t)Rd * dst.nt + (k0 - cOff)) * kTileBytes;
     const int nk8 = K / 8, total = kSplitRows * nk8;
     for (int it = tid; it < total; it += 256) {
@@ -397,15 +415,16 @@ __global__ void __launch_bounds__(256) k_oz_split(const double *M, int64_t ld, i
             for (int q = 0; q < 8; ++q) x[q] = p[(int64_t)q * ld];
         }
         uint32_t w[kImages][4];
-        const int em = max(emax[rl], 1);
+        const int em = KS ? emax[rl] : max(emax[rl], 1);
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
             const long long b = __double_as_longlong(x[q]);
-            const int e = max((int)((b >> 52) & 0x7ff), 1);
+            const int e = max((int)((b >> 52) & 0x7ff), 1) + (KS ? ksign * __ldg(ke + k8 * 8 + q) : 0);
             long long m = b & 0xfffffffffffffll;
             if ((b >> 52) & 0x7ff) m |= 0x10000000000000ll;
-            // x 2^(55 - exponent), |.| < 2^55, rounded to an integer
-            const int sh = em - e - 2;
+            // x 2^(55 - exponent), |.| < 2^55, rounded to an integer (a zero has
+            // no part in the scaled maximum)
+            const int sh = KS && m == 0 ? 0 : em - e - 2;
             if (sh <= 0) m <<= -sh;
             else m = sh > 60 ? 0 : (m + (1ll << (sh - 1))) >> sh;
             if (b < 0) m = -m;
@@ -442,11 +461,12 @@ __global__ void __launch_bounds__(256) k_oz_split(const double *M, int64_t ld, i
 
 cudaError_t oz_split(const double *M, int64_t ld, int32_t r0, int32_t r1, int32_t k0, int32_t k1, int trans, int tri,
                      const oz::Op &dst, int32_t rOff, int32_t cOff, int gs, cudaStream_t s, int32_t count, int32_t step,
-                     int32_t lim, int32_t wrap) {
+                     int32_t lim, int32_t wrap, const int32_t *kexp, int ksign) {
     if (r1 <= r0 || k1 <= k0 || count <= 0) return cudaSuccess;
     const int ng = ((k1 - 1 - cOff) >> gs) - ((k0 - cOff) >> gs) + 1;
     const dim3 grid((unsigned)((r1 - r0) * (kNB / kSplitRows)), (unsigned)ng, (unsigned)count);
-    k_oz_split<<<grid, 256, 0, s>>>(M, ld, r0, k0, k1, trans, tri, dst, rOff, cOff, gs, step, lim, wrap);
+    (kexp ? k_oz_split<true> : k_oz_split<false>)<<<grid, 256, 0, s>>>(M, ld, r0, k0, k1, trans, tri, dst, rOff, cOff, gs,
+                                                                       step, lim, wrap, kexp, ksign);
     return cudaGetLastError();
 }
 

@@ -37,9 +37,12 @@ struct Window {
 // only k >= r.  count > 1: the same for r0, r1, k0, k1 and cOff moved by step, 2
 // step, ... tiles; tiles from lim on are left out.  wrap > 0: M holds column
 // tile c at c mod wrap (the K tiles of a group then wrap at most at its ends).
+// kexp: K value k (counted over all K tiles, not wrapped) is taken times 2^(ksign
+// kexp[k]); the other operand takes the opposite sign.
 cudaError_t oz_split(const double *M, int64_t ld, int32_t r0, int32_t r1, int32_t k0, int32_t k1, int trans, int tri,
                      const oz::Op &dst, int32_t rOff, int32_t cOff, int gs, cudaStream_t s, int32_t count = 1,
-                     int32_t step = 0, int32_t lim = 1 << 28, int32_t wrap = 0);
+                     int32_t step = 0, int32_t lim = 1 << 28, int32_t wrap = 0, const int32_t *kexp = nullptr,
+                     int ksign = 1);
 // C(cRow, cCol) = alpha sum_k A(aRow, k) B(bRow, k)^T + beta C over a device
 // task list, or (tasks null) over the lower triangle of tiles from tile
 // (trail0, trail0) on with K tiles [0, trailK) (tc_tile_gemm's convention).

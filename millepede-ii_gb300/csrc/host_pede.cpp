@@ -17,6 +17,8 @@
 #include "../../include/mpgpu.h"
 #include "host_struct.h"
 
+void ctx_set_lean(mpgpu_ctx *c, bool lean);   // mpgpu_api.cu
+
 namespace {
 
 // measurement boundaries of one record (decodeNextMeasurement,
@@ -598,15 +600,18 @@ int32_t pede_run_admitted(mpgpu_ctx *ctxIn, const mpgpu_steer *st, const mpgpu_j
         // buffers of the constraint elimination and the preconditioner's
         // super-block inverses (about 40 KB per row)
         const int64_t dense = (st->metsol == 31 || st->metsol == 32) ? 2 * npad * npad + 5120 * npad : 0;
-        // iterative solves in sparse storage: the block-row copy (each block
-        // with its transpose, padded) and the vectors
+        // needed by the faster form of a solve only: the block-row copy of the
+        // sparse matrix (each block with its transpose, padded) and the vectors
         const int64_t iter = (st->metsol == 4 || st->metsol == 5) && st->matsto == 2
                                  ? 4 * nm + (32 + 5 * (int64_t)std::min(job->ncon, 64)) * nVar
                                  : 0;
         const int64_t stageCap = (int64_t)2 << 30;   // 2 x 8 GiB staging buffers at most (in doubles)
-        const int64_t bytes = 40 * nw + 8 * (std::min(stage, stageCap) + nm + dense + iter) + 64 * (int64_t)nVar +
+        const int64_t bytes = 40 * nw + 8 * (std::min(stage, stageCap) + nm + dense) + 64 * (int64_t)nVar +
                               ((int64_t)64 << 20);
-        if (!admit(bytes)) {
+        // a budget that does not hold the faster form gets the smaller one
+        const bool lean = iter > 0 && !admit(bytes + 8 * iter);
+        ctx_set_lean(ctx, lean);
+        if ((iter == 0 || lean) && !admit(bytes)) {
             res->exitCode = MPGPU_ERR_BUDGET;
             if (!ctxIn) mpgpu_destroy(ctx);
             return MPGPU_ERR_BUDGET;

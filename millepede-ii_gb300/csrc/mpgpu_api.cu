@@ -72,9 +72,7 @@ void free_layout(DevJob &j) {
     dfree(j.matD); dfree(j.gvec); dfree(j.gcnt); dfree(j.gpar); dfree(j.work);
     dfree(j.rowBlk0); dfree(j.blkJ); dfree(j.blkOff); dfree(j.blkLd);
     dfree(j.rowWidth);
-    dfree(j.br.val); dfree(j.br.col); dfree(j.br.stepBeg); dfree(j.br.itemBeg);
-    dfree(j.br.itemS0); dfree(j.br.itemS1); dfree(j.br.part); dfree(j.br.xp);
-    j.br = BlockRows();
+    block_rows_free(j);
 }
 
 void free_constraints(DevJob &j) {
@@ -151,6 +149,8 @@ extern "C" int32_t mpgpu_release(mpgpu_ctx *c) {
     c->j.nVar = 0;
     return MPGPU_OK;
 }
+
+void ctx_set_lean(mpgpu_ctx *c, bool lean) { c->lean = lean; }
 
 extern "C" const char *mpgpu_last_error(const mpgpu_ctx *c) { return c ? c->err.c_str() : ""; }
 

@@ -431,6 +431,21 @@ int32_t block_rows_build(mpgpu_ctx *c) {
     return MPGPU_OK;
 }
 
+int64_t block_rows_bytes(const BlockRows &b) {
+    if (b.R <= 0) return 0;
+    const int64_t L = (int64_t)b.nslot * b.R;
+    return 8 * b.nsteps * b.R * L + 4 * b.nsteps * b.nslot + (8 * (int64_t)b.R + 8) * b.nitem +
+           (16 + 8 * (int64_t)b.R) * b.nG;
+}
+
+void block_rows_free(DevJob &j) {
+    BlockRows &b = j.br;
+    for (void *p : {(void *)b.val, (void *)b.col, (void *)b.stepBeg, (void *)b.itemBeg, (void *)b.itemS0,
+                    (void *)b.itemS1, (void *)b.part, (void *)b.xp})
+        if (p) cudaFree(p);
+    b = BlockRows();
+}
+
 cudaError_t block_rows_spmv(const BlockRows &b, const double *xp, const int32_t *done, const BlockRowsCoef *coef,
                             cudaStream_t s) {
     const unsigned g = (unsigned)((b.nitem + kBrWarps - 1) / kBrWarps);

@@ -7,6 +7,7 @@
 #include "mpgpu_minres.cuh"
 
 struct mpgpu_ctx;
+struct DevJob;
 
 // Device arrays of the copy, kept (with their capacities) in the job between
 // the solves of a layout.
@@ -30,8 +31,11 @@ struct BlockRows {
 bool block_rows_fit(const mpgpu_ctx *c);
 // Builds the copy of the current matrix on the context's stream (in the job's br).
 int32_t block_rows_build(mpgpu_ctx *c);
-// part = item sums of A xp (xp padded, see block_rows_pad); nothing when
-// *done is set.  coef: work of one extra CTA (null: none)
+// its device memory, and giving it back
+int64_t block_rows_bytes(const BlockRows &b);
+void block_rows_free(DevJob &j);
+// part = item sums of A xp (xp padded: parameter i of group g at g R + i); nothing
+// when *done is set.  coef: work of one extra CTA (null: none)
 struct BlockRowsCoef {
     int32_t m;                // constraints
     int32_t nblk;             // partial dots per column

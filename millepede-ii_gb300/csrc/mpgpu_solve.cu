@@ -388,6 +388,7 @@ struct SparseBlocks {
     int64_t *colItemQ1 = nullptr;  // [nColItem] end
     int64_t *colItemBeg = nullptr; // [nG+1] first item of column group J
     double *colPart = nullptr;     // [nColItem * kSmallGroup]
+    int uniform = 0;               // every group has this many parameters (0: mixed)
 };
 
 // phase 1: warp per row group I: y_I = D_I x_I + sum_J A_IJ x_J, the
@@ -450,30 +451,33 @@ __global__ void k_spmv_cols(int32_t nG, const int32_t *aig, const int64_t *colSt
 }
 
 // the same two phases for row groups of at most 8 parameters of strongly
-// mixed sizes (others take the block-row copy, mpgpu_bspmv.cu).  Phase 1,
+// mixed sizes, or where the memory does not hold the block-row copy that the
+// others take (mpgpu_bspmv.cu).  Phase 1,
 // one thread per stored block (all blocks of all row groups, so the lanes
 // stay full whatever the row lengths): the block's rows times x_J into its
 // partial row sums (rowPart, 8 per block; the diagonal block adds both
 // triangles of its strictly-lower part there) and its columns times x_I
-// into tbuf (parameter-major per column group).  Phase 2: the partial row
-// sums of a group's blocks and the transposed products of its incoming
-// blocks summed by column items (long columns split over several warps),
-// then y = D x + the group's items in item order; no atomics, the sums are
-// reproducible.
+// into tbuf (parameter-major per column group).  G > 0: every group has G
+// parameters (loops fully unrolled); G = 0: at most 8, predicated.  Phase 2:
+// the partial row sums of a group's blocks and the transposed products of its
+// incoming blocks summed by column items (long columns split over several
+// warps), then y = D x + the group's items in item order; no atomics, the sums
+// are reproducible.
 constexpr int kSmallGroup = 8;
 
+template <int G>
 __global__ void __launch_bounds__(256) k_spmv_blocks(int64_t nb, const int32_t *brow, const int32_t *aig,
                                                      const int32_t *bcol, const int64_t *boff, const int32_t *bld,
                                                      const int64_t *tOff, const int32_t *tStr,
                                                      const double *matD, const double *x, double *tbuf,
                                                      double *rowPart) {
-    constexpr int M = kSmallGroup;
+    constexpr int M = G > 0 ? G : kSmallGroup;
     for (int64_t bl = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; bl < nb;
          bl += (int64_t)gridDim.x * blockDim.x) {
         const int32_t I = brow[bl], J = bcol[bl];
         const int32_t ia = aig[I - 1] - 1, ja = aig[J - 1] - 1;
-        const int np = aig[I] - 1 - ia;
-        const int nj = aig[J] - 1 - ja;
+        const int np = G > 0 ? G : aig[I] - 1 - ia;
+        const int nj = G > 0 ? G : aig[J] - 1 - ja;
         const double *blk = matD + boff[bl];
         const int32_t ld = bld[bl];
         double xi[M], sr[M];
@@ -1078,6 +1082,10 @@ __global__ void k_sub(int32_t n, double *a, const double *b) {
 }
 
 // ---------------------------------------------------------------- helpers
+// device memory that a context keeps between its iterative solves, at most, for
+// the block-row copy and for the vectors each (30,000 globals: 145 and 70 MB)
+constexpr int64_t kKeepBytes = (int64_t)4 << 30;
+
 struct Solver {
     mpgpu_ctx *c;
     DevJob &j;
@@ -1090,6 +1098,10 @@ struct Solver {
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
     }
     ~Solver() {
+        // the copy and the vectors stay for the next solve unless they are large:
+        // the data loop in between may need the memory
+        if (useRows && block_rows_bytes(j.br) > kKeepBytes) block_rows_free(j);
+        if (8 * j.cap[(const void *)&j.work] > kKeepBytes) dfree(j.work);
         // stream-ordered (cudaMallocAsync on the context's stream)
         if (partOwned) cudaFreeAsync(partOwned, s);
         dfree(wyPart); dfree(wyT);
@@ -1240,6 +1252,9 @@ struct Solver {
         }
         ciBeg[j.nG] = (int64_t)ciJ.size();
         sb.nColItem = (int64_t)ciJ.size();
+        int32_t minnp = maxnp;
+        for (int32_t I = 1; I <= j.nG; ++I) minnp = std::min(minnp, aig[I] - aig[I - 1]);
+        sb.uniform = (sb.smallGroups && minnp == maxnp) ? maxnp : 0;
         sb.nblk = nb;
         sb.tlen = tl;
         auto up = [&](auto *&d, const auto &h) -> cudaError_t {
@@ -1275,8 +1290,21 @@ struct Solver {
             MPG_CUDA(c, alloc_pmv(j.nVar));
             return MPGPU_OK;
         }
-        useRows = block_rows_fit(c);
-        return useRows ? block_rows_build(c) : build_blocks();
+        useRows = !c->lean && block_rows_fit(c);
+        if (useRows && block_rows_build(c) == MPGPU_OK) return MPGPU_OK;
+        return from_storage();
+    }
+
+    // the product from the stored matrix: layouts that the copy does not
+    // serve, or no memory for it (the copy takes twice the matrix, the
+    // transposed products 0.4 of it for groups of six)
+    int32_t from_storage() {
+        if (useRows) {
+            cudaGetLastError();
+            block_rows_free(j);
+        }
+        useRows = false;
+        return build_blocks();
     }
 
     // y = A x (full parameter space)
@@ -1285,8 +1313,22 @@ struct Solver {
             block_rows_product(j.br, j.aig, j.p2g, x, y, s);
         } else if (j.matsto == 2 && sb.smallGroups) {
             const unsigned gb = grid(sb.nblk);
-            k_spmv_blocks<<<gb, kThreads, 0, s>>>(sb.nblk, sb.brow, j.aig, sb.bcol, sb.boff, sb.bld, sb.tOff, sb.tStr,
-                                                  j.matD, x, sb.tbuf, sb.rowPart);
+            auto blocks = [&](auto g) {
+                k_spmv_blocks<decltype(g)::value><<<gb, kThreads, 0, s>>>(sb.nblk, sb.brow, j.aig, sb.bcol, sb.boff, sb.bld,
+                                                                          sb.tOff, sb.tStr, j.matD, x, sb.tbuf,
+                                                                          sb.rowPart);
+            };
+            switch (sb.uniform) {
+            case 1: blocks(std::integral_constant<int, 1>()); break;
+            case 2: blocks(std::integral_constant<int, 2>()); break;
+            case 3: blocks(std::integral_constant<int, 3>()); break;
+            case 4: blocks(std::integral_constant<int, 4>()); break;
+            case 5: blocks(std::integral_constant<int, 5>()); break;
+            case 6: blocks(std::integral_constant<int, 6>()); break;
+            case 7: blocks(std::integral_constant<int, 7>()); break;
+            case 8: blocks(std::integral_constant<int, 8>()); break;
+            default: blocks(std::integral_constant<int, 0>()); break;
+            }
             k_spmv_colitems<<<wgrid(sb.nColItem), kThreads, 0, s>>>(sb.nColItem, sb.colItemJ, sb.colItemQ0,
                                                                     sb.colItemQ1, j.aig, sb.rowStart, sb.rowPart,
                                                                     sb.colStart, sb.tBase, sb.tbuf, sb.colPart);
@@ -1563,16 +1605,26 @@ int32_t solve_minres(mpgpu_ctx *c, const double *consResiduals, double rtol, int
     if (rc) return rc;
     // workspace, kept by the job: vectors, partial sums, the reflections'
     // columns, the iteration's scalars
-    const bool fused = S.useRows && ncon <= kWyFused;
     const int64_t nv = ((int64_t)std::max(n, 1) + 1) / 2 * 2;   // vectors stay 16-byte aligned
-    const int64_t nxp = fused ? ((int64_t)j.nG * j.br.R + 1) / 2 * 2 : nv;
     const int nb = (int)std::min<int64_t>(kMrBlocks, (nfit + kThreads - 1) / kThreads + (nfit < 1));
     const int nbY1 = (int)std::min<int64_t>(kMrBlocks, ((int64_t)nfit * kY1Lanes + kY1Threads - 1) / kY1Threads + (nfit < 1));
     const int nbStep = (int)std::min<int64_t>(kStepBlocks, (n + kStepRows - 1) / kStepRows);
     const int64_t nUW = (int64_t)nbStep * 2 * kWyFused;
     const int64_t scalLen = (2 * sizeof(MinresState) + 2 * sizeof(QlpState) + sizeof(MinresFlags)) / 8 + 8;
-    const int64_t len = 16 * nv + nxp + 3 * kMrBlocks + kDotBlocks + 8 + nUW + 2 * kWyFused + scalLen + S.wy_len();
-    MPG_CUDA(c, dgrow(j, j.work, len));
+    auto padded = [&] { return S.useRows && ncon <= kWyFused ? ((int64_t)j.nG * j.br.R + 1) / 2 * 2 : nv; };
+    auto grow = [&] {
+        return dgrow(j, j.work, 16 * nv + padded() + 3 * kMrBlocks + kDotBlocks + 8 + nUW + 2 * kWyFused + scalLen +
+                                    S.wy_len());
+    };
+    cudaError_t eWork = grow();
+    if (eWork != cudaSuccess && S.useRows) {   // without the copy and the reflections' columns
+        rc = S.from_storage();
+        if (rc) return rc;
+        eWork = grow();
+    }
+    MPG_CUDA(c, eWork);
+    const bool fused = S.useRows && ncon <= kWyFused;
+    const int64_t nxp = padded();
     double *at = j.work;
     auto vec = [&](int64_t l) {
         double *p = at;

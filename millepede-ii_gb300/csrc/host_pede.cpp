@@ -600,18 +600,24 @@ int32_t pede_run_admitted(mpgpu_ctx *ctxIn, const mpgpu_steer *st, const mpgpu_j
         // buffers of the constraint elimination and the preconditioner's
         // super-block inverses (about 40 KB per row)
         const int64_t dense = (st->metsol == 31 || st->metsol == 32) ? 2 * npad * npad + 5120 * npad : 0;
-        // needed by the faster form of a solve only: the block-row copy of the
+        // needed by the faster form of a solve: the block-row copy of the
         // sparse matrix (each block with its transpose, padded) and the vectors
         const int64_t iter = (st->metsol == 4 || st->metsol == 5) && st->matsto == 2
                                  ? 4 * nm + (32 + 5 * (int64_t)std::min(job->ncon, 64)) * nVar
                                  : 0;
+        // the blocked FP64 inversion: the dense forms' buffers and the slices of
+        // its two operands, 24 bytes per element of up to 64 K tiles of 128
+        const int64_t inv = st->metsol == 12
+                                ? 2 * npad * npad + 5120 * npad + 6 * npad * std::min<int64_t>(64 * 128, npad + 384)
+                                : 0;
+        const int64_t more = 8 * (iter + inv);
         const int64_t stageCap = (int64_t)2 << 30;   // 2 x 8 GiB staging buffers at most (in doubles)
         const int64_t bytes = 40 * nw + 8 * (std::min(stage, stageCap) + nm + dense) + 64 * (int64_t)nVar +
                               ((int64_t)64 << 20);
         // a budget that does not hold the faster form gets the smaller one
-        const bool lean = iter > 0 && !admit(bytes + 8 * iter);
+        const bool lean = more > 0 && !admit(bytes + more);
         ctx_set_lean(ctx, lean);
-        if ((iter == 0 || lean) && !admit(bytes)) {
+        if ((more == 0 || lean) && !admit(bytes)) {
             res->exitCode = MPGPU_ERR_BUDGET;
             if (!ctxIn) mpgpu_destroy(ctx);
             return MPGPU_ERR_BUDGET;

@@ -358,7 +358,7 @@ int32_t dense_inverse_device(mpgpu_ctx *c, double *L, int64_t npad, int64_t n, i
     }
     // W: all K tiles up to 64 (C is read and written once per W tiles, 64 of
     // them take 400 us), fewer where the memory does not suffice
-    int32_t W = std::min(64, (np + 3) / 4 * 4);
+    int32_t W = c->lean ? 4 : std::min(64, (np + 3) / 4 * 4);
     oz::Op oa{}, ob{};
     if (mode == 0 && e == cudaSuccess) {
         for (;; W = std::max(4, W / 8 * 4)) {

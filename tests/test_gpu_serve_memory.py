@@ -32,3 +32,23 @@ def test_sparse_product_without_the_copy(mp, name, metsol):
     assert np.max(np.abs(got - want)) <= 1e-9 * np.max(np.abs(want))
     rc, _, _ = run(mp, d, b - 1, **st)
     assert rc == 42
+
+
+def test_slices_of_the_inverse(mp):
+    """The blocked FP64 inversion: the footprint holds the slices of both
+    operands (24 bytes per element, all K tiles below 64); in windows of four
+    K tiles where the budget does not, with the same solution."""
+    cfg = mp.gen_config("telescope", ntracks=20000, seed=22)
+    cfg.nmod = 80
+    d = mp.generate(cfg)
+    st = dict(metsol=12, matsto=1)
+    rc, full, jd = run(mp, d, 0, **st)
+    assert rc == 0
+    labels, want = jd.parameters()
+    npad = (len(labels) + 127) // 128 * 128
+    assert npad > 5 * 128
+    rc, b, jd = run(mp, d, full - 1, **st)
+    assert rc == 0 and full - b >= 2 * 24 * npad * npad
+    np.testing.assert_array_equal(jd.parameters()[1], want)   # the solution does not take the inverse
+    rc, _, _ = run(mp, d, b - 1, **st)
+    assert rc == 42

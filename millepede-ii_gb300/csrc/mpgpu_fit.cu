@@ -1909,11 +1909,20 @@ int fit_default_wpc(const FitParams &p) {
     FitParams q = p;
     q.onePerBlock = 0;
     int best = 0, bestW = 1;
+    // (the query counts by the kernel's limit: raised first, as for a launch)
+    if (smem_optin((const void *)fit_kernel(q)) != cudaSuccess) {
+        cudaGetLastError();   // the launch will report it
+        return bestW;
+    }
     for (int w = 1; w <= MPG_WARPS_FIT; w *= 2) {
         q.wpc = w;
         if (fit_warps_per_cta(q) != w) break;
         int perSM = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, fit_kernel(q), 32 * w, (size_t)fit_smem_per_warp(q) * w);
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, fit_kernel(q), 32 * w,
+                                                          (size_t)fit_smem_per_warp(q) * w) != cudaSuccess) {
+            cudaGetLastError();
+            break;
+        }
         if (perSM * w > best) {
             best = perSM * w;
             bestW = w;

@@ -192,8 +192,9 @@ int32_t mpgpu_write_mon(const char *path, int32_t header, int32_t mode, int32_t 
  * needs: class k < 7 up to 4 KB << k, class 7 beyond one CTA): records per
  * class, warps per CTA chosen on the first data loop (0: no loop yet, -1:
  * no candidate fitted), by the tuner for classes of several 100,000 records,
- * else one, and the tuner's sample times (ms) of 1, 2, 4 and 8 warps per CTA
- * (0: not sampled); arrays of MPGPU_FIT_BUCKETS (and 4x that for tuneMs).  No counterpart in the reference. */
+ * else the form with the most warps resident on an SM, and the tuner's sample
+ * times (ms) of 1, 2, 4 and 8 warps per CTA (0: not sampled); arrays of
+ * MPGPU_FIT_BUCKETS (and 4x that for tuneMs).  No counterpart in the reference. */
 #define MPGPU_FIT_BUCKETS 8
 int32_t mpgpu_fit_buckets(const mpgpu_ctx *ctx, int64_t *count, int32_t *wpc, double *tuneMs);
 
@@ -557,7 +558,10 @@ int32_t mpgpu_write_res_opts(const char *path, const mpgpu_result *res, const mp
  * counterpart in the reference, which runs one job per process).  maxActive
  * worker contexts run jobs concurrently on the device; a job is admitted
  * when its device footprint fits in budgetBytes next to the running jobs,
- * in submission order.  A job's result does not depend on the other jobs.
+ * in submission order.  A job's result does not depend on the other jobs.  A
+ * job whose faster solve (the block-row copy of a sparse matrix, the slices of
+ * the blocked inversion) exceeds the whole budget runs in the smaller form; one
+ * that exceeds it even so is refused.
  * ---------------------------------------------------------------- */
 typedef struct mpgpu_server mpgpu_server;
 typedef struct mpgpu_server_cfg {

@@ -644,7 +644,7 @@ __global__ void k_sub_vec(int64_t n, const double *b, const double *ax, double *
 
 // ---- the preconditioner's triangular solves by super-blocks of kSB rows:
 // X_b = L_bb^-1 of every diagonal super-block (from the 128-row inverse
-// blocks by block forward substitution in FP64 tile products), then each
+// blocks by doubling, build_super_inverse), then each
 // solve is nsb steps of (X_b times the block, update of the rows below or
 // the columns left) instead of np steps of 128 rows: a quarter of the
 // dependent launches of a CG iteration
@@ -707,7 +707,7 @@ __global__ void __launch_bounds__(256) k_sb_diag(const double *X, int64_t row0, 
 
 // v_R -= L[R][row0 .. row0 + kSB) z_b for the rows R >= row0 + kSB (there are
 // none below a shorter block), two rows per warp with all their loads issued at
-// once.  FP64-bound (512 multiply-adds per row, 8.8 us for 10,000 rows); with a
+// once.  FP64-bound (512 multiply-adds per row, 8.1 us for 10,000 rows); with a
 // row per warp and a loop of dependent loads 19.5 us, now 14.8.  (Four rows per
 // warp leave too few warps for a few thousand rows.)
 __global__ void __launch_bounds__(256) k_sb_fwd_upd(const double *L, int64_t ld, int64_t row0, int64_t npad,

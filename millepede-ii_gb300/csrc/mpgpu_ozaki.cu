@@ -2,7 +2,7 @@
 // tensor cores by error-free slices (the scheme of Ozaki, Ogita, Oishi & Rump
 // 2012, with the operands' rows scaled to fixed point).
 //
-// GB300's FP64 units give 2 multiply-adds per SM and clock (0.58 T/s), its
+// GB300's FP64 units give 2 multiply-adds per SM and clock (0.63 T/s), its
 // bf16 tensor cores some 4,000.  Every operand row is scaled by a power of two
 // over a group of at most 512 K values, rounded to 56-bit fixed point and cut
 // into eight balanced 7-bit digits, which bf16 holds exactly.  The products of

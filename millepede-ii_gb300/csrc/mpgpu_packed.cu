@@ -521,7 +521,7 @@ __global__ void __launch_bounds__(128) k_chdec_rows(int32_t i0, int32_t nb, doub
 // the leading i0 x i0 triangle: G(r, c) -= U(i, c) R(i, r), i from the last.
 // Tiles of 32 x 32: the work of a tile of 64 (65,000 clocks) was the time of
 // every launch with fewer tiles than SMs (61 us per block of 2,000 rows on
-// average, now 46; FP64 floor 36).
+// average, now 46; FP64 floor 34).
 constexpr int kCt = 32;
 __global__ void __launch_bounds__(256) k_chdec_update(int32_t i0, int32_t nb, double *g, const double *U,
                                                       const double *R, int64_t ld) {

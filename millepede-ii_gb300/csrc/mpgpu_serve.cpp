@@ -8,7 +8,9 @@
 // on the device (their kernels overlap on separate streams).  Each job's
 // matrix and vectors stay on the device across its iterations.  The device
 // arithmetic of one job does not depend on the others, so a job's result is
-// identical alone and in a mix.  Latency = submission to completion.
+// identical alone and in a mix (a budget too small for a job's faster solve
+// takes the smaller form, whose sums are in another order, whatever runs
+// beside it).  Latency = submission to completion.
 #include <chrono>
 #include <condition_variable>
 #include <cstdint>

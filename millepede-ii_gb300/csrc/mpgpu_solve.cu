@@ -160,7 +160,7 @@ __global__ void k_wy_apply(int32_t n, int32_t m, const double *V, const double *
 // element is read once and used for its row's sum and for its column's.  Pass 2
 // adds, per j, the row parts by column range and the column parts of the blocks
 // below j, eight threads per j.
-// FP64-bound: two multiply-adds per stored element (62 us for 6,000 rows; the
+// FP64-bound: two multiply-adds per stored element (57 us for 6,000 rows; the
 // matrix once takes 22 us).  Reading it once per row and once per column took
 // 248 + 85 us, now 99 + 15 (1,500 rows: 21 + 14 us, now 20 + 4).
 constexpr int kMvRows = 16;
@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(256) k_pmv_final(int32_t n, int64_t nb, const 
 // rows ilast and below in [1, ilast] get -2 Av_c v_i, the diagonal (kn,kn)
 // its combined term and rows > kn their -2 v_c Av_i parts.  Tiles of 16 rows x
 // 256 columns, a thread per column: the row's and the column's factors are
-// read once per tile.  FP64-bound: two multiply-adds per element (62 us for
+// read once per tile.  FP64-bound: two multiply-adds per element (57 us for
 // 6,000 rows, reading and writing the matrix 43 us); a warp per row took 210
 // us, now 104.
 constexpr int kQlRows = 16;
@@ -638,8 +638,8 @@ __global__ void k_mr_init(MinresState *S, QlpState *Q, MinresFlags *F, const dou
 // one (at most kMrBlocks values).  They are bound by launch and
 // synchronisation latency, not by their 0.2 MB vectors, and by FP64
 // instructions that every warp would repeat (a warp's FP64 instruction holds
-// the pipe for 16 clocks, a division about 30 of them), so the scalars are
-// formed by one warp.  At 30,000 globals and 18 constraints: product 35 to
+// its quarter of the SM for 64 clocks, and a division is about 30 of them), so
+// the scalars are formed by one warp.  At 30,000 globals and 18 constraints: product 35 to
 // 44 us (mpgpu_bspmv.cu), 9.8, 6.2 and 10.9 us.  The first form had 16
 // launches, with the sums in kernels of one CTA.
 constexpr int kMrBlocks = 1216;    // CTAs of the vector kernels (at most)
